@@ -56,6 +56,10 @@ PROTOTYPES = {
         C.c_int,
         [_p, _i64, _i64, _kvp, _p, _i32, _p, _i64, _i64, _i32, _p, _i32, _i32, _i32, _i32, _i32, _i32, _i32, _i32, _i32, _p, _p],
     ),
+    "dgpt_fmha_prefill_gated": (
+        C.c_int,
+        [_p, _i64, _i64, _kvp, _p, _i32, _p, _i64, _i64, _p, _i64, _i32, _i32, _i32, _i32, _i32, _i32, _i32, _i32, _p, _p],
+    ),
     "dgpt_decode_attn_workspace_bytes": (_sz, [_i32, _i32, _i32, _i32]),
     "dgpt_decode_attn": (
         C.c_int,
@@ -138,6 +142,10 @@ _NOT_LAUNCHING = {
 }
 
 
+# entry points that are another one with an addition in its kernels' epilogue: timed under that one's name
+_TIMED_AS = {"dgpt_fmha_prefill_gated": "dgpt_fmha_prefill"}
+
+
 class Stats:
     launches = 0
     timer = None
@@ -208,7 +216,7 @@ class _Lib:
             fn = getattr(raw, name)  # AttributeError if the symbol is not exported
             fn.restype = res
             fn.argtypes = args
-            setattr(self, name, fn if name in _NOT_LAUNCHING else self._wrap(name, fn))
+            setattr(self, name, fn if name in _NOT_LAUNCHING else self._wrap(_TIMED_AS.get(name, name), fn))
 
     @staticmethod
     def _wrap(name, fn):

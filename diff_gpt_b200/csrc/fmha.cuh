@@ -27,6 +27,10 @@ struct FmhaArgs {
   int keep_first = 0;       // with a window: keys j < keep_first are seen from every distance
   const void* hgate = nullptr;  // [B * Tq, H] in dtype: output of head h is multiplied by sigmoid(hgate)
   long long hgate_rs = 0;
+  // gate per output element (dgpt_fmha_prefill_gated), exclusive with hgate
+  const void* egate = nullptr;  // [B * Tq, H * D] in dtype: o = round(o) * round(sigmoid(egate))
+  long long egate_rs = 0;
+  int any_run = 0;  // the tensor-core kernels may take dense keys of any length, not only whole tiles (impl 0)
 };
 
 // What the tensor-core kernels need besides the three tensor maps.
@@ -51,6 +55,8 @@ struct TcParams {
   int kv_div;        // query heads per key/value head
   const void* hgate; // bf16 [B * Tq, H], or NULL
   long long hgate_rs;
+  const __nv_bfloat16* egate;  // [B * Tq, H * d_head], or NULL
+  long long egate_rs;
   int BH, group_bh;  // two-query-tile kernel: (batch, head) pairs in all, and how many are worked on at a time
 };
 
@@ -59,6 +65,39 @@ template <typename T>
 __device__ __forceinline__ float head_gate(const void* hgate, long long rs, long long row, int h) {
   if (hgate == nullptr) return 1.f;
   return 1.f / (1.f + expf(-Io<T>::ld(static_cast<const T*>(hgate) + row * rs + h)));
+}
+// One element through its gate, with the rounding points of a separate pass over the stored output (sigmoid_gate_kernel).
+template <typename T>
+__device__ __forceinline__ float gated(float o, float g) {
+  return Io<T>::round(o) * Io<T>::round(1.f / (1.f + __expf(-g)));
+}
+// bf16 keeps 8 bits of the sigmoid, so the two-instruction division (2 ulp of fp32) gives the same rounded value except
+// within 2e-7 of a rounding boundary; the full one cost a fifth of the short kernel (425 against 355 us on config 2's shape).
+template <>
+__device__ __forceinline__ float gated<__nv_bfloat16>(float o, float g) {
+  using B = Io<__nv_bfloat16>;
+  return B::round(o) * B::round(__fdividef(1.f, 1.f + __expf(-g)));
+}
+// N columns (a multiple of 8) of one output row, gated: the stored row never makes a second trip through memory.  (The
+// separate pass took 171 us for 131072 x 256 elements and 597 us for 228480 x 512.)
+template <int N>
+__device__ __forceinline__ void store_gated(__nv_bfloat16* dst, const float* v, float inv, const __nv_bfloat16* gate) {
+  uint4 raw[N / 8];  // all loads before the first store, which the compiler could not prove to be elsewhere
+#pragma unroll
+  for (int i = 0; i < N / 8; ++i) raw[i] = __ldg(reinterpret_cast<const uint4*>(gate) + i);
+#pragma unroll
+  for (int i = 0; i < N / 8; ++i) {
+    float g[8];
+    unpack16<__nv_bfloat16>(raw[i], g);
+#pragma unroll
+    for (int x = 0; x < 8; ++x) g[x] = gated<__nv_bfloat16>(v[8 * i + x] * inv, g[x]);
+    st16<__nv_bfloat16>(dst + 8 * i, g, 1.f);
+  }
+}
+// A row's gate of `bytes` on its way to L2 while the row's scores are worked on (loaded cold in the epilogue it is one more miss to memory per item).
+__device__ __forceinline__ void prefetch_gate(const __nv_bfloat16* gate, int bytes) {
+  const char* p = reinterpret_cast<const char*>(gate);
+  for (int i = 0; i < bytes; i += 64) asm volatile("prefetch.global.L2 [%0];" ::"l"(p + i));
 }
 // First key tile of `tile` keys inside the window of a query at position `first_q` (the query tile's lowest).
 __device__ __forceinline__ int window_first_tile(int window, int first_q, int tile) {

@@ -20,7 +20,8 @@ __global__ void __launch_bounds__(128)
 fmha_simt_kernel(const T* __restrict__ q, long long q_bs, long long q_rs, KvView kv, const int* __restrict__ kv_len,
                  int kv_len_all, void* __restrict__ o, long long o_bs, long long o_rs, int o_f32,
                  float* __restrict__ lse, int H, int Tq, int q_offset, int causal, float scale_log2, int window,
-                 int keep_first, int kv_div, const void* __restrict__ hgate, long long hgate_rs) {
+                 int keep_first, int kv_div, const void* __restrict__ hgate, long long hgate_rs,
+                 const T* __restrict__ egate, long long egate_rs) {
   constexpr int DP = D / SPLIT;       // elements per thread
   constexpr int BM = 128 / SPLIT;     // queries per CTA
   constexpr int VEC = Io<T>::kVec16;
@@ -136,8 +137,14 @@ fmha_simt_kernel(const T* __restrict__ q, long long q_bs, long long q_rs, KvView
     for (int d = 0; d < DP; ++d) op[d] = acc[d] * inv;
   } else {
     T* op = static_cast<T*>(o) + oo;
+    if (egate) {
+      const T* gp = egate + ((long long)b * Tq + qi) * egate_rs + (long long)h * D + part * DP;
 #pragma unroll
-    for (int d = 0; d < DP; ++d) Io<T>::st(op + d, acc[d] * inv);
+      for (int d = 0; d < DP; ++d) Io<T>::st(op + d, gated<T>(acc[d] * inv, Io<T>::ld(gp + d)));
+    } else {
+#pragma unroll
+      for (int d = 0; d < DP; ++d) Io<T>::st(op + d, acc[d] * inv);
+    }
   }
   if (lse && part == 0) {
     const int Hn = H;
@@ -155,7 +162,7 @@ static int fmha_simt_launch(const FmhaArgs& a, const KvView& kv, cudaStream_t st
                                                       a.kv_len_all, a.o, a.o_bs, a.o_rs, a.o_f32, a.lse, a.H, a.Tq,
                                                       a.q_offset, a.causal, scale_log2, a.window,
                                                       a.window > 0 ? a.keep_first : 0, a.kv_heads > 0 ? a.H / a.kv_heads : 1, a.hgate,
-                                                      a.hgate_rs);
+                                                      a.hgate_rs, static_cast<const T*>(a.egate), a.egate_rs);
   return launch_status("fmha_simt");
 }
 
@@ -187,11 +194,10 @@ int fmha_simt(const FmhaArgs& a, const KvView& kv, cudaStream_t st) {
 
 using namespace dgpt;
 
-extern "C" int dgpt_fmha_prefill(const void* q, int64_t q_batch_stride, int64_t q_row_stride,
-                                 const dgpt_kv_layout* kv, const int32_t* kv_len, int32_t kv_len_all, void* o,
-                                 int64_t o_batch_stride, int64_t o_row_stride, int32_t o_f32, float* lse, int32_t B,
-                                 int32_t H, int32_t Tq, int32_t D, int32_t q_offset, int32_t causal, int32_t dtype,
-                                 int32_t impl, int32_t max_ctas, int32_t* status, void* stream) {
+static int fmha_full(const void* q, int64_t q_batch_stride, int64_t q_row_stride, const dgpt_kv_layout* kv, const int32_t* kv_len,
+                     int32_t kv_len_all, void* o, int64_t o_batch_stride, int64_t o_row_stride, int32_t o_f32, float* lse,
+                     const void* egate, int64_t egate_rs, int32_t B, int32_t H, int32_t Tq, int32_t D, int32_t q_offset,
+                     int32_t causal, int32_t dtype, int32_t impl, int32_t max_ctas, int32_t* status, void* stream) {
   DGPT_REQUIRE(q && o, "fmha_prefill: NULL pointer");
   DGPT_REQUIRE(B >= 0 && H > 0 && Tq >= 0 && B <= 65535 && H <= 65535, "fmha_prefill: bad sizes");
   DGPT_REQUIRE(kv_len || kv_len_all >= 0, "fmha_prefill: kv length missing");
@@ -209,6 +215,12 @@ extern "C" int dgpt_fmha_prefill(const void* q, int64_t q_batch_stride, int64_t 
   a.B = B; a.H = H; a.Tq = Tq; a.D = D; a.q_offset = q_offset; a.causal = causal; a.dtype = dtype;
   a.status = status;
   a.max_ctas = max_ctas;
+  a.egate = egate; a.egate_rs = egate_rs;
+  a.pingpong = impl == 4;
+  // Dense keys that are not whole tiles: the tensor cores from 24 keys on (8 to 512 pairs of sequence and head; at 17 keys 6.5 us
+  // against 5.3 / 9.3 / 11.7 us for heads of 32 / 64 / 128 on the warp-level kernel, at 33 keys 6.3 against 7.5 / 13.7 / 19, at 777
+  // keys 19 to 27 against 90 to 555).
+  a.any_run = impl == 0 && (causal ? (long long)Tq + q_offset : kv_len ? (long long)kv->page_tokens : (long long)kv_len_all) >= 24;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const KvView view = make_view(kv);
   const bool tc_ok = fmha_tc_supported(a, *kv);
@@ -218,13 +230,31 @@ extern "C" int dgpt_fmha_prefill(const void* q, int64_t q_batch_stride, int64_t 
   const long long span = causal ? (long long)Tq + q_offset
                                 : (kv_len ? (long long)kv->max_pages * kv->page_tokens : (long long)kv_len_all);
   a.two_cta = impl == 3 || (impl == 0 && span < 1024);
-  a.pingpong = impl == 4;
   if (impl >= 2 && !tc_ok) {
     set_error("fmha_prefill: the tensor-core kernel does not cover dtype %d, head_dim %d with this layout", dtype, D);
     return DGPT_E_UNSUPPORTED;
   }
   if (tc_ok && impl != 1) return fmha_tc(a, *kv, st);
   return fmha_simt(a, view, st);
+}
+
+extern "C" int dgpt_fmha_prefill(const void* q, int64_t q_batch_stride, int64_t q_row_stride,
+                                 const dgpt_kv_layout* kv, const int32_t* kv_len, int32_t kv_len_all, void* o,
+                                 int64_t o_batch_stride, int64_t o_row_stride, int32_t o_f32, float* lse, int32_t B,
+                                 int32_t H, int32_t Tq, int32_t D, int32_t q_offset, int32_t causal, int32_t dtype,
+                                 int32_t impl, int32_t max_ctas, int32_t* status, void* stream) {
+  return fmha_full(q, q_batch_stride, q_row_stride, kv, kv_len, kv_len_all, o, o_batch_stride, o_row_stride, o_f32, lse, nullptr, 0, B, H,
+                   Tq, D, q_offset, causal, dtype, impl, max_ctas, status, stream);
+}
+
+extern "C" int dgpt_fmha_prefill_gated(const void* q, int64_t q_batch_stride, int64_t q_row_stride, const dgpt_kv_layout* kv,
+                                       const int32_t* kv_len, int32_t kv_len_all, void* o, int64_t o_batch_stride,
+                                       int64_t o_row_stride, const void* gate, int64_t gate_row_stride, int32_t B, int32_t H,
+                                       int32_t Tq, int32_t D, int32_t q_offset, int32_t causal, int32_t dtype, int32_t impl,
+                                       int32_t* status, void* stream) {
+  DGPT_REQUIRE(gate, "fmha_prefill_gated: NULL pointer");
+  return fmha_full(q, q_batch_stride, q_row_stride, kv, kv_len, kv_len_all, o, o_batch_stride, o_row_stride, 0, nullptr, gate,
+                   gate_row_stride, B, H, Tq, D, q_offset, causal, dtype, impl, 0, status, stream);
 }
 
 // Sliding-window attention for both entry points: `kv` with keys kv_ts elements apart, dense runs or pages.

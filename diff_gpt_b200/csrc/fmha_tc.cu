@@ -119,6 +119,8 @@ fmha_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__ C
   };
 
   float m = -INFINITY, l = 0.f;
+  if (!KEPT && p.egate && q0 + tid < p.Tq)
+    prefetch_gate(p.egate + ((long long)b * p.Tq + q0 + tid) * p.egate_rs + (long long)h * p.d_head, p.d_head * 2);
 
   if (tid == 0 && n_tiles > 0) {
     mbar_expect_tx(bar_q, kTileBytes);
@@ -281,6 +283,9 @@ fmha_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__ C
 #pragma unroll
           for (int d = 0; d < 32; d += 4)
             dst[d >> 2] = make_float4(v[d] * inv, v[d + 1] * inv, v[d + 2] * inv, v[d + 3] * inv);
+        } else if (!KEPT && p.egate) {
+          store_gated<32>(static_cast<__nv_bfloat16*>(p.o) + off + c * 32, v, inv,
+                          p.egate + ((long long)b * p.Tq + qi) * p.egate_rs + (long long)h * p.d_head + c * 32);
         } else {
           __nv_bfloat16* dst = static_cast<__nv_bfloat16*>(p.o) + off + c * 32;
 #pragma unroll
@@ -312,12 +317,13 @@ fmha_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__ C
 bool fmha_tc_supported(const FmhaArgs& a, const dgpt_kv_layout& kv) {
   if (a.dtype != DGPT_BF16 || (a.D != 32 && a.D != 64 && a.D != 128)) return false;
   const int pt = kv.page_tokens;
-  // One dense run of keys per sequence with a stated token stride (dgpt_fmha_window) may have any length: a tile never
-  // leaves the run's tensor, and what the box covers past its end arrives as zeros.
-  const bool run = a.kv_ts > 0 && kv.page_table == nullptr;
+  // One dense run of keys per sequence may have any length: a tile never leaves the run's tensor, and what the box covers
+  // past its end arrives as zeros.
+  const bool run = (a.kv_ts > 0 || a.any_run) && kv.page_table == nullptr;
   if (!run && !((pt >= tc::kBN && pt % tc::kBN == 0) || (pt >= 8 && pt < tc::kBN && tc::kBN % pt == 0))) return false;
   if (!run && kv.page_table == nullptr && pt < tc::kBN) return false;
   auto al16 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
+  if (a.egate && (!al16(a.egate) || a.egate_rs % 8 || a.pingpong)) return false;
   if (!al16(a.q) || !al16(a.o) || !al16(kv.k_base) || !al16(kv.v_base)) return false;
   if (a.q_rs % 8 || a.q_bs % 8 || a.o_rs % 8 || a.o_bs % 8 || kv.head_stride % 8 || kv.page_stride % 8) return false;
   if (a.q_rs <= 0 || kv.head_stride <= 0 || kv.page_stride <= 0) return false;
@@ -330,7 +336,7 @@ int fmha_tc(const FmhaArgs& a, const dgpt_kv_layout& kv, cudaStream_t st) {
   // engine fills what lies outside the tensor with zeros - Q K^T and P V see zero columns and are unchanged
   const int d_head = a.D;
   const int D = d_head == 32 ? 64 : d_head;
-  const bool run = a.kv_ts > 0 && kv.page_table == nullptr;
+  const bool run = (a.kv_ts > 0 || a.any_run) && kv.page_table == nullptr;
   TcMaps maps;
   CUtensorMap &mq = maps.q, &mk = maps.k, &mv = maps.v;
   {
@@ -371,6 +377,8 @@ int fmha_tc(const FmhaArgs& a, const dgpt_kv_layout& kv, cudaStream_t st) {
   p.kv_div = a.kv_heads > 0 ? a.H / a.kv_heads : 1;
   p.hgate = a.hgate;
   p.hgate_rs = a.hgate_rs;
+  p.egate = static_cast<const __nv_bfloat16*>(a.egate);
+  p.egate_rs = a.egate_rs;
   p.d_head = d_head;
   p.status = a.status;
   p.n_qt = (a.Tq + kBM - 1) / kBM;

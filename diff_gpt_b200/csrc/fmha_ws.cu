@@ -267,6 +267,8 @@ fmha_tc_ws_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant_
       const WsItem it = ws_item<KEPT>(p, bh, qt);
       const int n_tiles = it.n, klen = it.klen, q0 = it.q0, b = it.b, h = it.h;
       float m = -INFINITY, l = 0.f;
+      if (!KEPT && p.egate && half == 0 && q0 + row < p.Tq)
+        prefetch_gate(p.egate + ((long long)b * p.Tq + q0 + row) * p.egate_rs + (long long)h * p.d_head, p.d_head * 2);
       for (int j = 0; j < n_tiles; ++j) {
         const unsigned g = g0 + (unsigned)j, buf = g & 1u, ph = (g >> 1) & 1u;
         const int t0 = tile_of<KEPT>(j, it.n_window, it.tile0) * kBN;
@@ -429,6 +431,9 @@ fmha_tc_ws_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant_
 #pragma unroll
             for (int d = 0; d < 32; d += 4)
               dst[d >> 2] = make_float4(v[d] * inv, v[d + 1] * inv, v[d + 2] * inv, v[d + 3] * inv);
+          } else if (!KEPT && p.egate) {
+            store_gated<32>(static_cast<__nv_bfloat16*>(p.o) + off + c * 32, v, inv,
+                            p.egate + ((long long)b * p.Tq + qi) * p.egate_rs + (long long)h * p.d_head + half * (D / 2) + c * 32);
           } else {
             __nv_bfloat16* dst = static_cast<__nv_bfloat16*>(p.o) + off + c * 32;
 #pragma unroll

@@ -7,6 +7,8 @@
 //   mode 2:  out[m, n]     = bf16(resid[m, n] + acc[m, n])                    (the residual add of addmm, one rounding)
 //   mode 4:  out[m, n]     = bf16(xielu(acc[m, n]))   with alpha_p = alpha, alpha_n = limit
 //   mode 5:  out[m, n / 2] = bf16(silu(acc[m, n]) * acc[m, n + 1])   for even n  (interleaved gate / up)
+//   mode 6:  out[m, n]     = cap(bf16(acc[m, n]))   with cap = alpha: the head of a scoring forward, its soft-cap applied on the
+//            way out (a pass of its own over the stored logits took 214 us for 131072 x 512 of them)
 //   mode 3:  nothing is stored: row m keeps the best key of  key[m, n] = cap(bf16(acc[m, n])) / T + Gumbel noise(m, n)
 //            (no noise and T = 1 for an arg-max) in best[m], a 64-bit word (order-preserving key bits, ~n) raised with
 //            atomicMax - the tied-embedding head with the draw in its epilogue, so [M, N] logits never reach HBM
@@ -239,6 +241,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap ma, const __grid_constant__ C
             } else if (p.mode == 4) {
 #pragma unroll
               for (int x = 0; x < 8; ++x) v[8 * q + x] = xielu_fast(v[8 * q + x], p.alpha, p.limit);
+            } else if (p.mode == 6) {
+#pragma unroll
+              for (int x = 0; x < 8; ++x) v[8 * q + x] = softcap_value<__nv_bfloat16>(Io<__nv_bfloat16>::round(v[8 * q + x]), p.alpha);
             }
             st16<__nv_bfloat16>(dst + 8 * q, v + 8 * q, 1.f);
           }
@@ -339,8 +344,10 @@ int dgpt::linear_launch(const void* a, int64_t a_row_stride, const void* w, int6
                         const HeadDraw* draw, void* stream) {
   DGPT_REQUIRE(a && w && (out || epilogue == 3), "linear: NULL pointer");
   DGPT_REQUIRE(M >= 0 && N > 0 && K > 0, "linear: bad sizes");
-  DGPT_REQUIRE(epilogue >= 0 && epilogue <= 5,
-               "linear: epilogue must be 0 (store), 1 (SwiGLU of interleaved pairs), 2 (add), 3 (draw), 4 (xIELU) or 5 (SiLU gate)");
+  DGPT_REQUIRE(epilogue >= 0 && epilogue <= 6,
+               "linear: epilogue must be 0 (store), 1 (SwiGLU of interleaved pairs), 2 (add), 3 (draw), 4 (xIELU), 5 (SiLU gate) or 6 "
+               "(soft-cap)");
+  DGPT_REQUIRE(epilogue != 6 || alpha > 0.f, "linear: epilogue 6 needs a positive cap");
   DGPT_REQUIRE(epilogue != 2 || resid, "linear: epilogue 2 needs the matrix to add");
   DGPT_REQUIRE(epilogue != 3 || (draw && draw->best), "linear: epilogue 3 needs the draw parameters");
   if (dtype != DGPT_BF16) {
@@ -423,8 +430,8 @@ extern "C" int dgpt_linear(const void* a, int64_t a_row_stride, const void* w, i
                            int64_t out_row_stride, const void* resid, int64_t resid_row_stride, int32_t M, int32_t N,
                            int32_t K, int32_t epilogue, float alpha, float limit, int32_t dtype, int32_t* status,
                            void* stream) {
-  DGPT_REQUIRE((epilogue >= 0 && epilogue <= 2) || epilogue == 4 || epilogue == 5,
-               "linear: epilogue must be 0 (store), 1 (SwiGLU of interleaved pairs), 2 (add), 4 (xIELU) or 5 (SiLU gate)");
+  DGPT_REQUIRE(epilogue >= 0 && epilogue <= 6 && epilogue != 3,
+               "linear: epilogue must be 0 (store), 1 (SwiGLU of interleaved pairs), 2 (add), 4 (xIELU), 5 (SiLU gate) or 6 (soft-cap)");
   return linear_launch(a, a_row_stride, w, w_row_stride, out, out_row_stride, resid, resid_row_stride, M, N, K, epilogue, alpha,
                        limit, dtype, status, nullptr, stream);
 }

@@ -197,7 +197,9 @@ class ForwardPlan:
     every time, so a plan can be captured into a CUDA graph and replayed.
     """
 
-    def __init__(self, model: "GPT", n_seq: int, T: int, last_only: bool = False, want_logits: bool = True) -> None:
+    def __init__(self, model: "GPT", n_seq: int, T: int, last_only: bool = False, want_logits: bool = True,
+                 cap: float = 0.0) -> None:
+        """`cap`: soft-cap the logits as they are stored (0 = raw logits)."""
         emb = model.token_embedding_table.weight
         dev, dt = emb.device, emb.dtype
         C, V, L = model.n_embd, model.vocab_size, model.n_layer
@@ -217,6 +219,7 @@ class ForwardPlan:
         self.logits = buf(n_out, V) if want_logits else None
         # the tied-embedding head on the library's tcgen05 GEMM (bf16 with tileable sizes); fp32 stays on cuBLAS
         self.own_head = dt == torch.bfloat16 and C % 8 == 0 and V % 16 == 0
+        self.cap = cap
         self.status = torch.zeros(1, dtype=torch.int32, device=dev)
         # tcgen05 GEMM + SwiGLU epilogue: bf16 with tileable sizes, and enough rows to fill the tensor cores
         self.fused_ffn = FUSED_FFN and dt == torch.bfloat16 and C % 8 == 0 and n >= FUSED_FFN_MIN_ROWS
@@ -342,9 +345,8 @@ class ForwardPlan:
                 ops.fmha_prefill(
                     self.q, b.layouts[i], self.y, B=n_seq, H=H, Tq=T, D=D, q_batch_stride=T * C, q_row_stride=C,
                     o_batch_stride=T * C, o_row_stride=C, kv_len_all=b.kv_len, q_offset=b.q_offset, causal=True,
-                    impl=b.fmha_impl, status=self.status,
+                    impl=b.fmha_impl, status=self.status, gate=gv,
                 )
-                ops.sigmoid_gate(self.y, gv)
             part = self.parts[i]
             with region("gemm_proj"):
                 if partial is None:
@@ -369,10 +371,12 @@ class ForwardPlan:
         if self.logits is None:
             return None
         if self.own_head:
-            ops.linear(self.xn, W.emb, self.logits, status=self.status)
+            ops.linear(self.xn, W.emb, self.logits, softcap=self.cap, status=self.status)
         else:
             with region("gemm_logits"):
                 torch.mm(self.xn, W.emb.t(), out=self.logits)
+            if self.cap > 0:
+                ops.softcap_(self.logits, self.cap)
         return self.logits
 
 
@@ -582,10 +586,8 @@ class GPT(DeviceModel):
             bind.len1 = torch.full((B,), t0 + 1, dtype=torch.int32, device=dev)
             n_keys = t0 + 1
             bind.n_splits = _pick_splits(B * H, n_keys)
-        plan = ForwardPlan(self, B, T)
+        plan = ForwardPlan(self, B, T, cap=self.logit_softcap)
         logits = plan.run(idx.reshape(-1).to(torch.int32), bind)
-        if self.logit_softcap > 0:
-            ops.softcap_(logits, self.logit_softcap)
         if kv_cache is not None:
             kv_cache.pos = t0 + T
         return logits.view(B, T, V)

@@ -167,8 +167,21 @@ def fmha_prefill(
     impl: int = 0,
     status: torch.Tensor | None = None,
     max_ctas: int = 0,
+    gate: torch.Tensor | None = None,
 ) -> None:
-    _cuda(q, o, kv_len, lse, status)
+    """`gate`: 2-D view [B * Tq, H * D] in o's dtype; the output is multiplied by its sigmoid as `sigmoid_gate` would."""
+    _cuda(q, o, kv_len, lse, status, gate)
+    if gate is not None:
+        assert lse is None and max_ctas == 0 and o.dtype == gate.dtype == q.dtype and gate.stride(1) == 1
+        assert gate.shape == (B * Tq, H * D)
+        check(
+            lib.dgpt_fmha_prefill_gated(
+                q.data_ptr(), q_batch_stride, q_row_stride, C.byref(kv), _ptr(kv_len), kv_len_all, o.data_ptr(), o_batch_stride,
+                o_row_stride, gate.data_ptr(), gate.stride(0), B, H, Tq, D, q_offset, int(causal), dtype_code(q), impl, _ptr(status),
+                _stream(),
+            )
+        )
+        return
     o_f32 = int(o.dtype == torch.float32 and q.dtype != torch.float32)
     check(
         lib.dgpt_fmha_prefill(
@@ -269,22 +282,23 @@ def linear(
     add: torch.Tensor | None = None,
     xielu: tuple[float, float] | None = None,
     silu_gate: bool = False,
+    softcap: float = 0.0,
     status: torch.Tensor | None = None,
 ) -> None:
     """out = a @ w.T on the tcgen05 kernel (bf16).  swiglu=(alpha, limit): the SwiGLU of interleaved column pairs is
     applied in the epilogue and `out` has half as many columns as `w` has rows.  add=r: out = r + a @ w.T, rounded
     once (r may be `out`).  xielu=(alpha_p, alpha_n): that activation is applied in the epilogue.  silu_gate: column pairs
-    are (gate, up) and `out` = silu(gate) * up, half as many columns."""
+    are (gate, up) and `out` = silu(gate) * up, half as many columns.  softcap > 0: out = softcap * tanh(a @ w.T / softcap)."""
     _cuda(a, w, out, add, status)
-    assert (swiglu is not None) + (add is not None) + (xielu is not None) + silu_gate <= 1
+    assert (swiglu is not None) + (add is not None) + (xielu is not None) + silu_gate + (softcap > 0) <= 1
     M, K = a.shape
     N = w.shape[0]
     assert w.shape[1] == K and a.stride(1) == 1 and w.stride(1) == 1 and out.stride(1) == 1
     assert out.shape == (M, N // 2 if swiglu or silu_gate else N) and a.dtype == w.dtype == out.dtype
     if add is not None:
         assert add.shape == out.shape and add.dtype == out.dtype and add.stride(1) == 1
-    alpha, limit = swiglu or xielu or (0.0, 0.0)
-    epilogue = 1 if swiglu else 4 if xielu else 5 if silu_gate else 2 if add is not None else 0
+    alpha, limit = swiglu or xielu or (softcap, 0.0)
+    epilogue = 1 if swiglu else 4 if xielu else 5 if silu_gate else 6 if softcap > 0 else 2 if add is not None else 0
     check(
         lib.dgpt_linear(
             a.data_ptr(), a.stride(0), w.data_ptr(), w.stride(0), out.data_ptr(), out.stride(0), _ptr(add),

@@ -132,6 +132,15 @@ int dgpt_fmha_prefill(const void* q, int64_t q_batch_stride, int64_t q_row_strid
                       int32_t B, int32_t H, int32_t Tq, int32_t D, int32_t q_offset, int32_t causal,
                       int32_t dtype, int32_t impl, int32_t max_ctas, int32_t* status, void* stream);
 
+/* dgpt_fmha_prefill with the output gate of src/diff_gpt/model/mha.py:84 applied where the output is stored:
+ *   o[b,i,h,:] = round(o[b,i,h,:]) * round(sigmoid(gate[b*Tq + i, h*D + :])),   round = to `dtype`
+ * which is what dgpt_fmha_prefill followed by dgpt_sigmoid_gate gives, bit for bit, without the second pass.
+ * gate: device [B * Tq, H * D] in `dtype` with gate_row_stride (elements); impl 4 is not built with a gate. */
+int dgpt_fmha_prefill_gated(const void* q, int64_t q_batch_stride, int64_t q_row_stride, const dgpt_kv_layout* kv,
+                            const int32_t* kv_len, int32_t kv_len_all, void* o, int64_t o_batch_stride, int64_t o_row_stride,
+                            const void* gate, int64_t gate_row_stride, int32_t B, int32_t H, int32_t Tq, int32_t D,
+                            int32_t q_offset, int32_t causal, int32_t dtype, int32_t impl, int32_t* status, void* stream);
+
 /* Bytes of workspace dgpt_decode_attn needs for R rows, H heads, head_dim D and n_splits (a multiple of 16;
  * the workspace pointer itself must be 16-byte aligned). */
 size_t dgpt_decode_attn_workspace_bytes(int32_t R, int32_t H, int32_t D, int32_t n_splits);
@@ -217,9 +226,10 @@ int dgpt_softcap(void* logits, int64_t n, float cap, int32_t dtype, void* stream
  *   epilogue 2:  out[m, n]     = resid[m, n] + acc[m, n], rounded once (resid may be out itself)   out: [M, N]
  *   epilogue 4:  out[m, n]     = xielu(acc[m, n]) with alpha_p = alpha, alpha_n = limit (see dgpt_xielu)   out: [M, N]
  *   epilogue 5:  out[m, n / 2] = silu(acc[m, n]) * acc[m, n + 1] for even n, from the unrounded accumulator     out: [M, N / 2]
+ *   epilogue 6:  out[m, n]     = alpha * tanh(acc[m, n] / alpha), the rule of dgpt_softcap with cap = alpha > 0   out: [M, N]
  * Replaces nn.Linear of src/diff_gpt/model/feed_forward.py:10-14 followed by swi_glu.py:11-19 (epilogue 1), any
  * bias-free nn.Linear of the path (epilogue 0), or a projection with the residual add that follows it
- * (src/diff_gpt/model/block.py:98-106, epilogue 2).  resid is ignored for epilogues 0, 1, 4 and 5.  bf16 only; pointers 16-byte aligned, K and the row strides
+ * (src/diff_gpt/model/block.py:98-106, epilogue 2).  resid is ignored for epilogues 0, 1, 4, 5 and 6.  bf16 only; pointers 16-byte aligned, K and the row strides
  * multiples of 8 elements, N a multiple of 16.  status: device int32, set non-zero if a bounded wait ran out. */
 int dgpt_linear(const void* a, int64_t a_row_stride, const void* w, int64_t w_row_stride, void* out,
                 int64_t out_row_stride, const void* resid, int64_t resid_row_stride, int32_t M, int32_t N,
