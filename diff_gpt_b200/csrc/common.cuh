@@ -64,8 +64,12 @@ template <>
 struct Io<__nv_bfloat16> {
   static __device__ __forceinline__ float ld(const __nv_bfloat16* p) { return __bfloat162float(*p); }
   static __device__ __forceinline__ void st(__nv_bfloat16* p, float v) { *p = __float2bfloat16_rn(v); }
+  // To bf16 and back in one instruction: packed with a zero below it, the bf16 already sits where fp32 has it.  (The
+  // conversion of a single number runs at a quarter of the packed one's rate.)
   static __device__ __forceinline__ float round(float v) {
-    return __bfloat162float(__float2bfloat16_rn(v));
+    uint32_t r;
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(v), "f"(0.f));
+    return __uint_as_float(r);
   }
   static constexpr int kVec16 = 8;
 };

@@ -2,6 +2,7 @@
 // stream and the logit soft-cap with the reference's rounding points.
 #pragma once
 
+#include "activation.cuh"
 #include "common.cuh"
 
 namespace dgpt {
@@ -51,8 +52,8 @@ __device__ __forceinline__ float softcap_value(float x, float cap) {
 template <>
 __device__ __forceinline__ float softcap_value<__nv_bfloat16>(float x, float cap) {
   using B = Io<__nv_bfloat16>;
-  const float t = B::round(__fdividef(x, cap));
-  const float th = 1.f - __fdividef(2.f, __expf(2.f * fabsf(t)) + 1.f);  // e^{2|t|} = inf gives 1
+  const float t = B::round(x * rcp_fast(cap));
+  const float th = 1.f - 2.f * rcp_fast(exp_fast(2.f * fabsf(t)) + 1.f);  // e^{2|t|} = inf gives 1
   return B::round(cap * B::round(copysignf(th, t)));
 }
 
