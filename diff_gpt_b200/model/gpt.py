@@ -152,9 +152,28 @@ FUSED_FFN_MIN_ROWS = 256
 # kernel with two query tiles per CTA on 64 SMs, which it owns outright (it fills an SM's shared memory and TMEM)
 # while the HBM-bound per-row kernel has the other 84 to itself, 1249-1259 ms; on 48 or 80 SMs 1256-1262; the small
 # kernel (impl 3) on every SM, one CTA each, sharing the SMs with the per-row kernel, 1271-1275; the persistent kernel
-# with one query tile per CTA on 64 SMs 1267-1271, on 40 SMs 1288 (the phase becomes the longer one).
+# with one query tile per CTA on 64 SMs 1267-1271, on 40 SMs 1288 (the phase becomes the longer one).  Where the prompt
+# phase is the longer one it takes more SMs: see `prefix_ctas`.
 PREFIX_CTAS = 64
 PREFIX_IMPL = 4
+
+
+def prefix_ctas(units: int, key_tiles: int, own_us: float, n_sm: int) -> int:
+    """SMs for the shared-prompt phase: `units` work items (pairs of 128-query tiles) of `key_tiles` 128-key tiles, about 3.3 us a
+    tile, beside a per-row phase that takes `own_us` on the whole GPU and meanwhile advances on the SMs left over.  PREFIX_CTAS,
+    unless one SM per unit, or every SM, is estimated to be done earlier.  Measured per layer with the merge, us: 3 x 333 rows,
+    12 heads, 777 + 20 keys (72 units) on 64 SMs 42.5, on 72 34.1; 10 x 64 rows, 8 heads, 500 + 30 keys (80 units) 26.9 -> 19.0; 40 x
+    20 rows, 12 heads, 1000 + 40 keys (480 units) 148, on all 92; 4096 rows, 12 heads, 1024 + 128 keys (192 units) 282, on all 295."""
+
+    def estimate(ctas: int) -> float:
+        phase = -(-units // ctas) * key_tiles * 3.3
+        return phase + max(0.0, own_us - phase * min(1.0, 1.3 * (n_sm - ctas) / n_sm))
+
+    few = min(PREFIX_CTAS, n_sm)
+    many = min(units, n_sm)
+    return many if units > few and estimate(many) < 0.97 * estimate(few) else few
+
+
 SIDE_PRIORITY = -1  # stream of the shared-prompt attention phase: ahead of the per-row phase it runs beside
 
 
@@ -185,6 +204,8 @@ class KvBinding:
     n_splits: int = 1
     shared_layouts: list | None = None
     shared_len: torch.Tensor | None = None
+    shared_keys: int = 0  # the longest prompt, on the host
+    own_keys: int = 0  # mean number of a row's own keys over the run, on the host
     rows_per_series: int = 0
     fmha_impl: int = 0
     overlap_prefix: bool = False  # run the shared-prompt phase on a second stream beside the per-row phase
@@ -270,7 +291,11 @@ class ForwardPlan:
             self.part_lse = torch.empty((self.n, H), dtype=torch.float32, device=dev)
             self.side = torch.cuda.Stream(device=dev, priority=SIDE_PRIORITY)
             n_sm = torch.cuda.get_device_properties(dev).multi_processor_count
-            self.prefix_ctas = n_sm if PREFIX_CTAS is None else min(PREFIX_CTAS, n_sm)
+            rows, size = b.rows_per_series, self.q.element_size()
+            units = (self.n // rows) * H * (-(-rows // 256))
+            # the per-row phase: its bytes at the copy rate, and what a warp per (row, head) costs however few its keys
+            own_us = self.n * H * (2 * D * size * b.own_keys / 6.65e6 + 4e-4)
+            self.prefix_ctas = prefix_ctas(units, -(-b.shared_keys // 128), own_us, n_sm)
             # the persistent tensor-core kernel covers bf16 heads of 32, 64 or 128 in pages that tile its 128-key
             # blocks; other models leave the choice to the library (its warp-level kernel)
             pt = int(b.shared_layouts[0].page_tokens)
@@ -530,6 +555,8 @@ class GPT(DeviceModel):
             n_splits=1 if shared else _pick_splits(R * self.n_head, max_keys),
             shared_layouts=[cache.prefix_layout(l) for l in range(L)] if shared else None,
             shared_len=prompt_lens if shared else None,
+            shared_keys=cache.prefix_len,
+            own_keys=max(1, cache.max_new // 2),
             rows_per_series=cache.rows_per_series,
             fmha_impl=fmha_impl,
             overlap_prefix=overlap_prefix and shared,
@@ -632,11 +659,13 @@ def _sm_count() -> int:
 
 
 def _pick_splits(n_pairs: int, n_keys: int) -> int:
-    """Split the keys when (row, head) pairs alone cannot fill the GPU (16 warps on every multiprocessor)."""
-    target_warps = _sm_count() * 16
-    if n_pairs <= 0 or n_pairs >= target_warps or n_keys < 512:
+    """Split the keys when (row, head) pairs alone cannot fill the GPU: as many splits as leave one wave of CTAs, 16 warps on
+    every multiprocessor.  One more split makes a second wave of a few CTAs: 64 rows, 8 heads of 64, 3682 keys, us: 4 splits (512
+    CTAs of 592) 76, 5 splits (640) 96; 130 rows, 1400 keys: 2 splits 61, 3 splits 71."""
+    room = _sm_count() * 16
+    if n_pairs <= 0 or 2 * n_pairs > room or n_keys < 512:
         return 1
-    return max(1, min(-(-target_warps // n_pairs), n_keys // 256, 64))
+    return max(1, min(room // n_pairs, n_keys // 256, 64))
 
 
 def _ordinal_soft_ce(logits: torch.Tensor, targets: torch.Tensor, sigma: float, ignore_index: int = -100):
