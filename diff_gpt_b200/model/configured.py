@@ -11,7 +11,7 @@ import torch
 import torch.nn as nn
 import torch.nn.functional as F
 
-from .gpt import DeviceModel, _sm_count
+from .gpt import DeviceModel, SingleStep, _sm_count
 from .kv_cache import RowCache
 
 FUSED_FF_MIN_ROWS = 256  # rows from which the up projection runs on the library's GEMM with the activation fused
@@ -82,7 +82,8 @@ class ConfiguredModel(DeviceModel):
         return str(self.embed.device.type)
 
     def packed_weights(self):
-        stamp = tuple((p.data_ptr(), p._version, p.dtype) for p in self.parameters())
+        # every parameter is registered on the model itself: no walk through modules (0.3 ms a call with 139 of them)
+        stamp = tuple((p.data_ptr(), p._version, p.dtype) for p in self._parameters.values())
         if self._packed is None or self._packed.stamp != stamp:
             with torch.no_grad():
                 self._packed = self.pack(stamp)
@@ -97,8 +98,9 @@ class ConfiguredModel(DeviceModel):
         ...
 
     @abstractmethod
-    def step_binding(self, cache: RowCache, B: int, T: int):
-        """How the next T tokens of each sequence are bound to a cache that has room for them."""
+    def step_binding(self, cache: RowCache, B: int, T: int, numbers: torch.Tensor | None = None):
+        """How the next T tokens of each sequence are bound to a cache that has room for them.  `numbers` (int32 [4] on the device, B =
+        T = 1): slot, position and key count are its last three."""
 
     # ---- forward behind a cache ----------------------------------------------------------------
     def _step(self, idx: torch.Tensor, cache: RowCache, rows: torch.Tensor | None, tap: Callable | None = None) -> torch.Tensor:
@@ -123,6 +125,21 @@ class ConfiguredModel(DeviceModel):
     @torch.inference_mode()
     def logits_at(self, idx, cache, rows):
         return self._step(idx, cache, rows)
+
+    def single_step(self, cache: RowCache, old: SingleStep | None) -> SingleStep:
+        cache.ensure(1)
+        # the key splits change from one 128-key tile to the next, until every window is full
+        kind = -(-min(cache.slot + 1, cache.keep + 1 + cache.keep_first) // 128)
+        held = (self.packed_weights(), *cache.state.source.values(), *cache.store.values(), *self.step_tables(cache.pos + 1))
+        if old is not None and old.fits(kind, held):
+            return old
+        numbers = torch.zeros(4, dtype=torch.int32, device=self.embedding.device)
+        bind = self.step_binding(cache, 1, 1, numbers)
+        return SingleStep(self.new_plan(1, 1, rows=1), bind, numbers, kind, held, checks=True)
+
+    def step_tables(self, positions: int) -> tuple:
+        """Tables that a binding for this many positions points at."""
+        return ()
 
     def forward(self, idx: torch.Tensor, targets: torch.Tensor | None = None, kv_cache: RowCache | None = None):
         if not idx.is_cuda:

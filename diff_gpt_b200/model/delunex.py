@@ -440,13 +440,17 @@ class Delunex(ConfiguredModel):
     def new_plan(self, n_seq, T, **kw) -> DelunexPlan:
         return DelunexPlan(self, n_seq, T, **kw)
 
-    def step_binding(self, cache: LatentCache, B: int, T: int) -> LatentBinding:
+    def step_binding(self, cache: LatentCache, B: int, T: int, numbers: torch.Tensor | None = None) -> LatentBinding:
         dev = self.embedding.device
         slot = cache.slot
-        start = torch.full((B,), slot, dtype=torch.int32, device=dev)
+        if numbers is None:
+            start = torch.full((B,), slot, dtype=torch.int32, device=dev)
+            keys = start + 1
+        else:
+            start, keys = numbers[1:2], numbers[3:4]
         state = cache.state
         return LatentBinding(
-            layout=cache.layout, slot0=start, start1=torch.zeros_like(start), len1=start + 1, keys=slot + T, expand=True,
+            layout=cache.layout, slot0=start, start1=torch.zeros((B,), dtype=torch.int32, device=dev), len1=keys, keys=slot + T, expand=True,
             context=slot, latents=lambda layer, n: cache.span(layer, slot - n, slot + T), conv_in=state.source["conv"],
             conv_out=(state.source if T == 1 else state.target)["conv"],
         )

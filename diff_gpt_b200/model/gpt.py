@@ -83,6 +83,11 @@ class DeviceModel(BaseGPT):
     def logits_at(self, idx: torch.Tensor, cache, rows: torch.Tensor) -> torch.Tensor:
         """Run idx (1, T) behind what `cache` holds; the logits [len(rows), V] of the given places among the T tokens."""
 
+    def single_step(self, cache, old: "SingleStep | None") -> "SingleStep | None":
+        """The launches of one more token behind `cache`, which has room for it afterwards: `old` where it still fits, or None
+        where a single token takes the general path."""
+        return None
+
     # -- batched decode (DecodeRun) --
     @abstractmethod
     def paged_cache(self, n_series: int, rows_per_series: int, prefix_len: int, max_new: int, page_tokens: int, pool=None):
@@ -175,6 +180,32 @@ def prefix_ctas(units: int, key_tiles: int, own_us: float, n_sm: int) -> int:
 
 
 SIDE_PRIORITY = -1  # stream of the shared-prompt attention phase: ahead of the per-row phase it runs beside
+
+
+@dataclass
+class SingleStep:
+    """One token of one request: a plan and a binding whose changing numbers are read from `numbers` on the device (token, slot,
+    position, keys), so that the launches can be recorded once and replayed.
+
+    kind    host-side choices that the launches were made with (key splits)
+    held    what the launches point at; kept alive here and compared by `is`
+    """
+
+    plan: object
+    bind: object
+    numbers: torch.Tensor  # int32 [4]
+    kind: int
+    held: tuple
+    checks: bool  # the plan's status is read after every step
+    graph: torch.cuda.CUDAGraph | None = None
+    launches: int = 0
+    runs: int = 0
+
+    def fits(self, kind: int, held: tuple) -> bool:
+        return self.kind == kind and len(self.held) == len(held) and all(a is b for a, b in zip(self.held, held))
+
+    def enqueue(self) -> None:
+        self.plan.run(self.numbers[0:1], self.bind)
 
 
 # ---- how one forward call is bound to K/V storage ----------------------------------
@@ -523,6 +554,24 @@ class GPT(DeviceModel):
     @torch.inference_mode()
     def logits_at(self, idx: torch.Tensor, cache: KVCache, rows: torch.Tensor) -> torch.Tensor:
         return self(idx, kv_cache=cache)[0][0].index_select(0, rows)
+
+    def single_step(self, cache: KVCache, old: SingleStep | None) -> SingleStep | None:
+        t0, H, emb = cache.get_pos(), self.n_head, self.embedding
+        if t0 == 0:
+            return None
+        assert t0 + 1 <= self.freqs_cis.shape[0]
+        cache.ensure(t0 + 1, emb.dtype, emb.device)
+        splits = _pick_splits(H, t0 + 1)
+        held = (self.packed_weights(), cache.kv_cache)
+        if old is not None and old.fits(splits, held):
+            return old
+        numbers = torch.zeros(4, dtype=torch.int32, device=emb.device)
+        zero = torch.zeros(1, dtype=torch.int32, device=emb.device)
+        bind = KvBinding(
+            layouts=[cache.layer_layout(i) for i in range(self.n_layer)], pos0=numbers[2:3], slot0=numbers[1:2], decode=True, len0=zero,
+            start1=zero, len1=numbers[3:4], n_splits=splits,
+        )
+        return SingleStep(ForwardPlan(self, 1, 1, cap=self.logit_softcap), bind, numbers, splits, held, checks=False)
 
     def paged_cache(self, n_series, rows_per_series, prefix_len, max_new, page_tokens, pool=None) -> PagedKVCache:
         emb = self.embedding

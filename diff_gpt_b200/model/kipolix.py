@@ -507,12 +507,19 @@ class Kipolix(ConfiguredModel):
     def new_plan(self, n_seq, T, **kw) -> KipolixPlan:
         return KipolixPlan(self, n_seq, T, **kw)
 
-    def step_binding(self, cache: RowCache, B: int, T: int) -> RowBinding:
+    def step_tables(self, positions: int) -> tuple:
+        return tuple(self.tables(positions).values())
+
+    def step_binding(self, cache: RowCache, B: int, T: int, numbers: torch.Tensor | None = None) -> RowBinding:
         dev = self.embedding.device
         slot, state = cache.slot, cache.state
-        start = torch.full((B,), slot, dtype=torch.int32, device=dev)
+        if numbers is None:
+            start = torch.full((B,), slot, dtype=torch.int32, device=dev)
+            pos, keys = torch.full((B,), cache.pos, dtype=torch.int32, device=dev), start + 1
+        else:
+            start, pos, keys = numbers[1:2], numbers[2:3], numbers[3:4]
         return RowBinding(
-            layout=cache.layout, slot0=start, pos0=torch.full((B,), cache.pos, dtype=torch.int32, device=dev),
-            start1=torch.zeros_like(start), len1=start + 1, keys=slot + T, tables=self.tables(cache.pos + T), state_in=state.source,
-            state_out=state.source if T == 1 else state.target, context=slot, kv_layout=cache.kv_layout,
+            layout=cache.layout, slot0=start, pos0=pos, start1=torch.zeros((B,), dtype=torch.int32, device=dev), len1=keys, keys=slot + T,
+            tables=self.tables(cache.pos + T), state_in=state.source, state_out=state.source if T == 1 else state.target, context=slot,
+            kv_layout=cache.kv_layout,
         )

@@ -1,0 +1,82 @@
+"""Single tokens through StepRunner (recorded launches) against the general path behind a cache of its own, bit for bit."""
+
+import pytest
+import torch
+
+import delunex_cases
+import kipolix_cases
+
+pytestmark = pytest.mark.gpu
+
+
+def _model(family, dtype):
+    if family == "gpt":
+        from diff_gpt_b200 import GPT
+
+        torch.manual_seed(0)
+        m = GPT(vocab_size=128, n_embd=96, block_size=2048, n_head=3, n_layer=3)
+        for p in m.parameters():
+            torch.nn.init.normal_(p, std=0.1)
+        return m.to(dtype).cuda().eval(), 128
+    cases = {"delunex": delunex_cases, "kipolix": kipolix_cases}[family]
+    cfg = cases.CASES["wide"]
+    return cases.build(cfg, 5, dtype)[0], cfg["vocab"]
+
+
+def _plain(model, cache, ids):
+    idx = torch.tensor([ids], device="cuda")
+    return model.logits_at(idx, cache, torch.tensor([len(ids) - 1], device="cuda")).float().clone()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("family", ["gpt", "delunex", "kipolix"])
+def test_recorded_steps_equal_the_general_path(family, dtype):
+    """From the first token over 1200 tokens: every count of key splits, portions in between (which swap the state buffer), a
+    grown or moved cache, weights changed on the way, and a second request that takes the cache over."""
+    from diff_gpt_b200 import StepRunner
+
+    model, V = _model(family, dtype)
+    runner = StepRunner(model)
+    g = torch.Generator().manual_seed(1)
+    ids = torch.randint(0, V, (1300,), generator=g).tolist()
+    for n_tokens, portions in ((1300, {5: 3, 40: 120, 300: 40, 900: 150}), (30, {0: 7})):
+        cache = model.new_cache()
+        cache.reset()
+        at, part = 0, []
+        with torch.inference_mode():
+            while at < n_tokens:
+                n = min(portions.get(at, 1), n_tokens - at)
+                got = runner.step("r", ids[at : at + n], [n - 1])
+                part.append(torch.equal(got, _plain(model, cache, ids[at : at + n])))
+                at += n
+                if at == 700:
+                    w = model.token_embedding_table.weight if family == "gpt" else model.embed
+                    w.mul_(1.25)
+        assert all(part), [i for i, ok in enumerate(part) if not ok][:5]
+        assert any(one.graph is not None for one in runner._single.values())
+        runner.finish("r")
+    assert len(runner._free) == 1 and len(runner._single) <= 2
+
+
+def test_requests_on_their_own_streams():
+    """Two requests stepped from two streams without any wait between them give what they give alone."""
+    from diff_gpt_b200 import StepRunner
+
+    model, V = _model("kipolix", torch.bfloat16)
+    runner = StepRunner(model)
+    ids = {k: torch.randint(0, V, (60,), generator=torch.Generator().manual_seed(k)).tolist() for k in range(2)}
+    want = {}
+    for k, t in ids.items():
+        cache = model.new_cache()
+        with torch.inference_mode():
+            want[k] = torch.cat([_plain(model, cache, [x]) for x in t])
+    streams = [torch.cuda.Stream() for _ in ids]
+    got = {k: [] for k in ids}
+    torch.cuda.synchronize()
+    for i in range(60):
+        for k in ids:
+            with torch.cuda.stream(streams[k]):
+                got[k].append(runner.step(k, [ids[k][i]], [0]))
+    torch.cuda.synchronize()
+    for k in ids:
+        assert torch.equal(torch.cat(got[k]), want[k])
