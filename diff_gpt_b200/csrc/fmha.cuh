@@ -1,6 +1,7 @@
 // Argument block shared by the two prefill-attention kernels.
 #pragma once
 
+#include "activation.cuh"
 #include "common.cuh"
 
 namespace dgpt {
@@ -16,7 +17,7 @@ struct FmhaArgs {
   float* lse;
   int B, H, Tq, D, q_offset, causal, dtype;
   int* status;
-  int max_ctas;  // two-CTAs-per-SM kernel only: at most this many CTAs, looping over the query tiles (0 = one CTA per tile)
+  int max_ctas;  // at most this many CTAs, looping over the query tiles (0 = as many as fit)
   int two_cta;  // tensor-core path only: the 128-thread kernel with two CTAs per SM instead of the warp-specialised one
   int pingpong;  // tensor-core path only: the kernel with two query tiles per CTA
   // sliding-window form (dgpt_fmha_window); the defaults leave the kernels as dgpt_fmha_prefill uses them
@@ -71,12 +72,12 @@ template <typename T>
 __device__ __forceinline__ float gated(float o, float g) {
   return Io<T>::round(o) * Io<T>::round(1.f / (1.f + __expf(-g)));
 }
-// bf16 keeps 8 bits of the sigmoid, so the two-instruction division (2 ulp of fp32) gives the same rounded value except
+// bf16 keeps 8 bits of the sigmoid, so the one-instruction reciprocal (1 ulp of fp32) gives the same rounded value except
 // within 2e-7 of a rounding boundary; the full one cost a fifth of the short kernel (425 against 355 us on config 2's shape).
 template <>
 __device__ __forceinline__ float gated<__nv_bfloat16>(float o, float g) {
   using B = Io<__nv_bfloat16>;
-  return B::round(o) * B::round(__fdividef(1.f, 1.f + __expf(-g)));
+  return B::round(o) * B::round(rcp_fast(1.f + exp_fast(-g)));
 }
 // N columns (a multiple of 8) of one output row, gated: the stored row never makes a second trip through memory.  (The
 // separate pass took 171 us for 131072 x 256 elements and 597 us for 228480 x 512.)

@@ -194,6 +194,15 @@ int fmha_simt(const FmhaArgs& a, const KvView& kv, cudaStream_t st) {
 
 using namespace dgpt;
 
+// Every query tile in one round of one CTA per SM.
+static bool fmha_one_round(const FmhaArgs& a) {
+  static int n_sm[64] = {};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
+  if (n_sm[dev] == 0) cudaDeviceGetAttribute(&n_sm[dev], cudaDevAttrMultiProcessorCount, dev);
+  return (long long)a.B * a.H * ((a.Tq + 127) / 128) <= n_sm[dev];
+}
+
 static int fmha_full(const void* q, int64_t q_batch_stride, int64_t q_row_stride, const dgpt_kv_layout* kv, const int32_t* kv_len,
                      int32_t kv_len_all, void* o, int64_t o_batch_stride, int64_t o_row_stride, int32_t o_f32, float* lse,
                      const void* egate, int64_t egate_rs, int32_t B, int32_t H, int32_t Tq, int32_t D, int32_t q_offset,
@@ -224,12 +233,14 @@ static int fmha_full(const void* q, int64_t q_batch_stride, int64_t q_row_stride
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const KvView view = make_view(kv);
   const bool tc_ok = fmha_tc_supported(a, *kv);
-  // Which tensor-core kernel: the persistent warp-specialised one from 1024 keys on (measured against the small one on
-  // one to 256 sequences of 1024 to 3584 keys, heads of 32, 64 and 128: 5 to 65 % ahead; level at 512 keys); below
-  // that two smaller CTAs per SM, each done with its item after a few key tiles.
+  // Which tensor-core kernel: the persistent warp-specialised one from 640 keys on (5 to 65 % ahead from 1024; 32 sequences of 768, 12
+  // heads of 64, 111 against 115 us) and where one round of its CTAs holds every query tile, so that only the length of a tile's chain
+  // counts (8 heads of 64: 4 x 640 tokens 12 against 17 us, 3 x 768, 12 heads, 15 against 20; 128 tokens 7.0 against 7.2); else
+  // two smaller CTAs per SM, each done with its item after a few key tiles (256 x 512, 8 heads of 32, 285 against 291 us, 256 x 128 44
+  // against 57).
   const long long span = causal ? (long long)Tq + q_offset
                                 : (kv_len ? (long long)kv->max_pages * kv->page_tokens : (long long)kv_len_all);
-  a.two_cta = impl == 3 || (impl == 0 && span < 1024);
+  a.two_cta = impl == 3 || (impl == 0 && span < 640 && !fmha_one_round(a));
   if (impl >= 2 && !tc_ok) {
     set_error("fmha_prefill: the tensor-core kernel does not cover dtype %d, head_dim %d with this layout", dtype, D);
     return DGPT_E_UNSUPPORTED;
@@ -285,10 +296,11 @@ static int fmha_sliding(const char* what, const void* q, int64_t q_batch_stride,
   a.kv_heads = G; a.keep_first = keep_first;
   a.hgate = gate; a.hgate_rs = gate_row_stride;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  // The persistent kernel from 1024 keys on, as for full attention, unless the window leaves a query tile only a few key
-  // tiles (16 heads, 8192 tokens: window 128 39 against 46 us, 512 level, 1024 126 against 107 us; with kept first keys the
-  // persistent one is ahead at 256 and 512 too).
-  a.two_cta = impl == 3 || (impl == 0 && (n_keys < 1024 || (window > 0 && window <= 512 && keep_first == 0)));
+  // The persistent kernel as for full attention, unless the window leaves a query tile only a few key tiles (16 heads, 8192
+  // tokens: window 128 39 against 46 us, 512 level, 1024 126 against 107 us).  With kept first keys it is ahead from 512 keys on (256
+  // sequences, 16 heads of 128, 776 against 883 us; 8 x 2048, window 512, 143 against 156).
+  const bool short_keys = n_keys < (keep_first > 0 ? 512 : 640) && !fmha_one_round(a);
+  a.two_cta = impl == 3 || (impl == 0 && (short_keys || (window > 0 && window <= 512 && keep_first == 0)));
   const bool tc_ok = fmha_tc_supported(a, kv);
   if (impl >= 2 && !tc_ok) {
     set_error("%s: the tensor-core kernels do not cover dtype %d, head_dim %d with this layout", what, dtype, D);

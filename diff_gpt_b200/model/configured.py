@@ -147,7 +147,9 @@ class ConfiguredModel(DeviceModel):
         B, T = idx.shape
         with torch.inference_mode():
             cache = self.new_cache(B, T) if kv_cache is None else kv_cache
-            logits = self._step(idx, cache, None).view(B, T, self.vocab_size).clone()
+            logits = self._step(idx, cache, None).view(B, T, self.vocab_size)
+            if T == 1:  # the plan of a single token is kept and its buffer written again (a longer call's belongs to the caller)
+                logits = logits.clone()
         loss = None
         if targets is not None:
             loss = F.cross_entropy(logits.view(-1, self.vocab_size).float(), targets.view(-1))
