@@ -138,6 +138,106 @@ __global__ void depthmix_kernel(CandPtrs cands, int n_cands, const T* __restrict
 
 // Same algorithm with 16-byte accesses: lane l owns vectors l + 32*i (i < NV) of VEC elements each.
 // Used when n_embd is a multiple of VEC and every pointer is 16-byte aligned.
+// LPR = lanes that share a row: lane l of them owns vectors l + LPR*i.
+template <typename T, int NV, int LPR = 32>
+struct MixRow {
+  static constexpr int VEC = Io<T>::kVec16;
+  static constexpr int E = NV * VEC;
+  float acc[E], m, l;
+  __device__ __forceinline__ void clear() {
+#pragma unroll
+    for (int x = 0; x < E; ++x) acc[x] = 0.f;
+    m = -INFINITY;
+    l = 0.f;
+  }
+  // the only candidate: the mix is the identity
+  __device__ __forceinline__ void set(const float* v) {
+#pragma unroll
+    for (int x = 0; x < E; ++x) acc[x] = v[x];
+    l = 1.f;
+  }
+  // logit = rms_norm(v) . w = rsqrt(mean(v^2) + eps) * (v . w): both sums in one sweep and one
+  // interleaved butterfly.  (The reference rounds rms_norm(v) to the storage type before the
+  // product; for bf16 that changes the logit by ~1e-4 of its own rounding step.)
+  // A committed candidate does not change between mixes, so its norm factor is computed by the first mix that
+  // sees it and handed to the later ones: they skip the sum of squares and its half of the butterfly.  The
+  // factor is the same number either way (same code computed it), so results do not depend on the cache.
+  // Returns the norm factor.
+  __device__ __forceinline__ float add(const float* v, const float* wv, bool cached, float inv_cached, float mult, int C) {
+    float s4[4] = {0.f, 0.f, 0.f, 0.f}, d4[4] = {0.f, 0.f, 0.f, 0.f};
+    float inv;
+    float dr;
+    if (cached) {
+#pragma unroll
+      for (int x = 0; x < E; ++x) d4[x & 3] += v[x] * wv[x];
+      dr = (d4[0] + d4[1]) + (d4[2] + d4[3]);
+#pragma unroll
+      for (int o = LPR / 2; o > 0; o >>= 1) dr += __shfl_xor_sync(0xffffffffu, dr, o);
+      inv = inv_cached;
+    } else {
+#pragma unroll
+      for (int x = 0; x < E; ++x) {
+        s4[x & 3] += v[x] * v[x];
+        d4[x & 3] += v[x] * wv[x];
+      }
+      float ss = (s4[0] + s4[1]) + (s4[2] + s4[3]);
+      dr = (d4[0] + d4[1]) + (d4[2] + d4[3]);
+#pragma unroll
+      for (int o = LPR / 2; o > 0; o >>= 1) {
+        ss += __shfl_xor_sync(0xffffffffu, ss, o);
+        dr += __shfl_xor_sync(0xffffffffu, dr, o);
+      }
+      inv = rsqrtf(ss / (float)C + kRmsEps);
+    }
+    const float dot = Io<T>::round(dr * inv);
+    if (dot > m) {  // the same in all lanes of the row: the accumulator is rescaled only when the running maximum moves
+      const float resc = __expf(m - dot);
+      l *= resc;
+#pragma unroll
+      for (int x = 0; x < E; ++x) acc[x] *= resc;
+      m = dot;
+    }
+    const float pw = __expf(dot - m) * mult;
+    l += pw;
+#pragma unroll
+    for (int x = 0; x < E; ++x) acc[x] += pw * v[x];
+    return inv;
+  }
+  __device__ __forceinline__ void store(T* out_h, T* out_rn, long long row, int lane, int nvec, int C, bool row_ok = true) {
+    const float invl = 1.f / l;
+    float s4[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int x = 0; x < E; ++x) {
+      acc[x] = Io<T>::round(acc[x] * invl);
+      s4[x & 3] += acc[x] * acc[x];
+    }
+    float ss = (s4[0] + s4[1]) + (s4[2] + s4[3]);
+#pragma unroll
+    for (int o = LPR / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+    const float inv = rsqrtf(ss / (float)C + kRmsEps);
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+      const int j = lane + LPR * i;
+      if (j >= nvec || !row_ok) continue;
+      if (out_h) st16<T>(out_h + row * C + j * VEC, acc + i * VEC, 1.f);
+      if (out_rn) st16<T>(out_rn + row * C + j * VEC, acc + i * VEC, inv);
+    }
+  }
+};
+template <typename T, int NV, int LPR = 32>
+__device__ __forceinline__ void mix_weights(const T* w, int n_cands, int lane, int nvec, float* wv) {
+  constexpr int VEC = Io<T>::kVec16;
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    const int j = lane + LPR * i;
+#pragma unroll
+    for (int x = 0; x < VEC; ++x) wv[i * VEC + x] = 0.f;
+    if (n_cands > 1 && j < nvec) ld16<T>(w + j * VEC, wv + i * VEC);
+  }
+}
+
+// Few rows: a warp per row.  The candidates are reduced one after another, so the next one's row is fetched (as raw
+// 16-byte words) before the current one is reduced (two or three ahead were measured slower).
 template <typename T, int NV>
 __global__ void __launch_bounds__(128, 4)
 depthmix_vec_kernel(CandPtrs cands, int n_cands, const T* __restrict__ w, T* __restrict__ out_h,
@@ -149,114 +249,102 @@ depthmix_vec_kernel(CandPtrs cands, int n_cands, const T* __restrict__ w, T* __r
   if (row >= rows) return;
   const int lane = threadIdx.x & 31;
   const int nvec = C / VEC;
-  float acc[E], wv[E];
-#pragma unroll
-  for (int i = 0; i < NV; ++i) {
-    const int j = lane + 32 * i;
-#pragma unroll
-    for (int x = 0; x < VEC; ++x) acc[i * VEC + x] = wv[i * VEC + x] = 0.f;
-    if (n_cands > 1 && j < nvec) ld16<T>(w + j * VEC, wv + i * VEC);
-  }
-  float m = -INFINITY, l = 0.f;
-  // The candidates are reduced one after another (online softmax), so the rows of the next ones are
-  // fetched (as raw 16-byte words) before the current one is reduced, to keep loads in flight.
-#ifndef DGPT_MIX_AHEAD
-#define DGPT_MIX_AHEAD 1  // candidates in flight beyond the current one (2 and 3 measured slower)
-#endif
-  constexpr int AHEAD = DGPT_MIX_AHEAD;
-  uint4 nxt[AHEAD][NV];
-  float inv_nxt = 0.f;  // the cached norm factor of the candidate in nxt[0], when it has one (AHEAD == 1)
-  auto fetch = [&](int n, uint4* dst) {
-    if (AHEAD == 1 && cands.inv[n]) inv_nxt = cands.inv[n][row];
+  float wv[E];
+  mix_weights<T, NV>(w, n_cands, lane, nvec, wv);
+  MixRow<T, NV> mix;
+  mix.clear();
+  uint4 nxt[NV];
+  float inv_nxt = 0.f;  // the cached norm factor of the candidate in nxt, when it has one
+  auto fetch = [&](int n) {
+    if (cands.inv[n]) inv_nxt = cands.inv[n][row];
     const T* src = static_cast<const T*>(cands.p[n]) + row * C;
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
       const int j = lane + 32 * i;
-      dst[i] = j < nvec ? *reinterpret_cast<const uint4*>(src + j * VEC) : make_uint4(0u, 0u, 0u, 0u);
+      nxt[i] = j < nvec ? *reinterpret_cast<const uint4*>(src + j * VEC) : make_uint4(0u, 0u, 0u, 0u);
     }
   };
-#pragma unroll
-  for (int a = 0; a < AHEAD; ++a)
-    if (a < n_cands) fetch(a, nxt[a]);
+  fetch(0);
   for (int n = 0; n < n_cands; ++n) {
     float v[E];
-    const bool cached = AHEAD == 1 && cands.inv[n] != nullptr;  // warp-uniform
+    const bool cached = cands.inv[n] != nullptr;  // warp-uniform
     const float inv_cached = inv_nxt;
 #pragma unroll
-    for (int i = 0; i < NV; ++i) unpack16<T>(nxt[0][i], v + i * VEC);
-#pragma unroll
-    for (int a = 0; a + 1 < AHEAD; ++a) {
-#pragma unroll
-      for (int i = 0; i < NV; ++i) nxt[a][i] = nxt[a + 1][i];
-    }
-    if (n + AHEAD < n_cands) fetch(n + AHEAD, nxt[AHEAD - 1]);
+    for (int i = 0; i < NV; ++i) unpack16<T>(nxt[i], v + i * VEC);
+    if (n + 1 < n_cands) fetch(n + 1);
     if (n_cands == 1) {
-#pragma unroll
-      for (int x = 0; x < E; ++x) acc[x] = v[x];
-      l = 1.f;
+      mix.set(v);
       break;
     }
-    // logit = rms_norm(v) . w = rsqrt(mean(v^2) + eps) * (v . w): both sums in one sweep and one
-    // interleaved butterfly.  (The reference rounds rms_norm(v) to the storage type before the
-    // product; for bf16 that changes the logit by ~1e-4 of its own rounding step.)
-    // A committed candidate does not change between mixes, so its norm factor is computed by the first mix that
-    // sees it and handed to the later ones: they skip the sum of squares and its half of the butterfly.  The
-    // factor is the same number either way (same code computed it), so results do not depend on the cache.
-    float s4[4] = {0.f, 0.f, 0.f, 0.f}, d4[4] = {0.f, 0.f, 0.f, 0.f};
-    float inv;
-    float dr;
-    if (cached) {
+    const float inv = mix.add(v, wv, cached, inv_cached, (float)cands.mult[n], C);
+    if (!cached && n == inv_out_index && lane == 0) inv_out[row] = inv;
+  }
+  mix.store(out_h, out_rn, row, lane, nvec, C);
+}
+
+// Many rows, more than L2 holds: the candidates' pieces run kDepth ahead through cp.async into each lane's own places in shared memory
+// (no registers, no barrier), and a row of up to 32 vectors is shared by 16 lanes, so that a warp's butterflies and exponentials
+// serve two rows.  Measured against the kernel above (bf16, us): 131072 x 256, 3 and 6 candidates
+// 88 -> 69 and 141 -> 110 (with cached factors 103), 228480 x 512, 8 candidates 493 -> 466 (423), 30000 x 768, 13 candidates 142 -> 128 (115),
+// 400000 x 64, 4 candidates 297 -> 171.
+// A persistent form whose stream runs on from row to row was slower than that kernel (131072 x 256, 6 candidates: 180 against 141): the
+// chain of a row is bound by its arithmetic, and what helps is many warps.
+__host__ __device__ constexpr int mix_depth(int nv) { return nv <= 1 ? 8 : nv == 2 ? 6 : 4; }
+template <typename T, int NV, int LPR>
+__global__ void __launch_bounds__(128, 4)
+depthmix_ahead_kernel(CandPtrs cands, int n_cands, const T* __restrict__ w, T* __restrict__ out_h,
+                      T* __restrict__ out_rn, float* __restrict__ inv_out, int inv_out_index, long long rows, int C) {
+  constexpr int VEC = Io<T>::kVec16;
+  constexpr int E = NV * VEC;
+  constexpr int kDepth = mix_depth(NV);
+  __shared__ __align__(16) uint4 ring[4][kDepth][NV][32];
+  dep_wait();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & (LPR - 1);
+  const long long at = ((long long)blockIdx.x * 128 + threadIdx.x) / LPR;
+  const bool row_ok = at < rows;
+  const long long row = row_ok ? at : rows - 1;  // every lane takes part in the butterflies
+  const int nvec = C / VEC;
+  const uint4* place = &ring[warp][0][0][threadIdx.x & 31];
+  const uint32_t mine = (uint32_t)__cvta_generic_to_shared(place);
+  auto fetch = [&](int n) {  // a group per candidate, empty past the last
+    if (n < n_cands) {
+      const T* src = static_cast<const T*>(cands.p[n]) + row * C;
 #pragma unroll
-      for (int x = 0; x < E; ++x) d4[x & 3] += v[x] * wv[x];
-      dr = (d4[0] + d4[1]) + (d4[2] + d4[3]);
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) dr += __shfl_xor_sync(0xffffffffu, dr, o);
-      inv = inv_cached;
-    } else {
-#pragma unroll
-      for (int x = 0; x < E; ++x) {
-        s4[x & 3] += v[x] * v[x];
-        d4[x & 3] += v[x] * wv[x];
+      for (int i = 0; i < NV; ++i) {
+        const int j = lane + LPR * i;
+        if (j < nvec)
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(mine + (uint32_t)(((n % kDepth) * NV + i) * 512)), "l"(src + j * VEC) : "memory");
       }
-      float ss = (s4[0] + s4[1]) + (s4[2] + s4[3]);
-      dr = (d4[0] + d4[1]) + (d4[2] + d4[3]);
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        ss += __shfl_xor_sync(0xffffffffu, ss, o);
-        dr += __shfl_xor_sync(0xffffffffu, dr, o);
-      }
-      inv = rsqrtf(ss / (float)C + kRmsEps);
-      if (n == inv_out_index && lane == 0) inv_out[row] = inv;
     }
-    const float dot = Io<T>::round(dr * inv);
-    if (dot > m) {  // warp-uniform: the accumulator is rescaled only when the running maximum moves
-      const float resc = __expf(m - dot);
-      l *= resc;
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+#pragma unroll 1
+  for (int n = 0; n < kDepth; ++n) fetch(n);
+  // cached norm factors: lane l holds those of candidates l and l + LPR
+  float lo = 0.f, hi = 0.f;
+  if (lane < n_cands && cands.inv[lane]) lo = cands.inv[lane][row];
+  if (lane + LPR < n_cands && cands.inv[lane + LPR]) hi = cands.inv[lane + LPR][row];
+  float wv[E];
+  mix_weights<T, NV, LPR>(w, n_cands, lane, nvec, wv);
+  MixRow<T, NV, LPR> mix;
+  mix.clear();
+  for (int n = 0; n < n_cands; ++n) {
+    float v[E];
+    const bool cached = cands.inv[n] != nullptr;  // the same for every row
+    const float inv_cached = __shfl_sync(0xffffffffu, n < LPR ? lo : hi, n & (LPR - 1), LPR);
+    asm volatile("cp.async.wait_group %0;" ::"n"(kDepth - 1) : "memory");
 #pragma unroll
-      for (int x = 0; x < E; ++x) acc[x] *= resc;
-      m = dot;
+    for (int i = 0; i < NV; ++i)
+      unpack16<T>(lane + LPR * i < nvec ? place[((n % kDepth) * NV + i) * 32] : make_uint4(0u, 0u, 0u, 0u), v + i * VEC);
+    if (n_cands == 1) {
+      mix.set(v);
+      break;
     }
-    const float pw = __expf(dot - m) * (float)cands.mult[n];
-    l += pw;
-#pragma unroll
-    for (int x = 0; x < E; ++x) acc[x] += pw * v[x];
+    const float inv = mix.add(v, wv, cached, inv_cached, (float)cands.mult[n], C);
+    if (!cached && n == inv_out_index && lane == 0 && row_ok) inv_out[row] = inv;
+    fetch(n + kDepth);  // into the place whose values the sums have consumed
   }
-  const float invl = 1.f / l;
-  float s4[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-  for (int x = 0; x < E; ++x) {
-    acc[x] = Io<T>::round(acc[x] * invl);
-    s4[x & 3] += acc[x] * acc[x];
-  }
-  const float ss = warp_sum((s4[0] + s4[1]) + (s4[2] + s4[3]));
-  const float inv = rsqrtf(ss / (float)C + kRmsEps);
-#pragma unroll
-  for (int i = 0; i < NV; ++i) {
-    const int j = lane + 32 * i;
-    if (j >= nvec) continue;
-    if (out_h) st16<T>(out_h + row * C + j * VEC, acc + i * VEC, 1.f);
-    if (out_rn) st16<T>(out_rn + row * C + j * VEC, acc + i * VEC, inv);
-  }
+  mix.store(out_h, out_rn, row, lane, nvec, C, row_ok);
 }
 
 template <typename T>
@@ -281,14 +369,26 @@ static int depthmix_launch(const CandPtrs& cp, int n, const void* w, void* out_h
   }
   if (vec) {
     const int nv = (C / Io<T>::kVec16 + 31) / 32;
-#define DGPT_MIXV(N)                                                                              \
-  launch_dep(depthmix_vec_kernel<T, N>, dim3(grid), dim3(warps * 32), 0, st, cp, n, static_cast<const T*>(w), \
+#define DGPT_MIXV(K, G, ...)                                                                              \
+  launch_dep(K<T, __VA_ARGS__>, dim3(G), dim3(warps * 32), 0, st, cp, n, static_cast<const T*>(w), \
              static_cast<T*>(out_h), static_cast<T*>(out_rn), inv_out, inv_out_index, rows, C)
-    if (nv <= 1) DGPT_MIXV(1);
-    else if (nv <= 2) DGPT_MIXV(2);
-    else if (nv <= 3) DGPT_MIXV(3);
-    else if (nv <= 4) DGPT_MIXV(4);
-    else DGPT_MIXV(8);
+    // Ahead where the candidates do not fit L2 (126 MB): from memory the fetches in flight count, from L2 the extra trip through shared
+    // memory costs more than it hides (4096 x 768, 13 candidates: 20.1 against 17.9 us).
+    const int vecs = C / Io<T>::kVec16;
+    const bool from_memory = (double)rows * C * sizeof(T) * n > 128e6;
+    const unsigned pairs = (unsigned)((rows + 2 * warps - 1) / (2 * warps));
+    if (from_memory && vecs <= 32 && n <= 32) {
+      if (vecs <= 16) DGPT_MIXV(depthmix_ahead_kernel, pairs, 1, 16);
+      else DGPT_MIXV(depthmix_ahead_kernel, pairs, 2, 16);
+    } else if (from_memory && nv <= 4) {
+      if (nv <= 2) DGPT_MIXV(depthmix_ahead_kernel, grid, 2, 32);
+      else if (nv <= 3) DGPT_MIXV(depthmix_ahead_kernel, grid, 3, 32);
+      else DGPT_MIXV(depthmix_ahead_kernel, grid, 4, 32);
+    } else if (nv <= 1) DGPT_MIXV(depthmix_vec_kernel, grid, 1);
+    else if (nv <= 2) DGPT_MIXV(depthmix_vec_kernel, grid, 2);
+    else if (nv <= 3) DGPT_MIXV(depthmix_vec_kernel, grid, 3);
+    else if (nv <= 4) DGPT_MIXV(depthmix_vec_kernel, grid, 4);
+    else DGPT_MIXV(depthmix_vec_kernel, grid, 8);
 #undef DGPT_MIXV
     return launch_status("depthmix");
   }
