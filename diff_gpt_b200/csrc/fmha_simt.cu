@@ -6,7 +6,8 @@
 // of 32 keys are staged in shared memory as fp32 and read by every query thread
 // as broadcasts.  A query is owned by SPLIT adjacent lanes, each holding D/SPLIT
 // elements of q and of the output accumulator in registers.  Scores are produced
-// eight keys at a time so that the accumulator is rescaled once per eight keys.
+// eight keys at a time so that the accumulator is rescaled once per eight keys.  Where that leaves few CTAs, eight lanes share a
+// query instead, each with every eighth key, and merge at the end (heads up to 32).
 #include "common.cuh"
 #include "fmha.cuh"
 
@@ -15,24 +16,28 @@ namespace dgpt {
 constexpr int kSimtBN = 32;  // keys per shared-memory tile
 constexpr int kSimtKB = 8;   // keys per softmax update
 
-template <typename T, int D, int SPLIT>
+template <typename T, int D, int SPLIT, int KEYS>
 __global__ void __launch_bounds__(128)
 fmha_simt_kernel(const T* __restrict__ q, long long q_bs, long long q_rs, KvView kv, const int* __restrict__ kv_len,
                  int kv_len_all, void* __restrict__ o, long long o_bs, long long o_rs, int o_f32,
                  float* __restrict__ lse, int H, int Tq, int q_offset, int causal, float scale_log2, int window,
                  int keep_first, int kv_div, const void* __restrict__ hgate, long long hgate_rs,
                  const T* __restrict__ egate, long long egate_rs) {
-  constexpr int DP = D / SPLIT;       // elements per thread
-  constexpr int BM = 128 / SPLIT;     // queries per CTA
+  static_assert(SPLIT == 1 || KEYS == 1, "a query's lanes share its elements or its keys");
+  constexpr int DP = D / SPLIT;               // elements per thread
+  constexpr int BM = 128 / (SPLIT * KEYS);    // queries per CTA
   constexpr int VEC = Io<T>::kVec16;
-  __shared__ __align__(16) float Ks[kSimtBN][D];
-  __shared__ __align__(16) float Vs[kSimtBN][D];
+  constexpr int KB = KEYS > 1 ? kSimtBN / KEYS : kSimtKB;  // keys per softmax update
+  constexpr int PITCH = KEYS > 1 ? D + 4 : D;  // lanes that read KEYS rows side by side do not collide
+  __shared__ __align__(16) float Ks[kSimtBN][PITCH];
+  __shared__ __align__(16) float Vs[kSimtBN][PITCH];
 
   const int b = blockIdx.z, h = blockIdx.y;
   const int q0 = blockIdx.x * BM;
   const int tid = threadIdx.x;
-  const int qi = q0 + tid / SPLIT;
-  const int part = tid % SPLIT;
+  const int qi = q0 + tid / (SPLIT * KEYS);
+  const int part = tid % SPLIT;          // its elements
+  const int share = KEYS > 1 ? tid % KEYS : 0;  // its keys: share, share + KEYS, ... of a tile
   const bool q_ok = qi < Tq;
   const int klen = kv_len ? kv_len[b] : kv_len_all;
   int kmax = klen;
@@ -86,12 +91,12 @@ fmha_simt_kernel(const T* __restrict__ q, long long q_bs, long long q_rs, KvView
     }
     __syncthreads();
     const int jn = min(kSimtBN, kmax - j0);
-    for (int kb = 0; kb < jn; kb += kSimtKB) {
-      float s[kSimtKB];
+    for (int kb = 0; kb < jn; kb += KB * KEYS) {
+      float s[KB];
       float smax = -INFINITY;
 #pragma unroll
-      for (int kk = 0; kk < kSimtKB; ++kk) {
-        const float* kr = &Ks[kb + kk][part * DP];
+      for (int kk = 0; kk < KB; ++kk) {
+        const float* kr = &Ks[kb + kk * KEYS + share][part * DP];
         float dot = 0.f;
 #pragma unroll
         for (int d = 0; d < DP; d += 4) {
@@ -100,7 +105,7 @@ fmha_simt_kernel(const T* __restrict__ q, long long q_bs, long long q_rs, KvView
         }
 #pragma unroll
         for (int x = 1; x < SPLIT; x <<= 1) dot += __shfl_xor_sync(0xffffffffu, dot, x);
-        const int j = j0 + kb + kk;
+        const int j = j0 + kb + kk * KEYS + share;
         s[kk] = (q_ok && j < klen && j <= my_last && (j >= my_first || j < keep_first)) ? dot : -INFINITY;
         smax = fmaxf(smax, s[kk]);
       }
@@ -111,10 +116,10 @@ fmha_simt_kernel(const T* __restrict__ q, long long q_bs, long long q_rs, KvView
 #pragma unroll
       for (int d = 0; d < DP; ++d) acc[d] *= resc;
 #pragma unroll
-      for (int kk = 0; kk < kSimtKB; ++kk) {
+      for (int kk = 0; kk < KB; ++kk) {
         const float p = exp2f(s[kk] - mn);
         l += p;
-        const float* vr = &Vs[kb + kk][part * DP];
+        const float* vr = &Vs[kb + kk * KEYS + share][part * DP];
 #pragma unroll
         for (int d = 0; d < DP; d += 4) {
           const float4 vx = *reinterpret_cast<const float4*>(vr + d);
@@ -126,6 +131,18 @@ fmha_simt_kernel(const T* __restrict__ q, long long q_bs, long long q_rs, KvView
       }
       m = mn;
     }
+  }
+  if constexpr (KEYS > 1) {  // the shares of a query become one
+#pragma unroll
+    for (int x = 1; x < KEYS; x <<= 1) {
+      const float m2 = __shfl_xor_sync(0xffffffffu, m, x), l2 = __shfl_xor_sync(0xffffffffu, l, x), mn = fmaxf(m, m2);
+      const float f = m == -INFINITY ? 0.f : exp2f(m - mn), f2 = m2 == -INFINITY ? 0.f : exp2f(m2 - mn);
+      l = l * f + l2 * f2;
+#pragma unroll
+      for (int d = 0; d < DP; ++d) acc[d] = acc[d] * f + __shfl_xor_sync(0xffffffffu, acc[d], x) * f2;
+      m = mn;
+    }
+    if (share != 0) return;
   }
   if (!q_ok) return;
   float inv = l > 0.f ? 1.f / l : 0.f;
@@ -155,14 +172,20 @@ fmha_simt_kernel(const T* __restrict__ q, long long q_bs, long long q_rs, KvView
 template <typename T, int D>
 static int fmha_simt_launch(const FmhaArgs& a, const KvView& kv, cudaStream_t st) {
   constexpr int SPLIT = D > 64 ? D / 64 : 1;
-  constexpr int BM = 128 / SPLIT;
-  dim3 grid((unsigned)((a.Tq + BM - 1) / BM), (unsigned)a.H, (unsigned)a.B);
+  constexpr int KEYS = D <= 32 ? 8 : 1;
   const float scale_log2 = a.scale > 0.f ? a.scale * kLog2e : kLog2e / sqrtf((float)D);
-  fmha_simt_kernel<T, D, SPLIT><<<grid, 128, 0, st>>>(static_cast<const T*>(a.q), a.q_bs, a.q_rs, kv, a.kv_len,
-                                                      a.kv_len_all, a.o, a.o_bs, a.o_rs, a.o_f32, a.lse, a.H, a.Tq,
-                                                      a.q_offset, a.causal, scale_log2, a.window,
-                                                      a.window > 0 ? a.keep_first : 0, a.kv_heads > 0 ? a.H / a.kv_heads : 1, a.hgate,
-                                                      a.hgate_rs, static_cast<const T*>(a.egate), a.egate_rs);
+#define DGPT_SIMT(SS, KK)                                                                                                     \
+  fmha_simt_kernel<T, D, SS, KK><<<dim3((unsigned)((a.Tq + 128 / (SS * KK) - 1) / (128 / (SS * KK))), (unsigned)a.H, (unsigned)a.B), 128, 0, st>>>( \
+      static_cast<const T*>(a.q), a.q_bs, a.q_rs, kv, a.kv_len, a.kv_len_all, a.o, a.o_bs, a.o_rs, a.o_f32, a.lse, a.H, a.Tq, a.q_offset, \
+      a.causal, scale_log2, a.window, a.window > 0 ? a.keep_first : 0, a.kv_heads > 0 ? a.H / a.kv_heads : 1, a.hgate, a.hgate_rs, \
+      static_cast<const T*>(a.egate), a.egate_rs)
+  // Eight lanes share a query's keys where one lane per query leaves most SMs without a CTA.  (fp32, us: 100 and 1000
+  // queries, 4 heads of 16, 89 keys 10.0 -> 4.4 and 10.6 -> 5.7; 300 x 300, 8 heads of 32, 58 -> 17; 4000 queries, 128 CTAs, 11.3
+  // either way.)
+  const long long ctas = (long long)a.B * a.H * ((a.Tq + 128 / SPLIT - 1) / (128 / SPLIT));
+  if (KEYS > 1 && ctas <= 74) DGPT_SIMT(1, KEYS);
+  else DGPT_SIMT(SPLIT, 1);
+#undef DGPT_SIMT
   return launch_status("fmha_simt");
 }
 
