@@ -208,6 +208,13 @@ class SingleStep:
         self.plan.run(self.numbers[0:1], self.bind)
 
 
+def own_f32(M: int, N: int, K: int) -> bool:
+    """Whether an fp32 product runs on dgpt_linear_f32: up to 400 of its tiles (measured in us, cuBLAS / own: 100 x 256 x 64 3.63 / 2.62,
+    100 x 64 x 128 4.65 / 2.93, 400 x 512 x 64 3.95 / 3.93, 1000 x 256 x 64 3.99 / 4.69, 400 x 1024 x 256 9.4 / 13.2; its SwiGLU saves a launch of
+    1.6 besides).  cuBLAS has a matrix-vector kernel for one row, ahead from K = 128 on (1 x 64 x 128 1.97 / 2.81; K = 64 2.90 / 2.28)."""
+    return -(-M // 16) * -(-N // 32) <= 400 and (M > 1 or K <= 64) and K <= 512
+
+
 # ---- how one forward call is bound to K/V storage ----------------------------------
 @dataclass
 class KvBinding:
@@ -275,7 +282,9 @@ class ForwardPlan:
         self.status = torch.zeros(1, dtype=torch.int32, device=dev)
         # tcgen05 GEMM + SwiGLU epilogue: bf16 with tileable sizes, and enough rows to fill the tensor cores
         self.fused_ffn = FUSED_FFN and dt == torch.bfloat16 and C % 8 == 0 and n >= FUSED_FFN_MIN_ROWS
-        self.f = None if self.fused_ffn else buf(n, 4 * C)
+        self.f32 = dt == torch.float32 and C % 4 == 0
+        self.own_ffn1 = self.f32 and own_f32(n, 4 * C, C)
+        self.f = None if self.fused_ffn or self.own_ffn1 else buf(n, 4 * C)
         # norm factors of committed depth-mix candidates, carried from mix to mix (16-byte rows needed)
         self.cache_norms = CACHE_NORMS and (C * emb.element_size()) % 16 == 0
         self.norm_cache: dict[int, torch.Tensor] = {}
@@ -309,6 +318,17 @@ class ForwardPlan:
         ops.depthmix_cached(cands + [partial], inv_in + [None], w, None, self.u, inv_out, out_index)
         if inv_out is not None:
             known.add(cands[out_index].data_ptr())
+
+    def _linear(self, a: torch.Tensor, w_t: torch.Tensor, out: torch.Tensor, name: str, add: bool = False) -> None:
+        """out (+)= a @ w_t: a small fp32 model's on the library's kernel, others on cuBLAS."""
+        if self.f32 and own_f32(out.shape[0], out.shape[1], a.shape[1]):
+            ops.linear_f32(a, w_t.t(), out, add=out if add else None)
+            return
+        with region(name):
+            if add:
+                out.addmm_(a, w_t)
+            else:
+                torch.mm(a, w_t, out=out)
 
     def _decode_extras(self, b: KvBinding) -> None:
         m = self.model
@@ -359,8 +379,7 @@ class ForwardPlan:
             if (i + 1) % m.attn_res_layers_per_block == 0:
                 cands = cands + [partial]
                 partial = None
-            with region("gemm_qkvg"):
-                torch.mm(self.u, lw.wqkvg_t, out=self.qkvg)
+            self._linear(self.u, lw.wqkvg_t, self.qkvg, "gemm_qkvg")
             qv, kv_, vv, gv = (self.qkvg[:, j * C : (j + 1) * C] for j in range(4))
             ops.rope_qknorm_kvappend(
                 qv, kv_, vv, self.q, W.freqs_cis, b.layouts[i], b.pos0, b.slot0, b.step, n_seq, T, H, D, self.status
@@ -404,21 +423,23 @@ class ForwardPlan:
                     impl=b.fmha_impl, status=self.status, gate=gv,
                 )
             part = self.parts[i]
-            with region("gemm_proj"):
-                if partial is None:
-                    torch.mm(self.y, lw.wproj_t, out=part)
-                else:  # layers_per_block > 1: the running block sum keeps accumulating
+            if partial is None:
+                self._linear(self.y, lw.wproj_t, part, "gemm_proj")
+            else:  # layers_per_block > 1: the running block sum keeps accumulating
+                with region("gemm_proj"):
                     torch.addmm(partial, self.y, lw.wproj_t, out=part)
             partial = part
             self._mix(cands, partial, lw.w_mlp, known)
             if self.fused_ffn:  # first FFN GEMM with the SwiGLU in its epilogue (the [n, 4C] product never reaches HBM)
                 ops.linear(self.u, lw.w1, self.act, swiglu=(m.swiglu_alpha, m.swiglu_limit), status=self.status)
+            elif self.own_ffn1:
+                ops.linear_f32(self.u, lw.w1, self.act, swiglu=(m.swiglu_alpha, m.swiglu_limit))
             else:
                 with region("gemm_ffn1"):
                     torch.mm(self.u, lw.w1_t, out=self.f)
                 ops.swiglu(self.f, self.act, m.swiglu_alpha, m.swiglu_limit)
-            with region("gemm_ffn2"):  # cuBLAS: 6.6 / 9.8 us for the two n_embd-wide GEMMs against 10.4 / 14.4 us for dgpt_linear
-                partial.addmm_(self.act, lw.w2_t)
+            # bf16 on cuBLAS: 6.6 / 9.8 us for the two n_embd-wide GEMMs of 4096 rows against 9.5 / 14.4 us for dgpt_linear
+            self._linear(self.act, lw.w2_t, partial, "gemm_ffn2", add=True)
         final = partial
         if self.last is not None:
             self.last.copy_(partial.view(n_seq, T, C)[:, T - 1, :])
@@ -428,6 +449,8 @@ class ForwardPlan:
             return None
         if self.own_head:
             ops.linear(self.xn, W.emb, self.logits, softcap=self.cap, status=self.status)
+        elif self.f32 and own_f32(*self.logits.shape, C):
+            ops.linear_f32(self.xn, W.emb, self.logits, softcap=self.cap)
         else:
             with region("gemm_logits"):
                 torch.mm(self.xn, W.emb.t(), out=self.logits)

@@ -308,6 +308,34 @@ def linear(
     )
 
 
+def linear_f32(
+    a: torch.Tensor,
+    w: torch.Tensor,
+    out: torch.Tensor,
+    *,
+    swiglu: tuple[float, float] | None = None,
+    add: torch.Tensor | None = None,
+    softcap: float = 0.0,
+) -> None:
+    """`linear` in fp32 on the CUDA cores, for small models: out = a @ w.T, with the same meaning of swiglu, add and softcap."""
+    _cuda(a, w, out, add)
+    assert (swiglu is not None) + (add is not None) + (softcap > 0) <= 1
+    M, K = a.shape
+    N = w.shape[0]
+    assert w.shape[1] == K and a.stride(1) == 1 and w.stride(1) == 1 and out.stride(1) == 1
+    assert out.shape == (M, N // 2 if swiglu else N) and a.dtype == w.dtype == out.dtype == torch.float32
+    if add is not None:
+        assert add.shape == out.shape and add.dtype == out.dtype and add.stride(1) == 1
+    alpha, limit = swiglu or (softcap, 0.0)
+    epilogue = 1 if swiglu else 6 if softcap > 0 else 2 if add is not None else 0
+    check(
+        lib.dgpt_linear_f32(
+            a.data_ptr(), a.stride(0), w.data_ptr(), w.stride(0), out.data_ptr(), out.stride(0), _ptr(add),
+            0 if add is None else add.stride(0), M, N, K, epilogue, alpha, limit, _stream(),
+        )
+    )
+
+
 def integrate_tokens(
     tokens: torch.Tensor, n_chan: int, vocab_size: int, scale: torch.Tensor, order: torch.Tensor, state: torch.Tensor
 ) -> torch.Tensor:

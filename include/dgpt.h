@@ -218,6 +218,15 @@ int dgpt_sigmoid_gate(void* y, int64_t y_row_stride, const void* gate, int64_t g
  * Replaces src/diff_gpt/model/gpt.py:182-186.  logits: device [n] */
 int dgpt_softcap(void* logits, int64_t n, float cap, int32_t dtype, void* stream);
 
+/* Linear layer in fp32 on the CUDA cores, for small models (K a few hundred at most, any M and N):
+ *   epilogue 0 (store), 1 (SwiGLU), 2 (add resid, which may be out) and 6 (soft-cap with cap = alpha) as dgpt_linear's, nothing rounded
+ *   in between.  a, w: device fp32, 16-byte aligned, K and their row strides multiples of 4; out, resid: any strides.
+ * Replaces nn.Linear of src/diff_gpt/model/mha.py:20-27 and feed_forward.py:10-14 (with swi_glu.py:11-19), block.py:98-106 and the head
+ * with its cap (gpt.py:181-186). */
+int dgpt_linear_f32(const float* a, int64_t a_row_stride, const float* w, int64_t w_row_stride, float* out,
+                    int64_t out_row_stride, const float* resid, int64_t resid_row_stride, int32_t M, int32_t N, int32_t K,
+                    int32_t epilogue, float alpha, float limit, void* stream);
+
 /* Linear layer on the tcgen05 tensor cores, optionally with the SwiGLU of the feed-forward block in its epilogue:
  *   acc[m, n] = sum_k a[m, k] * w[n, k]                     (w as nn.Linear stores it: [N, K])
  *   epilogue 0:  out[m, n]     = acc[m, n]                  out: [M, N]
