@@ -33,7 +33,7 @@ import torch.nn.functional as F
 
 from .. import ops
 from .._lib import region
-from .configured import FUSED_FF_MIN_ROWS, ConfiguredModel, fp32_reductions, pick_latent_splits, round_up
+from .configured import FUSED_FF_MIN_ROWS, ConfiguredModel, fp32_reductions, linear, pick_latent_splits, round_up
 from .kv_cache import LatentCache, PagedLatentCache
 
 EXPAND_MIN_TOKENS = 32  # query tokens per sequence from which keys and values are expanded
@@ -219,7 +219,7 @@ class DelunexPlan:
         self.xn = torch.empty((n_out, C), dtype=self.dt, device=self.dev)
         self.logits = torch.empty((n_out, V), dtype=self.dt, device=self.dev) if want_logits else None
         self.own_head = self.dt == torch.bfloat16 and C % 8 == 0 and V % 16 == 0
-        self.fused_ff = self.dt == torch.bfloat16 and C % 8 == 0 and n >= FUSED_FF_MIN_ROWS
+        self.fused_ff = self.dt == torch.bfloat16 and C % 8 == 0 and (n >= FUSED_FF_MIN_ROWS or n == 1)
         self.status = torch.zeros(1, dtype=torch.int32, device=self.dev)
 
     def _buf(self, name: str, *shape: int, dtype=None) -> torch.Tensor:
@@ -240,8 +240,7 @@ class DelunexPlan:
         """self.y = mixer(self.h)"""
         n, n_seq, T, H, D, r = self.n, self.n_seq, self.T, lw.H, lw.D, lw.r
         proj = self._buf("proj", n, lw.w_in_t.shape[1])
-        with region("gemm_in"):
-            torch.mm(self.h, lw.w_in_t, out=proj)
+        linear(self.h, lw.w_in_t, proj, "gemm_in", self.status)
         q, gate = proj[:, : H * D], proj[:, lw.gate_col : lw.gate_col + H]
         if lw.owner == i:
             ops.latent_append(
@@ -273,8 +272,7 @@ class DelunexPlan:
             )
             with region("gemm_absorb"):
                 torch.bmm(oa.view(n, H, r).transpose(0, 1), lw.w_uv_t, out=o.view(n, H, D).transpose(0, 1))
-        with region("gemm_proj"):
-            torch.mm(o, lw.w_o_t, out=self.y)
+        linear(o, lw.w_o_t, self.y, "gemm_proj", self.status)
 
     def _feed_forward(self, lw: _PackedLayer) -> None:
         """self.y = W_down xielu(W_up self.u)"""
@@ -287,8 +285,7 @@ class DelunexPlan:
             with region("gemm_up"):
                 torch.mm(self.u, lw.w_up.t(), out=up)
             ops.xielu(up, act, *lw.act)
-        with region("gemm_down"):
-            torch.mm(act, lw.w_down_t, out=self.y)
+        linear(act, lw.w_down_t, self.y, "gemm_down", self.status)
 
     def run(self, ids32: torch.Tensor, b: LatentBinding, rows: torch.Tensor | None = None,
             tap: Callable[[int, torch.Tensor], None] | None = None) -> torch.Tensor | None:

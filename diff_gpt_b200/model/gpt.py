@@ -281,7 +281,8 @@ class ForwardPlan:
         self.cap = cap
         self.status = torch.zeros(1, dtype=torch.int32, device=dev)
         # tcgen05 GEMM + SwiGLU epilogue: bf16 with tileable sizes, and enough rows to fill the tensor cores
-        self.fused_ffn = FUSED_FFN and dt == torch.bfloat16 and C % 8 == 0 and n >= FUSED_FFN_MIN_ROWS
+        self.one_row = dt == torch.bfloat16 and C % 16 == 0 and n == 1  # see dgpt_linear: ahead of cuBLAS at every size
+        self.fused_ffn = FUSED_FFN and dt == torch.bfloat16 and C % 8 == 0 and (n >= FUSED_FFN_MIN_ROWS or self.one_row)
         self.f32 = dt == torch.float32 and C % 4 == 0
         self.own_ffn1 = self.f32 and own_f32(n, 4 * C, C)
         self.f = None if self.fused_ffn or self.own_ffn1 else buf(n, 4 * C)
@@ -320,9 +321,12 @@ class ForwardPlan:
             known.add(cands[out_index].data_ptr())
 
     def _linear(self, a: torch.Tensor, w_t: torch.Tensor, out: torch.Tensor, name: str, add: bool = False) -> None:
-        """out (+)= a @ w_t: a small fp32 model's on the library's kernel, others on cuBLAS."""
+        """out (+)= a @ w_t: a small fp32 model's and a lone bf16 row on the library's kernels, others on cuBLAS."""
         if self.f32 and own_f32(out.shape[0], out.shape[1], a.shape[1]):
             ops.linear_f32(a, w_t.t(), out, add=out if add else None)
+            return
+        if self.one_row:
+            ops.linear(a, w_t.t(), out, add=out if add else None, status=self.status)
             return
         with region(name):
             if add:

@@ -37,7 +37,7 @@ import torch.nn.functional as F
 
 from .. import ops
 from .._lib import region
-from .configured import FUSED_FF_MIN_ROWS, ConfiguredModel, fp32_reductions, pick_latent_splits, round_up
+from .configured import FUSED_FF_MIN_ROWS, ConfiguredModel, fp32_reductions, linear, pick_latent_splits, round_up
 from .kv_cache import PagedRowCache, RowCache, StateSpec
 from .rope import rotation_table
 
@@ -277,7 +277,7 @@ class KipolixPlan:
         self.xn = torch.empty((n_out, C), dtype=self.dt, device=self.dev)
         self.logits = torch.empty((n_out, V), dtype=self.dt, device=self.dev) if want_logits else None
         self.own_head = self.dt == torch.bfloat16 and C % 8 == 0 and V % 16 == 0
-        self.fused_ff = self.dt == torch.bfloat16 and C % 8 == 0 and n >= FUSED_FF_MIN_ROWS
+        self.fused_ff = self.dt == torch.bfloat16 and C % 8 == 0 and (n >= FUSED_FF_MIN_ROWS or n == 1)
         self.status = torch.zeros(1, dtype=torch.int32, device=self.dev)
 
     def _buf(self, name: str, *shape: int, dtype=None) -> torch.Tensor:
@@ -335,8 +335,7 @@ class KipolixPlan:
             with region("gemm_up"):
                 torch.mm(self.h, lw.w_gu.t(), out=gu)
             ops.silu_mul(gu, act)
-        with region("gemm_down"):
-            torch.mm(act, lw.w_down_t, out=self.y)
+        linear(act, lw.w_down_t, self.y, "gemm_down", self.status)
 
     def run(self, ids32: torch.Tensor, b: RowBinding, rows: torch.Tensor | None = None,
             tap: Callable[[int, torch.Tensor], None] | None = None) -> torch.Tensor | None:
@@ -358,11 +357,9 @@ class KipolixPlan:
         for k, i in enumerate(runs):
             lw = W.layers[i]
             proj = self._buf("proj", self.n, lw.w_in_t.shape[1])
-            with region("gemm_in"):
-                torch.mm(self.h, lw.w_in_t, out=proj)
+            linear(self.h, lw.w_in_t, proj, "gemm_in", self.status)
             o = (self._retention if isinstance(lw.m, Retention) else self._attention)(k, lw, proj, b)
-            with region("gemm_proj"):
-                torch.mm(o, lw.w_o_t, out=self.y)
+            linear(o, lw.w_o_t, self.y, "gemm_proj", self.status)
             sub = lw.sub1
             if lw.sub2 is not None:
                 nxt = lw.sub2

@@ -10,6 +10,8 @@ pytestmark = pytest.mark.gpu
 FORMS = {
     "one CTA, 64": (100, 272, 136), "one CTA, 128": (33, 9584, 72), "pair, 128": (300, 272, 200), "pair, 192": (1990, 1584, 72),
     "pair, 256": (1990, 2256, 72), "pair, several rounds": (4500, 2320, 328), "one row": (1, 16, 8),
+    "one row, shared K": (1, 528, 1032), "one row, a warp a pair": (1, 4752, 264), "two rows, shared K": (2, 1008, 5456),
+    "two rows, a warp a pair": (2, 4752, 520), "three rows": (3, 48, 24),
 }
 
 
