@@ -34,7 +34,7 @@ def fp32_reductions():
 def linear(a: torch.Tensor, w_t: torch.Tensor, out: torch.Tensor, name: str, status: torch.Tensor) -> None:
     """out = a @ w_t, on cuBLAS but for a single bf16 row (dgpt_linear, us: 1024 x 1024 4.8 -> 2.3, 1024 x 2736 8.1 -> 3.4)."""
     K, N = w_t.shape
-    if a.shape[0] == 1 and a.dtype == torch.bfloat16 and K % 8 == 0 and N % 16 == 0:
+    if a.shape[0] == 1 and a.dtype == torch.bfloat16 and K % 8 == 0 and N % 16 == 0 and w_t.data_ptr() % 16 == 0:
         ops.linear(a, w_t.t(), out, status=status)
         return
     with region(name):
@@ -138,16 +138,17 @@ class ConfiguredModel(DeviceModel):
     def logits_at(self, idx, cache, rows):
         return self._step(idx, cache, rows)
 
-    def single_step(self, cache: RowCache, old: SingleStep | None) -> SingleStep:
+    def single_step(self, cache: RowCache, old: SingleStep | None, stream: torch.cuda.Stream) -> SingleStep:
         cache.ensure(1)
         # the key splits change from one 128-key tile to the next, until every window is full
         kind = -(-min(cache.slot + 1, cache.keep + 1 + cache.keep_first) // 128)
         held = (self.packed_weights(), *cache.state.source.values(), *cache.store.values(), *self.step_tables(cache.pos + 1))
         if old is not None and old.fits(kind, held):
             return old
-        numbers = torch.zeros(4, dtype=torch.int32, device=self.embedding.device)
-        bind = self.step_binding(cache, 1, 1, numbers)
-        return SingleStep(self.new_plan(1, 1, rows=1), bind, numbers, kind, held, checks=True)
+        with torch.cuda.stream(stream):
+            numbers = torch.zeros(4, dtype=torch.int32, device=self.embedding.device)
+            bind = self.step_binding(cache, 1, 1, numbers)
+            return SingleStep(self.new_plan(1, 1, rows=1), bind, numbers, kind, held, checks=True)
 
     def step_tables(self, positions: int) -> tuple:
         """Tables that a binding for this many positions points at."""

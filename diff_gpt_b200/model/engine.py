@@ -548,12 +548,12 @@ class StepRunner:
     def _one(self, cache, token: int) -> torch.Tensor | None:
         state = getattr(cache, "state", None)
         key = (cache, 0 if state is None else state.current)  # a portion of several tokens changes the buffer
-        one = self.model.single_step(cache, self._single.get(key))
+        if self._stream is None:
+            self._stream = torch.cuda.Stream(device=self.model.embedding.device)
+        one = self.model.single_step(cache, self._single.get(key), self._stream)
         if one is None:
             return None
         self._single[key] = one
-        if self._stream is None:
-            self._stream = torch.cuda.Stream(device=self.model.embedding.device)
         caller, mine = torch.cuda.current_stream(), self._stream
         mine.wait_stream(caller)
         with torch.cuda.stream(mine):

@@ -83,9 +83,9 @@ class DeviceModel(BaseGPT):
     def logits_at(self, idx: torch.Tensor, cache, rows: torch.Tensor) -> torch.Tensor:
         """Run idx (1, T) behind what `cache` holds; the logits [len(rows), V] of the given places among the T tokens."""
 
-    def single_step(self, cache, old: "SingleStep | None") -> "SingleStep | None":
+    def single_step(self, cache, old: "SingleStep | None", stream: torch.cuda.Stream) -> "SingleStep | None":
         """The launches of one more token behind `cache`, which has room for it afterwards: `old` where it still fits, or None
-        where a single token takes the general path."""
+        where a single token takes the general path.  What it allocates for itself belongs to `stream`, where it will run."""
         return None
 
     # -- batched decode (DecodeRun) --
@@ -281,9 +281,12 @@ class ForwardPlan:
         self.cap = cap
         self.status = torch.zeros(1, dtype=torch.int32, device=dev)
         # tcgen05 GEMM + SwiGLU epilogue: bf16 with tileable sizes, and enough rows to fill the tensor cores
-        self.one_row = dt == torch.bfloat16 and C % 16 == 0 and n == 1  # see dgpt_linear: ahead of cuBLAS at every size
+        # parameters may be views into a larger buffer: the kernels that take the small products want 16-byte aligned rows
+        packed = model.packed_weights()
+        aligned = all(t.data_ptr() % 16 == 0 for l in packed.layers for t in (l.wproj_t, l.w1, l.w2_t)) and packed.emb.data_ptr() % 16 == 0
+        self.one_row = dt == torch.bfloat16 and C % 16 == 0 and n == 1 and aligned  # see dgpt_linear: ahead of cuBLAS at every size
         self.fused_ffn = FUSED_FFN and dt == torch.bfloat16 and C % 8 == 0 and (n >= FUSED_FFN_MIN_ROWS or self.one_row)
-        self.f32 = dt == torch.float32 and C % 4 == 0
+        self.f32 = dt == torch.float32 and C % 4 == 0 and aligned
         self.own_ffn1 = self.f32 and own_f32(n, 4 * C, C)
         self.f = None if self.fused_ffn or self.own_ffn1 else buf(n, 4 * C)
         # norm factors of committed depth-mix candidates, carried from mix to mix (16-byte rows needed)
@@ -582,7 +585,7 @@ class GPT(DeviceModel):
     def logits_at(self, idx: torch.Tensor, cache: KVCache, rows: torch.Tensor) -> torch.Tensor:
         return self(idx, kv_cache=cache)[0][0].index_select(0, rows)
 
-    def single_step(self, cache: KVCache, old: SingleStep | None) -> SingleStep | None:
+    def single_step(self, cache: KVCache, old: SingleStep | None, stream: torch.cuda.Stream) -> SingleStep | None:
         t0, H, emb = cache.get_pos(), self.n_head, self.embedding
         if t0 == 0:
             return None
@@ -592,13 +595,14 @@ class GPT(DeviceModel):
         held = (self.packed_weights(), cache.kv_cache)
         if old is not None and old.fits(splits, held):
             return old
-        numbers = torch.zeros(4, dtype=torch.int32, device=emb.device)
-        zero = torch.zeros(1, dtype=torch.int32, device=emb.device)
-        bind = KvBinding(
-            layouts=[cache.layer_layout(i) for i in range(self.n_layer)], pos0=numbers[2:3], slot0=numbers[1:2], decode=True, len0=zero,
-            start1=zero, len1=numbers[3:4], n_splits=splits,
-        )
-        return SingleStep(ForwardPlan(self, 1, 1, cap=self.logit_softcap), bind, numbers, splits, held, checks=False)
+        with torch.cuda.stream(stream):
+            numbers = torch.zeros(4, dtype=torch.int32, device=emb.device)
+            zero = torch.zeros(1, dtype=torch.int32, device=emb.device)
+            bind = KvBinding(
+                layouts=[cache.layer_layout(i) for i in range(self.n_layer)], pos0=numbers[2:3], slot0=numbers[1:2], decode=True,
+                len0=zero, start1=zero, len1=numbers[3:4], n_splits=splits,
+            )
+            return SingleStep(ForwardPlan(self, 1, 1, cap=self.logit_softcap), bind, numbers, splits, held, checks=False)
 
     def paged_cache(self, n_series, rows_per_series, prefix_len, max_new, page_tokens, pool=None) -> PagedKVCache:
         emb = self.embedding

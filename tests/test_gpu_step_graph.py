@@ -80,3 +80,29 @@ def test_requests_on_their_own_streams():
     torch.cuda.synchronize()
     for k in ids:
         assert torch.equal(torch.cat(got[k]), want[k])
+
+
+@pytest.mark.parametrize("family,dtype", [("gpt", torch.float32), ("gpt", torch.bfloat16), ("delunex", torch.bfloat16), ("kipolix", torch.bfloat16)])
+def test_parameters_that_are_views_off_16_bytes(family, dtype):
+    """Layer weights four or two bytes off a 16-byte boundary (views into one buffer) give what aligned ones give, up to the order of
+    the sums: single tokens and short prompts took any alignment before the kernels for few rows."""
+    model, V = _model(family, dtype)
+    ids = torch.randint(0, V, (1, 12), generator=torch.Generator().manual_seed(3)).cuda()
+
+    def run():
+        cache = model.new_cache()
+        cache.reset()
+        rows = torch.tensor([0], device="cuda")
+        with torch.inference_mode():
+            first = model.logits_at(ids[:, :11], cache, torch.tensor([10], device="cuda")).float().clone()
+            return torch.cat([first, model.logits_at(ids[:, 11:], cache, rows).float()])
+
+    want = run()
+    table = model.token_embedding_table.weight if family == "gpt" else None
+    for name, p in model.named_parameters():
+        if p.dim() == 2 and p.shape[0] > 1 and p is not table and name not in ("embed", "head", "bigram"):
+            flat = torch.empty(p.numel() + 1, dtype=dtype, device="cuda")
+            flat[1:].copy_(p.detach().reshape(-1))
+            p.data = flat[1:].view(p.shape)
+    got = run()
+    assert (got - want).abs().max().item() <= (1e-5 if dtype == torch.float32 else 3e-2) * want.abs().max().item()
