@@ -31,6 +31,9 @@ struct FmhaArgs {
   // gate per output element (dgpt_fmha_prefill_gated), exclusive with hgate
   const void* egate = nullptr;  // [B * Tq, H * D] in dtype: o = round(o) * round(sigmoid(egate))
   long long egate_rs = 0;
+  // Probabilities as a bf16 pair, high and low part: two-CTAs-per-SM kernel only, for calls whose other route is the warp-level kernel
+  // with its probabilities in fp32
+  int split_p = 0;
   int any_run = 0;  // the tensor-core kernels may take dense keys of any length, not only whole tiles (impl 0)
 };
 

@@ -263,7 +263,12 @@ static int fmha_full(const void* q, int64_t q_batch_stride, int64_t q_row_stride
   // against 57).
   const long long span = causal ? (long long)Tq + q_offset
                                 : (kv_len ? (long long)kv->max_pages * kv->page_tokens : (long long)kv_len_all);
-  a.two_cta = impl == 3 || (impl == 0 && span < 640 && !fmha_one_round(a));
+  // The other route of dense keys that are not whole tiles is the warp-level kernel, whose probabilities are fp32: here they keep 16
+  // bits as a pair.  Error against float64, rope and norm included, of 4 x 12 heads of 64 x 777 tokens: 0.003236 there, 0.003236 with the
+  // pair, 0.0035 with one bf16; the whole layer 337 us there, 66 with the pair (1 x 8 heads x 8191: 3896 and 300; 2 x 16 heads of 128 x 1500:
+  // 1669 and 89).
+  a.split_p = a.any_run && kv->page_table == nullptr && kv->page_tokens % 128 != 0;
+  a.two_cta = impl == 3 || a.split_p || (impl == 0 && span < 640 && !fmha_one_round(a));
   if (impl >= 2 && !tc_ok) {
     set_error("fmha_prefill: the tensor-core kernel does not cover dtype %d, head_dim %d with this layout", dtype, D);
     return DGPT_E_UNSUPPORTED;

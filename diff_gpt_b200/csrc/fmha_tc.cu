@@ -22,7 +22,8 @@ namespace tc {
 constexpr int kTmemCols = 256;    // S/P: [0,128), O tile: [128, 128 + D)
 
 
-template <int D, bool KEPT>
+// SPLIT: a probability is the sum of two bf16 numbers (16 bits of it), and P V two products; P takes all of S's columns.
+template <int D, bool KEPT, bool SPLIT>
 __global__ void __launch_bounds__(128, 2)
 fmha_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__ CUtensorMap mk,
                const __grid_constant__ CUtensorMap mv, const TcParams p) {
@@ -217,7 +218,7 @@ fmha_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__ C
     float rowsum = 0.f;
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
-      uint32_t packed[16];
+      uint32_t packed[16], low[SPLIT ? 16 : 1];
 #pragma unroll
       for (int i = 0; i < 32; i += 2) {
         const float p0 = ex2(fmaf(sv[c * 32 + i], p.scale_log2, -m_use));      // -inf -> 0
@@ -225,8 +226,14 @@ fmha_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__ C
         rowsum += p0 + p1;
         const __nv_bfloat162 pk = __floats2bfloat162_rn(p0, p1);
         packed[i >> 1] = *reinterpret_cast<const uint32_t*>(&pk);
+        if constexpr (SPLIT) {
+          const float h0 = __uint_as_float(packed[i >> 1] << 16), h1 = __uint_as_float(packed[i >> 1] & 0xffff0000u);
+          const __nv_bfloat162 rest = __floats2bfloat162_rn(p0 - h0, p1 - h1);
+          low[i >> 1] = *reinterpret_cast<const uint32_t*>(&rest);
+        }
       }
       tmem_st16(lane_addr + c * 16, packed);  // P overwrites S, which this row now holds in registers
+      if constexpr (SPLIT) tmem_st16(lane_addr + 64 + c * 16, low);
     }
     l = l * alpha + rowsum;
     tc_wait_st();
@@ -242,6 +249,11 @@ fmha_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__ C
       for (int ks = 0; ks < kBN / 16; ++ks)
         umma_ts(tmem + 128, tmem + ks * 8, smem_desc(aV + ks * 2048, kSubBytes, 1024), kIdescPV,
                 (j > 0 || ks > 0) ? 1u : 0u);
+      if constexpr (SPLIT) {
+#pragma unroll
+        for (int ks = 0; ks < kBN / 16; ++ks)
+          umma_ts(tmem + 128, tmem + 64 + ks * 8, smem_desc(aV + ks * 2048, kSubBytes, 1024), kIdescPV, 1u);
+      }
       umma_commit(bar_o);
       pend_o = (int)par;
     }
@@ -402,16 +414,18 @@ int fmha_tc(const FmhaArgs& a, const dgpt_kv_layout& kv, cudaStream_t st) {
   }
   // one CTA per work item, or fewer CTAs that loop over the items when the caller wants the kernel on few SMs
   const unsigned n_cta = (a.max_ctas > 0 && a.max_ctas < p.n_work) ? (unsigned)a.max_ctas : (unsigned)p.n_work;
-#define DGPT_TC(DD, KK)                                                                                           \
+#define DGPT_TC(...)                                                                                              \
   do {                                                                                                            \
-    e = cudaFuncSetAttribute(fmha_tc_kernel<DD, KK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);     \
-    if (e == cudaSuccess) fmha_tc_kernel<DD, KK><<<n_cta, 128, smem, st>>>(mq, mk, mv, p);                        \
+    e = cudaFuncSetAttribute(fmha_tc_kernel<__VA_ARGS__>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
+    if (e == cudaSuccess) fmha_tc_kernel<__VA_ARGS__><<<n_cta, 128, smem, st>>>(mq, mk, mv, p);                   \
   } while (0)
   const bool kept = p.keep_first > 0;
-  if (D == 64 && kept) DGPT_TC(64, true);
-  else if (D == 64) DGPT_TC(64, false);
-  else if (kept) DGPT_TC(128, true);
-  else DGPT_TC(128, false);
+  if (a.split_p && D == 64) DGPT_TC(64, false, true);
+  else if (a.split_p) DGPT_TC(128, false, true);
+  else if (D == 64 && kept) DGPT_TC(64, true, false);
+  else if (D == 64) DGPT_TC(64, false, false);
+  else if (kept) DGPT_TC(128, true, false);
+  else DGPT_TC(128, false, false);
 #undef DGPT_TC
   if (e != cudaSuccess) {
     set_error("fmha_tc: cudaFuncSetAttribute: %s", cudaGetErrorString(e));

@@ -50,6 +50,17 @@ def test_dense_keys_of_any_length(T, cap, D):
     assert bool(((got - want).abs() <= bound).all())
 
 
+@pytest.mark.parametrize("D", [32, 64, 128])
+@pytest.mark.parametrize("T", [33, 127, 300, 777, 1400])
+def test_probabilities_of_dense_keys_keep_more_than_bf16(T, D):
+    """Against the warp-level kernel (probabilities in fp32): sums that agree to 2^-16 or so round to different bf16 numbers in
+    under one of a hundred places, a step of 2^-8 each: 5e-4 in the norm.  Probabilities rounded to bf16 give 1.4e-3."""
+    B, H = 2, 3
+    q, _, _, lay = _inputs(B, H, T, D, T, torch.bfloat16)
+    a, b = (_attend(q, lay, B, H, T, D, impl=impl).float() for impl in (0, 1))
+    assert ((a - b).norm() / b.norm()).item() <= 5e-4
+
+
 @pytest.mark.parametrize("dt,D,T,cap,impl", [
     (torch.bfloat16, 32, 130, 256, 2), (torch.bfloat16, 32, 130, 256, 3), (torch.bfloat16, 64, 77, 77, 0), (torch.bfloat16, 128, 300, 384, 2),
     (torch.bfloat16, 128, 300, 384, 3), (torch.bfloat16, 64, 1100, 1100, 0), (torch.bfloat16, 16, 40, 40, 0), (torch.float32, 16, 90, 90, 0),
