@@ -251,7 +251,7 @@ static int fmha_full(const void* q, int64_t q_batch_stride, int64_t q_row_stride
   a.pingpong = impl == 4;
   // Dense keys that are not whole tiles: the tensor cores from 24 keys on (8 to 512 pairs of sequence and head; at 17 keys 6.5 us
   // against 5.3 / 9.3 / 11.7 us for heads of 32 / 64 / 128 on the warp-level kernel, at 33 keys 6.3 against 7.5 / 13.7 / 19, at 777
-  // keys 19 to 27 against 90 to 555).
+  // keys 19 to 27 against 90 to 555; with one bf16 part per probability - the second part's product is a quarter of a tile's MMAs more).
   a.any_run = impl == 0 && (causal ? (long long)Tq + q_offset : kv_len ? (long long)kv->page_tokens : (long long)kv_len_all) >= 24;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const KvView view = make_view(kv);

@@ -2,13 +2,16 @@
 // shared-prompt phase of the Monte-Carlo decode (all trajectories of a series against the prompt K/V).
 //
 // Three kernels share the tensor maps and parameters built here:
-//   fmha_tc_ws_kernel (fmha_ws.cu, impl = 2 of dgpt_fmha_prefill, chosen from 1024 keys on): persistent, warp-specialised,
+//   fmha_tc_ws_kernel (fmha_ws.cu, impl = 2 of dgpt_fmha_prefill, chosen from 640 keys on and where one round of its
+//                     CTAs holds every query tile): persistent, warp-specialised,
 //                     one query tile per work item, scores double-buffered in TMEM
 //   fmha_tc_pp_kernel (fmha_pp.cu, impl = 4): persistent, two query tiles per work item
 //   fmha_tc_kernel    (below, impl = 3): the small one
 //
 // fmha_tc_kernel (impl = 3 of dgpt_fmha_prefill; the earlier, simpler form): 128 threads, no
-// fixed roles, 256 TMEM columns and two CTAs per SM so that one CTA's softmax overlaps the other's MMAs.
+// fixed roles, 256 TMEM columns and two CTAs per SM so that one CTA's softmax overlaps the other's MMAs.  Made persistent, with a
+// loader's and an issuer's warp, it took 303 us where this form takes 285 (256 x 8 heads of 32 x 512): the softmax of one warp, 4000
+// clocks a tile, is what bounds it.
 //
 // No cluster launch and no multicast.  Every wait on an mbarrier is bounded in clock cycles; if one runs
 // out the CTA stores the code of the waiting site in a status word, raises a CTA-wide abort flag so the
