@@ -190,7 +190,6 @@ sample_kernel(const T* __restrict__ logits, long long stride, int V, float cap, 
     const int chunk = (V + kSampleThreads - 1) / kSampleThreads;
     const int a = tid * chunk, bnd = min(V, a + chunk);
     float mine = 0.f;
-    int last_kept = -1;
     for (int i = a; i < bnd; ++i) {
       bool kept = true;
       if (filt) {
@@ -200,7 +199,6 @@ sample_kernel(const T* __restrict__ logits, long long stride, int V, float cap, 
       const float w = kept ? __expf((z[i] - zmax) * inv_t) : 0.f;
       z[i] = w;  // own chunk only: reuse the staging buffer for the weights
       mine += w;
-      if (kept) last_kept = i;
     }
     float W;
     const float incl = block_scan_incl(mine, scratch, &W);
@@ -210,24 +208,33 @@ sample_kernel(const T* __restrict__ logits, long long stride, int V, float cap, 
                                         (uint32_t)(step + step_base), 0u, seed_lo, seed_hi);
     const float u = (float)(bits >> 8) * (1.0f / 16777216.0f);
     const float target = u * W;
-    if (tid == 0) sh_int[1] = -1;
+    // Owner of the target: see walk_owner below.
+    if (tid == 0) {
+      sh_int[0] = kSampleThreads;
+      sh_int[1] = -1;
+    }
     __syncthreads();
-    if (mine > 0.f && excl <= target && target < incl) {
-      const float local = target - excl;
+    if (mine > 0.f && target < incl) atomicMin(&sh_int[0], tid);
+    if (mine > 0.f && target == target) atomicMax(&sh_int[1], tid);
+    __syncthreads();
+    const int first = sh_int[0], last = sh_int[1];
+    __syncthreads();
+    if (tid == (first < kSampleThreads ? first : last)) {
+      const float local = first < kSampleThreads ? fmaxf(target - excl, 0.f) : INFINITY;
       float c = 0.f;
-      int pick = last_kept;
+      int pick = -1;
       for (int i = a; i < bnd; ++i) {
         c += z[i];
-        if (z[i] > 0.f && c > local) {
+        if (z[i] > 0.f) {
           pick = i;
-          break;
+          if (c > local) break;
         }
       }
       sh_int[1] = pick;
     }
     __syncthreads();
     token = sh_int[1];
-    if (token < 0) token = best.i;  // unreachable unless W is not finite
+    if (token < 0) token = best.i;  // W is not a number
   }
   if (tid == 0) {
     out_tok[r] = token;
@@ -244,6 +251,18 @@ sample_kernel(const T* __restrict__ logits, long long stride, int V, float cap, 
 // (needed where token order matters) are free of bank conflicts.  The bisection stops as soon as all
 // keys left in the bracket are equal, which takes about log2(distinct keys) sweeps instead of 30.
 constexpr int kWarpRows = 4;
+
+// Which lane's chunk an inverse-CDF walk ends in, and how far into it: the first lane with mass whose inclusive sum lies above
+// `tgt`; the last lane with mass where the rounded target reaches the total.  A lane's chunk begins at incl - mine, which is
+// rounded and may lie above the previous lane's inclusive sum: a target in that gap belongs to the chunk's first token, so the
+// distance is clamped at 0.  (Asked for excl <= tgt as well, such a target had no owner, about one draw in a million.)
+// Returns -1 where no lane has mass or the target is not a number; `local` = INFINITY takes the chunk's last token.
+__device__ __forceinline__ int walk_owner(float mine, float incl, float tgt, float* local) {
+  const unsigned above = __ballot_sync(0xffffffffu, mine > 0.f && tgt < incl);
+  const unsigned mass = __ballot_sync(0xffffffffu, mine > 0.f && tgt == tgt);
+  *local = above ? fmaxf(tgt - (incl - mine), 0.f) : INFINITY;
+  return above ? __ffs(above) - 1 : 31 - __clz(mass);
+}
 
 template <typename T>
 __global__ void __launch_bounds__(32 * kWarpRows)
@@ -356,16 +375,15 @@ sample_warp_kernel(const T* __restrict__ logits, long long stride, int R, int V,
           if (lane >= o) incl += t;
         }
         const float W = __shfl_sync(0xffffffffu, incl, 31);
-        const float excl = incl - mine;
         const float target = fmaxf(top_p, 1e-30f) * Z;
         for (int a = 0; a < kAttempts && !done; ++a) {
           const uint32_t bits = philox4x32_10((uint32_t)traj, (uint32_t)((unsigned long long)traj >> 32),
                                               (uint32_t)(step + step_base), (uint32_t)a, seed_lo, seed_hi);
           const float tgt = (float)(bits >> 8) * (1.0f / 16777216.0f) * W;
-          const bool own = mine > 0.f && excl <= tgt && tgt < incl;
+          float local;
+          const int who = walk_owner(mine, incl, tgt, &local);
           int pick = best.i;
-          if (own) {
-            const float local = tgt - excl;
+          if (lane == who) {
             float c = 0.f;
             for (int i = c0; i < c1; ++i) {
               const float ev = at(i);
@@ -375,8 +393,7 @@ sample_warp_kernel(const T* __restrict__ logits, long long stride, int R, int V,
               if (w > 0.f && c > local) break;
             }
           }
-          const unsigned who = __ballot_sync(0xffffffffu, own);
-          pick = __shfl_sync(0xffffffffu, pick, who ? __ffs(who) - 1 : 0);
+          pick = __shfl_sync(0xffffffffu, pick, max(who, 0));
           if (!filt) {
             token = pick;
             done = true;
@@ -488,7 +505,6 @@ sample_warp_kernel(const T* __restrict__ logits, long long stride, int R, int V,
       __syncwarp();  // chunks below were written by other lanes
       const float inv_t = 1.f / temperature;
       float mine = 0.f;
-      int last_kept = -1;
       for (int i = c0; i < c1; ++i) {
         const float ev = at(i);
         bool kept = true;
@@ -499,7 +515,6 @@ sample_warp_kernel(const T* __restrict__ logits, long long stride, int R, int V,
         const float w = !kept ? 0.f : (temperature == 1.f ? ev : __expf(__logf(ev) * inv_t));
         at(i) = w;
         mine += w;
-        if (kept) last_kept = i;
       }
       float incl = mine;
 #pragma unroll
@@ -508,28 +523,23 @@ sample_warp_kernel(const T* __restrict__ logits, long long stride, int R, int V,
         if (lane >= o) incl += t;
       }
       const float W = __shfl_sync(0xffffffffu, incl, 31);
-      const float excl = incl - mine;
-
       const uint32_t bits = philox4x32_10((uint32_t)traj, (uint32_t)((unsigned long long)traj >> 32),
                                           (uint32_t)(step + step_base), (uint32_t)kAttempts, seed_lo, seed_hi);
       const float u = (float)(bits >> 8) * (1.0f / 16777216.0f);
       const float tgt = u * W;
-      const bool own = mine > 0.f && excl <= tgt && tgt < incl;
-      int pick = last_kept;
-      if (own) {
-        const float local = tgt - excl;
+      float local;
+      const int who = walk_owner(mine, incl, tgt, &local);
+      int pick = best.i;
+      if (lane == who) {
         float c = 0.f;
         for (int i = c0; i < c1; ++i) {
           const float w = at(i);
           c += w;
-          if (w > 0.f && c > local) {
-            pick = i;
-            break;
-          }
+          if (w > 0.f) pick = i;
+          if (w > 0.f && c > local) break;
         }
       }
-      const unsigned who = __ballot_sync(0xffffffffu, own);
-      if (who) token = __shfl_sync(0xffffffffu, pick, __ffs(who) - 1);
+      token = __shfl_sync(0xffffffffu, pick, max(who, 0));
       }
     }
   }
