@@ -22,6 +22,7 @@ honoured by running the same forward eagerly and handing it the device logits.
 
 from __future__ import annotations
 
+import threading
 from typing import Callable, Generator
 
 import torch
@@ -514,6 +515,10 @@ class StepRunner:
     changes: the weights, the cache's storage or state buffer, the key splits.  All of them run on one stream of the runner,
     between two waits with the caller's, so that requests stepped from several streams never share cuBLAS's workspace at
     the same time.
+
+    Different requests may be stepped from different threads: one thread at a time enqueues on the runner's stream (what
+    another put there meanwhile would be recorded instead of run), and a thread records only after it has run a step
+    itself, so that its cuBLAS handle and workspace exist before.
     """
 
     def __init__(self, model: DeviceModel) -> None:
@@ -522,13 +527,16 @@ class StepRunner:
         self._free: list = []
         self._single: dict = {}  # (cache, state buffer): its SingleStep
         self._stream: torch.cuda.Stream | None = None
+        self._lock = threading.Lock()  # the dictionaries, and what is enqueued on the runner's stream
+        self._ran = threading.local()
 
     def _cache(self, request):
-        if request not in self._live:
-            cache = self._free.pop() if self._free else self.model.new_cache()
-            cache.reset()
-            self._live[request] = cache
-        return self._live[request]
+        with self._lock:
+            cache = self._live.get(request)
+            if cache is None:
+                cache = self._live[request] = self._free.pop() if self._free else self.model.new_cache()
+                cache.reset()
+            return cache
 
     @torch.inference_mode()
     def step(self, request, tokens: list[int], want: list[int]) -> torch.Tensor:
@@ -546,20 +554,27 @@ class StepRunner:
         return self.model.logits_at(idx, cache, rows).to(torch.float32, copy=True)
 
     def _one(self, cache, token: int) -> torch.Tensor | None:
+        with self._lock:
+            one, out = self._enqueue_one(cache, token)
+        if one is not None and one.checks and int(one.plan.status.item()):
+            raise RuntimeError(f"device-side status {int(one.plan.status.item())}: a cache slot was out of range, or a bounded wait ran out")
+        return out
+
+    def _enqueue_one(self, cache, token: int):
         state = getattr(cache, "state", None)
         key = (cache, 0 if state is None else state.current)  # a portion of several tokens changes the buffer
         if self._stream is None:
             self._stream = torch.cuda.Stream(device=self.model.embedding.device)
         one = self.model.single_step(cache, self._single.get(key), self._stream)
         if one is None:
-            return None
+            return None, None
         self._single[key] = one
         caller, mine = torch.cuda.current_stream(), self._stream
         mine.wait_stream(caller)
         with torch.cuda.stream(mine):
             slot = cache.pos if state is None else cache.slot
             one.numbers.copy_(torch.tensor([token, slot, cache.pos, slot + 1], dtype=torch.int32))
-            if one.graph is None and one.runs > 0:
+            if one.graph is None and one.runs > 0 and getattr(self._ran, "eager", False):
                 before = _lib.stats.launches
                 graph = torch.cuda.CUDAGraph()
                 graph.capture_begin(capture_error_mode="thread_local")
@@ -570,6 +585,7 @@ class StepRunner:
                 one.graph, one.launches, _lib.stats.launches = graph, _lib.stats.launches - before, before
             if one.graph is None:
                 one.enqueue()
+                self._ran.eager = True
             else:
                 one.graph.replay()
                 _lib.stats.launches += one.launches
@@ -578,14 +594,13 @@ class StepRunner:
         caller.wait_stream(mine)
         out.record_stream(caller)
         cache.pos += 1
-        if one.checks and int(one.plan.status.item()):
-            raise RuntimeError(f"device-side status {int(one.plan.status.item())}: a cache slot was out of range, or a bounded wait ran out")
-        return out
+        return one, out
 
     def finish(self, request) -> None:
-        cache = self._live.pop(request, None)
-        if cache is not None:
-            self._free.append(cache)
+        with self._lock:
+            cache = self._live.pop(request, None)
+            if cache is not None:
+                self._free.append(cache)
 
 
 def _generate_generic(model, tokens, num_samples, G, sampler, seed, force_schedule):

@@ -1,0 +1,117 @@
+"""StepRunner's host logic without a GPU: streams, graphs and the model are stand-ins that note who is inside."""
+
+import contextlib
+import threading
+import time
+from types import SimpleNamespace
+
+import pytest
+import torch
+
+
+class _Logits:
+    def to(self, *a, **k):
+        return SimpleNamespace(record_stream=lambda s: None)
+
+
+class _Busy:
+    """What is enqueued on the runner's stream: only one thread may be at it."""
+
+    def __init__(self):
+        self.inside, self.overlaps = set(), 0
+
+    def work(self):
+        me = threading.get_ident()
+        self.overlaps += bool(self.inside - {me})
+        self.inside.add(me)
+        time.sleep(0.002)
+        self.inside.discard(me)
+
+
+@pytest.fixture
+def cuda(monkeypatch):
+    class Graph:
+        def capture_begin(self, **k):
+            pass
+
+        def capture_end(self):
+            pass
+
+        def replay(self):
+            pass
+
+    stream = SimpleNamespace(wait_stream=lambda other: None)
+    monkeypatch.setattr(torch.cuda, "Stream", lambda **k: stream)
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda *a: stream)
+    monkeypatch.setattr(torch.cuda, "stream", lambda s: contextlib.nullcontext())
+    monkeypatch.setattr(torch.cuda, "CUDAGraph", Graph)
+
+
+def _model(busy):
+    from diff_gpt_b200.model.gpt import SingleStep
+
+    class Cache:
+        def reset(self):
+            self.pos = 0
+
+    class Plan:
+        logits = _Logits()
+
+        def run(self, ids, bind):
+            busy.work()
+
+    class Model:
+        vocab_size, embedding = 8, torch.zeros(1)
+
+        def new_cache(self):
+            return Cache()
+
+        def single_step(self, cache, old, stream):
+            return old or SingleStep(Plan(), None, torch.zeros(4, dtype=torch.int32), 0, (), checks=False)
+
+    return Model()
+
+
+def _in_thread(fn):
+    err = []
+
+    def go():
+        try:
+            fn()
+        except Exception as e:  # noqa: BLE001
+            err.append(e)
+
+    t = threading.Thread(target=go)
+    t.start()
+    return t, err
+
+
+def test_one_thread_at_a_time_on_the_runners_stream(cuda):
+    from diff_gpt_b200 import StepRunner
+
+    busy = _Busy()
+    runner = StepRunner(_model(busy))
+    threads = [_in_thread(lambda r=r: [runner.step(r, [1], [0]) for _ in range(8)]) for r in range(4)]
+    for t, err in threads:
+        t.join()
+        assert not err
+    assert busy.overlaps == 0
+    assert sorted(c.pos for c in runner._live.values()) == [8] * 4
+
+
+def test_a_thread_records_only_after_a_step_of_its_own(cuda):
+    """Thread B takes over a request that A has begun: B's first step runs as launches, its second is recorded."""
+    from diff_gpt_b200 import StepRunner
+
+    runner = StepRunner(_model(_Busy()))
+    runner.step("r", [1], [0])
+    seen = []
+
+    def b():
+        for _ in range(2):
+            runner.step("r", [1], [0])
+            seen.append(next(iter(runner._single.values())).graph is not None)
+
+    t, err = _in_thread(b)
+    t.join()
+    assert not err and seen == [False, True]
