@@ -424,11 +424,14 @@ class ForwardPlan:
                         prefix_o=po, prefix_lse=pl, workspace=self.workspace, n_splits=b.n_splits,
                     )
             else:
+                own_gate = b.fmha_impl != 4  # the kernel with two query tiles per CTA is not built with one
                 ops.fmha_prefill(
                     self.q, b.layouts[i], self.y, B=n_seq, H=H, Tq=T, D=D, q_batch_stride=T * C, q_row_stride=C,
                     o_batch_stride=T * C, o_row_stride=C, kv_len_all=b.kv_len, q_offset=b.q_offset, causal=True,
-                    impl=b.fmha_impl, status=self.status, gate=gv,
+                    impl=b.fmha_impl, status=self.status, gate=gv if own_gate else None,
                 )
+                if not own_gate:
+                    ops.sigmoid_gate(self.y, gv)
             part = self.parts[i]
             if partial is None:
                 self._linear(self.y, lw.wproj_t, part, "gemm_proj")
