@@ -278,7 +278,7 @@ class DelunexPlan:
         """self.y = W_down xielu(W_up self.u)"""
         ff = lw.w_up.shape[0]
         act = self._buf("act", self.n, ff)
-        if self.fused_ff and ff % 16 == 0 and (self.n > 1 or lw.w_up.data_ptr() % 16 == 0):
+        if self.fused_ff and ff % 16 == 0 and (self.n > 1 or ops.rows16(lw.w_up)):
             ops.linear(self.u, lw.w_up, act, xielu=lw.act, status=self.status)
         else:
             up = self._buf("up", self.n, ff)

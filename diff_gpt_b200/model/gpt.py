@@ -281,9 +281,8 @@ class ForwardPlan:
         self.cap = cap
         self.status = torch.zeros(1, dtype=torch.int32, device=dev)
         # tcgen05 GEMM + SwiGLU epilogue: bf16 with tileable sizes, and enough rows to fill the tensor cores
-        # parameters may be views into a larger buffer: the kernels that take the small products want 16-byte aligned rows
-        packed = model.packed_weights()
-        aligned = all(t.data_ptr() % 16 == 0 for l in packed.layers for t in (l.wproj_t, l.w1, l.w2_t)) and packed.emb.data_ptr() % 16 == 0
+        # parameters may be views: rows that the kernels for small products do not take stay on cuBLAS
+        aligned = model.packed_weights().rows16
         self.one_row = dt == torch.bfloat16 and C % 16 == 0 and n == 1 and aligned  # see dgpt_linear: ahead of cuBLAS at every size
         self.fused_ffn = FUSED_FFN and dt == torch.bfloat16 and C % 8 == 0 and (n >= FUSED_FFN_MIN_ROWS or self.one_row)
         self.f32 = dt == torch.float32 and C % 4 == 0 and aligned
@@ -485,6 +484,7 @@ class _Packed:
     emb: torch.Tensor
     freqs_cis: torch.Tensor
     layers: list
+    rows16: bool  # every matrix lies as the linear kernels want it
     stamp: tuple
 
     @property
@@ -561,7 +561,8 @@ class GPT(DeviceModel):
                 )
             emb = self.token_embedding_table.weight.detach()
             table = self.freqs_cis.to(emb.dtype).contiguous()
-        self._packed = _Packed(emb=emb, freqs_cis=table, layers=layers, stamp=stamp)
+        rows16 = ops.rows16(emb) and all(ops.rows16(w) for l in layers for w in (l.w1, l.wproj_t.t(), l.w2_t.t()))
+        self._packed = _Packed(emb=emb, freqs_cis=table, layers=layers, rows16=rows16, stamp=stamp)
         return self._packed
 
     @classmethod

@@ -273,6 +273,12 @@ def attn_merge(
     )
 
 
+def rows16(w: torch.Tensor) -> bool:
+    """Whether a matrix's rows lie as the linear kernels want them: elements side by side, every row on a 16-byte boundary.
+    (Parameters may be views: slices of a wider buffer, transposed, off a boundary.)"""
+    return w.stride(1) == 1 and w.data_ptr() % 16 == 0 and w.stride(0) * w.element_size() % 16 == 0
+
+
 def linear(
     a: torch.Tensor,
     w: torch.Tensor,
