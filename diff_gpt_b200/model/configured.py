@@ -188,3 +188,6 @@ class ConfiguredModel(DeviceModel):
                 new = torch.multinomial(F.softmax(logits.float(), dim=-1), num_samples=1, generator=rng)
             out[:, cur] = new.reshape(-1)
         return out
+
+
+ConfiguredModel.step_path = ((ConfiguredModel, "logits_at"), (ConfiguredModel, "_step"))

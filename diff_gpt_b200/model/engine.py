@@ -544,7 +544,7 @@ class StepRunner:
         assert len(tokens) > 0 and all(0 <= t < self.model.vocab_size for t in tokens), "tokens must be ids of the vocabulary"
         assert all(0 <= w < len(tokens) for w in want), "wanted places must lie among the tokens of the step"
         cache = self._cache(request)
-        if len(tokens) == 1 and len(want) == 1 and _lib.stats.timer is None:
+        if len(tokens) == 1 and len(want) == 1 and _lib.stats.timer is None and self.model.single_step_allowed():
             out = self._one(cache, int(tokens[0]))
             if out is not None:
                 return out

@@ -25,6 +25,7 @@ from dataclasses import dataclass
 import torch
 import torch.nn as nn
 import torch.nn.functional as F
+from torch.nn.modules.module import _has_any_global_hook
 
 from .. import ops
 from .._lib import region
@@ -82,6 +83,20 @@ class DeviceModel(BaseGPT):
     @abstractmethod
     def logits_at(self, idx: torch.Tensor, cache, rows: torch.Tensor) -> torch.Tensor:
         """Run idx (1, T) behind what `cache` holds; the logits [len(rows), V] of the given places among the T tokens."""
+
+    # (class, method) that `logits_at` goes through up to the launches, itself first
+    step_path: tuple = ()
+
+    def single_step_allowed(self) -> bool:
+        """Whether a token through `logits_at` is this library's launches and nothing else: none of the methods on the way
+        replaced by a subclass or on the object and, where the module is called, no hook on it."""
+        for cls, name in self.step_path:
+            if name == "__call__":
+                if self._forward_hooks or self._forward_pre_hooks or self._compiled_call_impl or _has_any_global_hook():
+                    return False
+            if getattr(type(self), name) is not getattr(cls, name) or name in self.__dict__:
+                return False
+        return bool(self.step_path)
 
     def single_step(self, cache, old: "SingleStep | None", stream: torch.cuda.Stream) -> "SingleStep | None":
         """The launches of one more token behind `cache`, which has room for it afterwards: `old` where it still fits, or None
@@ -727,6 +742,8 @@ class GPT(DeviceModel):
     def device_type(self) -> str:
         return str(self.freqs_cis.device.type)
 
+
+GPT.step_path = ((GPT, "logits_at"), (nn.Module, "__call__"), (GPT, "forward"), (GPT, "_infer"))
 
 _SM_COUNT: dict[int, int] = {}
 

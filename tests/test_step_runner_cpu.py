@@ -66,6 +66,9 @@ def _model(busy):
         def new_cache(self):
             return Cache()
 
+        def single_step_allowed(self):
+            return True
+
         def single_step(self, cache, old, stream):
             return old or SingleStep(Plan(), None, torch.zeros(4, dtype=torch.int32), 0, (), checks=False)
 
@@ -115,3 +118,37 @@ def test_a_thread_records_only_after_a_step_of_its_own(cuda):
     t, err = _in_thread(b)
     t.join()
     assert not err and seen == [False, True]
+
+
+def test_replaced_methods_and_hooks_keep_the_general_path():
+    import delunex_cases
+    from diff_gpt_b200 import GPT
+    from diff_gpt_b200.model.registry import model_class
+
+    kw = dict(vocab_size=64, n_embd=32, n_head=2, n_layer=1)
+    cfg = delunex_cases.CASES["tiny"]
+    other = model_class(cfg)
+    assert GPT(**kw).single_step_allowed() and other.from_config(cfg).single_step_allowed()
+
+    class Own(GPT):
+        def forward(self, *a, **k):
+            return super().forward(*a, **k)
+
+    class OwnOther(other):
+        def logits_at(self, *a):
+            return super().logits_at(*a)
+
+    assert not Own(**kw).single_step_allowed() and not OwnOther.from_config(cfg).single_step_allowed()
+    m = GPT(**kw)
+    m.forward = lambda *a, **k: None
+    assert not m.single_step_allowed()
+    for add in (m.register_forward_hook, m.register_forward_pre_hook, torch.nn.modules.module.register_module_forward_hook):
+        m = GPT(**kw)
+        h = (getattr(m, add.__name__) if hasattr(m, add.__name__) else add)(lambda *a: None)
+        assert not m.single_step_allowed()
+        h.remove()
+        assert m.single_step_allowed()
+    # the module itself is not called on the way to the other models' logits
+    m = other.from_config(cfg)
+    m.register_forward_hook(lambda *a: None)
+    assert m.single_step_allowed()
