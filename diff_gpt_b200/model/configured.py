@@ -141,7 +141,7 @@ class ConfiguredModel(DeviceModel):
     def single_step(self, cache: RowCache, old: SingleStep | None, stream: torch.cuda.Stream) -> SingleStep:
         cache.ensure(1)
         # the key splits change from one 128-key tile to the next, until every window is full
-        kind = -(-min(cache.slot + 1, cache.keep + 1 + cache.keep_first) // 128)
+        kind = (-(-min(cache.slot + 1, cache.keep + 1 + cache.keep_first) // 128),)
         held = (self.packed_weights(), *cache.state.source.values(), *cache.store.values(), *self.step_tables(cache.pos + 1))
         if old is not None and old.fits(kind, held):
             return old

@@ -512,7 +512,7 @@ class StepRunner:
     A single token whose logits are wanted is a hundred launches of a few microseconds each, which take the host three times
     as long as the GPU (Kipolix, 8 layers: 1.4 ms a token, of which the GPU was busy 0.4).  So the second such step of a
     cache records its launches as a graph, and the following ones replay it until something that the launches were made for
-    changes: the weights, the cache's storage or state buffer, the key splits.  All of them run on one stream of the runner,
+    changes: the weights, the cache's storage or state buffer, the key splits, the numbers a GPT carries (soft-cap, SwiGLU).  All of them run on one stream of the runner,
     between two waits with the caller's, so that requests stepped from several streams never share cuBLAS's workspace at
     the same time.
 

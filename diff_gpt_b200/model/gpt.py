@@ -202,21 +202,21 @@ class SingleStep:
     """One token of one request: a plan and a binding whose changing numbers are read from `numbers` on the device (token, slot,
     position, keys), so that the launches can be recorded once and replayed.
 
-    kind    host-side choices that the launches were made with (key splits)
+    kind    host-side choices and numbers that the launches were made with (key splits, soft-cap, ...)
     held    what the launches point at; kept alive here and compared by `is`
     """
 
     plan: object
     bind: object
     numbers: torch.Tensor  # int32 [4]
-    kind: int
+    kind: tuple
     held: tuple
     checks: bool  # the plan's status is read after every step
     graph: torch.cuda.CUDAGraph | None = None
     launches: int = 0
     runs: int = 0
 
-    def fits(self, kind: int, held: tuple) -> bool:
+    def fits(self, kind: tuple, held: tuple) -> bool:
         return self.kind == kind and len(self.held) == len(held) and all(a is b for a, b in zip(self.held, held))
 
     def enqueue(self) -> None:
@@ -611,8 +611,9 @@ class GPT(DeviceModel):
         assert t0 + 1 <= self.freqs_cis.shape[0]
         cache.ensure(t0 + 1, emb.dtype, emb.device)
         splits = _pick_splits(H, t0 + 1)
+        kind = (splits, self.logit_softcap, self.swiglu_alpha, self.swiglu_limit, self.attn_res_layers_per_block)
         held = (self.packed_weights(), cache.kv_cache)
-        if old is not None and old.fits(splits, held):
+        if old is not None and old.fits(kind, held):
             return old
         with torch.cuda.stream(stream):
             numbers = torch.zeros(4, dtype=torch.int32, device=emb.device)
@@ -621,7 +622,7 @@ class GPT(DeviceModel):
                 layouts=[cache.layer_layout(i) for i in range(self.n_layer)], pos0=numbers[2:3], slot0=numbers[1:2], decode=True,
                 len0=zero, start1=zero, len1=numbers[3:4], n_splits=splits,
             )
-            return SingleStep(ForwardPlan(self, 1, 1, cap=self.logit_softcap), bind, numbers, splits, held, checks=False)
+            return SingleStep(ForwardPlan(self, 1, 1, cap=self.logit_softcap), bind, numbers, kind, held, checks=False)
 
     def paged_cache(self, n_series, rows_per_series, prefix_len, max_new, page_tokens, pool=None) -> PagedKVCache:
         emb = self.embedding
