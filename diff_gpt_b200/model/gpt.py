@@ -223,11 +223,21 @@ class SingleStep:
         self.plan.run(self.numbers[0:1], self.bind)
 
 
-def own_f32(M: int, N: int, K: int) -> bool:
-    """Whether an fp32 product runs on dgpt_linear_f32: up to 400 of its tiles (measured in us, cuBLAS / own: 100 x 256 x 64 3.63 / 2.62,
-    100 x 64 x 128 4.65 / 2.93, 400 x 512 x 64 3.95 / 3.93, 1000 x 256 x 64 3.99 / 4.69, 400 x 1024 x 256 9.4 / 13.2; its SwiGLU saves a launch of
-    1.6 besides).  cuBLAS has a matrix-vector kernel for one row, ahead from K = 128 on (1 x 64 x 128 1.97 / 2.81; K = 64 2.90 / 2.28)."""
-    return -(-M // 16) * -(-N // 32) <= 400 and (M > 1 or K <= 64) and K <= 512
+def own_f32(M: int, N: int, K: int, ends: bool = False) -> bool:
+    """Whether an fp32 product runs on dgpt_linear_f32; `ends`: it ends in an addition, a SwiGLU or a soft-cap, which cuBLAS leaves to
+    a pass of its own (or a slower kernel).  Measured over C = 64 to 512 (K = C or 2 C, N = C to 4 C), us, cuBLAS / own:
+    more than 16 rows, up to 400 tiles: 100 x 256 x 64 3.63 / 2.62, 100 x 64 x 128 4.65 / 2.93, 400 x 512 x 64 3.95 / 3.93, none over 3 % behind;
+    beyond 1000 x 256 x 64 3.99 / 4.69, 400 x 1024 x 256 9.4 / 13.2.
+    Up to 16 rows cuBLAS has kernels for few rows: 2 x 512 x 512 3.67 / 6.66, 8 x 256 x 256 3.29 / 4.16, 2 x 64 x 64 2.04 / 2.34.  Own there:
+    with an ending up to K = 128 (2 x 512 x 128 SwiGLU 3.57 / 3.48, 8 x 256 x 64 2.9 / 2.3), from 8 wide rows on (8 x 1024 x 256 6.43 / 4.25,
+    8 x 2048 x 512 9.63 / 7.00), and one row up to K = 64 (1 x 256 x 64 2.90 / 2.28; 1 x 64 x 128 1.97 / 2.81)."""
+    if -(-M // 16) * -(-N // 32) > 400 or K > 512:
+        return False
+    if M > 16:
+        return True
+    if M == 1:
+        return K <= 64
+    return (ends and K <= 128) or (M >= 8 and N >= 1024 and K >= 256)
 
 
 # ---- how one forward call is bound to K/V storage ----------------------------------
@@ -301,7 +311,7 @@ class ForwardPlan:
         self.one_row = dt == torch.bfloat16 and C % 16 == 0 and n == 1 and aligned  # see dgpt_linear: ahead of cuBLAS at every size
         self.fused_ffn = FUSED_FFN and dt == torch.bfloat16 and C % 8 == 0 and (n >= FUSED_FFN_MIN_ROWS or self.one_row)
         self.f32 = dt == torch.float32 and C % 4 == 0 and aligned
-        self.own_ffn1 = self.f32 and own_f32(n, 4 * C, C)
+        self.own_ffn1 = self.f32 and own_f32(n, 4 * C, C, ends=True)
         self.f = None if self.fused_ffn or self.own_ffn1 else buf(n, 4 * C)
         # norm factors of committed depth-mix candidates, carried from mix to mix (16-byte rows needed)
         self.cache_norms = CACHE_NORMS and (C * emb.element_size()) % 16 == 0
@@ -339,7 +349,7 @@ class ForwardPlan:
 
     def _linear(self, a: torch.Tensor, w_t: torch.Tensor, out: torch.Tensor, name: str, add: bool = False) -> None:
         """out (+)= a @ w_t: a small fp32 model's and a lone bf16 row on the library's kernels, others on cuBLAS."""
-        if self.f32 and own_f32(out.shape[0], out.shape[1], a.shape[1]):
+        if self.f32 and own_f32(out.shape[0], out.shape[1], a.shape[1], ends=add):
             ops.linear_f32(a, w_t.t(), out, add=out if add else None)
             return
         if self.one_row:
@@ -473,7 +483,7 @@ class ForwardPlan:
             return None
         if self.own_head:
             ops.linear(self.xn, W.emb, self.logits, softcap=self.cap, status=self.status)
-        elif self.f32 and own_f32(*self.logits.shape, C):
+        elif self.f32 and own_f32(*self.logits.shape, C, ends=self.cap > 0):
             ops.linear_f32(self.xn, W.emb, self.logits, softcap=self.cap)
         else:
             with region("gemm_logits"):
