@@ -501,7 +501,7 @@ struct GemmOperands {
 template <int BN, int CG, int EPI>
 static int gemm_launch(const GemmOperands& o, const GemmParams& p, int n_sm, int dev, cudaStream_t st) {
   constexpr uint32_t kSmem = gemm_smem(BN, CG, EPI);
-  static_assert(kSmem <= kGSmemMax && gemm_stages(BN, CG, EPI) >= 4 && 2 * gemm_stages(BN, CG, EPI) + 5 <= 24, "shared memory of the GEMM");
+  static_assert(kSmem <= kGSmemMax && gemm_stages(BN, CG, EPI) >= 3 && 2 * gemm_stages(BN, CG, EPI) + 5 <= 24, "shared memory of the GEMM");
   auto kernel = gemm_tc_kernel<BN, CG, EPI>;
   static bool ready[64] = {};
   if (!ready[dev]) {
@@ -535,31 +535,39 @@ static int gemm_launch(const GemmOperands& o, const GemmParams& p, int n_sm, int
   return launch_status("linear");
 }
 
-// Which tile: the form with the least estimated time, rounds of tiles x clocks of one.  A k-block of 64 takes 2 BN clocks of
-// the tensor cores in either form; bringing it in takes its bytes per SM at about 40 a clock, which is what the SMs get from L2 when
-// all of them ask; and an epilogue that runs beside the next tile's product takes about 10 clocks a column.
+// Which tile: the form with the least estimated time in clocks, rounds of tiles x clocks of one.  A k-block of 64 takes 2 BN clocks
+// of the tensor cores in either form; bringing it in takes its bytes per SM at 56 a clock; an epilogue that runs beside the next tile's product
+// takes about 16 clocks a column; and a pair costs 4000 more (its launch, and barriers across SMs at both ends), which single CTAs of up
+// to 256 columns save where there is little to do.  Over 289 layers of 3 to 65536 rows, N 256 to 16384 and K 128 to 2048, every form measured, the
+// one chosen is 0.3 % behind the best on average.  (Without the single CTAs of 256 and 192 columns, no charge for a pair and 40 bytes a clock it
+// was 7 %: 300 x 10912 x 2048 SiLU gate 26.1 -> 18.2 us, 512 x 512 x 256 6.0 -> 4.8, 1000 x 1024 x 512 7.3 -> 6.1, 4096 x 3072 x 768 SwiGLU 20.9 either way.)
 template <int EPI>
 static int gemm_run(const GemmOperands& o, const GemmParams& p, int n_sm, int dev, cudaStream_t st) {
   const int n_kb = (p.K + kGK - 1) / kGK;
   int bn = 0, cg = 0;
   double best = 1e300;
-  const int forms[5][2] = {{256, 2}, {192, 2}, {128, 2}, {128, 1}, {64, 1}};
+  const int forms[7][2] = {{256, 2}, {192, 2}, {128, 2}, {256, 1}, {192, 1}, {128, 1}, {64, 1}};
   for (const auto& f : forms) {
     if (f[1] == 2 && p.M <= kGM) continue;  // half of the pair would have no rows
     const long long tiles = (long long)((p.M + f[1] * kGM - 1) / (f[1] * kGM)) * ((p.N + f[0] - 1) / f[0]);
     const long long slots = n_sm / f[1];
-    const double block = fmax(2.0 * f[0], gemm_stage_bytes(f[0], f[1]) / 40.0);
-    const double cost = (double)((tiles + slots - 1) / slots) * fmax(n_kb * block, 10.0 * f[0]);
+    const double block = fmax(2.0 * f[0], gemm_stage_bytes(f[0], f[1]) / 56.0);
+    const double cost = (double)((tiles + slots - 1) / slots) * fmax(n_kb * block, 16.0 * f[0]) + (f[1] == 2 ? 4000.0 : 0.0);
     if (cost < best * 0.999) {
       best = cost;
       bn = f[0];
       cg = f[1];
     }
   }
-  if (cg == 1) return bn == 128 ? gemm_launch<128, 1, EPI>(o, p, n_sm, dev, st) : gemm_launch<64, 1, EPI>(o, p, n_sm, dev, st);
-  if (bn == 256) return gemm_launch<256, 2, EPI>(o, p, n_sm, dev, st);
-  if (bn == 192) return gemm_launch<192, 2, EPI>(o, p, n_sm, dev, st);
-  return gemm_launch<128, 2, EPI>(o, p, n_sm, dev, st);
+  if (cg == 2) {
+    if (bn == 256) return gemm_launch<256, 2, EPI>(o, p, n_sm, dev, st);
+    if (bn == 192) return gemm_launch<192, 2, EPI>(o, p, n_sm, dev, st);
+    return gemm_launch<128, 2, EPI>(o, p, n_sm, dev, st);
+  }
+  if (bn == 256) return gemm_launch<256, 1, EPI>(o, p, n_sm, dev, st);
+  if (bn == 192) return gemm_launch<192, 1, EPI>(o, p, n_sm, dev, st);
+  if (bn == 128) return gemm_launch<128, 1, EPI>(o, p, n_sm, dev, st);
+  return gemm_launch<64, 1, EPI>(o, p, n_sm, dev, st);
 }
 
 }  // namespace tc

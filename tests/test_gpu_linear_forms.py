@@ -1,18 +1,31 @@
-"""Every tile form of dgpt_linear (single CTAs of 64 and 128 columns, CTA pairs of 128, 192 and 256) with every storing epilogue, at
-sizes that end inside a tile in each direction."""
+"""Every tile form of dgpt_linear (single CTAs of 64, 128, 192 and 256 columns, CTA pairs of 128, 192 and 256) with every storing epilogue,
+at sizes that end inside a tile in each direction."""
 
 import pytest
 import torch
 
 pytestmark = pytest.mark.gpu
 
-# the form that the sizes lead to on 148 multiprocessors: see gemm_run
+# (M, N, K) and the form that gemm_run takes for them on 148 multiprocessors: columns of a tile, CTAs of one
 FORMS = {
-    "one CTA, 64": (100, 272, 136), "one CTA, 128": (33, 9584, 72), "pair, 128": (300, 272, 200), "pair, 192": (1990, 1584, 72),
-    "pair, 256": (1990, 2256, 72), "pair, several rounds": (4500, 2320, 328), "one row": (1, 16, 8),
-    "one row, shared K": (1, 528, 1032), "one row, a warp a pair": (1, 4752, 264), "two rows, shared K": (2, 1008, 5456),
-    "two rows, a warp a pair": (2, 4752, 520), "three rows": (3, 48, 24),
+    "one CTA, 64": ((100, 272, 136), (64, 1)), "one CTA, 64, two rows of tiles": ((300, 272, 200), (64, 1)),
+    "one CTA, 128": ((33, 9584, 72), (128, 1)), "one CTA, 192": ((1990, 1584, 72), (192, 1)), "one CTA, 256": ((1990, 2256, 72), (256, 1)),
+    "one CTA, 256, several rounds": ((4500, 2320, 328), (256, 1)), "pair, 128": ((555, 2064, 2056), (128, 2)),
+    "pair, 192": ((1100, 2064, 2056), (192, 2)), "pair, 256": ((1100, 3088, 1032), (256, 2)), "pair, several rounds": ((4500, 2320, 1032), (256, 2)),
+    "one row": ((1, 16, 8), None), "one row, shared K": ((1, 528, 1032), None), "one row, a warp a pair": ((1, 4752, 264), None),
+    "two rows, shared K": ((2, 1008, 5456), None), "two rows, a warp a pair": ((2, 4752, 520), None), "three rows": ((3, 48, 24), (64, 1)),
 }
+
+
+def _form(M, N, K):
+    """gemm_run's rule, restated: the least of rounds x clocks of a tile, 4000 more for a pair."""
+    best = []
+    for bn, cg in ((256, 2), (192, 2), (128, 2), (256, 1), (192, 1), (128, 1), (64, 1)):
+        if cg == 1 or M > 128:
+            tiles = -(-M // (128 * cg)) * -(-N // bn)
+            block = max(2 * bn, (16384 + bn // cg * 128) / 56)
+            best.append((-(-tiles // (148 // cg)) * max(-(-K // 64) * block, 16 * bn) + 4000 * (cg - 1), (bn, cg)))
+    return min(best, key=lambda x: x[0])[1]
 
 
 @pytest.mark.parametrize("form", FORMS)
@@ -24,7 +37,8 @@ def test_every_form_and_epilogue(form, epilogue):
     absolute in the tangent (its exponential form)."""
     from diff_gpt_b200 import ops
 
-    M, N, K = FORMS[form]
+    (M, N, K), taken = FORMS[form]
+    assert taken is None or _form(M, N, K) == taken
     g = torch.Generator(device="cuda").manual_seed(M + N + K)
     a = torch.randn(M, K, generator=g, device="cuda").bfloat16()
     w = (torch.randn(N, K, generator=g, device="cuda") * 0.3).bfloat16()
