@@ -155,9 +155,21 @@ fmha_simt_kernel(const T* __restrict__ q, long long q_bs, long long q_rs, KvView
   } else {
     T* op = static_cast<T*>(o) + oo;
     if (egate) {
+      // All of the row's gate before the first store, which the compiler cannot prove to be elsewhere: loaded one by one between the
+      // stores it took 16.2 us for 4 x 8 heads of 64 x 17 fp32 queries, where a separate pass over the output takes 11.2 in all.
       const T* gp = egate + ((long long)b * Tq + qi) * egate_rs + (long long)h * D + part * DP;
+      float g[DP];
+      if ((reinterpret_cast<uintptr_t>(gp) & 15) == 0) {
 #pragma unroll
-      for (int d = 0; d < DP; ++d) Io<T>::st(op + d, gated<T>(acc[d] * inv, Io<T>::ld(gp + d)));
+        for (int d = 0; d < DP; d += VEC) ld16<T>(gp + d, g + d);
+      } else {
+#pragma unroll
+        for (int d = 0; d < DP; ++d) g[d] = Io<T>::ld(gp + d);
+      }
+#pragma unroll
+      for (int d = 0; d < DP; ++d) g[d] = gated<T>(acc[d] * inv, g[d]);
+#pragma unroll
+      for (int d = 0; d < DP; ++d) Io<T>::st(op + d, g[d]);
     } else {
 #pragma unroll
       for (int d = 0; d < DP; ++d) Io<T>::st(op + d, acc[d] * inv);
@@ -226,6 +238,15 @@ static bool fmha_one_round(const FmhaArgs& a) {
   return (long long)a.B * a.H * ((a.Tq + 127) / 128) <= n_sm[dev];
 }
 
+// Whether the warp-level kernel applies the output gate itself.  One lane gates a query's whole row there, in fp32 with a full division
+// per element, which hundreds of short CTAs cannot hide; a pass of its own takes 1.4 to 2 us more than its launch hides.  Measured in us,
+// pass / epilogue: fp32 4 x 8 heads of 64 x 17 11.2 / 13.4, 1 x 4 heads of 128 x 8 7.9 / 10.7, 256 x 8 heads of 32 x 8 18.2 / 24.1, of 16 x 2
+// 10.2 / 12.4; but heads of 16, 64 x 12 x 8, 7.9 / 6.9, 1 x 4 x 89 within 0.4 of no gate at all.  bf16 256 x 8 heads of 64 x 2 1.15 times the pass, x 8 level.
+static bool simt_own_gate(const FmhaArgs& a) {
+  const long long pairs = (long long)a.B * a.H;
+  return a.dtype == DGPT_BF16 ? a.Tq >= 8 || pairs <= 512 : a.D <= 16 && pairs <= 1024;
+}
+
 static int fmha_full(const void* q, int64_t q_batch_stride, int64_t q_row_stride, const dgpt_kv_layout* kv, const int32_t* kv_len,
                      int32_t kv_len_all, void* o, int64_t o_batch_stride, int64_t o_row_stride, int32_t o_f32, float* lse,
                      const void* egate, int64_t egate_rs, int32_t B, int32_t H, int32_t Tq, int32_t D, int32_t q_offset,
@@ -274,6 +295,11 @@ static int fmha_full(const void* q, int64_t q_batch_stride, int64_t q_row_stride
     return DGPT_E_UNSUPPORTED;
   }
   if (tc_ok && impl != 1) return fmha_tc(a, *kv, st);
+  if (egate && !simt_own_gate(a) && (B == 1 || o_batch_stride == (int64_t)Tq * o_row_stride)) {
+    a.egate = nullptr;
+    if (const int e = fmha_simt(a, view, st)) return e;
+    return dgpt_sigmoid_gate(o, o_row_stride, egate, egate_rs, (int64_t)B * Tq, H * D, dtype, stream);
+  }
   return fmha_simt(a, view, st);
 }
 
