@@ -270,10 +270,11 @@ static int fmha_full(const void* q, int64_t q_batch_stride, int64_t q_row_stride
   a.max_ctas = max_ctas;
   a.egate = egate; a.egate_rs = egate_rs;
   a.pingpong = impl == 4;
-  // Dense keys that are not whole tiles: the tensor cores from 24 keys on (8 to 512 pairs of sequence and head; at 17 keys 6.5 us
-  // against 5.3 / 9.3 / 11.7 us for heads of 32 / 64 / 128 on the warp-level kernel, at 33 keys 6.3 against 7.5 / 13.7 / 19, at 777
-  // keys 19 to 27 against 90 to 555; with one bf16 part per probability - the second part's product is a quarter of a tile's MMAs more).
-  a.any_run = impl == 0 && (causal ? (long long)Tq + q_offset : kv_len ? (long long)kv->page_tokens : (long long)kv_len_all) >= 24;
+  // Dense keys that are not whole tiles: the tensor cores from 24 keys on, heads of 32 from 33 (bf16, us, warp-level / tensor cores: heads of
+  // 64 x 24 keys, 4 to 2048 pairs of sequence and head, 9.3 to 82 / 7.3 to 51, of 128 12 to 129 / 8.8 to 62; of 32 x 24 3.6 to 40 / 7.2 to 50,
+  // x 40 10 to 64 / 7.1 to 49; 777 keys 90 to 555 / 19 to 27).
+  const long long dense_keys = causal ? (long long)Tq + q_offset : kv_len ? (long long)kv->page_tokens : (long long)kv_len_all;
+  a.any_run = impl == 0 && dense_keys >= (D == 32 ? 33 : 24);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const KvView view = make_view(kv);
   const bool tc_ok = fmha_tc_supported(a, *kv);
