@@ -272,9 +272,10 @@ static int fmha_full(const void* q, int64_t q_batch_stride, int64_t q_row_stride
   a.pingpong = impl == 4;
   // Dense keys that are not whole tiles: the tensor cores from 24 keys on, heads of 32 from 33 (bf16, us, warp-level / tensor cores: heads of
   // 64 x 24 keys, 4 to 2048 pairs of sequence and head, 9.3 to 82 / 7.3 to 51, of 128 12 to 129 / 8.8 to 62; of 32 x 24 3.6 to 40 / 7.2 to 50,
-  // x 40 10 to 64 / 7.1 to 49; 777 keys 90 to 555 / 19 to 27).
+  // x 40 10 to 64 / 7.1 to 49; 777 keys 90 to 555 / 19 to 27).  An output that is stored in fp32 would show that a probability there has
+  // 16 bits: it keeps the warp-level kernel.
   const long long dense_keys = causal ? (long long)Tq + q_offset : kv_len ? (long long)kv->page_tokens : (long long)kv_len_all;
-  a.any_run = impl == 0 && dense_keys >= (D == 32 ? 33 : 24);
+  a.any_run = impl == 0 && !o_f32 && dense_keys >= (D == 32 ? 33 : 24);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const KvView view = make_view(kv);
   const bool tc_ok = fmha_tc_supported(a, *kv);
