@@ -388,8 +388,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap ma, const __grid_constant__ C
                 lo = xielu_fast(lo, p.alpha, p.limit);
                 hi = xielu_fast(hi, p.alpha, p.limit);
               } else if constexpr (EPI == 6) {
-                lo = softcap_value<__nv_bfloat16>(Io<__nv_bfloat16>::round(lo), p.alpha);
-                hi = softcap_value<__nv_bfloat16>(Io<__nv_bfloat16>::round(hi), p.alpha);
+                lo = softcap_logit(Io<__nv_bfloat16>::round(lo), p.alpha);
+                hi = softcap_logit(Io<__nv_bfloat16>::round(hi), p.alpha);
               }
               w[k] = pack_bf16(lo, hi);
             }

@@ -102,8 +102,8 @@ __global__ void __launch_bounds__(32 * kGvWarps) gemv_kernel(const GemvParams p)
         lo = xielu_fast(lo, p.alpha, p.limit);
         hi = xielu_fast(hi, p.alpha, p.limit);
       } else if constexpr (EPI == 6) {
-        lo = softcap_value<__nv_bfloat16>(B::round(lo), p.alpha);
-        hi = softcap_value<__nv_bfloat16>(B::round(hi), p.alpha);
+        lo = softcap_logit(B::round(lo), p.alpha);
+        hi = softcap_logit(B::round(hi), p.alpha);
       }
       *reinterpret_cast<__nv_bfloat162*>(p.out + (long long)m * p.out_rs + 2 * pair) = __floats2bfloat162_rn(lo, hi);
     }
