@@ -156,32 +156,39 @@ struct MixRow {
     for (int x = 0; x < E; ++x) acc[x] = v[x];
     l = 1.f;
   }
+  // This lane's share of a . b, four running sums.  Where 16 lanes hold a row, each vector's sum is taken by itself and then added:
+  // vectors l and l + 16 are lane l's and lane l + 16's of a row held by 32, which a butterfly adds first.
+  __device__ __forceinline__ static float lanes(const float* a, const float* b) {
+    constexpr int kParts = LPR == 32 ? 1 : NV, kLen = E / kParts;
+    static_assert(LPR == 32 || (LPR == 16 && NV <= 2), "order of the sums");
+    float sum = 0.f;
+#pragma unroll
+    for (int i = 0; i < kParts; ++i) {
+      float s4[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int x = 0; x < kLen; ++x) s4[x & 3] += a[i * kLen + x] * b[i * kLen + x];
+      const float part = (s4[0] + s4[1]) + (s4[2] + s4[3]);
+      sum = i == 0 ? part : sum + part;
+    }
+    return sum;
+  }
   // logit = rms_norm(v) . w = rsqrt(mean(v^2) + eps) * (v . w): both sums in one sweep and one
   // interleaved butterfly.  (The reference rounds rms_norm(v) to the storage type before the
   // product; for bf16 that changes the logit by ~1e-4 of its own rounding step.)
   // A committed candidate does not change between mixes, so its norm factor is computed by the first mix that
-  // sees it and handed to the later ones: they skip the sum of squares and its half of the butterfly.  The
-  // factor is the same number either way (same code computed it), so results do not depend on the cache.
+  // sees it and handed to the later ones: they skip the sum of squares and its half of the butterfly.  Every form of the kernel
+  // adds in the order of 32 lanes a row (see `lanes`), so the factor is the same number whichever mix computed it, and results
+  // do not depend on the cache.
   // Returns the norm factor.
   __device__ __forceinline__ float add(const float* v, const float* wv, bool cached, float inv_cached, float mult, int C) {
-    float s4[4] = {0.f, 0.f, 0.f, 0.f}, d4[4] = {0.f, 0.f, 0.f, 0.f};
     float inv;
-    float dr;
+    float dr = lanes(v, wv);
     if (cached) {
-#pragma unroll
-      for (int x = 0; x < E; ++x) d4[x & 3] += v[x] * wv[x];
-      dr = (d4[0] + d4[1]) + (d4[2] + d4[3]);
 #pragma unroll
       for (int o = LPR / 2; o > 0; o >>= 1) dr += __shfl_xor_sync(0xffffffffu, dr, o);
       inv = inv_cached;
     } else {
-#pragma unroll
-      for (int x = 0; x < E; ++x) {
-        s4[x & 3] += v[x] * v[x];
-        d4[x & 3] += v[x] * wv[x];
-      }
-      float ss = (s4[0] + s4[1]) + (s4[2] + s4[3]);
-      dr = (d4[0] + d4[1]) + (d4[2] + d4[3]);
+      float ss = lanes(v, v);
 #pragma unroll
       for (int o = LPR / 2; o > 0; o >>= 1) {
         ss += __shfl_xor_sync(0xffffffffu, ss, o);
@@ -205,13 +212,9 @@ struct MixRow {
   }
   __device__ __forceinline__ void store(T* out_h, T* out_rn, long long row, int lane, int nvec, int C, bool row_ok = true) {
     const float invl = 1.f / l;
-    float s4[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-    for (int x = 0; x < E; ++x) {
-      acc[x] = Io<T>::round(acc[x] * invl);
-      s4[x & 3] += acc[x] * acc[x];
-    }
-    float ss = (s4[0] + s4[1]) + (s4[2] + s4[3]);
+    for (int x = 0; x < E; ++x) acc[x] = Io<T>::round(acc[x] * invl);
+    float ss = lanes(acc, acc);
 #pragma unroll
     for (int o = LPR / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
     const float inv = rsqrtf(ss / (float)C + kRmsEps);
