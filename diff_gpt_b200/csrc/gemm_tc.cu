@@ -249,6 +249,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap ma, const __grid_constant__ C
           }
         }
       }
+      // The commits of the last MMAs arrive on bar_empty, in a pair from the other SM: the CTA stays until they have.
+      for (int i = 0; ok && i < kStages; ++i)
+        if (last[i] >= 0) ok = wait_or_abort(bar_empty + 8 * i, (uint32_t)last[i], abort_flag, 36);
       if (!ok || *abort_flag) {
         if (p.status) atomicExch(p.status, *abort_flag ? *abort_flag : 32);
         if (rank == 0)
