@@ -133,6 +133,14 @@ __device__ __forceinline__ uint32_t in_leader(uint32_t addr) {  // the same shar
   asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(r) : "r"(addr));
   return r;
 }
+__device__ __forceinline__ uint32_t in_other(uint32_t addr, uint32_t rank) {  // and in the pair's other CTA
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank ^ 1u));
+  return r;
+}
+__device__ __forceinline__ void store_cluster(uint32_t addr, uint32_t v) {
+  asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
+}
 __device__ __forceinline__ void arrive_cluster(uint32_t bar) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
 }
@@ -180,6 +188,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap ma, const __grid_constant__ C
   uint64_t* bars = reinterpret_cast<uint64_t*>(staging + kGEpiWarps * kTileBytes);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 24);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  volatile uint32_t* loaded = tmem_slot + 2;  // in the leader: blocks that each CTA of the pair has asked for, once it has stopped
   const uint32_t a0 = smem_u32(smem);
   const uint32_t bar_full = smem_u32(bars), bar_empty = bar_full + 8 * kStages, bar_accf = bar_empty + 8 * kStages,
                  bar_acce = bar_accf + 16, bar_drain = bar_acce + 16;
@@ -193,6 +202,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap ma, const __grid_constant__ C
 
   if (tid == 0) {
     *abort_flag = 0;
+    loaded[0] = loaded[1] = 0;
     for (int i = 0; i < kStages; ++i) {
       mbar_init(bar_full + 8 * i, 1);
       mbar_init(bar_empty + 8 * i, 1);
@@ -229,7 +239,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap ma, const __grid_constant__ C
       int last[kStages];  // parity of the newest load per slot (for the drain on failure)
       for (int i = 0; i < kStages; ++i) last[i] = -1;
       int s = 0;
-      uint32_t ph = 0;
+      uint32_t ph = 0, blocks = 0;
       bool ok = true;
       for (int tile = worker; ok && tile < n_tiles; tile += workers) {
         const GemmTile t = gemm_tile(tile, tiles_m, tiles_n);
@@ -243,6 +253,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap ma, const __grid_constant__ C
           tma_load_2d<CG>(dst, &ma, full + 8 * s, kb * kGK, row);
           tma_load_2d<CG>(dst + kGABytes, &mw, full + 8 * s, kb * kGK, col);
           last[s] = (int)ph;
+          ++blocks;
           if (++s == kStages) {
             s = 0;
             ph ^= 1u;
@@ -254,10 +265,11 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap ma, const __grid_constant__ C
         if (last[i] >= 0) ok = wait_or_abort(bar_empty + 8 * i, (uint32_t)last[i], abort_flag, 36);
       if (!ok || *abort_flag) {
         if (p.status) atomicExch(p.status, *abort_flag ? *abort_flag : 32);
-        if (rank == 0)
+        if (CG == 1)
           for (int i = 0; i < kStages; ++i)
             if (last[i] >= 0) mbar_wait(bar_full + 8 * i, (uint32_t)last[i]);  // bounded: let copies in flight land
       }
+      if constexpr (CG == 2) store_cluster(in_leader(smem_u32(tmem_slot + 2) + 4 * rank), blocks);
     }
   } else if (warp == kGEpiWarps) {
     // ================= MMA issuer =================
@@ -442,7 +454,23 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap ma, const __grid_constant__ C
   }
   tc_fence_before();
   __syncwarp();
+  if (CG == 2 && lane == 0 && *abort_flag) store_cluster(in_other(smem_u32(tmem_slot + 1), rank), (uint32_t)*abort_flag);
+  __syncwarp();
   sync_ctas<CG>();  // no CTA of a pair leaves while the other may still signal it or read its operands
+  if (CG == 2 && *abort_flag) {  // the same in both CTAs: a wait has run out somewhere, and nobody issues copies any more
+    if (rank == 0 && tid == 0) {
+      // Both CTAs' copies report to the leader's barriers.  A slot's last block may have been asked for by the other CTA alone, one ahead
+      // at most (the next needs that one's MMAs): its phase is still to be opened.
+      for (uint32_t i = 0; i < (uint32_t)kStages; ++i) {
+        const uint32_t own = (loaded[0] + kStages - 1 - i) / kStages, other = (loaded[1] + kStages - 1 - i) / kStages;
+        if (other > own) mbar_expect_tx(bar_full + 8 * i, kStageBytes);
+        const uint32_t n = other > own ? other : own;
+        if (n > 0) mbar_wait(bar_full + 8 * i, (n - 1) & 1u);  // bounded
+      }
+    }
+    __syncwarp();
+    sync_ctas<CG>();
+  }
   if (warp == 0) {
     if constexpr (CG == 2) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
     else tmem_dealloc(tmem, 512);
