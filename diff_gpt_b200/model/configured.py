@@ -138,11 +138,14 @@ class ConfiguredModel(DeviceModel):
     def logits_at(self, idx, cache, rows):
         return self._step(idx, cache, rows)
 
+    def cache_storage(self, cache: RowCache) -> tuple:
+        return tuple(cache.store.values())
+
     def single_step(self, cache: RowCache, old: SingleStep | None, stream: torch.cuda.Stream) -> SingleStep:
         cache.ensure(1)
         # the key splits change from one 128-key tile to the next, until every window is full
         kind = (-(-min(cache.slot + 1, cache.keep + 1 + cache.keep_first) // 128),)
-        held = (self.packed_weights(), *cache.state.source.values(), *cache.store.values(), *self.step_tables(cache.pos + 1))
+        held = (self.packed_weights(), *cache.state.source.values(), *self.cache_storage(cache), *self.step_tables(cache.pos + 1))
         if old is not None and old.fits(kind, held):
             return old
         with torch.cuda.stream(stream):

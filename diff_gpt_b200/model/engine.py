@@ -512,9 +512,11 @@ class StepRunner:
     A single token whose logits are wanted is a hundred launches of a few microseconds each, which take the host three times
     as long as the GPU (Kipolix, 8 layers: 1.4 ms a token, of which the GPU was busy 0.4).  So the second such step of a
     cache records its launches as a graph, and the following ones replay it until something that the launches were made for
-    changes: the weights, the cache's storage or state buffer, the key splits, the numbers a GPT carries (soft-cap, SwiGLU).  All of them run on one stream of the runner,
-    between two waits with the caller's, so that requests stepped from several streams never share cuBLAS's workspace at
-    the same time.
+    changes: the weights, the cache's storage or state buffer, the key splits, the numbers a GPT carries (soft-cap, SwiGLU).
+    A cache has two recordings at most (a GPT's one), and there are as many caches as requests were live at one time; a
+    recording that holds replaced weights or outgrown storage goes with the next step.  All of them run on one stream of the
+    runner, between two waits with the caller's, so that requests stepped from several streams never share cuBLAS's workspace
+    at the same time.
 
     Different requests may be stepped from different threads: one thread at a time enqueues on the runner's stream (what
     another put there meanwhile would be recorded instead of run), and a thread records only after it has run a step
@@ -551,7 +553,20 @@ class StepRunner:
         dev = self.model.embedding.device
         idx = torch.tensor([tokens], dtype=torch.int64, device=dev)
         rows = torch.tensor(want, dtype=torch.int64, device=dev)
-        return self.model.logits_at(idx, cache, rows).to(torch.float32, copy=True)
+        out = self.model.logits_at(idx, cache, rows).to(torch.float32, copy=True)
+        if self._single:
+            with self._lock:
+                self._drop_stale(cache)
+        return out
+
+    def _drop_stale(self, cache) -> None:
+        """Let go of what recordings hold that nothing else does any more: replaced weights, and storage that `cache` has outgrown."""
+        weights, storage = self.model.last_packed, self.model.cache_storage(cache)
+        stale = [k for k, one in self._single.items() if not one.current(weights, storage if k[0] is cache else ())]
+        if stale:
+            self._stream.synchronize()  # their memory belongs to other streams
+        for key in stale:
+            del self._single[key]
 
     def _one(self, cache, token: int) -> torch.Tensor | None:
         with self._lock:
@@ -565,10 +580,13 @@ class StepRunner:
         key = (cache, 0 if state is None else state.current)  # a portion of several tokens changes the buffer
         if self._stream is None:
             self._stream = torch.cuda.Stream(device=self.model.embedding.device)
-        one = self.model.single_step(cache, self._single.get(key), self._stream)
+        old = self._single.get(key)
+        one = self.model.single_step(cache, old, self._stream)
         if one is None:
             return None, None
-        self._single[key] = one
+        if one is not old:
+            self._drop_stale(cache)
+            self._single[key] = one
         caller, mine = torch.cuda.current_stream(), self._stream
         mine.wait_stream(caller)
         with torch.cuda.stream(mine):

@@ -75,6 +75,11 @@ class DeviceModel(BaseGPT):
         """Weights as the kernels want them, `head` [V, C] (the output head; the token table where they are tied) among
         them; the same object until a parameter is modified or moved."""
 
+    @property
+    def last_packed(self):
+        """What `packed_weights` gave last, without a look at the parameters."""
+        return self._packed
+
     # -- requests fed step by step --
     @abstractmethod
     def new_cache(self, batch_size: int = 1, seq_len: int = 0):
@@ -97,6 +102,10 @@ class DeviceModel(BaseGPT):
             if getattr(type(self), name) is not getattr(cls, name) or name in self.__dict__:
                 return False
         return bool(self.step_path)
+
+    def cache_storage(self, cache) -> tuple:
+        """The tensors of a cache from `new_cache` that are replaced when it grows."""
+        return ()
 
     def single_step(self, cache, old: "SingleStep | None", stream: torch.cuda.Stream) -> "SingleStep | None":
         """The launches of one more token behind `cache`, which has room for it afterwards: `old` where it still fits, or None
@@ -203,7 +212,7 @@ class SingleStep:
     position, keys), so that the launches can be recorded once and replayed.
 
     kind    host-side choices and numbers that the launches were made with (key splits, soft-cap, ...)
-    held    what the launches point at; kept alive here and compared by `is`
+    held    what the launches point at, the packed weights first; kept alive here and compared by `is`
     """
 
     plan: object
@@ -218,6 +227,10 @@ class SingleStep:
 
     def fits(self, kind: tuple, held: tuple) -> bool:
         return self.kind == kind and len(self.held) == len(held) and all(a is b for a, b in zip(self.held, held))
+
+    def current(self, weights, storage: tuple) -> bool:
+        """Whether it still holds these weights, and this storage of its cache."""
+        return self.held[0] is weights and all(any(t is h for h in self.held) for t in storage)
 
     def enqueue(self) -> None:
         self.plan.run(self.numbers[0:1], self.bind)
@@ -610,6 +623,9 @@ class GPT(DeviceModel):
         return KVCache(batch_size=batch_size, num_heads=self.n_head, seq_len=max(seq_len, 1),
                        head_dim=self.n_embd // self.n_head, num_layers=self.n_layer)
 
+    def cache_storage(self, cache: KVCache) -> tuple:
+        return (cache.kv_cache,)
+
     @torch.inference_mode()
     def logits_at(self, idx: torch.Tensor, cache: KVCache, rows: torch.Tensor) -> torch.Tensor:
         return self(idx, kv_cache=cache)[0][0].index_select(0, rows)
@@ -622,7 +638,7 @@ class GPT(DeviceModel):
         cache.ensure(t0 + 1, emb.dtype, emb.device)
         splits = _pick_splits(H, t0 + 1)
         kind = (splits, self.logit_softcap, self.swiglu_alpha, self.swiglu_limit, self.attn_res_layers_per_block)
-        held = (self.packed_weights(), cache.kv_cache)
+        held = (self.packed_weights(), *self.cache_storage(cache))
         if old is not None and old.fits(kind, held):
             return old
         with torch.cuda.stream(stream):

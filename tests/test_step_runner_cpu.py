@@ -1,8 +1,10 @@
 """StepRunner's host logic without a GPU: streams, graphs and the model are stand-ins that note who is inside."""
 
 import contextlib
+import gc
 import threading
 import time
+import weakref
 from types import SimpleNamespace
 
 import pytest
@@ -12,6 +14,10 @@ import torch
 class _Logits:
     def to(self, *a, **k):
         return SimpleNamespace(record_stream=lambda s: None)
+
+
+class _Storage:
+    """Stands for a cache's tensor, or for packed weights."""
 
 
 class _Busy:
@@ -40,7 +46,7 @@ def cuda(monkeypatch):
         def replay(self):
             pass
 
-    stream = SimpleNamespace(wait_stream=lambda other: None)
+    stream = SimpleNamespace(wait_stream=lambda other: None, synchronize=lambda: None)
     monkeypatch.setattr(torch.cuda, "Stream", lambda **k: stream)
     monkeypatch.setattr(torch.cuda, "current_stream", lambda *a: stream)
     monkeypatch.setattr(torch.cuda, "stream", lambda s: contextlib.nullcontext())
@@ -51,6 +57,9 @@ def _model(busy):
     from diff_gpt_b200.model.gpt import SingleStep
 
     class Cache:
+        def __init__(self):
+            self.storage = _Storage()
+
         def reset(self):
             self.pos = 0
 
@@ -63,14 +72,27 @@ def _model(busy):
     class Model:
         vocab_size, embedding = 8, torch.zeros(1)
 
+        def __init__(self):
+            self.last_packed = _Storage()
+
         def new_cache(self):
             return Cache()
 
         def single_step_allowed(self):
             return True
 
+        def cache_storage(self, cache):
+            return (cache.storage,)
+
         def single_step(self, cache, old, stream):
-            return old or SingleStep(Plan(), None, torch.zeros(4, dtype=torch.int32), 0, (), checks=False)
+            held = (self.last_packed, cache.storage)
+            if old is not None and old.fits((0,), held):
+                return old
+            return SingleStep(Plan(), None, torch.zeros(4, dtype=torch.int32), (0,), held, checks=False)
+
+        def logits_at(self, idx, cache, rows):
+            cache.pos += idx.shape[1]
+            return torch.zeros(rows.numel(), 8)
 
     return Model()
 
@@ -152,3 +174,22 @@ def test_replaced_methods_and_hooks_keep_the_general_path():
     m = other.from_config(cfg)
     m.register_forward_hook(lambda *a: None)
     assert m.single_step_allowed()
+
+
+@pytest.mark.parametrize("tokens", [[1], [1, 2, 3]])
+def test_replaced_weights_and_outgrown_storage_are_let_go(cuda, tokens):
+    """By the next step, a single token or a portion: the storage of that request's cache, and the weights that every recording held."""
+    from diff_gpt_b200 import StepRunner
+
+    model = _model(_Busy())
+    runner = StepRunner(model)
+    for r in ("a", "b"):
+        for _ in range(3):
+            runner.step(r, [1], [0])
+    cache = runner._live["a"]
+    storage, weights = weakref.ref(cache.storage), weakref.ref(model.last_packed)
+    cache.storage, model.last_packed = _Storage(), _Storage()
+    runner.step("a", tokens, [0])
+    gc.collect()
+    assert storage() is None and weights() is None
+    assert all(one.held[0] is model.last_packed for one in runner._single.values())
