@@ -34,7 +34,7 @@ struct FmhaArgs {
   // Probabilities as a bf16 pair, high and low part: two-CTAs-per-SM kernel only, for calls whose other route is the warp-level kernel
   // with its probabilities in fp32
   int split_p = 0;
-  int any_run = 0;  // the tensor-core kernels may take dense keys of any length, not only whole tiles (impl 0)
+  int any_run = 0;  // the tensor-core kernels may take dense keys of any length, not only whole tiles (impl 0, output not fp32)
 };
 
 // What the tensor-core kernels need besides the three tensor maps.

@@ -13,9 +13,9 @@
 //            (no noise and T = 1 for an arg-max) in best[m], a 64-bit word (order-preserving key bits, ~n) raised with
 //            atomicMax - the tied-embedding head with the draw in its epilogue, so [M, N] logits never reach HBM
 //
-// Persistent, warp-specialised CTAs of 320 threads, one per SM.  A tile is 128 CG x BN outputs, made by one CTA (CG = 1) or by a
-// CTA pair (CG = 2: one tcgen05.mma of M = 256 over both SMs; each CTA stages its 128 rows of A and half of the W rows, so a
-// pair reads W once where two single CTAs read it twice).  Tiles are taken round robin, eight rows of tiles at a time, so that
+// Persistent, warp-specialised CTAs of 576 threads, one per SM.  A tile is 128 CG x BN outputs, made by one CTA (CG = 1, BN = 64 to 256)
+// or by a CTA pair (CG = 2, BN = 128 to 256: one tcgen05.mma of M = 256 over both SMs; each CTA stages its 128 rows of A and half of the W
+// rows, so a pair reads W once where two single CTAs read it twice).  Tiles are taken round robin, eight rows of tiles at a time, so that
 // what is in flight shares both operands in L2:
 //   warp 17, lane 0 loader: TMA loads of the A and W blocks (64 of K), 128-byte swizzle, a ring of up to 8 stages; both CTAs of a
 //                   pair report their bytes to the leader's barrier

@@ -13,8 +13,9 @@ reference names and shapes; the arithmetic of a forward pass is enqueued by
     attention (+gate) -> out-proj GEMM -> depth-mix+rmsnorm -> FFN GEMM -> swiglu ->
     FFN GEMM (+residual)] x L -> rmsnorm -> tied-embedding GEMM -> soft-cap
 
-with the GEMMs on cuBLAS (torch.mm / addmm_) and everything else in this
-library.  There is no CPU implementation: CPU tensors raise.
+Large bf16 products without an epilogue, and large fp32 ones, are on cuBLAS (torch.mm / addmm_).  The bf16 head and feed-forward
+up projection, products of one bf16 row, those of small fp32 models (`own_f32`) and everything else are this library's.
+There is no CPU implementation: CPU tensors raise.
 """
 
 from __future__ import annotations
@@ -314,7 +315,7 @@ class ForwardPlan:
         self.xn = buf(n_out, C)
         self.last = buf(n_out, C) if (last_only and T > 1) else None
         self.logits = buf(n_out, V) if want_logits else None
-        # the tied-embedding head on the library's tcgen05 GEMM (bf16 with tileable sizes); fp32 stays on cuBLAS
+        # the tied-embedding head on the library's tcgen05 GEMM (bf16 with tileable sizes); fp32: see own_f32
         self.own_head = dt == torch.bfloat16 and C % 8 == 0 and V % 16 == 0
         self.cap = cap
         self.status = torch.zeros(1, dtype=torch.int32, device=dev)

@@ -118,9 +118,11 @@ int dgpt_rope_qknorm_kvappend(const void* q, const void* k, const void* v, int64
  * in that mode `o` may be requested in fp32 (o_f32 != 0) regardless of `dtype`.
  * q: device, element (b,i,h,d) at b*q_batch_stride + i*q_row_stride + h*D + d;  o likewise.
  * kv: sequence index = b;  kv_len: device int32 [B] or NULL (then kv_len_all is used).
- * impl: 0 = choose (bf16 with D = 64 or 128 runs on the tcgen05 tensor cores, everything else takes
- * the warp-level online-softmax kernel; of the two tensor-core kernels the warp-specialised one is taken
- * from 1024 keys on, the two-CTAs-per-SM one below), 1 = warp-level kernel, 2 = warp-specialised
+ * impl: 0 = choose (bf16 with D = 32, 64 or 128 and whole tiles of 128 keys, or pages that make them up, runs on the tcgen05
+ * tensor cores: the warp-specialised kernel from 640 keys on and where one CTA per SM holds every query tile, the two-CTAs-per-SM
+ * one otherwise.  Dense keys of any other length run on the two-CTAs-per-SM one with each probability as a pair of bf16 numbers,
+ * from 24 keys on (D = 32: 33) and unless the output is fp32.  Everything else takes the warp-level online-softmax kernel),
+ * 1 = warp-level kernel, 2 = warp-specialised
  * tensor-core kernel or fail, 3 = tensor-core kernel with two CTAs per SM or fail, 4 = persistent tensor-core kernel
  * with two query tiles per CTA or fail.
  * max_ctas: 0, or a cap on the CTAs of the two-CTAs-per-SM kernel, which then loop over the query tiles - for a
@@ -134,8 +136,10 @@ int dgpt_fmha_prefill(const void* q, int64_t q_batch_stride, int64_t q_row_strid
 
 /* dgpt_fmha_prefill with the output gate of src/diff_gpt/model/mha.py:84 applied where the output is stored:
  *   o[b,i,h,:] = round(o[b,i,h,:]) * round(sigmoid(gate[b*Tq + i, h*D + :])),   round = to `dtype`
- * which is what dgpt_fmha_prefill followed by dgpt_sigmoid_gate gives, bit for bit, without the second pass.
- * gate: device [B * Tq, H * D] in `dtype` with gate_row_stride (elements); impl 4 is not built with a gate. */
+ * which is what dgpt_fmha_prefill followed by dgpt_sigmoid_gate gives: bit for bit in fp32; in bf16 except where the sigmoid lies
+ * within 2e-7 of a rounding boundary.  The second pass is saved, but for short fp32 rows, where it is the faster way.
+ * gate: device [B * Tq, H * D] in `dtype` with gate_row_stride (elements).  The tensor-core kernels want it 16-byte aligned with a
+ * stride that is a multiple of 8 (impl 0 takes the warp-level kernel otherwise); impl 4 is not built with a gate. */
 int dgpt_fmha_prefill_gated(const void* q, int64_t q_batch_stride, int64_t q_row_stride, const dgpt_kv_layout* kv,
                             const int32_t* kv_len, int32_t kv_len_all, void* o, int64_t o_batch_stride, int64_t o_row_stride,
                             const void* gate, int64_t gate_row_stride, int32_t B, int32_t H, int32_t Tq, int32_t D,
@@ -235,7 +239,8 @@ int dgpt_linear_f32(const float* a, int64_t a_row_stride, const float* w, int64_
  *   epilogue 2:  out[m, n]     = resid[m, n] + acc[m, n], rounded once (resid may be out itself)   out: [M, N]
  *   epilogue 4:  out[m, n]     = xielu(acc[m, n]) with alpha_p = alpha, alpha_n = limit (see dgpt_xielu)   out: [M, N]
  *   epilogue 5:  out[m, n / 2] = silu(acc[m, n]) * acc[m, n + 1] for even n, from the unrounded accumulator     out: [M, N / 2]
- *   epilogue 6:  out[m, n]     = alpha * tanh(acc[m, n] / alpha), the rule of dgpt_softcap with cap = alpha > 0   out: [M, N]
+ *   epilogue 6:  out[m, n]     = alpha * tanh(acc[m, n] / alpha), the rule of dgpt_softcap with cap = alpha > 0 (the tangent within 4e-6 of its
+ *                value before it is rounded)   out: [M, N]
  * Replaces nn.Linear of src/diff_gpt/model/feed_forward.py:10-14 followed by swi_glu.py:11-19 (epilogue 1), any
  * bias-free nn.Linear of the path (epilogue 0), or a projection with the residual add that follows it
  * (src/diff_gpt/model/block.py:98-106, epilogue 2).  resid is ignored for epilogues 0, 1, 4, 5 and 6.  bf16 only; pointers 16-byte aligned, K and the row strides
