@@ -195,7 +195,9 @@ static int fmha_simt_launch(const FmhaArgs& a, const KvView& kv, cudaStream_t st
   // queries, 4 heads of 16, 89 keys 10.0 -> 4.4 and 10.6 -> 5.7; 300 x 300, 8 heads of 32, 58 -> 17; 4000 queries, 128 CTAs, 11.3
   // either way.)
   const long long ctas = (long long)a.B * a.H * ((a.Tq + 128 / SPLIT - 1) / (128 / SPLIT));
-  if (KEYS > 1 && ctas <= 74) DGPT_SIMT(1, KEYS);
+  // Not in bf16 where the log-sum-exp is asked for too (the prompt a batch of rows shares): the order of its sums would follow the
+  // number of rows, and a shard of the batch is to give what the whole gives.
+  if (KEYS > 1 && ctas <= 74 && !(sizeof(T) == 2 && a.lse)) DGPT_SIMT(1, KEYS);
   else DGPT_SIMT(SPLIT, 1);
 #undef DGPT_SIMT
   return launch_status("fmha_simt");
@@ -291,7 +293,8 @@ static int fmha_full(const void* q, int64_t q_batch_stride, int64_t q_row_stride
   // pair, 0.0035 with one bf16; the whole layer 337 us there, 66 with the pair (1 x 8 heads x 8191: 3896 and 300; 2 x 16 heads of 128 x 1500:
   // 1669 and 89).
   a.split_p = a.any_run && kv->page_table == nullptr && kv->page_tokens % 128 != 0;
-  a.two_cta = impl == 3 || a.split_p || (impl == 0 && span < 640 && !fmha_one_round(a));
+  // (With a log-sum-exp the number of rows is no reason: see fmha_simt_launch.)
+  a.two_cta = impl == 3 || a.split_p || (impl == 0 && span < 640 && (lse || !fmha_one_round(a)));
   if (impl >= 2 && !tc_ok) {
     set_error("fmha_prefill: the tensor-core kernel does not cover dtype %d, head_dim %d with this layout", dtype, D);
     return DGPT_E_UNSUPPORTED;

@@ -616,7 +616,7 @@ extern "C" int dgpt_bounded_wait_probe(int32_t arrive, int64_t limit_cycles, int
 int dgpt::linear_launch(const void* a, int64_t a_row_stride, const void* w, int64_t w_row_stride, void* out,
                         int64_t out_row_stride, const void* resid, int64_t resid_row_stride, int32_t M, int32_t N,
                         int32_t K, int32_t epilogue, float alpha, float limit, int32_t dtype, int32_t* status,
-                        const HeadDraw* draw, void* stream) {
+                        const HeadDraw* draw, bool tiles, void* stream) {
   DGPT_REQUIRE(a && w && (out || epilogue == 3), "linear: NULL pointer");
   DGPT_REQUIRE(M >= 0 && N > 0 && K > 0, "linear: bad sizes");
   DGPT_REQUIRE(epilogue >= 0 && epilogue <= 6,
@@ -641,7 +641,7 @@ int dgpt::linear_launch(const void* a, int64_t a_row_stride, const void* w, int6
     return DGPT_E_UNSUPPORTED;
   }
   // The rows of W are read once either way, and nothing waits for tiles (16384 x 1024 in us: one row 13.0 -> 8.0, two 10.3, four 13.2).
-  if (M <= kGemvMaxRows && epilogue != 3)
+  if (M <= kGemvMaxRows && epilogue != 3 && !tiles)
     return gemv_launch(a, a_row_stride, w, w_row_stride, out, out_row_stride, resid, resid_row_stride, M, N, K, epilogue, alpha, limit,
                        static_cast<cudaStream_t>(stream));
   static int n_sm[64] = {};
@@ -683,8 +683,10 @@ extern "C" int dgpt_linear(const void* a, int64_t a_row_stride, const void* w, i
                            int64_t out_row_stride, const void* resid, int64_t resid_row_stride, int32_t M, int32_t N,
                            int32_t K, int32_t epilogue, float alpha, float limit, int32_t dtype, int32_t* status,
                            void* stream) {
+  const bool tiles = epilogue >= 0 && (epilogue & DGPT_LINEAR_TILES) != 0;
+  if (tiles) epilogue &= ~DGPT_LINEAR_TILES;
   DGPT_REQUIRE(epilogue >= 0 && epilogue <= 6 && epilogue != 3,
                "linear: epilogue must be 0 (store), 1 (SwiGLU of interleaved pairs), 2 (add), 4 (xIELU), 5 (SiLU gate) or 6 (soft-cap)");
   return linear_launch(a, a_row_stride, w, w_row_stride, out, out_row_stride, resid, resid_row_stride, M, N, K, epilogue, alpha,
-                       limit, dtype, status, nullptr, stream);
+                       limit, dtype, status, nullptr, tiles, stream);
 }

@@ -17,11 +17,12 @@ struct HeadDraw {
   unsigned long long* best = nullptr;   // [M], zero before the launch
 };
 
-// dgpt_linear with the fourth epilogue reachable (draw != nullptr, epilogue == 3, out may be NULL).
+// dgpt_linear with the fourth epilogue reachable (draw != nullptr, epilogue == 3, out may be NULL).  `tiles`: no kernel of its own for
+// one or two rows.
 int linear_launch(const void* a, int64_t a_row_stride, const void* w, int64_t w_row_stride, void* out,
                   int64_t out_row_stride, const void* resid, int64_t resid_row_stride, int32_t M, int32_t N, int32_t K,
                   int32_t epilogue, float alpha, float limit, int32_t dtype, int32_t* status, const HeadDraw* draw,
-                  void* stream);
+                  bool tiles, void* stream);
 
 // One or two rows, every epilogue but the draw (gemv.cu); the arguments have passed linear_launch's checks.
 constexpr int kGemvMaxRows = 2;

@@ -53,8 +53,9 @@ extern "C" int dgpt_lmhead_sample(const void* xn, int64_t xn_row_stride, const v
   const bool nucleus = top_p < 1.f && temperature > 0.f;
   if (nucleus || logits_out) {
     DGPT_REQUIRE(logits_out, "lmhead_sample: a top-p filter needs the logits buffer (a row's whole distribution)");
+    // tiles for every number of rows: a shard of a batch draws from the logits that the whole would have
     if (int e = linear_launch(xn, xn_row_stride, emb, emb_row_stride, logits_out, logits_row_stride, nullptr, 0, R, V, C, 0,
-                              0.f, 0.f, dtype, status, nullptr, stream))
+                              0.f, 0.f, dtype, status, nullptr, true, stream))
       return e;
     return dgpt_sample(logits_out, logits_row_stride, R, V, cap, temperature, top_p, seed, traj_id0, traj_ids, step_base,
                        step_ptr, force_schedule, force_group_rows, force_group_stride, out_tokens, out_masks,
@@ -80,7 +81,7 @@ extern "C" int dgpt_lmhead_sample(const void* xn, int64_t xn_row_stride, const v
   d.step_ptr = step_ptr;
   d.best = static_cast<unsigned long long*>(workspace);
   if (int e = linear_launch(xn, xn_row_stride, emb, emb_row_stride, nullptr, 0, nullptr, 0, R, V, C, 3, 0.f, 0.f, dtype, status,
-                            &d, stream))
+                            &d, true, stream))
     return e;
   const int fg = force_group_rows > 0 ? force_group_rows : 1;
   head_finish_kernel<<<(R + 255) / 256, 256, 0, st>>>(d.best, R, step_ptr, force_schedule, fg, force_group_stride, out_tokens,

@@ -144,7 +144,7 @@ class DiffGPT:
         S, _rows, columns = values.shape
         tokens, state, scale, orders_dev = self._encode_on_device(values)
         prompts = tokens.reshape(S, -1)  # row-major: (time, channel)
-        generated, _ = self._get_engine().generate_many(prompts, num_samples, max_new_points * columns, sampler)
+        generated, _ = self._get_engine().generate_many(prompts, num_samples, max_new_points * columns, sampler, whole_job=True)
         V = self.model.vocab_size
         out = torch.empty((S, num_samples, max_new_points, columns), dtype=torch.float64, device=generated.device)
         for s in range(S):

@@ -31,10 +31,10 @@ def fp32_reductions():
         m.allow_bf16_reduced_precision_reduction = was
 
 
-def linear(a: torch.Tensor, w_t: torch.Tensor, out: torch.Tensor, name: str, status: torch.Tensor) -> None:
-    """out = a @ w_t, on cuBLAS but for a single bf16 row (dgpt_linear, us: 1024 x 1024 4.8 -> 2.3, 1024 x 2736 8.1 -> 3.4)."""
+def linear(a: torch.Tensor, w_t: torch.Tensor, out: torch.Tensor, name: str, status: torch.Tensor, few_rows: bool = True) -> None:
+    """out = a @ w_t, on cuBLAS but (with `few_rows`) for a single bf16 row (dgpt_linear, us: 1024 x 1024 4.8 -> 2.3, 1024 x 2736 8.1 -> 3.4)."""
     K, N = w_t.shape
-    if a.shape[0] == 1 and a.dtype == torch.bfloat16 and K % 8 == 0 and N % 16 == 0 and ops.rows16(w_t.t()):
+    if few_rows and a.shape[0] == 1 and a.dtype == torch.bfloat16 and K % 8 == 0 and N % 16 == 0 and ops.rows16(w_t.t()):
         ops.linear(a, w_t.t(), out, status=status)
         return
     with region(name):

@@ -200,8 +200,9 @@ class DelunexPlan:
     """Buffers for one (n_seq, T) forward and the launch sequence that fills them (see `ForwardPlan`)."""
 
     def __init__(self, model: "Delunex", n_seq: int, T: int, last_only: bool = False, want_logits: bool = True,
-                 rows: int | None = None) -> None:
-        """`rows`: the number of rows whose logits are asked for by index at each run (overrides last_only)."""
+                 rows: int | None = None, few_rows: bool = True) -> None:
+        """`rows`: the number of rows whose logits are asked for by index at each run (overrides last_only).  `few_rows`: see
+        `DeviceModel.prefill_plan`."""
         cfg, emb = model.config, model.embedding
         self.model, self.n_seq, self.T, self.n = model, n_seq, T, n_seq * T
         self.dev, self.dt = emb.device, emb.dtype
@@ -219,7 +220,8 @@ class DelunexPlan:
         self.xn = torch.empty((n_out, C), dtype=self.dt, device=self.dev)
         self.logits = torch.empty((n_out, V), dtype=self.dt, device=self.dev) if want_logits else None
         self.own_head = self.dt == torch.bfloat16 and C % 8 == 0 and V % 16 == 0
-        self.fused_ff = self.dt == torch.bfloat16 and C % 8 == 0 and (n >= FUSED_FF_MIN_ROWS or n == 1)
+        self.few_rows = few_rows
+        self.fused_ff = self.dt == torch.bfloat16 and C % 8 == 0 and (n >= FUSED_FF_MIN_ROWS or (few_rows and n == 1))
         self.status = torch.zeros(1, dtype=torch.int32, device=self.dev)
 
     def _buf(self, name: str, *shape: int, dtype=None) -> torch.Tensor:
@@ -240,7 +242,7 @@ class DelunexPlan:
         """self.y = mixer(self.h)"""
         n, n_seq, T, H, D, r = self.n, self.n_seq, self.T, lw.H, lw.D, lw.r
         proj = self._buf("proj", n, lw.w_in_t.shape[1])
-        linear(self.h, lw.w_in_t, proj, "gemm_in", self.status)
+        linear(self.h, lw.w_in_t, proj, "gemm_in", self.status, self.few_rows)
         q, gate = proj[:, : H * D], proj[:, lw.gate_col : lw.gate_col + H]
         if lw.owner == i:
             ops.latent_append(
@@ -272,7 +274,7 @@ class DelunexPlan:
             )
             with region("gemm_absorb"):
                 torch.bmm(oa.view(n, H, r).transpose(0, 1), lw.w_uv_t, out=o.view(n, H, D).transpose(0, 1))
-        linear(o, lw.w_o_t, self.y, "gemm_proj", self.status)
+        linear(o, lw.w_o_t, self.y, "gemm_proj", self.status, self.few_rows)
 
     def _feed_forward(self, lw: _PackedLayer) -> None:
         """self.y = W_down xielu(W_up self.u)"""
@@ -285,7 +287,7 @@ class DelunexPlan:
             with region("gemm_up"):
                 torch.mm(self.u, lw.w_up.t(), out=up)
             ops.xielu(up, act, *lw.act)
-        linear(act, lw.w_down_t, self.y, "gemm_down", self.status)
+        linear(act, lw.w_down_t, self.y, "gemm_down", self.status, self.few_rows)
 
     def run(self, ids32: torch.Tensor, b: LatentBinding, rows: torch.Tensor | None = None,
             tap: Callable[[int, torch.Tensor], None] | None = None) -> torch.Tensor | None:
@@ -333,7 +335,7 @@ class DelunexPlan:
         if self.logits is None:
             return None
         if self.own_head:
-            ops.linear(self.xn, W.emb, self.logits, status=self.status)
+            ops.linear(self.xn, W.emb, self.logits, tiles=not self.few_rows, status=self.status)
         else:
             with region("gemm_logits"):
                 torch.mm(self.xn, W.emb.t(), out=self.logits)
@@ -411,7 +413,7 @@ class Delunex(ConfiguredModel):
         return PagedLatentCache(self.ranks, self.keep, self.n_layer, self.config.taps, self.n_embd, n_series, rows_per_series,
                                 prefix_len, max_new, emb.dtype, emb.device, page_tokens=page_tokens)
 
-    def prefill_plan(self, cache, members, P, fmha_impl):
+    def prefill_plan(self, cache, members, P, fmha_impl, few_rows=True):
         dev = cache.prefix_table.device
         n = len(members)
         table = cache.prefix_table[torch.tensor(members, device=dev)].contiguous()
@@ -422,9 +424,9 @@ class Delunex(ConfiguredModel):
             layout=layouts.__getitem__, slot0=zero, start1=zero, len1=torch.ones(n, dtype=torch.int32, device=dev), keys=P,
             expand=True, conv_in=states if P == 1 else None, conv_out=states, fmha_impl=fmha_impl if fmha_impl <= 3 else 0,
         )
-        return bind, DelunexPlan(self, n, P, last_only=True)
+        return bind, DelunexPlan(self, n, P, last_only=True, few_rows=few_rows)
 
-    def decode_plan(self, cache, prompt_lens, max_keys, step, shared, fmha_impl, overlap_prefix, want_logits):
+    def decode_plan(self, cache, prompt_lens, max_keys, step, shared, fmha_impl, overlap_prefix, want_logits, few_rows=True):
         R, dev = cache.n_rows, prompt_lens.device
         slot0 = torch.full((R,), cache.suffix_slot0, dtype=torch.int32, device=dev)
         layouts = {layer: cache.layout(layer, cache.row_table) for layer in self.ranks}
@@ -432,7 +434,7 @@ class Delunex(ConfiguredModel):
             layout=layouts.__getitem__, slot0=slot0, start1=slot0, len0=prompt_lens.repeat_interleave(cache.rows_per_series).contiguous(),
             len1=torch.ones(R, dtype=torch.int32, device=dev), step=step, keys=max_keys, conv_in=cache.rows, conv_out=cache.rows,
         )
-        return bind, DelunexPlan(self, R, 1, want_logits=want_logits)
+        return bind, DelunexPlan(self, R, 1, want_logits=want_logits, few_rows=few_rows)
 
     def new_plan(self, n_seq, T, **kw) -> DelunexPlan:
         return DelunexPlan(self, n_seq, T, **kw)

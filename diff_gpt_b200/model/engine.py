@@ -52,13 +52,13 @@ class DecodeRun:
 
     @staticmethod
     def key_for(model, prompt_lens, num_samples, max_tokens, sampler, seed, has_force, page_tokens, use_graph,
-                fmha_impl, overlap_prefix, shared_prefix=None, fused_head=True, prefill_shared=False) -> tuple:
+                fmha_impl, overlap_prefix, shared_prefix=None, fused_head=True, prefill_shared=False, whole_job=True) -> tuple:
         spec = (1.0, 1.0) if sampler is None else (sampler.native_spec() if isinstance(sampler, Sampler) else None)
         emb = model.embedding
         return (
             id(model), str(emb.device), emb.dtype, tuple(prompt_lens), num_samples, max_tokens, spec,
             None if spec is not None else id(sampler), seed, has_force, page_tokens, use_graph, fmha_impl,
-            overlap_prefix, shared_prefix, fused_head, prefill_shared,
+            overlap_prefix, shared_prefix, fused_head, prefill_shared, whole_job,
         )
 
     def __init__(
@@ -80,7 +80,9 @@ class DecodeRun:
         shared_prefix: bool | None = None,
         fused_head: bool = True,
         prefill_group=None,
+        whole_job: bool = True,
     ) -> None:
+        """`whole_job`: False for what may be a shard: no kernels whose bf16 sums are ordered otherwise for one or two rows."""
         self.model = model
         emb = model.embedding
         if not emb.is_cuda:
@@ -103,7 +105,7 @@ class DecodeRun:
         self.prompt_lens = lens
         self.key = self.key_for(
             model, lens, N, G, sampler, seed, force_schedules is not None, page_tokens, use_graph, fmha_impl,
-            overlap_prefix, shared_prefix, fused_head, prefill_group is not None,
+            overlap_prefix, shared_prefix, fused_head, prefill_group is not None, whole_job,
         )
         self.packed = model.packed_weights()  # the graph holds these tensors' addresses
         self.cache = model.paged_cache(S, N, max(lens), G, page_tokens, kv_pool)
@@ -137,7 +139,7 @@ class DecodeRun:
                 groups.setdefault(n, []).append(s)
         self.prefills = []
         for P, members in groups.items():
-            bind, plan = model.prefill_plan(self.cache, members, P, fmha_impl)
+            bind, plan = model.prefill_plan(self.cache, members, P, fmha_impl, few_rows=whole_job)
             self.prefills.append((P, members, torch.tensor(members, device=dev), bind, plan))
 
         # ---- decode plan ----
@@ -159,7 +161,8 @@ class DecodeRun:
             else:
                 self.head_ws = torch.empty(max(1, ops.lmhead_workspace_bytes(self.R) // 8), dtype=torch.int64, device=dev)
         self.bind, self.plan = model.decode_plan(
-            self.cache, self.prefix_lens, max(lens) + G, self.step, shared, fmha_impl, overlap_prefix, want_logits=not self.lmhead
+            self.cache, self.prefix_lens, max(lens) + G, self.step, shared, fmha_impl, overlap_prefix, want_logits=not self.lmhead,
+            few_rows=whole_job,
         )
         self.graph = None
         self.done = 0  # tokens produced so far per row
@@ -369,6 +372,7 @@ class Engine:
         overlap_prefix: bool = True,
         shared_prefix: bool | None = None,
         prefill_group=None,
+        whole_job: bool = False,
     ) -> tuple[torch.Tensor, torch.Tensor]:
         """Decode every prompt `num_samples` times.
 
@@ -378,9 +382,12 @@ class Engine:
 
         Returns (tokens, masks): int32 device tensors of shape (S, num_samples, G); masks are 1 where a
         token was sampled and 0 where it was forced.  `traj_offset`/`series_offset` shift the ids that key
-        the random stream, so a shard of the trajectories reproduces exactly its part of the full run;
+        the random stream, so a shard of the trajectories draws what its part of the full run draws, for a bf16 model token
+        for token.  (fp32 products go to kernels by their number of rows, which order their sums differently: logits
+        equal to 1e-6 or so, and a draw that falls that close to a seam between two tokens may go to the other.)
         `shared_prefix` (None = decide from `num_samples`) fixes whether the prompt's keys are read once per series
-        by the tensor-core phase or per row, so that a shard can take the path the whole job takes.
+        by the tensor-core phase or per row, so that a shard can take the path the whole job takes; `whole_job` says that
+        this is no shard, and lets one or two rows take kernels of their own.
         `num_samples == 0` (a rank without work) returns empty tensors.  `prefill_group`: a process group whose ranks
         decode different trajectories of these same prompts; each rank then prefills only its share of the prompts
         and the ranks exchange the prompt K/V (every rank of the group must make the call).
@@ -405,7 +412,7 @@ class Engine:
         lens = [int(prompts.shape[1])] * S if on_device else [len(p) for p in prompts]
         key = DecodeRun.key_for(
             self.model, lens, num_samples, G, sampler, seed, force_schedules is not None, page_tokens, use_graph,
-            fmha_impl, overlap_prefix, shared_prefix, True, prefill_group is not None,
+            fmha_impl, overlap_prefix, shared_prefix, True, prefill_group is not None, whole_job,
         )
         run = self._run
         if run is not None and run.key == key and run.reusable():
@@ -415,7 +422,7 @@ class Engine:
             run = DecodeRun(
                 self.model, prompts, num_samples, G, sampler, seed, force_schedules, traj_offset=traj_offset,
                 series_offset=series_offset, page_tokens=page_tokens, use_graph=use_graph, fmha_impl=fmha_impl,
-                overlap_prefix=overlap_prefix, shared_prefix=shared_prefix, prefill_group=prefill_group,
+                overlap_prefix=overlap_prefix, shared_prefix=shared_prefix, prefill_group=prefill_group, whole_job=whole_job,
             )
             self._run = run
         run.start()
@@ -489,7 +496,7 @@ class Engine:
             sched = kwargs.get("force_schedule")
             toks, mk = self.generate_many(
                 [tokens], num_samples, kwargs.get("max_tokens"), kwargs.get("sampler"), kwargs.get("seed", 42),
-                None if sched is None else [sched],
+                None if sched is None else [sched], whole_job=True,
             )
             toks, mk = toks[0].cpu().tolist(), mk[0].cpu().tolist()  # the only read-back
             for i in range(num_samples):

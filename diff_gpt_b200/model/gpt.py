@@ -119,12 +119,13 @@ class DeviceModel(BaseGPT):
         """The cache of a decode run: prompt pages shared by a series' rows, private pages per row."""
 
     @abstractmethod
-    def prefill_plan(self, cache, members: list[int], P: int, fmha_impl: int):
-        """(binding, plan) that prefills the P-token prompts of the series `members` into `cache`."""
+    def prefill_plan(self, cache, members: list[int], P: int, fmha_impl: int, few_rows: bool = True):
+        """(binding, plan) that prefills the P-token prompts of the series `members` into `cache`.  `few_rows`: one or two rows may
+        run on kernels of their own, whose bf16 sums have another order than a larger batch's."""
 
     @abstractmethod
     def decode_plan(self, cache, prompt_lens: torch.Tensor, max_keys: int, step: torch.Tensor, shared: bool, fmha_impl: int,
-                    overlap_prefix: bool, want_logits: bool):
+                    overlap_prefix: bool, want_logits: bool, few_rows: bool = True):
         """(binding, plan) of one decode step of all rows; `step` is the device counter of generated tokens."""
 
 
@@ -296,8 +297,8 @@ class ForwardPlan:
     """
 
     def __init__(self, model: "GPT", n_seq: int, T: int, last_only: bool = False, want_logits: bool = True,
-                 cap: float = 0.0) -> None:
-        """`cap`: soft-cap the logits as they are stored (0 = raw logits)."""
+                 cap: float = 0.0, few_rows: bool = True) -> None:
+        """`cap`: soft-cap the logits as they are stored (0 = raw logits).  `few_rows`: see `DeviceModel.prefill_plan`."""
         emb = model.token_embedding_table.weight
         dev, dt = emb.device, emb.dtype
         C, V, L = model.n_embd, model.vocab_size, model.n_layer
@@ -322,7 +323,8 @@ class ForwardPlan:
         # tcgen05 GEMM + SwiGLU epilogue: bf16 with tileable sizes, and enough rows to fill the tensor cores
         # parameters may be views: rows that the kernels for small products do not take stay on cuBLAS
         aligned = model.packed_weights().rows16
-        self.one_row = dt == torch.bfloat16 and C % 16 == 0 and n == 1 and aligned  # see dgpt_linear: ahead of cuBLAS at every size
+        self.few_rows = few_rows
+        self.one_row = few_rows and dt == torch.bfloat16 and C % 16 == 0 and n == 1 and aligned  # see dgpt_linear: ahead of cuBLAS at every size
         self.fused_ffn = FUSED_FFN and dt == torch.bfloat16 and C % 8 == 0 and (n >= FUSED_FFN_MIN_ROWS or self.one_row)
         self.f32 = dt == torch.float32 and C % 4 == 0 and aligned
         self.own_ffn1 = self.f32 and own_f32(n, 4 * C, C, ends=True)
@@ -496,7 +498,7 @@ class ForwardPlan:
         if self.logits is None:
             return None
         if self.own_head:
-            ops.linear(self.xn, W.emb, self.logits, softcap=self.cap, status=self.status)
+            ops.linear(self.xn, W.emb, self.logits, softcap=self.cap, tiles=not self.few_rows, status=self.status)
         elif self.f32 and own_f32(*self.logits.shape, C, ends=self.cap > 0):
             ops.linear_f32(self.xn, W.emb, self.logits, softcap=self.cap)
         else:
@@ -656,7 +658,7 @@ class GPT(DeviceModel):
         return PagedKVCache(self.n_layer, self.n_head, self.n_embd // self.n_head, n_series, rows_per_series, prefix_len, max_new,
                             emb.dtype, emb.device, page_tokens=page_tokens, pool=pool)
 
-    def prefill_plan(self, cache, members, P, fmha_impl):
+    def prefill_plan(self, cache, members, P, fmha_impl, few_rows=True):
         idx = torch.tensor(members, device=cache.prefix_table.device)
         table = cache.prefix_table[idx].contiguous()
         zero = torch.zeros(len(members), dtype=torch.int32, device=table.device)
@@ -664,9 +666,9 @@ class GPT(DeviceModel):
             layouts=[cache._layout(l, table) for l in range(self.n_layer)], pos0=zero, slot0=zero, kv_len=P, q_offset=0,
             fmha_impl=fmha_impl,
         )
-        return bind, ForwardPlan(self, len(members), P, last_only=True)
+        return bind, ForwardPlan(self, len(members), P, last_only=True, few_rows=few_rows)
 
-    def decode_plan(self, cache, prompt_lens, max_keys, step, shared, fmha_impl, overlap_prefix, want_logits):
+    def decode_plan(self, cache, prompt_lens, max_keys, step, shared, fmha_impl, overlap_prefix, want_logits, few_rows=True):
         R, L = cache.n_rows, self.n_layer
         row_len = prompt_lens.repeat_interleave(cache.rows_per_series)
         slot0 = torch.full((R,), cache.suffix_slot0, dtype=torch.int32, device=row_len.device)
@@ -688,7 +690,7 @@ class GPT(DeviceModel):
             fmha_impl=fmha_impl,
             overlap_prefix=overlap_prefix and shared,
         )
-        return bind, ForwardPlan(self, R, 1, want_logits=want_logits)
+        return bind, ForwardPlan(self, R, 1, want_logits=want_logits, few_rows=few_rows)
 
     # ---- the reference contract --------------------------------------------------------
     def forward(

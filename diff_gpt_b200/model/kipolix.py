@@ -260,8 +260,9 @@ class KipolixPlan:
     """Buffers for one (n_seq, T) forward and the launch sequence that fills them (see `ForwardPlan`)."""
 
     def __init__(self, model: "Kipolix", n_seq: int, T: int, last_only: bool = False, want_logits: bool = True,
-                 rows: int | None = None) -> None:
-        """`rows`: the number of rows whose logits are asked for by index at each run (overrides last_only)."""
+                 rows: int | None = None, few_rows: bool = True) -> None:
+        """`rows`: the number of rows whose logits are asked for by index at each run (overrides last_only).  `few_rows`: see
+        `DeviceModel.prefill_plan`."""
         cfg, emb = model.config, model.embedding
         self.model, self.n_seq, self.T, self.n = model, n_seq, T, n_seq * T
         self.dev, self.dt = emb.device, emb.dtype
@@ -277,7 +278,8 @@ class KipolixPlan:
         self.xn = torch.empty((n_out, C), dtype=self.dt, device=self.dev)
         self.logits = torch.empty((n_out, V), dtype=self.dt, device=self.dev) if want_logits else None
         self.own_head = self.dt == torch.bfloat16 and C % 8 == 0 and V % 16 == 0
-        self.fused_ff = self.dt == torch.bfloat16 and C % 8 == 0 and (n >= FUSED_FF_MIN_ROWS or n == 1)
+        self.few_rows = few_rows
+        self.fused_ff = self.dt == torch.bfloat16 and C % 8 == 0 and (n >= FUSED_FF_MIN_ROWS or (few_rows and n == 1))
         self.status = torch.zeros(1, dtype=torch.int32, device=self.dev)
 
     def _buf(self, name: str, *shape: int, dtype=None) -> torch.Tensor:
@@ -335,7 +337,7 @@ class KipolixPlan:
             with region("gemm_up"):
                 torch.mm(self.h, lw.w_gu.t(), out=gu)
             ops.silu_mul(gu, act)
-        linear(act, lw.w_down_t, self.y, "gemm_down", self.status)
+        linear(act, lw.w_down_t, self.y, "gemm_down", self.status, self.few_rows)
 
     def run(self, ids32: torch.Tensor, b: RowBinding, rows: torch.Tensor | None = None,
             tap: Callable[[int, torch.Tensor], None] | None = None) -> torch.Tensor | None:
@@ -357,9 +359,9 @@ class KipolixPlan:
         for k, i in enumerate(runs):
             lw = W.layers[i]
             proj = self._buf("proj", self.n, lw.w_in_t.shape[1])
-            linear(self.h, lw.w_in_t, proj, "gemm_in", self.status)
+            linear(self.h, lw.w_in_t, proj, "gemm_in", self.status, self.few_rows)
             o = (self._retention if isinstance(lw.m, Retention) else self._attention)(k, lw, proj, b)
-            linear(o, lw.w_o_t, self.y, "gemm_proj", self.status)
+            linear(o, lw.w_o_t, self.y, "gemm_proj", self.status, self.few_rows)
             sub = lw.sub1
             if lw.sub2 is not None:
                 nxt = lw.sub2
@@ -382,7 +384,7 @@ class KipolixPlan:
         if self.logits is None:
             return None
         if self.own_head:
-            ops.linear(self.xn, W.head, self.logits, status=self.status)
+            ops.linear(self.xn, W.head, self.logits, tiles=not self.few_rows, status=self.status)
         else:
             with region("gemm_logits"):
                 torch.mm(self.xn, W.head.t(), out=self.logits)
@@ -475,7 +477,7 @@ class Kipolix(ConfiguredModel):
         return PagedRowCache(self.row_widths, self.keep, self.state_specs, n_series, rows_per_series, prefix_len, max_new, emb.dtype,
                              emb.device, page_tokens=page_tokens, keep_first=self.keep_first)
 
-    def prefill_plan(self, cache, members, P, fmha_impl):
+    def prefill_plan(self, cache, members, P, fmha_impl, few_rows=True):
         dev = cache.prefix_table.device
         n = len(members)
         table = cache.prefix_table[torch.tensor(members, device=dev)].contiguous()
@@ -487,9 +489,9 @@ class Kipolix(ConfiguredModel):
             tables=self.tables(P), state_in=states if P == 1 else None, state_out=states, context=0,
             kv_layout=lambda k, D, v_col: cache.kv_layout(k, table, D, v_col), fmha_impl=fmha_impl if fmha_impl <= 3 else 0,
         )
-        return bind, KipolixPlan(self, n, P, last_only=True)
+        return bind, KipolixPlan(self, n, P, last_only=True, few_rows=few_rows)
 
-    def decode_plan(self, cache, prompt_lens, max_keys, step, shared, fmha_impl, overlap_prefix, want_logits):
+    def decode_plan(self, cache, prompt_lens, max_keys, step, shared, fmha_impl, overlap_prefix, want_logits, few_rows=True):
         R, dev = cache.n_rows, prompt_lens.device
         slot0 = torch.full((R,), cache.suffix_slot0, dtype=torch.int32, device=dev)
         row_len = prompt_lens.repeat_interleave(cache.rows_per_series).contiguous()
@@ -499,7 +501,7 @@ class Kipolix(ConfiguredModel):
             len1=torch.ones(R, dtype=torch.int32, device=dev), step=step, keys=max_keys, tables=self.tables(max_keys),
             state_in=cache.states, state_out=cache.states,
         )
-        return bind, KipolixPlan(self, R, 1, want_logits=want_logits)
+        return bind, KipolixPlan(self, R, 1, want_logits=want_logits, few_rows=few_rows)
 
     def new_plan(self, n_seq, T, **kw) -> KipolixPlan:
         return KipolixPlan(self, n_seq, T, **kw)

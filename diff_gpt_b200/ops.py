@@ -289,9 +289,10 @@ def linear(
     xielu: tuple[float, float] | None = None,
     silu_gate: bool = False,
     softcap: float = 0.0,
+    tiles: bool = False,
     status: torch.Tensor | None = None,
 ) -> None:
-    """out = a @ w.T on the tcgen05 kernel (bf16).  swiglu=(alpha, limit): the SwiGLU of interleaved column pairs is
+    """out = a @ w.T on the tcgen05 kernel (bf16), one or two rows on a kernel of their own unless `tiles`.  swiglu=(alpha, limit): the SwiGLU of interleaved column pairs is
     applied in the epilogue and `out` has half as many columns as `w` has rows.  add=r: out = r + a @ w.T, rounded
     once (r may be `out`).  xielu=(alpha_p, alpha_n): that activation is applied in the epilogue.  silu_gate: column pairs
     are (gate, up) and `out` = silu(gate) * up, half as many columns.  softcap > 0: out = softcap * tanh(a @ w.T / softcap)."""
@@ -305,6 +306,7 @@ def linear(
         assert add.shape == out.shape and add.dtype == out.dtype and add.stride(1) == 1
     alpha, limit = swiglu or xielu or (softcap, 0.0)
     epilogue = 1 if swiglu else 4 if xielu else 5 if silu_gate else 6 if softcap > 0 else 2 if add is not None else 0
+    epilogue += 256 if tiles else 0  # DGPT_LINEAR_TILES
     check(
         lib.dgpt_linear(
             a.data_ptr(), a.stride(0), w.data_ptr(), w.stride(0), out.data_ptr(), out.stride(0), _ptr(add),

@@ -241,10 +241,13 @@ int dgpt_linear_f32(const float* a, int64_t a_row_stride, const float* w, int64_
  *   epilogue 5:  out[m, n / 2] = silu(acc[m, n]) * acc[m, n + 1] for even n, from the unrounded accumulator     out: [M, N / 2]
  *   epilogue 6:  out[m, n]     = alpha * tanh(acc[m, n] / alpha), the rule of dgpt_softcap with cap = alpha > 0 (the tangent within 4e-6 of its
  *                value before it is rounded)   out: [M, N]
+ * One or two rows run on a kernel of their own, whose sums have another order.  With DGPT_LINEAR_TILES added to the epilogue they take
+ * the tiles too, so that a row's result is the same bit for bit whatever the number of rows.
  * Replaces nn.Linear of src/diff_gpt/model/feed_forward.py:10-14 followed by swi_glu.py:11-19 (epilogue 1), any
  * bias-free nn.Linear of the path (epilogue 0), or a projection with the residual add that follows it
  * (src/diff_gpt/model/block.py:98-106, epilogue 2).  resid is ignored for epilogues 0, 1, 4, 5 and 6.  bf16 only; pointers 16-byte aligned, K and the row strides
  * multiples of 8 elements, N a multiple of 16.  status: device int32, set non-zero if a bounded wait ran out. */
+#define DGPT_LINEAR_TILES 256
 int dgpt_linear(const void* a, int64_t a_row_stride, const void* w, int64_t w_row_stride, void* out,
                 int64_t out_row_stride, const void* resid, int64_t resid_row_stride, int32_t M, int32_t N,
                 int32_t K, int32_t epilogue, float alpha, float limit, int32_t dtype, int32_t* status,
