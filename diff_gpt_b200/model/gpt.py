@@ -194,7 +194,9 @@ def prefix_ctas(units: int, key_tiles: int, own_us: float, n_sm: int) -> int:
     tile, beside a per-row phase that takes `own_us` on the whole GPU and meanwhile advances on the SMs left over.  PREFIX_CTAS,
     unless one SM per unit, or every SM, is estimated to be done earlier.  Measured per layer with the merge, us: 3 x 333 rows,
     12 heads, 777 + 20 keys (72 units) on 64 SMs 42.5, on 72 34.1; 10 x 64 rows, 8 heads, 500 + 30 keys (80 units) 26.9 -> 19.0; 40 x
-    20 rows, 12 heads, 1000 + 40 keys (480 units) 148, on all 92; 4096 rows, 12 heads, 1024 + 128 keys (192 units) 282, on all 295."""
+    20 rows, 12 heads, 1000 + 40 keys (480 units) 148, on all 92; 4096 rows, 12 heads, 1024 + 128 keys (192 units) 282, on all 295.  The rate a
+    tile is that of heads of 64; with heads of 32 no step of twelve such jobs got slower (4 layers, us: 40 x 20 rows 505 -> 393, 20 x 33
+    rows, 1400 keys 438 -> 360, 10 x 64 217 -> 176, 4096 rows 405 -> 400)."""
 
     def estimate(ctas: int) -> float:
         phase = -(-units // ctas) * key_tiles * 3.3
