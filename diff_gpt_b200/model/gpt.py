@@ -247,14 +247,15 @@ def own_f32(M: int, N: int, K: int, ends: bool = False) -> bool:
     beyond 1000 x 256 x 64 3.99 / 4.69, 400 x 1024 x 256 9.4 / 13.2.
     Up to 16 rows cuBLAS has kernels for few rows: 2 x 512 x 512 3.67 / 6.66, 8 x 256 x 256 3.29 / 4.16, 2 x 64 x 64 2.04 / 2.34.  Own there:
     with an ending up to K = 128 (2 x 512 x 128 SwiGLU 3.57 / 3.48, 8 x 256 x 64 2.9 / 2.3), from 8 wide rows on (8 x 1024 x 256 6.43 / 4.25,
-    8 x 2048 x 512 9.63 / 7.00), and one row up to K = 64 (1 x 256 x 64 2.90 / 2.28; 1 x 64 x 128 1.97 / 2.81)."""
+    8 x 2048 x 512 9.63 / 7.00), one row up to K = 64 (1 x 256 x 64 2.90 / 2.28; 1 x 64 x 128 1.97 / 2.81), and from 5 rows on up to K = 64, level
+    by itself (8 x 256 x 64 2.41 / 2.48) and 1 to 3 % ahead in a whole forecast of 5 to 12 futures."""
     if -(-M // 16) * -(-N // 32) > 400 or K > 512:
         return False
     if M > 16:
         return True
     if M == 1:
         return K <= 64
-    return (ends and K <= 128) or (M >= 8 and N >= 1024 and K >= 256)
+    return (ends and K <= 128) or (M >= 5 and K <= 64) or (M >= 8 and N >= 1024 and K >= 256)
 
 
 # ---- how one forward call is bound to K/V storage ----------------------------------
