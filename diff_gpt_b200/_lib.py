@@ -38,6 +38,22 @@ class KvLayout(C.Structure):
     ]
 
 
+class SmallGptModel(C.Structure):
+    _fields_ = [
+        ("emb", C.c_void_p), ("weights", C.c_void_p), ("cs_table", C.c_void_p),
+        ("C", C.c_int32), ("H", C.c_int32), ("L", C.c_int32), ("V", C.c_int32), ("table_len", C.c_int32), ("layers_per_block", C.c_int32),
+        ("swiglu_alpha", C.c_float), ("swiglu_limit", C.c_float),
+    ]
+
+
+class SmallGptDraw(C.Structure):
+    _fields_ = [
+        ("traj_ids", C.c_void_p), ("force_schedule", C.c_void_p), ("force_group_stride", C.c_int64), ("out_tokens", C.c_void_p),
+        ("history", C.c_void_p), ("history_stride", C.c_int64), ("seed", C.c_uint64), ("force_group_rows", C.c_int32),
+        ("cap", C.c_float), ("temperature", C.c_float), ("top_p", C.c_float),
+    ]
+
+
 _p, _i32, _i64, _f32, _u64, _sz = C.c_void_p, C.c_int32, C.c_int64, C.c_float, C.c_uint64, C.c_size_t
 _kvp = C.POINTER(KvLayout)
 
@@ -78,6 +94,11 @@ PROTOTYPES = {
     "dgpt_step_advance": (C.c_int, [_p, _i32, _p]),
     "dgpt_linear": (C.c_int, [_p, _i64, _p, _i64, _p, _i64, _p, _i64, _i32, _i32, _i32, _i32, _f32, _f32, _i32, _p, _p]),
     "dgpt_linear_f32": (C.c_int, [_p, _i64, _p, _i64, _p, _i64, _p, _i64, _i32, _i32, _i32, _i32, _f32, _f32, _p]),
+    "dgpt_small_gpt_supported": (C.c_int, [_i32, _i32, _i32, _i32, _i32]),
+    "dgpt_small_gpt": (
+        C.c_int,
+        [C.POINTER(SmallGptModel), _kvp, _i64, _p, _p, _p, _p, _p, _p, _p, _i32, _i32, _i32, _i32, _p, _f32, _i32, C.POINTER(SmallGptDraw), _p, _p],
+    ),
     "dgpt_integrate_tokens": (C.c_int, [_p, _i64, _i32, _i32, _i32, _i32, _p, _p, _p, _i32, _p, _p]),
     "dgpt_encode_series": (C.c_int, [_p, _i64, _i32, _i32, _i32, _i32, _p, _i32, _i32, _p, _p, _p, _p, _p]),
     "dgpt_bounded_wait_probe": (C.c_int, [_i32, _i64, _p, _p]),
@@ -139,7 +160,7 @@ PROTOTYPES = {
 }
 _NOT_LAUNCHING = {
     "dgpt_last_error", "dgpt_version", "dgpt_decode_attn_workspace_bytes", "dgpt_decode_attn_static_capacity_bytes",
-    "dgpt_lmhead_workspace_bytes", "dgpt_latent_attn_workspace_bytes", "dgpt_retention_workspace_bytes",
+    "dgpt_small_gpt_supported", "dgpt_lmhead_workspace_bytes", "dgpt_latent_attn_workspace_bytes", "dgpt_retention_workspace_bytes",
 }
 
 

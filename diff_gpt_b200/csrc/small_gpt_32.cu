@@ -1,0 +1,8 @@
+// dgpt_small_gpt, models 32 wide (see small_gpt.cu)
+#include "small_gpt.cuh"
+
+namespace dgpt {
+
+int small_gpt_32(const SmallGpt& p, int M, int grid, cudaStream_t st) { return small_gpt_pick<32>(p, M, grid, st); }
+
+}  // namespace dgpt

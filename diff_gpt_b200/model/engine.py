@@ -305,6 +305,9 @@ class DecodeRun:
                 self._sample(logits, slice(0, self.R), row_stride=logits.stride(0))
                 self.done += 1
             return
+        if getattr(self.plan, "whole", False):  # a small fp32 model: all the steps are one launch
+            self._advance_whole(n_steps)
+            return
         if self.use_graph and self.graph is None:
             # warm the forward (cuBLAS handles, lazy module loads) without touching tokens or the counter
             self.plan.run(self.tokens, self.bind)
@@ -330,6 +333,33 @@ class DecodeRun:
                 _lib.stats.launches += self.graph_launches
             else:
                 self._body()
+        self.done += n_steps
+
+    def _advance_whole(self, n_steps: int) -> None:
+        """All the steps of a small fp32 model in one launch; a run to its end, the usual case, is recorded."""
+
+        def enqueue():
+            draw = ops.small_gpt_draw(
+                cap=self.cap, temperature=self.temperature, top_p=self.top_p, seed=self.seed, traj_ids=self.traj_ids, tokens=self.tokens,
+                history=self.history, force_schedule=self.force, force_group_rows=self.N,
+                force_group_stride=self.G if self.force is not None else 0,
+            )
+            self.plan.run_whole(self.tokens, self.bind, n_steps, draw)
+            ops.step_advance(self.step, n_steps)
+
+        if not self.use_graph or n_steps != self.G - 1:
+            enqueue()
+        elif self.graph is None:
+            enqueue()  # the first time by itself: what a launch sets up once is not for a recording
+            before = _lib.stats.launches
+            self.graph = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(self.graph):
+                enqueue()
+            self.graph_launches = _lib.stats.launches - before
+            _lib.stats.launches = before
+        else:
+            self.graph.replay()
+            _lib.stats.launches += self.graph_launches
         self.done += n_steps
 
     def check_status(self) -> None:

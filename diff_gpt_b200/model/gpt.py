@@ -258,6 +258,23 @@ def own_f32(M: int, N: int, K: int, ends: bool = False) -> bool:
     return (ends and K <= 128) or (M >= 5 and K <= 64) or (M >= 8 and N >= 1024 and K >= 256)
 
 
+def whole_f32(C: int, H: int, L: int, V: int, n_seq: int, T: int, keys: int) -> bool:
+    """Whether a forward of an fp32 model runs as one launch of dgpt_small_gpt: `T` tokens of each of `n_seq` sequences behind one another,
+    or one token of `n_seq` rows (T = 1), none of which sees more than `keys` keys.
+    Decode steps, us a step, one launch per product / one for all: 2 layers of 64, 148 rows, 60 keys 69 / 14, 1900 keys 167 / 38; up to two
+    rows a multiprocessor ahead at every number of keys (4 layers of 128, 296 rows, 1900 keys 406 / 260), up to four below a thousand
+    (12 layers of 128, 592 rows, 900 keys 1193 / 1073, 1900 keys level), up to eight where the model is narrow (64, 1000 rows, 300 keys
+    101 / 76, 900 keys 141 / 146; 128, 60 keys 211 / 189, 300 keys 246 / 295).  Every CTA reads all weights and its rows' prompt by itself.
+    Whole sequences, us a call with its host work: 2 layers of 64, 1 x 256 tokens 520 / 256, 1 x 1024 590 / 979; 4 layers of 128, 1 x 128
+    855 / 365, 1 x 512 983 / 1334; many sequences pay while their CTAs are two a multiprocessor (8 x 256 565 / 382, 32 x 64 578 / 247)."""
+    if not ops.small_gpt_supported(C, H, L, V, keys):
+        return False
+    sms = _sm_count()
+    if T == 1:
+        return keys <= 2048 if n_seq <= 2 * sms else keys <= 1024 if n_seq <= 4 * sms else n_seq <= 8 * sms and C <= 64 and keys <= 512
+    return T <= (256 if C <= 64 else 128) and keys <= 1024 and n_seq * -(-min(T, 128) // 8) <= 2 * sms
+
+
 # ---- how one forward call is bound to K/V storage ----------------------------------
 @dataclass
 class KvBinding:
@@ -300,8 +317,9 @@ class ForwardPlan:
     """
 
     def __init__(self, model: "GPT", n_seq: int, T: int, last_only: bool = False, want_logits: bool = True,
-                 cap: float = 0.0, few_rows: bool = True) -> None:
-        """`cap`: soft-cap the logits as they are stored (0 = raw logits).  `few_rows`: see `DeviceModel.prefill_plan`."""
+                 cap: float = 0.0, few_rows: bool = True, keys: int | None = None) -> None:
+        """`cap`: soft-cap the logits as they are stored (0 = raw logits).  `few_rows`: see `DeviceModel.prefill_plan`.  `keys`: the
+        most keys that a token sees, where the kernel of small fp32 models may run the whole forward (see whole_f32)."""
         emb = model.token_embedding_table.weight
         dev, dt = emb.device, emb.dtype
         C, V, L = model.n_embd, model.vocab_size, model.n_layer
@@ -311,18 +329,25 @@ class ForwardPlan:
         def buf(*shape, dtype=dt):
             return torch.empty(shape, dtype=dtype, device=dev)
 
+        n_out = n_seq if last_only else n
+        self.cap = cap
+        self.status = torch.zeros(1, dtype=torch.int32, device=dev)
+        self.logits = buf(n_out, V) if want_logits else None
+        self.keys = keys
+        self.whole = (
+            keys is not None and want_logits and dt == torch.float32 and emb.is_contiguous() and whole_f32(C, model.n_head, L, V, n_seq, T, keys)
+        )
+        self.side = None
+        if self.whole:
+            return
         self.x, self.u, self.q, self.y = buf(n, C), buf(n, C), buf(n, C), buf(n, C)
         self.qkvg = buf(n, 4 * C)
         self.parts = [buf(n, C) for _ in range(L)]
         self.act = buf(n, 2 * C)
-        n_out = n_seq if last_only else n
         self.xn = buf(n_out, C)
         self.last = buf(n_out, C) if (last_only and T > 1) else None
-        self.logits = buf(n_out, V) if want_logits else None
         # the tied-embedding head on the library's tcgen05 GEMM (bf16 with tileable sizes); fp32: see own_f32
         self.own_head = dt == torch.bfloat16 and C % 8 == 0 and V % 16 == 0
-        self.cap = cap
-        self.status = torch.zeros(1, dtype=torch.int32, device=dev)
         # tcgen05 GEMM + SwiGLU epilogue: bf16 with tileable sizes, and enough rows to fill the tensor cores
         # parameters may be views: rows that the kernels for small products do not take stay on cuBLAS
         aligned = model.packed_weights().rows16
@@ -339,7 +364,6 @@ class ForwardPlan:
         self.prefix_lse = None
         self.part_o = None
         self.part_lse = None
-        self.side = None
         self.prefix_on_tc = False
         self.prefix_ctas = 0
         self.workspace = None
@@ -407,7 +431,20 @@ class ForwardPlan:
             nbytes = ops.decode_attn_workspace_bytes(self.n, H, D, b.n_splits)
             self.workspace = torch.empty(nbytes // 4, dtype=torch.float32, device=dev)
 
+    def run_whole(self, ids32: torch.Tensor, b: KvBinding, n_steps: int = 1, draw=None) -> torch.Tensor:
+        """The forward in one launch (`whole`), or `n_steps` decode steps with their draws."""
+        first = b.layouts[0]
+        stride = (b.layouts[1].k_base - first.k_base) // 4 if len(b.layouts) > 1 else 0
+        decode = {"len0": b.len0, "start1": b.start1, "len1": b.len1} if b.decode else {"T": self.T, "last_only": self.last_only}
+        ops.small_gpt(
+            self.model.packed_weights().whole(self.model), first, stride, ids32, b.pos0, b.slot0, b.step, self.logits, self.status,
+            max_keys=self.keys, logit_cap=self.cap, n_steps=n_steps, draw=draw, **decode,
+        )
+        return self.logits
+
     def run(self, ids32: torch.Tensor, b: KvBinding) -> torch.Tensor | None:
+        if self.whole:
+            return self.run_whole(ids32, b)
         m = self.model
         C, H, L = m.n_embd, m.n_head, m.n_layer
         D = C // H
@@ -530,10 +567,30 @@ class _Packed:
     layers: list
     rows16: bool  # every matrix lies as the linear kernels want it
     stamp: tuple
+    columns: torch.Tensor | None  # the same weights as dgpt_small_gpt reads them, where it is built for the model
+
+    def whole(self, m: "GPT"):
+        return ops.small_gpt_model(
+            self.emb, self.columns, self.freqs_cis, H=m.n_head, L=m.n_layer, layers_per_block=m.attn_res_layers_per_block,
+            swiglu=(m.swiglu_alpha, m.swiglu_limit),
+        )
 
     @property
     def head(self) -> torch.Tensor:
         return self.emb
+
+
+def _small_gpt_columns(layers: list, emb: torch.Tensor) -> torch.Tensor:
+    """Weights of all layers and the head as dgpt_small_gpt reads them (see include/dgpt.h)."""
+
+    def words(w: torch.Tensor) -> torch.Tensor:  # [N, K] -> [K / 4 / S][N][S][4]
+        N, K = w.shape
+        S = max(1, min(256 // N, K // 4))
+        return w.reshape(N, K // 4 // S, S, 4).transpose(0, 1).reshape(-1)
+
+    flat = [words(w) for l in layers for w in (l.wqkvg_t.t(), l.wproj_t.t(), l.w1, l.w2_t.t())]
+    flat += [words(F.pad(rows, (0, 0, 0, 256 - rows.shape[0]))) for rows in emb.split(256)]
+    return torch.cat(flat + [v for l in layers for v in (l.w_attn, l.w_mlp)])
 
 
 class GPT(DeviceModel):
@@ -605,8 +662,11 @@ class GPT(DeviceModel):
                 )
             emb = self.token_embedding_table.weight.detach()
             table = self.freqs_cis.to(emb.dtype).contiguous()
+            columns = None
+            if emb.dtype == torch.float32 and ops.small_gpt_supported(self.n_embd, self.n_head, self.n_layer, self.vocab_size):
+                columns = _small_gpt_columns(layers, emb)
         rows16 = ops.rows16(emb) and all(ops.rows16(w) for l in layers for w in (l.w1, l.wproj_t.t(), l.w2_t.t()))
-        self._packed = _Packed(emb=emb, freqs_cis=table, layers=layers, rows16=rows16, stamp=stamp)
+        self._packed = _Packed(emb=emb, freqs_cis=table, layers=layers, rows16=rows16, stamp=stamp, columns=columns)
         return self._packed
 
     @classmethod
@@ -643,7 +703,9 @@ class GPT(DeviceModel):
         assert t0 + 1 <= self.freqs_cis.shape[0]
         cache.ensure(t0 + 1, emb.dtype, emb.device)
         splits = _pick_splits(H, t0 + 1)
-        kind = (splits, self.logit_softcap, self.swiglu_alpha, self.swiglu_limit, self.attn_res_layers_per_block)
+        keys = -(-(t0 + 1) // 256) * 256  # a plan serves many tokens
+        whole = whole_f32(self.n_embd, H, self.n_layer, self.vocab_size, 1, 1, keys) and keys
+        kind = (splits, whole, self.logit_softcap, self.swiglu_alpha, self.swiglu_limit, self.attn_res_layers_per_block)
         held = (self.packed_weights(), *self.cache_storage(cache))
         if old is not None and old.fits(kind, held):
             return old
@@ -654,7 +716,7 @@ class GPT(DeviceModel):
                 layouts=[cache.layer_layout(i) for i in range(self.n_layer)], pos0=numbers[2:3], slot0=numbers[1:2], decode=True,
                 len0=zero, start1=zero, len1=numbers[3:4], n_splits=splits,
             )
-            return SingleStep(ForwardPlan(self, 1, 1, cap=self.logit_softcap), bind, numbers, kind, held, checks=False)
+            return SingleStep(ForwardPlan(self, 1, 1, cap=self.logit_softcap, keys=keys), bind, numbers, kind, held, checks=False)
 
     def paged_cache(self, n_series, rows_per_series, prefix_len, max_new, page_tokens, pool=None) -> PagedKVCache:
         emb = self.embedding
@@ -669,7 +731,7 @@ class GPT(DeviceModel):
             layouts=[cache._layout(l, table) for l in range(self.n_layer)], pos0=zero, slot0=zero, kv_len=P, q_offset=0,
             fmha_impl=fmha_impl,
         )
-        return bind, ForwardPlan(self, len(members), P, last_only=True, few_rows=few_rows)
+        return bind, ForwardPlan(self, len(members), P, last_only=True, few_rows=few_rows, keys=None if fmha_impl else P)
 
     def decode_plan(self, cache, prompt_lens, max_keys, step, shared, fmha_impl, overlap_prefix, want_logits, few_rows=True):
         R, L = cache.n_rows, self.n_layer
@@ -693,7 +755,7 @@ class GPT(DeviceModel):
             fmha_impl=fmha_impl,
             overlap_prefix=overlap_prefix and shared,
         )
-        return bind, ForwardPlan(self, R, 1, want_logits=want_logits, few_rows=few_rows)
+        return bind, ForwardPlan(self, R, 1, want_logits=want_logits, few_rows=few_rows, keys=None if fmha_impl else max_keys)
 
     # ---- the reference contract --------------------------------------------------------
     def forward(
@@ -725,17 +787,16 @@ class GPT(DeviceModel):
         dt = self.token_embedding_table.weight.dtype
         t0 = 0 if kv_cache is None else kv_cache.get_pos()
         assert t0 + T <= self.freqs_cis.shape[0]
+        plan = ForwardPlan(self, B, T, cap=self.logit_softcap, keys=t0 + T)
         if kv_cache is None:
-            scratch = KVCache(batch_size=B, num_heads=H, seq_len=T, head_dim=D, num_layers=1)
+            # every layer reuses the same scratch K/V, unless one kernel's CTAs work on different layers at one time
+            scratch = KVCache(batch_size=B, num_heads=H, seq_len=T, head_dim=D, num_layers=L if plan.whole else 1)
             scratch.ensure(T, dt, dev)
-            layouts = [scratch.layer_layout(0)] * L  # every layer reuses the same scratch K/V
-            store = scratch
+            layouts = [scratch.layer_layout(i if plan.whole else 0) for i in range(L)]
         else:
             assert not isinstance(kv_cache, PagedKVCache), "PagedKVCache is driven by the Engine"
             kv_cache.ensure(t0 + T, dt, dev)
             layouts = [kv_cache.layer_layout(i) for i in range(L)]
-            store = kv_cache
-        del store
         start = torch.full((B,), t0, dtype=torch.int32, device=dev)
         bind = KvBinding(layouts=layouts, pos0=start, slot0=start, kv_len=t0 + T, q_offset=t0)
         if T == 1 and t0 > 0:
@@ -745,7 +806,6 @@ class GPT(DeviceModel):
             bind.len1 = torch.full((B,), t0 + 1, dtype=torch.int32, device=dev)
             n_keys = t0 + 1
             bind.n_splits = _pick_splits(B * H, n_keys)
-        plan = ForwardPlan(self, B, T, cap=self.logit_softcap)
         logits = plan.run(idx.reshape(-1).to(torch.int32), bind)
         if kv_cache is not None:
             kv_cache.pos = t0 + T

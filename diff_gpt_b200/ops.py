@@ -344,6 +344,84 @@ def linear_f32(
     )
 
 
+def small_gpt_supported(C_: int, H: int, L: int, V: int, max_keys: int = 1) -> bool:
+    return bool(lib.dgpt_small_gpt_supported(C_, H, L, V, max_keys))
+
+
+def small_gpt_model(emb: torch.Tensor, weights: torch.Tensor, cs_table: torch.Tensor, *, H: int, L: int, layers_per_block: int,
+                    swiglu: tuple[float, float]) -> _lib.SmallGptModel:
+    """Descriptor of a small fp32 GPT; `weights` as include/dgpt.h lays them out."""
+    _cuda(emb, weights, cs_table)
+    V, Cdim = emb.shape
+    assert emb.dtype == weights.dtype == cs_table.dtype == torch.float32
+    assert emb.is_contiguous() and weights.is_contiguous() and cs_table.is_contiguous()
+    assert weights.numel() == L * (11 * Cdim * Cdim + 2 * Cdim) + -(-V // 256) * 256 * Cdim
+    m = _lib.SmallGptModel(emb.data_ptr(), weights.data_ptr(), cs_table.data_ptr(), Cdim, H, L, V, cs_table.shape[0], layers_per_block, *swiglu)
+    m._keep = (emb, weights, cs_table)
+    return m
+
+
+def small_gpt_draw(
+    *,
+    cap: float,
+    temperature: float,
+    top_p: float,
+    seed: int,
+    traj_ids: torch.Tensor,
+    tokens: torch.Tensor,
+    history: torch.Tensor,
+    force_schedule: torch.Tensor | None = None,
+    force_group_rows: int = 1,
+    force_group_stride: int = 0,
+) -> _lib.SmallGptDraw:
+    """Descriptor of the draw that ends a decode step of `small_gpt`."""
+    _cuda(traj_ids, tokens, history, force_schedule)
+    assert traj_ids.dtype == torch.int64 and tokens.dtype == history.dtype == torch.int32
+    d = _lib.SmallGptDraw(traj_ids.data_ptr(), _ptr(force_schedule), force_group_stride, tokens.data_ptr(), history.data_ptr(), history.stride(0),
+                          seed & 0xFFFFFFFFFFFFFFFF, force_group_rows, cap, temperature, top_p)
+    d._keep = (traj_ids, force_schedule, tokens, history)
+    return d
+
+
+def small_gpt(
+    model: _lib.SmallGptModel,
+    kv: KvLayout,
+    kv_layer_stride: int,
+    ids: torch.Tensor,
+    pos0: torch.Tensor,
+    slot0: torch.Tensor,
+    step: torch.Tensor | None,
+    logits: torch.Tensor,
+    status: torch.Tensor,
+    *,
+    max_keys: int,
+    T: int = 0,
+    last_only: bool = False,
+    len0: torch.Tensor | None = None,
+    start1: torch.Tensor | None = None,
+    len1: torch.Tensor | None = None,
+    logit_cap: float = 0.0,
+    n_steps: int = 1,
+    draw: _lib.SmallGptDraw | None = None,
+) -> None:
+    """Whole forwards of a small fp32 GPT: T tokens of each sequence of `pos0`, or (T = 0) `n_steps` decode steps of its rows, none
+    of which sees more than `max_keys` keys."""
+    _cuda(ids, pos0, slot0, step, logits, status, len0, start1, len1)
+    assert ids.dtype == torch.int32 and ids.is_contiguous() and logits.is_contiguous() and logits.dtype == torch.float32
+    n_seq = pos0.numel()
+    assert ids.numel() >= n_seq * max(T, 1) and slot0.numel() == n_seq and logits.shape[-1] == model.V
+    assert logits.numel() >= (n_seq if last_only or T == 0 else n_seq * T) * model.V
+    for t in (pos0, slot0, step, len0, start1, len1):
+        assert t is None or (t.dtype == torch.int32 and t.is_contiguous())
+    check(
+        lib.dgpt_small_gpt(
+            C.byref(model), C.byref(kv), kv_layer_stride, ids.data_ptr(), pos0.data_ptr(), slot0.data_ptr(), _ptr(step), _ptr(len0),
+            _ptr(start1), _ptr(len1), n_seq, T, max_keys, int(last_only), logits.data_ptr(), logit_cap, n_steps,
+            None if draw is None else C.byref(draw), status.data_ptr(), _stream(),
+        )
+    )
+
+
 def integrate_tokens(
     tokens: torch.Tensor, n_chan: int, vocab_size: int, scale: torch.Tensor, order: torch.Tensor, state: torch.Tensor
 ) -> torch.Tensor:

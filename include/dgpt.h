@@ -231,6 +231,56 @@ int dgpt_linear_f32(const float* a, int64_t a_row_stride, const float* w, int64_
                     int64_t out_row_stride, const float* resid, int64_t resid_row_stride, int32_t M, int32_t N, int32_t K,
                     int32_t epilogue, float alpha, float limit, void* stream);
 
+/* A small fp32 GPT as dgpt_small_gpt wants it.
+ * weights: device fp32, 16-byte aligned.  Matrices [N][K] laid out as [K / 4 / S][N][S][4], S = max(1, min(256 / N, K / 4)), one behind the other: per layer q, k, v and output
+ * gate (N = 4 C, K = C), output projection (C, C), feed-forward up (4 C, C; gate and linear columns interleaved) and down (C, 2 C); then
+ * the head, 256 rows of it at a time (the last block filled up with zeros); then per layer the depth mix's two vectors [C] (attention,
+ * feed-forward).
+ * emb: device fp32 [V, C]; cs_table: device fp32 [table_len, C / H / 2, 2] (cos, sin). */
+typedef struct dgpt_small_gpt_model {
+  const float* emb;
+  const float* weights;
+  const float* cs_table;
+  int32_t C, H, L, V, table_len, layers_per_block;
+  float swiglu_alpha, swiglu_limit;
+} dgpt_small_gpt_model;
+
+/* The draw at the end of a decode step, the rule of dgpt_sample: out_tokens device int32 [n_seq], history device int32
+ * [n_seq, history_stride], traj_ids device int64 [n_seq] (these three not NULL). */
+typedef struct dgpt_small_gpt_draw {
+  const int64_t* traj_ids;
+  const int32_t* force_schedule;
+  int64_t force_group_stride;
+  int32_t* out_tokens;
+  int32_t* history;
+  int64_t history_stride;
+  uint64_t seed;
+  int32_t force_group_rows;
+  float cap, temperature, top_p;
+} dgpt_small_gpt_draw;
+
+/* 1 where dgpt_small_gpt is built for such a model (C = 32, 64 or 128 with heads of 8, 16 or 32, up to 16 layers, V a multiple of 4 up to
+ * 4096; logits and the places of max_keys keys must fit in shared memory), else 0. */
+int dgpt_small_gpt_supported(int32_t C, int32_t H, int32_t L, int32_t V, int32_t max_keys);
+
+/* Whole forwards of a small fp32 GPT in one launch: every call of src/diff_gpt/model/gpt.py:140-186 (block.py:88-109, mha.py:41-86,
+ * feed_forward.py:10-14) from token ids to logits.
+ *   T > 0    tokens ids[s * T + t] of n_seq sequences, t < T, at position pos0[s] + step + t and slot slot0[s] + step + t, each seeing
+ *            the cache's slots up to its own.  logits: [n_seq * T, V], or with last_only the last token's, [n_seq, V].  (More than 128 tokens
+ *            a sequence are one launch per 128.)
+ *   T == 0   one token ids[r] of each of n_seq rows, at pos0[r] + step and slot0[r] + step, seeing slots [0, len0[r]) and
+ *            [start1[r], start1[r] + len1[r] + step), as dgpt_decode_attn (len0, start1 NULL: none, 0); logits [n_seq, V].  With a draw,
+ *            n_steps of them: step i runs at step + i, draws for column step + i + 1 and goes on with the token drawn; *step_ptr is not
+ *            advanced.  The logits of the last step remain.
+ * kv: layer 0's storage; layer l's lies l * kv_layer_stride elements behind it, through the same page table.  logit_cap > 0: logits are
+ * stored soft-capped.  Rows do not depend on one another.  max_keys: the most keys that any token of the call sees.  status: device
+ * int32, set to 1 if a position or slot is out of range (nothing is written there) or a token sees more keys than that (they are left
+ * out), to 2 if a bounded wait ran out. */
+int dgpt_small_gpt(const dgpt_small_gpt_model* model, const dgpt_kv_layout* kv, int64_t kv_layer_stride, const int32_t* ids,
+                   const int32_t* pos0, const int32_t* slot0, const int32_t* step_ptr, const int32_t* len0, const int32_t* start1,
+                   const int32_t* len1, int32_t n_seq, int32_t T, int32_t max_keys, int32_t last_only, float* logits, float logit_cap, int32_t n_steps,
+                   const dgpt_small_gpt_draw* draw, int32_t* status, void* stream);
+
 /* Linear layer on the tcgen05 tensor cores, optionally with the SwiGLU of the feed-forward block in its epilogue:
  *   acc[m, n] = sum_k a[m, k] * w[n, k]                     (w as nn.Linear stores it: [N, K])
  *   epilogue 0:  out[m, n]     = acc[m, n]                  out: [M, N]
