@@ -603,6 +603,9 @@ class StepRunner:
         if stale:
             self._stream.synchronize()  # their memory belongs to other streams
         for key in stale:
+            if self._single[key].last is not None:
+                self._single[key].last.synchronize()
+        for key in stale:
             del self._single[key]
 
     def _one(self, cache, token: int) -> torch.Tensor | None:
@@ -624,6 +627,8 @@ class StepRunner:
         if one is not old:
             self._drop_stale(cache)
             self._single[key] = one
+        if one.graph is not None and getattr(one.plan, "whole", False):
+            return one, self._replay_here(one, cache, token)
         caller, mine = torch.cuda.current_stream(), self._stream
         mine.wait_stream(caller)
         with torch.cuda.stream(mine):
@@ -650,6 +655,22 @@ class StepRunner:
         out.record_stream(caller)
         cache.pos += 1
         return one, out
+
+    def _replay_here(self, one, cache, token: int) -> torch.Tensor:
+        """A recorded token of one launch, which needs nothing of cuBLAS's: on the caller's stream, behind the stream it ran on last.
+        (The change of streams and its two waits are 35 us of a token's 105.)"""
+        if one.last is None or one.last.cuda_stream != ops._stream():
+            caller = torch.cuda.current_stream()
+            caller.wait_stream(self._stream if one.last is None else one.last)
+            for t in (one.numbers, one.plan.logits, one.plan.status):
+                t.record_stream(caller)
+            one.last = caller
+        one.numbers.copy_(torch.tensor([token, cache.pos, cache.pos, cache.pos + 1], dtype=torch.int32))
+        one.graph.replay()
+        _lib.stats.launches += one.launches
+        one.runs += 1
+        cache.pos += 1
+        return one.plan.logits.to(torch.float32, copy=True)
 
     def finish(self, request) -> None:
         with self._lock:

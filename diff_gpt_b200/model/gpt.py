@@ -228,6 +228,7 @@ class SingleStep:
     graph: torch.cuda.CUDAGraph | None = None
     launches: int = 0
     runs: int = 0
+    last: torch.cuda.Stream | None = None  # where it was replayed last, if not on the runner's stream
 
     def fits(self, kind: tuple, held: tuple) -> bool:
         return self.kind == kind and len(self.held) == len(held) and all(a is b for a, b in zip(self.held, held))
@@ -580,6 +581,17 @@ class _Packed:
         return self.emb
 
 
+def _parameters(module: nn.Module) -> list:
+    """Every parameter in the tree as it is now, a tied one as often as it occurs.  (`parameters()` names and compares them on its way:
+    50 us a call for 2 layers, which a recorded token pays every time.)"""
+    found, below = [], [module]
+    while below:
+        m = below.pop()
+        found += [p for p in m._parameters.values() if p is not None]
+        below += [c for c in m._modules.values() if c is not None]
+    return found
+
+
 def _small_gpt_columns(layers: list, emb: torch.Tensor) -> torch.Tensor:
     """Weights of all layers and the head as dgpt_small_gpt reads them (see include/dgpt.h)."""
 
@@ -640,8 +652,7 @@ class GPT(DeviceModel):
     # ---- weights as the kernels want them -------------------------------------------
     def packed_weights(self) -> _Packed:
         """Fused QKVG weight and transposed views, rebuilt when a parameter was modified or moved."""
-        params = [p for p in self.parameters()]
-        stamp = tuple((p.data_ptr(), p._version, p.dtype) for p in params) + (self.freqs_cis.data_ptr(),)
+        stamp = tuple([(p.data_ptr(), p._version, p.dtype) for p in _parameters(self)]) + (self.freqs_cis.data_ptr(),)
         if self._packed is not None and self._packed.stamp == stamp:
             return self._packed
         layers = []
@@ -844,10 +855,11 @@ _SM_COUNT: dict[int, int] = {}
 def _sm_count() -> int:
     """Multiprocessors of the current CUDA device (148 on a B200); that figure is assumed where no device is present,
     so the split policy can be examined on a CPU box."""
-    if not torch.cuda.is_available():
-        return 148
-    dev = torch.cuda.current_device()
+    dev = torch._C._cuda_getDevice() if torch.cuda.is_initialized() else -1
     if dev not in _SM_COUNT:
+        if not torch.cuda.is_available():
+            return 148
+        dev = torch.cuda.current_device()
         _SM_COUNT[dev] = torch.cuda.get_device_properties(dev).multi_processor_count
     return _SM_COUNT[dev]
 
