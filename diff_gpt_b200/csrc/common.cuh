@@ -28,9 +28,20 @@ int launch_status(const char* what);  // cudaGetLastError -> DGPT_OK / DGPT_E_CU
 // dep_wait() before it touches anything the previous kernel wrote.  dep_wait() is a no-op otherwise.
 bool dep_launch_enabled();
 __device__ __forceinline__ void dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// The next kernel may be made resident from here on (it waits for this one's end in its own dep_wait).
+__device__ __forceinline__ void dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void dep_begin() {
+  dep_launch();
+  dep_wait();
+}
+
+// Rows up to which the kernels of a token's chain are launched dependent.  Such a chain is bound by the time from one kernel's end to the
+// next one's first instruction: a Kipolix token (8 layers, 88 launches) 400 -> 358 us with its host work.  With more rows the blocks made
+// resident early take room from the kernel that is still running (see dep_launch_enabled).
+constexpr long long kFewRows = 4;
 
 template <typename... P, typename... A>
-inline void launch_dep(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
+inline void launch_few(bool few, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
@@ -38,10 +49,14 @@ inline void launch_dep(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem,
   cfg.stream = st;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = dep_launch_enabled() ? 1 : 0;
+  attr[0].val.programmaticStreamSerializationAllowed = few || dep_launch_enabled() ? 1 : 0;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);  // errors surface through launch_status()
+}
+template <typename... P, typename... A>
+inline void launch_dep(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
+  launch_few(false, kernel, grid, block, smem, st, static_cast<A&&>(args)...);
 }
 
 constexpr float kRmsEps = 1.1920928955078125e-07f;  // FLT_EPSILON: F.rms_norm's default eps

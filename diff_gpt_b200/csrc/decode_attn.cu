@@ -54,7 +54,7 @@ decode_attn_kernel(const T* __restrict__ q, long long q_stride, KvView kv, const
                    float* __restrict__ part_lse, int n_splits, int R, int H, float scale_log2) {
   using Cfg = DecodeCfg<T, D>;
   constexpr int VEC = Cfg::VEC, LPT = Cfg::LPT, TPW = Cfg::TPW;
-  dep_wait();
+  dep_begin();
   const long long rh = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (rh >= (long long)R * H) return;
   const int r = (int)(rh / H), h = (int)(rh - (long long)r * H);
@@ -215,6 +215,7 @@ __global__ void decode_combine_kernel(const float* __restrict__ ws_ml, const flo
                                       const float* __restrict__ prefix_o, const float* __restrict__ prefix_lse,
                                       const T* __restrict__ gate, long long gate_stride, T* __restrict__ y,
                                       long long y_stride, int R, int H, int D) {
+  dep_begin();
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long RH = (long long)R * H;
   if (idx >= RH * D) return;
@@ -307,14 +308,14 @@ static int decode_launch(const void* q, long long q_stride, const KvView& kv, co
                q_stride, kv, len0, start1, len1, step_ptr, prefix_o, prefix_lse, static_cast<const T*>(gate), gate_stride,
                static_cast<T*>(y), y_stride, ws_ml, ws_o, part_o, part_lse, n_splits, R, H, scale_log2);
   else
-    launch_dep(decode_attn_kernel<T, D, kDecLoads, kDecMinCtas>, grid, dim3(128), 0, st, static_cast<const T*>(q),
+    launch_few(R <= kFewRows, decode_attn_kernel<T, D, kDecLoads, kDecMinCtas>, grid, dim3(128), 0, st, static_cast<const T*>(q),
                q_stride, kv, len0, start1, len1, step_ptr, prefix_o, prefix_lse, static_cast<const T*>(gate), gate_stride,
                static_cast<T*>(y), y_stride, ws_ml, ws_o, part_o, part_lse, n_splits, R, H, scale_log2);
   if (int e = launch_status("decode_attn")) return e;
   if (n_splits > 1) {
     const long long n = RH * D;
-    decode_combine_kernel<T><<<(unsigned)((n + 255) / 256), 256, 0, st>>>(
-        ws_ml, ws_o, n_splits, prefix_o, prefix_lse, static_cast<const T*>(gate), gate_stride, static_cast<T*>(y),
+    launch_few(
+        R <= kFewRows, decode_combine_kernel<T>, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, st, ws_ml, ws_o, n_splits, prefix_o, prefix_lse, static_cast<const T*>(gate), gate_stride, static_cast<T*>(y),
         y_stride, R, H, D);
     return launch_status("decode_combine");
   }

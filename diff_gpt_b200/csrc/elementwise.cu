@@ -39,6 +39,7 @@ bool dep_launch_enabled() {
 template <typename T>
 __global__ void embed_rmsnorm_kernel(const int* __restrict__ ids, const T* __restrict__ emb,
                                      T* __restrict__ out, long long n_tokens, int C, int V) {
+  dep_launch();
   const long long tok = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (tok >= n_tokens) return;
   const int lane = threadIdx.x & 31;
@@ -247,7 +248,7 @@ depthmix_vec_kernel(CandPtrs cands, int n_cands, const T* __restrict__ w, T* __r
                     T* __restrict__ out_rn, float* __restrict__ inv_out, int inv_out_index, long long rows, int C) {
   constexpr int VEC = Io<T>::kVec16;
   constexpr int E = NV * VEC;
-  dep_wait();
+  dep_begin();
   const long long row = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (row >= rows) return;
   const int lane = threadIdx.x & 31;
@@ -373,7 +374,7 @@ static int depthmix_launch(const CandPtrs& cp, int n, const void* w, void* out_h
   if (vec) {
     const int nv = (C / Io<T>::kVec16 + 31) / 32;
 #define DGPT_MIXV(K, G, ...)                                                                              \
-  launch_dep(K<T, __VA_ARGS__>, dim3(G), dim3(warps * 32), 0, st, cp, n, static_cast<const T*>(w), \
+  launch_few(rows <= kFewRows, K<T, __VA_ARGS__>, dim3(G), dim3(warps * 32), 0, st, cp, n, static_cast<const T*>(w), \
              static_cast<T*>(out_h), static_cast<T*>(out_rn), inv_out, inv_out_index, rows, C)
     // Ahead where the candidates do not fit L2 (126 MB): from memory the fetches in flight count, from L2 the extra trip through shared
     // memory costs more than it hides (4096 x 768, 13 candidates: 20.1 against 17.9 us).

@@ -24,15 +24,29 @@ constexpr int kGvWarps = 4, kGvAhead = 4;  // pieces of each row in flight
 template <int MM, int EPI, bool SHARE>
 __global__ void __launch_bounds__(32 * kGvWarps) gemv_kernel(const GemvParams p) {
   __shared__ float sums[kGvWarps][2 * MM];
-  dep_wait();
+  dep_launch();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int pair = SHARE ? blockIdx.x : blockIdx.x * kGvWarps + warp;
-  if (!SHARE && 2 * pair >= p.N) return;
+  if (!SHARE && 2 * pair >= p.N) {
+    dep_wait();  // no CTA ends before the kernel it depends on
+    return;
+  }
   const int first = SHARE ? warp : 0, step = SHARE ? kGvWarps : 1;  // of the pieces of 256 columns
   const __nv_bfloat16* w0 = p.w + (long long)(2 * pair) * p.w_rs;
   const __nv_bfloat16* w1 = w0 + p.w_rs;
   float acc[2 * MM] = {};
   const int n_pieces = (p.K + 255) / 256;
+  // The weights of the first round come from memory into L2 while the kernel before is still at work.  (Into L2 only: should that kernel
+  // have written them, the loads behind the wait see it.)
+#pragma unroll
+  for (int u = 0; u < kGvAhead; ++u) {
+    const int k = (first + u * step) * 256 + lane * 8;
+    if (k < p.K && (lane & 7) == 0) {  // a line of 128 bytes
+      asm volatile("prefetch.global.L2 [%0];" ::"l"(w0 + k));
+      asm volatile("prefetch.global.L2 [%0];" ::"l"(w1 + k));
+    }
+  }
+  dep_wait();
   for (int c0 = first; c0 < n_pieces; c0 += step * kGvAhead) {
     uint4 r0[kGvAhead], r1[kGvAhead];
 #pragma unroll
@@ -117,11 +131,11 @@ static void gemv_run(const GemvParams& p, cudaStream_t st) {
   const bool share = pairs < 148 * 16 && p.K >= 512;
   const dim3 grid((unsigned)(share ? pairs : (pairs + kGvWarps - 1) / kGvWarps)), block(32 * kGvWarps);
   if (p.M == 1) {
-    if (share) launch_dep(gemv_kernel<1, EPI, true>, grid, block, 0, st, p);
-    else launch_dep(gemv_kernel<1, EPI, false>, grid, block, 0, st, p);
+    if (share) launch_few(true, gemv_kernel<1, EPI, true>, grid, block, 0, st, p);
+    else launch_few(true, gemv_kernel<1, EPI, false>, grid, block, 0, st, p);
   } else {
-    if (share) launch_dep(gemv_kernel<2, EPI, true>, grid, block, 0, st, p);
-    else launch_dep(gemv_kernel<2, EPI, false>, grid, block, 0, st, p);
+    if (share) launch_few(true, gemv_kernel<2, EPI, true>, grid, block, 0, st, p);
+    else launch_few(true, gemv_kernel<2, EPI, false>, grid, block, 0, st, p);
   }
 }
 

@@ -36,6 +36,7 @@ embed_streams_kernel(const int* __restrict__ ids, const int* prev_in, int* prev_
                      T* __restrict__ h, int Tn, int C) {
   extern __shared__ __align__(16) float su[];
   __shared__ float scratch[40];
+  dep_launch();  // (launched the plain way: what came before a token's chain is complete when the chain begins)
   const long long row = blockIdx.x;
   const int s = (int)(row / Tn), t = (int)(row - (long long)s * Tn);
   const int id = min(max(ids[row], 0), V - 1);
@@ -72,6 +73,7 @@ streams_step_kernel(const float* x, long long x_stride, const T* __restrict__ y,
                     float* x_new, long long x_new_stride, T* __restrict__ h, int C) {
   extern __shared__ __align__(16) float su[];
   __shared__ float scratch[40], sm[SM * SM + 2 * SM];
+  dep_begin();
   const long long row = blockIdx.x;
   for (int i = threadIdx.x; i < SM * SM + 2 * SM; i += blockDim.x) {  // unused streams get zeros
     float v = 0.f;
@@ -132,6 +134,7 @@ streams_final_kernel(const float* __restrict__ x, long long x_stride, const T* _
                      const int* __restrict__ row_index, T* __restrict__ h, long long n, int C) {
   extern __shared__ __align__(16) float su[];
   __shared__ float scratch[40];
+  dep_begin();
   const long long row = blockIdx.x;
   long long src = row_index ? (long long)row_index[row] : row;
   src = src < 0 ? 0 : (src >= n ? n - 1 : src);
@@ -219,7 +222,7 @@ extern "C" int dgpt_streams_step(const float* x, int64_t x_stream_stride, const 
                   al16(x_new) && al16(h);
   const int th = row_threads(v4 ? C / 4 : C);
 #define DGPT_SS(TT, VV, SS)                                                                                             \
-  streams_step_kernel<TT, VV, SS><<<(unsigned)rows, th, smem, st>>>(x, x_stream_stride, static_cast<const TT*>(y), mix, out, a, \
+  launch_few(rows <= kFewRows, streams_step_kernel<TT, VV, SS>, dim3((unsigned)rows), dim3(th), smem, st, x, x_stream_stride, static_cast<const TT*>(y), mix, out, a, \
                                                                     S, w, eps, x_new, x_new_stream_stride, static_cast<TT*>(h), C)
 #define DGPT_SSV(TT, VV)              \
   do {                                \
@@ -252,7 +255,7 @@ extern "C" int dgpt_streams_final(const float* x, int64_t x_stream_stride, const
   const bool v4 = C % 4 == 0 && x_stream_stride % 4 == 0 && al16(x) && al16(y) && al16(w) && al16(h);
   const int th = row_threads(v4 ? C / 4 : C);
 #define DGPT_SF(TT, VV)                                                                                                  \
-  streams_final_kernel<TT, VV><<<(unsigned)n_out, th, smem, st>>>(x, x_stream_stride, static_cast<const TT*>(y), mix, out, S, w, \
+  launch_few(n_out <= kFewRows, streams_final_kernel<TT, VV>, dim3((unsigned)n_out), dim3(th), smem, st, x, x_stream_stride, static_cast<const TT*>(y), mix, out, S, w, \
                                                                   eps, row_index, static_cast<TT*>(h), (long long)n, C)
   if (dtype == DGPT_F32) {
     if (v4) DGPT_SF(float, 4);

@@ -50,6 +50,7 @@ template <typename T, int NV>
 __global__ void latent_append_kernel(const T* __restrict__ in, long long in_rs, const float* __restrict__ w, float eps, int r_norm,
                                      KvView kv, const int* __restrict__ slot0, const int* __restrict__ step_ptr, int n_seq, int Tn,
                                      int r, T* __restrict__ flat, int* status) {
+  dep_begin();
   const long long tok = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (tok >= (long long)n_seq * Tn) return;
   const int lane = threadIdx.x & 31;
@@ -223,6 +224,7 @@ template <typename T>
 __global__ void __launch_bounds__(128) latent_combine_kernel(const LatentArgs a) {
   __shared__ float wt[kLatMaxSplits];
   __shared__ float scratch[40];
+  dep_begin();
   const long long RH = (long long)a.n_seq * a.Tn * a.H;
   const long long rh = blockIdx.x;
   const long long row = rh / a.H;
@@ -313,7 +315,7 @@ extern "C" int dgpt_latent_append(const void* in, int64_t in_row_stride, const f
   const bool wide = r == r_norm && in_row_stride % vec == 0 && al16(in) && al16(w) && al16(flat) && kv->page_stride % vec == 0;
   const int nv = wide ? (r / vec + 31) / 32 : 0;
 #define DGPT_LA(TT, NV)                                                                                                          \
-  latent_append_kernel<TT, NV><<<grid, 256, 0, st>>>(static_cast<const TT*>(in), in_row_stride, w, eps, r_norm, view, seq_slot0, \
+  launch_few(n <= kFewRows, latent_append_kernel<TT, NV>, dim3(grid), dim3(256), 0, st, static_cast<const TT*>(in), in_row_stride, w, eps, r_norm, view, seq_slot0, \
                                                      step_ptr, n_seq, T, r, static_cast<TT*>(flat), status)
 #define DGPT_LAT(TT)                    \
   do {                                  \
@@ -386,8 +388,8 @@ static int row_attn(const char* what, const void* q, int64_t q_row_stride, const
   else e = latent_simt_launch<__nv_bfloat16>(a, st);
   if (e || n_splits == 1) return e;
   const long long RH = R * H;
-  if (dtype == DGPT_F32) latent_combine_kernel<float><<<(unsigned)RH, 128, 0, st>>>(a);
-  else latent_combine_kernel<__nv_bfloat16><<<(unsigned)RH, 128, 0, st>>>(a);
+  const auto combine = dtype == DGPT_F32 ? latent_combine_kernel<float> : latent_combine_kernel<__nv_bfloat16>;
+  launch_few(R <= kFewRows, combine, dim3((unsigned)RH), dim3(128), 0, st, a);
   return launch_status("latent_combine");
 }
 

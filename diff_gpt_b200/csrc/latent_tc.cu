@@ -210,7 +210,7 @@ latent_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
-  dep_wait();
+  dep_begin();
 
   if (warp == 5) {
     // ================= loader =================
@@ -562,7 +562,7 @@ static int lt_launch(const CUtensorMap& mq, const CUtensorMap& mc, const LtParam
     set_error("latent_attn: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
     return DGPT_E_CUDA;
   }
-  launch_dep(latent_tc_kernel<NB, HS, SHARED>, dim3(grid), dim3(kLtThreads), smem, st, mq, mc, p);
+  launch_few(p.n_rows <= kFewRows, latent_tc_kernel<NB, HS, SHARED>, dim3(grid), dim3(kLtThreads), smem, st, mq, mc, p);
   return launch_status("latent_attn");
 }
 

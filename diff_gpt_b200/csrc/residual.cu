@@ -49,6 +49,7 @@ __device__ __forceinline__ FVec<VEC> depth_sum(const float* __restrict__ slab, l
 template <typename T, int VEC>
 __global__ void embed_scale_kernel(const int* __restrict__ ids, const T* __restrict__ emb, float* __restrict__ out,
                                    long long n, int C, int V, float scale) {
+  dep_launch();
   const int cv = C / VEC;
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n * cv) return;
@@ -69,6 +70,7 @@ __global__ void __launch_bounds__(kRowThreads)
 norm_add_kernel(const T* __restrict__ y, const float* __restrict__ w, float eps, const float* x, float* out, T* __restrict__ u,
                 int C) {
   __shared__ float scratch[40];
+  dep_begin();
   const long long row = blockIdx.x;
   const int cv = C / VEC;
   FVec<VEC> r[NV];
@@ -106,6 +108,7 @@ __global__ void __launch_bounds__(128)
 depth_avg_conv_kernel(const float* __restrict__ slab, long long term_stride, int terms, const float* __restrict__ coef,
                       const float* __restrict__ cw, int taps, const float* state_in, float* state_out, float* x_out,
                       T* __restrict__ h_out, int n_seq, int Tn, int seg, int n_seg, int C) {
+  dep_begin();
   const int cv = C / VEC;
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= (long long)n_seq * n_seg * cv) return;
@@ -170,6 +173,7 @@ layer_tail_kernel(const T* __restrict__ y, const float* __restrict__ nw, float e
                   long long term_stride, int terms, const float* __restrict__ coef, const float* __restrict__ cw, int taps,
                   float* state, float* __restrict__ x_out, T* __restrict__ h_out, int C) {
   __shared__ float scratch[40];
+  dep_begin();
   const long long row = blockIdx.x;
   const int cv = C / VEC;
   FVec<VEC> r[NV];
@@ -225,6 +229,7 @@ depth_avg_norm_kernel(const float* __restrict__ slab, long long term_stride, int
                       const float* __restrict__ w, float eps, const int* __restrict__ row_index, T* __restrict__ out,
                       long long n, int C) {
   __shared__ float scratch[40];
+  dep_begin();
   const long long row = blockIdx.x;
   long long src = row_index ? (long long)row_index[row] : row;
   src = src < 0 ? 0 : (src >= n ? n - 1 : src);
@@ -289,11 +294,11 @@ using namespace dgpt;
 #define DGPT_ROW_DISPATCH(KERNEL, TT, VV, ...)                                                                     \
   do {                                                                                                             \
     const int cv_ = C / VV, th_ = row_threads(cv_), nv_ = (cv_ + th_ - 1) / th_;                                   \
-    if (nv_ <= 1) KERNEL<TT, VV, 1><<<(unsigned)rows_, th_, 0, st>>>(__VA_ARGS__);                                 \
-    else if (nv_ <= 2) KERNEL<TT, VV, 2><<<(unsigned)rows_, th_, 0, st>>>(__VA_ARGS__);                            \
-    else if (nv_ <= 4) KERNEL<TT, VV, 4><<<(unsigned)rows_, th_, 0, st>>>(__VA_ARGS__);                            \
-    else if (nv_ <= 8) KERNEL<TT, VV, 8><<<(unsigned)rows_, th_, 0, st>>>(__VA_ARGS__);                            \
-    else if (nv_ <= 16) KERNEL<TT, VV, 16><<<(unsigned)rows_, th_, 0, st>>>(__VA_ARGS__);                          \
+    if (nv_ <= 1) launch_few(rows_ <= kFewRows, KERNEL<TT, VV, 1>, dim3((unsigned)rows_), dim3(th_), 0, st, __VA_ARGS__);                                 \
+    else if (nv_ <= 2) launch_few(rows_ <= kFewRows, KERNEL<TT, VV, 2>, dim3((unsigned)rows_), dim3(th_), 0, st, __VA_ARGS__);                            \
+    else if (nv_ <= 4) launch_few(rows_ <= kFewRows, KERNEL<TT, VV, 4>, dim3((unsigned)rows_), dim3(th_), 0, st, __VA_ARGS__);                            \
+    else if (nv_ <= 8) launch_few(rows_ <= kFewRows, KERNEL<TT, VV, 8>, dim3((unsigned)rows_), dim3(th_), 0, st, __VA_ARGS__);                            \
+    else if (nv_ <= 16) launch_few(rows_ <= kFewRows, KERNEL<TT, VV, 16>, dim3((unsigned)rows_), dim3(th_), 0, st, __VA_ARGS__);                          \
     else {                                                                                                         \
       set_error(#KERNEL ": width %d is not built", C);                                                             \
       return DGPT_E_UNSUPPORTED;                                                                                   \
@@ -365,7 +370,7 @@ extern "C" int dgpt_depth_avg_conv(const float* slab, int64_t term_stride, int32
   const long long work = (long long)n_seq * n_seg * cv;
   const unsigned grid = (unsigned)((work + 127) / 128);
 #define DGPT_DC(TT, VV, TP)                                                                                               \
-  depth_avg_conv_kernel<TT, VV, TP><<<grid, 128, 0, st>>>(slab, term_stride, terms, coef, conv_w, taps, state_in, state_out, \
+  launch_few((long long)n_seq * T <= kFewRows, depth_avg_conv_kernel<TT, VV, TP>, dim3(grid), dim3(128), 0, st, slab, term_stride, terms, coef, conv_w, taps, state_in, state_out, \
                                                           x_out, static_cast<TT*>(h_out), n_seq, T, seg, n_seg, C)
 #define DGPT_DCT(TT, VV)                \
   do {                                  \

@@ -39,6 +39,7 @@ __device__ __forceinline__ float silu_value(float z) { return z / (1.f + expf(-z
 template <typename T>
 __global__ void __launch_bounds__(kRetThreads) retention_decode_kernel(const RetentionArgs a) {
   extern __shared__ __align__(16) float ret_smem[];
+  dep_begin();
   const int dim = a.dim, e = a.vdim, cols = e >> 2;
   const int groups = kRetThreads / cols;
   float* sq = ret_smem;             // [dim]
@@ -218,7 +219,7 @@ static int retention_recurrent(const RetentionArgs& a, cudaStream_t st) {
   if (fused) {
     const int groups = kRetThreads / (e / 4);
     const size_t smem = ((size_t)2 * a.dim_pad + (size_t)groups * e) * 4;
-    retention_decode_kernel<T><<<(unsigned)(a.n_seq * a.H), kRetThreads, smem, st>>>(a);
+    launch_few(a.n_seq <= kFewRows, retention_decode_kernel<T>, dim3((unsigned)(a.n_seq * a.H)), dim3(kRetThreads), smem, st, a);
     return launch_status("retention_decode");
   }
   // the widest slice of value columns whose state fits; a few CTAs per head are welcome while there are few heads

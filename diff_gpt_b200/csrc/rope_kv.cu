@@ -109,7 +109,7 @@ __global__ void rope_qknorm_kvappend_vec_kernel(const T* __restrict__ q, const T
   constexpr int VEC = Io<T>::kVec16;
   constexpr int LPH = D / VEC;
   static_assert(LPH >= 1 && LPH <= 32 && (LPH & (LPH - 1)) == 0, "unsupported head_dim");
-  dep_wait();
+  dep_begin();
   const long long unit = ((long long)blockIdx.x * blockDim.x + threadIdx.x) / LPH;  // (token, head)
   const int e = threadIdx.x % LPH;
   const long long total = (long long)n_seq * T_len * H;
@@ -163,7 +163,7 @@ static int rope_vec_launch(const void* q, const void* k, const void* v, long lon
   constexpr int LPH = D / Io<T>::kVec16;
   const long long threads = (long long)n_seq * T_len * H * LPH;
   const unsigned grid = (unsigned)((threads + 255) / 256);
-  launch_dep(rope_qknorm_kvappend_vec_kernel<T, D>, dim3(grid), dim3(256), 0, st, static_cast<const T*>(q),
+  launch_few((long long)n_seq * T_len <= kFewRows, rope_qknorm_kvappend_vec_kernel<T, D>, dim3(grid), dim3(256), 0, st, static_cast<const T*>(q),
              static_cast<const T*>(k), static_cast<const T*>(v), in_stride, static_cast<T*>(q_out), q_out_stride,
              static_cast<const T*>(cs), table_len, view, pos0, slot0, step_ptr, n_seq, T_len, H, status);
   return launch_status("rope_qknorm_kvappend");
@@ -289,6 +289,7 @@ template <typename T>
 __global__ void __launch_bounds__(kRowsThreads)
 proj_norm_rope_append_kernel(const T* __restrict__ in, T* __restrict__ q_out, const KvView kv, const ProjArgs a) {
   __shared__ float scratch[40], scratch2[40];
+  dep_begin();
   const long long tok = blockIdx.x;
   const int s = (int)(tok / a.Tn), t = (int)(tok - (long long)s * a.Tn), tid = threadIdx.x;
   const int step = a.step_ptr ? *a.step_ptr : 0;
@@ -345,7 +346,8 @@ static int proj_launch(const void* in, void* q_out, const KvView& view, const Pr
   T* q = static_cast<T*>(q_out);
   const int nv = (a.HD + a.GD + 32 * Io<T>::kVec16 - 1) / (32 * Io<T>::kVec16);
   const unsigned grid = (unsigned)((n_tok + 7) / 8);
-  if (n_tok < 148 * 8 || nv > 16) proj_norm_rope_append_kernel<T><<<(unsigned)n_tok, kRowsThreads, 0, st>>>(x, q, view, a);  // few tokens: a CTA each
+  if (n_tok < 148 * 8 || nv > 16) 
+    launch_few(n_tok <= kFewRows, proj_norm_rope_append_kernel<T>, dim3((unsigned)n_tok), dim3(kRowsThreads), 0, st, x, q, view, a);  // few tokens: a CTA each
   else if (nv <= 2) proj_norm_rope_append_warp_kernel<T, 2><<<grid, 256, 0, st>>>(x, q, view, a, n_tok);
   else if (nv <= 4) proj_norm_rope_append_warp_kernel<T, 4><<<grid, 256, 0, st>>>(x, q, view, a, n_tok);
   else if (nv <= 6) proj_norm_rope_append_warp_kernel<T, 6><<<grid, 256, 0, st>>>(x, q, view, a, n_tok);
