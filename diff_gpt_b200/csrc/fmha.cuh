@@ -121,6 +121,10 @@ __device__ __forceinline__ int tile_of(int j, int n_window, int tile0) {
 // warp-level kernel (fmha_simt.cu)
 int fmha_simt(const FmhaArgs& a, const KvView& kv, cudaStream_t st);
 
+// short sequences with small heads (fmha_mma.cu); `keys`: the most that a query sees
+bool fmha_mma_supported(const FmhaArgs& a, const KvView& kv, long long keys);
+int fmha_mma(const FmhaArgs& a, const KvView& kv, long long keys, cudaStream_t st);
+
 // tcgen05 / TMEM kernel (fmha_tc.cu)
 bool fmha_tc_supported(const FmhaArgs& a, const dgpt_kv_layout& kv);
 int fmha_tc(const FmhaArgs& a, const dgpt_kv_layout& kv, cudaStream_t st);

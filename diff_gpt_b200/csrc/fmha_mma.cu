@@ -1,0 +1,340 @@
+// Attention of short sequences with small heads (bf16, head_dim 32 or 64) with the products in registers: mma.sync on fragments, the keys and
+// values of a (sequence, head) in shared memory as a whole.
+//
+// What bounds such heads is not the tensor pipe but the softmax: a 128 x 128 tile of scores is 16384 exponentials, 1024 clocks of the
+// SM's exponential units, where its two products are 256 clocks of tcgen05 (head_dim 32).  The tcgen05 kernel spends 4600 clocks on such
+// a tile: each of its few softmax warps waits for a commit, a TMEM load, a barrier, one after the other.  Here a warp is on its own from
+// its rows' first score to their last output - scores and probabilities never leave its registers - and sixteen of them fill the SM's
+// pipes among themselves.
+//   A warp takes 16 MT rows and walks over their keys 32 at a time: MT x 4 tiles of 16 x 8 scores, exponentials against a running maximum
+//   that only moves when it is exceeded by 2^4 (one vote a step; 2^8 left the
+//   largest probabilities further from a whole power of two: error against float64 0.00306 instead of 0.00303), probabilities rounded to bf16 as the A operand of the second
+//   product.  MT = 2 for heads of 32, so that each key fragment read from shared memory serves 32 rows; heads of 64 have registers for 16.
+//   SPLIT: each probability as a pair of bf16 numbers, two second products (see fmha_full).
+//   CTAs of 8 warps, two an SM; blocks of rows are dealt to the warps in snake order, so that under the causal rule short and long rows
+//   come together.
+// Measured with the gate, us, tcgen05 kernels / this: 256 x 8 heads of 32 x 512 keys 326 / 238, x 256 133 / 110, x 128 52 / 70; 64 x 8 x 512 88 / 67;
+// 1 x 8 x 512 10.7 / 17; keys that are not whole tiles (pairs) 256 x 8 x 200 161 / 106; heads of 64 184 / 158, x 33 59 / 46, whole tiles level.
+#include "fmha.cuh"
+
+namespace dgpt {
+
+constexpr int kMmWarps = 8, kMmThreads = 32 * kMmWarps, kMmKeys = 32;  // keys of a step
+
+struct MmaArgs {
+  const __nv_bfloat16* q;
+  long long q_bs, q_rs;
+  KvView kv;
+  const int* kv_len;
+  int kv_len_all;
+  __nv_bfloat16* o;
+  long long o_bs, o_rs;
+  const __nv_bfloat16* gate;
+  long long gate_rs;
+  int H, Tq, q_offset, causal, splits, room;  // room: keys that fit
+  float scale_log2;
+};
+
+template <int D>
+__device__ __forceinline__ uint32_t mm_at(int row, int chunk) {  // byte offset of 8 columns of a row: eight rows side by side do not collide
+  return D == 32 ? row * 64 + ((chunk ^ ((row >> 1) & 3)) << 4) : row * 128 + ((chunk ^ (row & 7)) << 4);
+}
+__device__ __forceinline__ void ldsm4(uint32_t addr, uint32_t (&r)[4]) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
+}
+__device__ __forceinline__ void ldsm4t(uint32_t addr, uint32_t (&r)[4]) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(addr));
+}
+__device__ __forceinline__ void mma16816(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
+  const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
+  return *reinterpret_cast<const uint32_t*>(&v);
+}
+__device__ __forceinline__ float mm_ex2(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
+template <int D, int MT, bool SPLIT>
+__global__ void __launch_bounds__(kMmThreads, 2) fmha_mma_kernel(const __grid_constant__ MmaArgs p) {
+  constexpr int KS = D / 16, NT = kMmKeys / 8, OT = D / 8, kChunks = D / 8, kRows = 16 * MT;
+  extern __shared__ __align__(1024) uint8_t smem[];
+  const uint32_t sK = (uint32_t)__cvta_generic_to_shared(smem), sV = sK + (uint32_t)p.room * D * 2;
+  const int j = blockIdx.x % p.splits, bh = blockIdx.x / p.splits, h = bh % p.H, b = bh / p.H;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int n_blk = (p.Tq + kRows - 1) / kRows, G = p.splits * kMmWarps, me = j * kMmWarps + warp;
+  const int cap = p.kv.page_table ? p.kv.max_pages * p.kv.page_tokens : p.kv.page_tokens;
+  const int klen = min(min(p.kv_len ? p.kv_len[b] : p.kv_len_all, cap), p.room);
+  // keys that the CTA's last rows see
+  int last_blk = 0;
+  for (int r = 0; r * G < n_blk; ++r) last_blk = max(last_blk, min(n_blk - 1, (r & 1) ? r * G + G - 1 - j * kMmWarps : r * G + j * kMmWarps + kMmWarps - 1));
+  const int need = max(0, p.causal ? min(klen, p.q_offset + min(p.Tq, (last_blk + 1) * kRows)) : klen);
+  const int rows = (need + kMmKeys - 1) / kMmKeys * kMmKeys;
+  const __nv_bfloat16 *kb = static_cast<const __nv_bfloat16*>(p.kv.k), *vb = static_cast<const __nv_bfloat16*>(p.kv.v);
+#pragma unroll 2
+  for (int i = threadIdx.x; i < rows * kChunks; i += kMmThreads) {
+    const int row = i / kChunks, c = i - row * kChunks;
+    long long off = -1;
+    if (row < need) {
+      const int lp = p.kv.page_table ? row / p.kv.page_tokens : 0;
+      const long long pg = p.kv.page_table ? (long long)p.kv.page_table[(long long)b * p.kv.max_pages + lp] : (long long)b;
+      if (!(p.kv.page_table && (pg < 0 || (p.kv.n_pages > 0 && pg >= p.kv.n_pages))))
+        off = pg * p.kv.page_stride + (long long)h * p.kv.head_stride + (long long)(row - lp * p.kv.page_tokens) * (p.kv.token_stride ? p.kv.token_stride : D) + c * 8;
+    }
+    const uint32_t at = mm_at<D>(row, c);
+    const int bytes = off >= 0 ? 16 : 0;  // 0: filled with zeros, so that 0 * x stays 0
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(sK + at), "l"(kb + (off >= 0 ? off : 0)), "r"(bytes) : "memory");
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(sV + at), "l"(vb + (off >= 0 ? off : 0)), "r"(bytes) : "memory");
+  }
+  asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
+  __syncthreads();
+
+#pragma unroll 1
+  for (int r = 0; r * G < n_blk; ++r) {
+    const int blk = (r & 1) ? r * G + G - 1 - me : r * G + me;
+    if (blk >= n_blk) continue;
+    const int r0 = blk * kRows;
+    uint32_t qa[MT][KS][4];
+#pragma unroll
+    for (int m = 0; m < MT; ++m) {
+      const __nv_bfloat16* q0 = p.q + (long long)b * p.q_bs + (long long)min(r0 + 16 * m + g, p.Tq - 1) * p.q_rs + h * D + 2 * t;
+      const __nv_bfloat16* q1 = p.q + (long long)b * p.q_bs + (long long)min(r0 + 16 * m + g + 8, p.Tq - 1) * p.q_rs + h * D + 2 * t;
+#pragma unroll
+      for (int k = 0; k < KS; ++k) {
+        qa[m][k][0] = __ldg(reinterpret_cast<const uint32_t*>(q0 + 16 * k));
+        qa[m][k][1] = __ldg(reinterpret_cast<const uint32_t*>(q1 + 16 * k));
+        qa[m][k][2] = __ldg(reinterpret_cast<const uint32_t*>(q0 + 16 * k + 8));
+        qa[m][k][3] = __ldg(reinterpret_cast<const uint32_t*>(q1 + 16 * k + 8));
+      }
+    }
+    float o[MT][OT][4], top[MT][2], l[MT][2];
+#pragma unroll
+    for (int m = 0; m < MT; ++m) {
+      top[m][0] = top[m][1] = -INFINITY;
+      l[m][0] = l[m][1] = 0.f;
+#pragma unroll
+      for (int n = 0; n < OT; ++n) o[m][n][0] = o[m][n][1] = o[m][n][2] = o[m][n][3] = 0.f;
+    }
+    const int end = p.causal ? min(klen, p.q_offset + min(p.Tq, r0 + kRows)) : klen;
+#pragma unroll 1
+    for (int k0 = 0; k0 < end; k0 += kMmKeys) {
+      float s[MT][NT][4];
+#pragma unroll
+      for (int n = 0; n < NT; ++n) {
+#pragma unroll
+        for (int m = 0; m < MT; ++m) s[m][n][0] = s[m][n][1] = s[m][n][2] = s[m][n][3] = 0.f;
+#pragma unroll
+        for (int kk = 0; kk < KS / 2; ++kk) {
+          uint32_t kf[4];
+          ldsm4(sK + mm_at<D>(k0 + 8 * n + (lane & 7), 4 * kk + (lane >> 3)), kf);
+#pragma unroll
+          for (int m = 0; m < MT; ++m) {
+            mma16816(s[m][n], qa[m][2 * kk], kf[0], kf[1]);
+            mma16816(s[m][n], qa[m][2 * kk + 1], kf[2], kf[3]);
+          }
+        }
+      }
+      if (k0 + kMmKeys > klen || (p.causal && k0 + kMmKeys - 1 > p.q_offset + r0)) {
+#pragma unroll
+        for (int m = 0; m < MT; ++m) {
+#pragma unroll
+          for (int n = 0; n < NT; ++n) {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              const int key = k0 + 8 * n + 2 * t + (e & 1), row = r0 + 16 * m + g + (e >> 1) * 8;
+              if (key >= klen || (p.causal && key > p.q_offset + row)) s[m][n][e] = -INFINITY;
+            }
+          }
+        }
+      }
+      // exponents against the running maxima; if one exceeds its row's by 2^4 the maxima move (always so at a row's first keys)
+      float most = -INFINITY;
+#pragma unroll
+      for (int m = 0; m < MT; ++m) {
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const float ref = top[m][e];
+          float mx = fmaxf(s[m][0][2 * e], s[m][0][2 * e + 1]);
+#pragma unroll
+          for (int n = 1; n < NT; ++n) mx = fmaxf(mx, fmaxf(s[m][n][2 * e], s[m][n][2 * e + 1]));
+          most = fmaxf(most, ref == -INFINITY ? INFINITY : fmaf(mx, p.scale_log2, -ref));
+        }
+      }
+      if (__any_sync(0xffffffffu, most > 4.f)) {
+#pragma unroll
+        for (int m = 0; m < MT; ++m) {
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            float mx = fmaxf(s[m][0][2 * e], s[m][0][2 * e + 1]);
+#pragma unroll
+            for (int n = 1; n < NT; ++n) mx = fmaxf(mx, fmaxf(s[m][n][2 * e], s[m][n][2 * e + 1]));
+            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+            const float now = fmaxf(top[m][e], mx * p.scale_log2);
+            const float alpha = now == -INFINITY ? 1.f : mm_ex2(top[m][e] - now);
+            top[m][e] = now;
+            l[m][e] *= alpha;
+#pragma unroll
+            for (int n = 0; n < OT; ++n) {
+              o[m][n][2 * e] *= alpha;
+              o[m][n][2 * e + 1] *= alpha;
+            }
+          }
+        }
+      }
+#pragma unroll
+      for (int m = 0; m < MT; ++m) {
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const float ref = top[m][e] == -INFINITY ? 0.f : top[m][e];
+#pragma unroll
+          for (int n = 0; n < NT; ++n) {
+            s[m][n][2 * e] = mm_ex2(fmaf(s[m][n][2 * e], p.scale_log2, -ref));
+            s[m][n][2 * e + 1] = mm_ex2(fmaf(s[m][n][2 * e + 1], p.scale_log2, -ref));
+          }
+        }
+      }
+#pragma unroll
+      for (int kk = 0; kk < NT / 2; ++kk) {
+        uint32_t pa[MT][4], pl[SPLIT ? MT : 1][4];
+#pragma unroll
+        for (int m = 0; m < MT; ++m) {
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const float x = s[m][2 * kk + (e >> 1)][2 * (e & 1)], y = s[m][2 * kk + (e >> 1)][2 * (e & 1) + 1];
+            pa[m][e] = pack_bf16(x, y);
+            const float xr = __uint_as_float(pa[m][e] << 16), yr = __uint_as_float(pa[m][e] & 0xffff0000u);
+            if constexpr (SPLIT) {
+              pl[m][e] = pack_bf16(x - xr, y - yr);
+              l[m][e & 1] += x + y;
+            } else {
+              l[m][e & 1] += xr + yr;  // the sum of what the second product weighs the values with
+            }
+          }
+        }
+#pragma unroll
+        for (int n = 0; n < OT / 2; ++n) {
+          uint32_t vf[4];
+          ldsm4t(sV + mm_at<D>(k0 + 16 * kk + ((lane >> 3) & 1) * 8 + (lane & 7), 2 * n + (lane >> 4)), vf);
+#pragma unroll
+          for (int m = 0; m < MT; ++m) {
+            mma16816(o[m][2 * n], pa[m], vf[0], vf[1]);
+            mma16816(o[m][2 * n + 1], pa[m], vf[2], vf[3]);
+            if constexpr (SPLIT) {
+              mma16816(o[m][2 * n], pl[m], vf[0], vf[1]);
+              mma16816(o[m][2 * n + 1], pl[m], vf[2], vf[3]);
+            }
+          }
+        }
+      }
+    }
+    // ---- the rows' results: four lanes hold a row in pairs of columns; they swap them so that each has 16 bytes in a run ----
+#pragma unroll
+    for (int m = 0; m < MT; ++m) {
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        float sum = l[m][e];
+        sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+        sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+        const float inv = sum > 0.f ? 1.f / sum : 0.f;
+        const int row = r0 + 16 * m + g + 8 * e;
+#pragma unroll
+        for (int n4 = 0; n4 < OT; n4 += 4) {
+          uint32_t v[4];
+#pragma unroll
+          for (int n = 0; n < 4; ++n) v[n] = pack_bf16(o[m][n4 + n][2 * e] * inv, o[m][n4 + n][2 * e + 1] * inv);
+          auto pick = [&](int i) { return i == 0 ? v[0] : i == 1 ? v[1] : i == 2 ? v[2] : v[3]; };
+          uint32_t w[4];
+          const uint32_t a0 = pick(t), a1 = __shfl_xor_sync(0xffffffffu, pick(t ^ 1), 1), a2 = __shfl_xor_sync(0xffffffffu, pick(t ^ 2), 2),
+                         a3 = __shfl_xor_sync(0xffffffffu, pick(t ^ 3), 3);  // a_i: from lane t ^ i of the four
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const int x = i ^ t;
+            w[i] = x == 0 ? a0 : x == 1 ? a1 : x == 2 ? a2 : a3;
+          }
+          if (row < p.Tq) {
+            const int col = h * D + 8 * (n4 + t);
+            uint4 out = make_uint4(w[0], w[1], w[2], w[3]);
+            if (p.gate) {
+              const uint4 graw = __ldg(reinterpret_cast<const uint4*>(p.gate + ((long long)b * p.Tq + row) * p.gate_rs + col));
+              float x[8], gv[8];
+              unpack16<__nv_bfloat16>(out, x);
+              unpack16<__nv_bfloat16>(graw, gv);
+#pragma unroll
+              for (int i = 0; i < 8; ++i) x[i] = gated<__nv_bfloat16>(x[i], gv[i]);
+              st16<__nv_bfloat16>(p.o + (long long)b * p.o_bs + (long long)row * p.o_rs + col, x, 1.f);
+            } else {
+              *reinterpret_cast<uint4*>(p.o + (long long)b * p.o_bs + (long long)row * p.o_rs + col) = out;
+            }
+          }
+        }
+      }
+    }
+  }
+}
+
+// What the kernel covers: whole sequences or portions without window, log-sum-exp or fp32 output, `keys` of them at most.
+bool fmha_mma_supported(const FmhaArgs& a, const KvView& kv, long long keys) {
+  auto al16 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
+  return a.dtype == DGPT_BF16 && (a.D == 32 || a.D == 64) && !a.lse && !a.o_f32 && a.window == 0 && !a.hgate &&
+         (a.kv_heads == 0 || a.kv_heads == a.H) && a.max_ctas == 0 && keys >= 1 && keys * a.D * 4 <= 96 * 1024 && al16(a.q) && al16(a.o) &&
+         al16(a.egate) && a.egate_rs % 8 == 0 && (kv.token_stride == 0 || kv.token_stride % 8 == 0) && (a.scale == 0.f);
+}
+
+template <int D, int MT, bool SPLIT>
+static int fmha_mma_launch(const MmaArgs& p, unsigned grid, size_t smem, cudaStream_t st) {
+  cudaError_t e = cudaFuncSetAttribute(fmha_mma_kernel<D, MT, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) {
+    set_error("fmha_mma: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
+    return DGPT_E_CUDA;
+  }
+  fmha_mma_kernel<D, MT, SPLIT><<<grid, kMmThreads, smem, st>>>(p);
+  return launch_status("fmha_mma");
+}
+
+int fmha_mma(const FmhaArgs& a, const KvView& kv, long long keys, cudaStream_t st) {
+  MmaArgs p;
+  p.q = static_cast<const __nv_bfloat16*>(a.q);
+  p.q_bs = a.q_bs;
+  p.q_rs = a.q_rs;
+  p.kv = kv;
+  p.kv_len = a.kv_len;
+  p.kv_len_all = a.kv_len_all;
+  p.o = static_cast<__nv_bfloat16*>(a.o);
+  p.o_bs = a.o_bs;
+  p.o_rs = a.o_rs;
+  p.gate = static_cast<const __nv_bfloat16*>(a.egate);
+  p.gate_rs = a.egate_rs;
+  p.H = a.H;
+  p.Tq = a.Tq;
+  p.q_offset = a.q_offset;
+  p.causal = a.causal;
+  p.scale_log2 = kLog2e / sqrtf((float)a.D);
+  p.room = (int)((keys + kMmKeys - 1) / kMmKeys * kMmKeys);
+  int dev = 0, sms = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (sms <= 0) sms = 148;
+  // one CTA a (sequence, head), or several that share its rows where that leaves room for more CTAs
+  const int rows = a.D == 32 ? 32 : 16, most = (a.Tq + rows * kMmWarps - 1) / (rows * kMmWarps);
+  const long long pairs = (long long)a.B * a.H;
+  long long splits = pairs > 0 ? 2ll * sms / pairs : 1;
+  p.splits = (int)(splits < 1 ? 1 : splits > most ? most : splits);
+  if (pairs * p.splits > 0x7fffffffll) {
+    set_error("fmha_mma: too many sequences");
+    return DGPT_E_ARG;
+  }
+  const unsigned grid = (unsigned)(pairs * p.splits);
+  const size_t smem = (size_t)p.room * a.D * 4;
+  if (a.D == 32) return a.split_p ? fmha_mma_launch<32, 2, true>(p, grid, smem, st) : fmha_mma_launch<32, 2, false>(p, grid, smem, st);
+  return a.split_p ? fmha_mma_launch<64, 1, true>(p, grid, smem, st) : fmha_mma_launch<64, 1, false>(p, grid, smem, st);
+}
+
+}  // namespace dgpt

@@ -249,6 +249,18 @@ static bool simt_own_gate(const FmhaArgs& a) {
   return a.dtype == DGPT_BF16 ? a.Tq >= 8 || pairs <= 512 : a.D <= 16 && pairs <= 1024;
 }
 
+// Whether the kernel with its products in registers is ahead of the tcgen05 kernels (us, those / this).  Heads of 32 over whole tiles: from 256
+// keys and 192 pairs of sequence and head on (16 x 12 x 256 keys 17.8 / 15.7, 256 x 8 x 512 326 / 238, x 128 52 / 70, 1 x 8 x 512 10.7 / 17).  Keys that
+// are not whole tiles, whose probabilities are pairs: up to half a tile (256 x 8 heads of 64 x 33 59 / 46, x 64 62 / 59; of 32 54 / 48) and behind
+// the first tile (x 200 184 / 158; of 32 161 / 106); in between the one tile is all there is to do (x 100 67 / 78).  Few heads of 32 stay: 4 x 8 x 200
+// level, 1 x 8 x 200 10.9 / 11.3.
+static bool fmha_prefers_mma(const FmhaArgs& a, long long keys) {
+  const long long pairs = (long long)a.B * a.H;
+  if (a.D == 32 && pairs < 192) return false;
+  if (a.split_p) return keys <= 64 || (keys > 128 && keys <= (a.D == 32 ? 768 : 320));
+  return a.D == 32 && keys >= 256 && keys <= 768;
+}
+
 static int fmha_full(const void* q, int64_t q_batch_stride, int64_t q_row_stride, const dgpt_kv_layout* kv, const int32_t* kv_len,
                      int32_t kv_len_all, void* o, int64_t o_batch_stride, int64_t o_row_stride, int32_t o_f32, float* lse,
                      const void* egate, int64_t egate_rs, int32_t B, int32_t H, int32_t Tq, int32_t D, int32_t q_offset,
@@ -299,6 +311,7 @@ static int fmha_full(const void* q, int64_t q_batch_stride, int64_t q_row_stride
     set_error("fmha_prefill: the tensor-core kernel does not cover dtype %d, head_dim %d with this layout", dtype, D);
     return DGPT_E_UNSUPPORTED;
   }
+  if (impl == 0 && tc_ok && fmha_prefers_mma(a, span) && fmha_mma_supported(a, view, span)) return fmha_mma(a, view, span, st);
   if (tc_ok && impl != 1) return fmha_tc(a, *kv, st);
   if (egate && !simt_own_gate(a) && (B == 1 || o_batch_stride == (int64_t)Tq * o_row_stride)) {
     a.egate = nullptr;
