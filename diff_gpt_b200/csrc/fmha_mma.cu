@@ -6,16 +6,18 @@
 // a tile: each of its few softmax warps waits for a commit, a TMEM load, a barrier, one after the other.  Here a warp is on its own from
 // its rows' first score to their last output - scores and probabilities never leave its registers - and sixteen of them fill the SM's
 // pipes among themselves.
-//   A warp takes 16 MT rows and walks over their keys 32 at a time: MT x 4 tiles of 16 x 8 scores, exponentials against a running maximum
-//   that only moves when it is exceeded by 2^4 (one vote a step; 2^8 left the
-//   largest probabilities further from a whole power of two: error against float64 0.00306 instead of 0.00303), probabilities rounded to bf16 as the A operand of the second
-//   product.  MT = 2 for heads of 32, so that each key fragment read from shared memory serves 32 rows; heads of 64 have registers for 16.
+//   A warp takes 16 rows and walks over their keys 32 at a time: four tiles of 16 x 8 scores, exponentials against a running maximum that only
+//   moves when it is exceeded by 2^4 (one vote a step; 2^8 left the largest probabilities further from a whole power of two: error against
+//   float64 0.00306 instead of 0.00303), probabilities rounded to bf16 as the A operand of the second product.  (32 rows a warp, which
+//   read half the fragments, 221 us where 16 take 198: the steps are latency, and 24 warps hide more of it than 16.  The next step's scores
+//   issued ahead of a step's exponentials: 242.)
 //   SPLIT: each probability as a pair of bf16 numbers, two second products (see fmha_full).
-//   CTAs of 8 warps, two an SM; blocks of rows are dealt to the warps in snake order, so that under the causal rule short and long rows
+//   CTAs of 8 warps, three an SM (heads of 64: two); blocks of rows are dealt to the warps in snake order, so that under the causal rule short and long rows
 //   come together.
-// Measured with the gate, us, tcgen05 kernels / this: 256 x 8 heads of 32 x 512 keys 326 / 238, x 256 133 / 110, x 128 52 / 70; 64 x 8 x 512 88 / 67;
-// 1 x 8 x 512 10.7 / 17; keys that are not whole tiles (pairs) 256 x 8 x 200 161 / 106; heads of 64 184 / 158, x 33 59 / 46, whole tiles level.
+// Measured with the gate, us, tcgen05 kernels / this: 256 x 8 heads of 32 x 512 keys 328 / 198 (44 % of the exponential units, 38 % of the tensor
+// pipe, 0.56 instructions a clock and scheduler), x 256 133 / 79, x 128 52 / 39; the choice between them is in fmha_simt.cu.
 #include "fmha.cuh"
+#include "tcgen05.cuh"
 
 namespace dgpt {
 
@@ -40,15 +42,15 @@ __device__ __forceinline__ uint32_t mm_at(int row, int chunk) {  // byte offset 
   return D == 32 ? row * 64 + ((chunk ^ ((row >> 1) & 3)) << 4) : row * 128 + ((chunk ^ (row & 7)) << 4);
 }
 __device__ __forceinline__ void ldsm4(uint32_t addr, uint32_t (&r)[4]) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
+  asm("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
 }
 __device__ __forceinline__ void ldsm4t(uint32_t addr, uint32_t (&r)[4]) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+  asm("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
                : "r"(addr));
 }
 __device__ __forceinline__ void mma16816(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
                : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
                : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
@@ -62,9 +64,9 @@ __device__ __forceinline__ float mm_ex2(float x) {
   return y;
 }
 
-template <int D, int MT, bool SPLIT>
-__global__ void __launch_bounds__(kMmThreads, 2) fmha_mma_kernel(const __grid_constant__ MmaArgs p) {
-  constexpr int KS = D / 16, NT = kMmKeys / 8, OT = D / 8, kChunks = D / 8, kRows = 16 * MT;
+template <int D, bool SPLIT>
+__global__ void __launch_bounds__(kMmThreads, D == 32 ? 3 : 2) fmha_mma_kernel(const __grid_constant__ MmaArgs p) {
+  constexpr int KS = D / 16, NT = kMmKeys / 8, OT = D / 8, kChunks = D / 8, kRows = 16;
   extern __shared__ __align__(1024) uint8_t smem[];
   const uint32_t sK = (uint32_t)__cvta_generic_to_shared(smem), sV = sK + (uint32_t)p.room * D * 2;
   const int j = blockIdx.x % p.splits, bh = blockIdx.x / p.splits, h = bh % p.H, b = bh / p.H;
@@ -78,6 +80,13 @@ __global__ void __launch_bounds__(kMmThreads, 2) fmha_mma_kernel(const __grid_co
   const int need = max(0, p.causal ? min(klen, p.q_offset + min(p.Tq, (last_blk + 1) * kRows)) : klen);
   const int rows = (need + kMmKeys - 1) / kMmKeys * kMmKeys;
   const __nv_bfloat16 *kb = static_cast<const __nv_bfloat16*>(p.kv.k), *vb = static_cast<const __nv_bfloat16*>(p.kv.v);
+  // queries and gates of the CTA's rows on their way to L2 under the keys' loads
+  for (int i = threadIdx.x; i < n_blk * kRows; i += kMmThreads) {
+    const int blk = i / kRows, r = blk / G, in = (r & 1) ? G - 1 - (blk - r * G) : blk - r * G;
+    if (in / kMmWarps != j || i >= p.Tq) continue;
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(p.q + (long long)b * p.q_bs + (long long)i * p.q_rs + h * D));
+    if (p.gate) asm volatile("prefetch.global.L2 [%0];" ::"l"(p.gate + ((long long)b * p.Tq + i) * p.gate_rs + h * D));
+  }
 #pragma unroll 2
   for (int i = threadIdx.x; i < rows * kChunks; i += kMmThreads) {
     const int row = i / kChunks, c = i - row * kChunks;
@@ -96,183 +105,156 @@ __global__ void __launch_bounds__(kMmThreads, 2) fmha_mma_kernel(const __grid_co
   asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
   __syncthreads();
 
+  // this lane's place in a fragment's rows: the swizzle repeats every 8 rows, so it is the same for every step
+  uint32_t k_at[KS / 2], v_at[OT / 2];
+#pragma unroll
+  for (int kk = 0; kk < KS / 2; ++kk) k_at[kk] = mm_at<D>(lane & 7, 4 * kk + (lane >> 3));
+#pragma unroll
+  for (int n = 0; n < OT / 2; ++n) v_at[n] = mm_at<D>(((lane >> 3) & 1) * 8 + (lane & 7), 2 * n + (lane >> 4));
+
 #pragma unroll 1
   for (int r = 0; r * G < n_blk; ++r) {
     const int blk = (r & 1) ? r * G + G - 1 - me : r * G + me;
     if (blk >= n_blk) continue;
     const int r0 = blk * kRows;
-    uint32_t qa[MT][KS][4];
-#pragma unroll
-    for (int m = 0; m < MT; ++m) {
-      const __nv_bfloat16* q0 = p.q + (long long)b * p.q_bs + (long long)min(r0 + 16 * m + g, p.Tq - 1) * p.q_rs + h * D + 2 * t;
-      const __nv_bfloat16* q1 = p.q + (long long)b * p.q_bs + (long long)min(r0 + 16 * m + g + 8, p.Tq - 1) * p.q_rs + h * D + 2 * t;
+    uint32_t qa[KS][4];
+    {
+      const __nv_bfloat16* q0 = p.q + (long long)b * p.q_bs + (long long)min(r0 + g, p.Tq - 1) * p.q_rs + h * D + 2 * t;
+      const __nv_bfloat16* q1 = p.q + (long long)b * p.q_bs + (long long)min(r0 + g + 8, p.Tq - 1) * p.q_rs + h * D + 2 * t;
 #pragma unroll
       for (int k = 0; k < KS; ++k) {
-        qa[m][k][0] = __ldg(reinterpret_cast<const uint32_t*>(q0 + 16 * k));
-        qa[m][k][1] = __ldg(reinterpret_cast<const uint32_t*>(q1 + 16 * k));
-        qa[m][k][2] = __ldg(reinterpret_cast<const uint32_t*>(q0 + 16 * k + 8));
-        qa[m][k][3] = __ldg(reinterpret_cast<const uint32_t*>(q1 + 16 * k + 8));
+        qa[k][0] = __ldg(reinterpret_cast<const uint32_t*>(q0 + 16 * k));
+        qa[k][1] = __ldg(reinterpret_cast<const uint32_t*>(q1 + 16 * k));
+        qa[k][2] = __ldg(reinterpret_cast<const uint32_t*>(q0 + 16 * k + 8));
+        qa[k][3] = __ldg(reinterpret_cast<const uint32_t*>(q1 + 16 * k + 8));
       }
     }
-    float o[MT][OT][4], top[MT][2], l[MT][2];
+    float o[OT][4], top[2] = {-INFINITY, -INFINITY}, lsum[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-    for (int m = 0; m < MT; ++m) {
-      top[m][0] = top[m][1] = -INFINITY;
-      l[m][0] = l[m][1] = 0.f;
-#pragma unroll
-      for (int n = 0; n < OT; ++n) o[m][n][0] = o[m][n][1] = o[m][n][2] = o[m][n][3] = 0.f;
-    }
+    for (int n = 0; n < OT; ++n) o[n][0] = o[n][1] = o[n][2] = o[n][3] = 0.f;
     const int end = p.causal ? min(klen, p.q_offset + min(p.Tq, r0 + kRows)) : klen;
 #pragma unroll 1
     for (int k0 = 0; k0 < end; k0 += kMmKeys) {
-      float s[MT][NT][4];
+      const uint32_t kk0 = sK + k0 * (D * 2), vk0 = sV + k0 * (D * 2);
+      float s[NT][4];
 #pragma unroll
       for (int n = 0; n < NT; ++n) {
-#pragma unroll
-        for (int m = 0; m < MT; ++m) s[m][n][0] = s[m][n][1] = s[m][n][2] = s[m][n][3] = 0.f;
+        s[n][0] = s[n][1] = s[n][2] = s[n][3] = 0.f;
 #pragma unroll
         for (int kk = 0; kk < KS / 2; ++kk) {
           uint32_t kf[4];
-          ldsm4(sK + mm_at<D>(k0 + 8 * n + (lane & 7), 4 * kk + (lane >> 3)), kf);
-#pragma unroll
-          for (int m = 0; m < MT; ++m) {
-            mma16816(s[m][n], qa[m][2 * kk], kf[0], kf[1]);
-            mma16816(s[m][n], qa[m][2 * kk + 1], kf[2], kf[3]);
-          }
+          ldsm4(kk0 + k_at[kk] + 8 * n * (D * 2), kf);
+          mma16816(s[n], qa[2 * kk], kf[0], kf[1]);
+          mma16816(s[n], qa[2 * kk + 1], kf[2], kf[3]);
         }
       }
       if (k0 + kMmKeys > klen || (p.causal && k0 + kMmKeys - 1 > p.q_offset + r0)) {
 #pragma unroll
-        for (int m = 0; m < MT; ++m) {
+        for (int n = 0; n < NT; ++n) {
 #pragma unroll
-          for (int n = 0; n < NT; ++n) {
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              const int key = k0 + 8 * n + 2 * t + (e & 1), row = r0 + 16 * m + g + (e >> 1) * 8;
-              if (key >= klen || (p.causal && key > p.q_offset + row)) s[m][n][e] = -INFINITY;
-            }
+          for (int e = 0; e < 4; ++e) {
+            const int key = k0 + 8 * n + 2 * t + (e & 1), row = r0 + g + (e >> 1) * 8;
+            if (key >= klen || (p.causal && key > p.q_offset + row)) s[n][e] = -INFINITY;
           }
         }
       }
       // exponents against the running maxima; if one exceeds its row's by 2^4 the maxima move (always so at a row's first keys)
-      float most = -INFINITY;
+      float mx[2], most = -INFINITY;
 #pragma unroll
-      for (int m = 0; m < MT; ++m) {
+      for (int e = 0; e < 2; ++e) {
+        mx[e] = fmaxf(s[0][2 * e], s[0][2 * e + 1]);
 #pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const float ref = top[m][e];
-          float mx = fmaxf(s[m][0][2 * e], s[m][0][2 * e + 1]);
-#pragma unroll
-          for (int n = 1; n < NT; ++n) mx = fmaxf(mx, fmaxf(s[m][n][2 * e], s[m][n][2 * e + 1]));
-          most = fmaxf(most, ref == -INFINITY ? INFINITY : fmaf(mx, p.scale_log2, -ref));
-        }
+        for (int n = 1; n < NT; ++n) mx[e] = fmaxf(mx[e], fmaxf(s[n][2 * e], s[n][2 * e + 1]));
+        most = fmaxf(most, top[e] == -INFINITY ? INFINITY : fmaf(mx[e], p.scale_log2, -top[e]));
       }
       if (__any_sync(0xffffffffu, most > 4.f)) {
 #pragma unroll
-        for (int m = 0; m < MT; ++m) {
+        for (int e = 0; e < 2; ++e) {
+          float m = fmaxf(mx[e], __shfl_xor_sync(0xffffffffu, mx[e], 1));
+          m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 2));
+          const float now = fmaxf(top[e], m * p.scale_log2), alpha = now == -INFINITY ? 1.f : mm_ex2(top[e] - now);
+          top[e] = now;
+          lsum[2 * e] *= alpha;
+          lsum[2 * e + 1] *= alpha;
 #pragma unroll
-          for (int e = 0; e < 2; ++e) {
-            float mx = fmaxf(s[m][0][2 * e], s[m][0][2 * e + 1]);
-#pragma unroll
-            for (int n = 1; n < NT; ++n) mx = fmaxf(mx, fmaxf(s[m][n][2 * e], s[m][n][2 * e + 1]));
-            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
-            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
-            const float now = fmaxf(top[m][e], mx * p.scale_log2);
-            const float alpha = now == -INFINITY ? 1.f : mm_ex2(top[m][e] - now);
-            top[m][e] = now;
-            l[m][e] *= alpha;
-#pragma unroll
-            for (int n = 0; n < OT; ++n) {
-              o[m][n][2 * e] *= alpha;
-              o[m][n][2 * e + 1] *= alpha;
-            }
+          for (int n = 0; n < OT; ++n) {
+            o[n][2 * e] *= alpha;
+            o[n][2 * e + 1] *= alpha;
           }
         }
       }
+      const uint64_t scale2 = tc::pack2(p.scale_log2, p.scale_log2);
 #pragma unroll
-      for (int m = 0; m < MT; ++m) {
+      for (int e = 0; e < 2; ++e) {
+        const float ref = top[e] == -INFINITY ? 0.f : -top[e];
+        const uint64_t ref2 = tc::pack2(ref, ref);
 #pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const float ref = top[m][e] == -INFINITY ? 0.f : top[m][e];
-#pragma unroll
-          for (int n = 0; n < NT; ++n) {
-            s[m][n][2 * e] = mm_ex2(fmaf(s[m][n][2 * e], p.scale_log2, -ref));
-            s[m][n][2 * e + 1] = mm_ex2(fmaf(s[m][n][2 * e + 1], p.scale_log2, -ref));
-          }
+        for (int n = 0; n < NT; ++n) {
+          float x, y;
+          tc::unpack2(tc::fma2(tc::pack2(s[n][2 * e], s[n][2 * e + 1]), scale2, ref2), x, y);
+          s[n][2 * e] = mm_ex2(x);
+          s[n][2 * e + 1] = mm_ex2(y);
         }
       }
 #pragma unroll
       for (int kk = 0; kk < NT / 2; ++kk) {
-        uint32_t pa[MT][4], pl[SPLIT ? MT : 1][4];
+        uint32_t pa[4], pl[4];
 #pragma unroll
-        for (int m = 0; m < MT; ++m) {
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const float x = s[m][2 * kk + (e >> 1)][2 * (e & 1)], y = s[m][2 * kk + (e >> 1)][2 * (e & 1) + 1];
-            pa[m][e] = pack_bf16(x, y);
-            const float xr = __uint_as_float(pa[m][e] << 16), yr = __uint_as_float(pa[m][e] & 0xffff0000u);
-            if constexpr (SPLIT) {
-              pl[m][e] = pack_bf16(x - xr, y - yr);
-              l[m][e & 1] += x + y;
-            } else {
-              l[m][e & 1] += xr + yr;  // the sum of what the second product weighs the values with
-            }
-          }
+        for (int e = 0; e < 4; ++e) {
+          const float x = s[2 * kk + (e >> 1)][2 * (e & 1)], y = s[2 * kk + (e >> 1)][2 * (e & 1) + 1];
+          pa[e] = pack_bf16(x, y);
+          if constexpr (SPLIT) pl[e] = pack_bf16(x - __uint_as_float(pa[e] << 16), y - __uint_as_float(pa[e] & 0xffff0000u));
         }
+        // the rows' sums, of what the values are weighed with: a product with ones
+        mma16816(lsum, pa, 0x3f803f80u, 0x3f803f80u);
+        if constexpr (SPLIT) mma16816(lsum, pl, 0x3f803f80u, 0x3f803f80u);
 #pragma unroll
         for (int n = 0; n < OT / 2; ++n) {
           uint32_t vf[4];
-          ldsm4t(sV + mm_at<D>(k0 + 16 * kk + ((lane >> 3) & 1) * 8 + (lane & 7), 2 * n + (lane >> 4)), vf);
-#pragma unroll
-          for (int m = 0; m < MT; ++m) {
-            mma16816(o[m][2 * n], pa[m], vf[0], vf[1]);
-            mma16816(o[m][2 * n + 1], pa[m], vf[2], vf[3]);
-            if constexpr (SPLIT) {
-              mma16816(o[m][2 * n], pl[m], vf[0], vf[1]);
-              mma16816(o[m][2 * n + 1], pl[m], vf[2], vf[3]);
-            }
+          ldsm4t(vk0 + v_at[n] + 16 * kk * (D * 2), vf);
+          mma16816(o[2 * n], pa, vf[0], vf[1]);
+          mma16816(o[2 * n + 1], pa, vf[2], vf[3]);
+          if constexpr (SPLIT) {
+            mma16816(o[2 * n], pl, vf[0], vf[1]);
+            mma16816(o[2 * n + 1], pl, vf[2], vf[3]);
           }
         }
       }
     }
     // ---- the rows' results: four lanes hold a row in pairs of columns; they swap them so that each has 16 bytes in a run ----
 #pragma unroll
-    for (int m = 0; m < MT; ++m) {
+    for (int e = 0; e < 2; ++e) {
+      const float sum = lsum[2 * e];  // the same in all four lanes
+      const float inv = sum > 0.f ? 1.f / sum : 0.f;
+      const int row = r0 + g + 8 * e;
 #pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        float sum = l[m][e];
-        sum += __shfl_xor_sync(0xffffffffu, sum, 1);
-        sum += __shfl_xor_sync(0xffffffffu, sum, 2);
-        const float inv = sum > 0.f ? 1.f / sum : 0.f;
-        const int row = r0 + 16 * m + g + 8 * e;
+      for (int n4 = 0; n4 < OT; n4 += 4) {
+        uint32_t v[4];
 #pragma unroll
-        for (int n4 = 0; n4 < OT; n4 += 4) {
-          uint32_t v[4];
+        for (int n = 0; n < 4; ++n) v[n] = pack_bf16(o[n4 + n][2 * e] * inv, o[n4 + n][2 * e + 1] * inv);
+        auto pick = [&](int i) { return i == 0 ? v[0] : i == 1 ? v[1] : i == 2 ? v[2] : v[3]; };
+        uint32_t w[4];
+        const uint32_t a0 = pick(t), a1 = __shfl_xor_sync(0xffffffffu, pick(t ^ 1), 1), a2 = __shfl_xor_sync(0xffffffffu, pick(t ^ 2), 2),
+                       a3 = __shfl_xor_sync(0xffffffffu, pick(t ^ 3), 3);  // a_i: from lane t ^ i of the four
 #pragma unroll
-          for (int n = 0; n < 4; ++n) v[n] = pack_bf16(o[m][n4 + n][2 * e] * inv, o[m][n4 + n][2 * e + 1] * inv);
-          auto pick = [&](int i) { return i == 0 ? v[0] : i == 1 ? v[1] : i == 2 ? v[2] : v[3]; };
-          uint32_t w[4];
-          const uint32_t a0 = pick(t), a1 = __shfl_xor_sync(0xffffffffu, pick(t ^ 1), 1), a2 = __shfl_xor_sync(0xffffffffu, pick(t ^ 2), 2),
-                         a3 = __shfl_xor_sync(0xffffffffu, pick(t ^ 3), 3);  // a_i: from lane t ^ i of the four
+        for (int i = 0; i < 4; ++i) {
+          const int x = i ^ t;
+          w[i] = x == 0 ? a0 : x == 1 ? a1 : x == 2 ? a2 : a3;
+        }
+        if (row < p.Tq) {
+          const int col = h * D + 8 * (n4 + t);
+          const uint4 out = make_uint4(w[0], w[1], w[2], w[3]);
+          __nv_bfloat16* dst = p.o + (long long)b * p.o_bs + (long long)row * p.o_rs + col;
+          if (p.gate) {
+            const uint4 graw = __ldg(reinterpret_cast<const uint4*>(p.gate + ((long long)b * p.Tq + row) * p.gate_rs + col));
+            float x[8], gv[8];
+            unpack16<__nv_bfloat16>(out, x);
+            unpack16<__nv_bfloat16>(graw, gv);
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const int x = i ^ t;
-            w[i] = x == 0 ? a0 : x == 1 ? a1 : x == 2 ? a2 : a3;
-          }
-          if (row < p.Tq) {
-            const int col = h * D + 8 * (n4 + t);
-            uint4 out = make_uint4(w[0], w[1], w[2], w[3]);
-            if (p.gate) {
-              const uint4 graw = __ldg(reinterpret_cast<const uint4*>(p.gate + ((long long)b * p.Tq + row) * p.gate_rs + col));
-              float x[8], gv[8];
-              unpack16<__nv_bfloat16>(out, x);
-              unpack16<__nv_bfloat16>(graw, gv);
-#pragma unroll
-              for (int i = 0; i < 8; ++i) x[i] = gated<__nv_bfloat16>(x[i], gv[i]);
-              st16<__nv_bfloat16>(p.o + (long long)b * p.o_bs + (long long)row * p.o_rs + col, x, 1.f);
-            } else {
-              *reinterpret_cast<uint4*>(p.o + (long long)b * p.o_bs + (long long)row * p.o_rs + col) = out;
-            }
+            for (int i = 0; i < 8; ++i) x[i] = gated<__nv_bfloat16>(x[i], gv[i]);
+            st16<__nv_bfloat16>(dst, x, 1.f);
+          } else {
+            *reinterpret_cast<uint4*>(dst) = out;
           }
         }
       }
@@ -288,14 +270,14 @@ bool fmha_mma_supported(const FmhaArgs& a, const KvView& kv, long long keys) {
          al16(a.egate) && a.egate_rs % 8 == 0 && (kv.token_stride == 0 || kv.token_stride % 8 == 0) && (a.scale == 0.f);
 }
 
-template <int D, int MT, bool SPLIT>
+template <int D, bool SPLIT>
 static int fmha_mma_launch(const MmaArgs& p, unsigned grid, size_t smem, cudaStream_t st) {
-  cudaError_t e = cudaFuncSetAttribute(fmha_mma_kernel<D, MT, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = cudaFuncSetAttribute(fmha_mma_kernel<D, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) {
     set_error("fmha_mma: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
     return DGPT_E_CUDA;
   }
-  fmha_mma_kernel<D, MT, SPLIT><<<grid, kMmThreads, smem, st>>>(p);
+  fmha_mma_kernel<D, SPLIT><<<grid, kMmThreads, smem, st>>>(p);
   return launch_status("fmha_mma");
 }
 
@@ -323,7 +305,7 @@ int fmha_mma(const FmhaArgs& a, const KvView& kv, long long keys, cudaStream_t s
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if (sms <= 0) sms = 148;
   // one CTA a (sequence, head), or several that share its rows where that leaves room for more CTAs
-  const int rows = a.D == 32 ? 32 : 16, most = (a.Tq + rows * kMmWarps - 1) / (rows * kMmWarps);
+  const int rows = 16, most = (a.Tq + rows * kMmWarps - 1) / (rows * kMmWarps);
   const long long pairs = (long long)a.B * a.H;
   long long splits = pairs > 0 ? 2ll * sms / pairs : 1;
   p.splits = (int)(splits < 1 ? 1 : splits > most ? most : splits);
@@ -333,8 +315,8 @@ int fmha_mma(const FmhaArgs& a, const KvView& kv, long long keys, cudaStream_t s
   }
   const unsigned grid = (unsigned)(pairs * p.splits);
   const size_t smem = (size_t)p.room * a.D * 4;
-  if (a.D == 32) return a.split_p ? fmha_mma_launch<32, 2, true>(p, grid, smem, st) : fmha_mma_launch<32, 2, false>(p, grid, smem, st);
-  return a.split_p ? fmha_mma_launch<64, 1, true>(p, grid, smem, st) : fmha_mma_launch<64, 1, false>(p, grid, smem, st);
+  if (a.D == 32) return a.split_p ? fmha_mma_launch<32, true>(p, grid, smem, st) : fmha_mma_launch<32, false>(p, grid, smem, st);
+  return a.split_p ? fmha_mma_launch<64, true>(p, grid, smem, st) : fmha_mma_launch<64, false>(p, grid, smem, st);
 }
 
 }  // namespace dgpt

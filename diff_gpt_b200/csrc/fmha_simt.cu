@@ -249,16 +249,15 @@ static bool simt_own_gate(const FmhaArgs& a) {
   return a.dtype == DGPT_BF16 ? a.Tq >= 8 || pairs <= 512 : a.D <= 16 && pairs <= 1024;
 }
 
-// Whether the kernel with its products in registers is ahead of the tcgen05 kernels (us, those / this).  Heads of 32 over whole tiles: from 256
-// keys and 192 pairs of sequence and head on (16 x 12 x 256 keys 17.8 / 15.7, 256 x 8 x 512 326 / 238, x 128 52 / 70, 1 x 8 x 512 10.7 / 17).  Keys that
-// are not whole tiles, whose probabilities are pairs: up to half a tile (256 x 8 heads of 64 x 33 59 / 46, x 64 62 / 59; of 32 54 / 48) and behind
-// the first tile (x 200 184 / 158; of 32 161 / 106); in between the one tile is all there is to do (x 100 67 / 78).  Few heads of 32 stay: 4 x 8 x 200
-// level, 1 x 8 x 200 10.9 / 11.3.
+// Whether the kernel with its products in registers is ahead of the tcgen05 kernels (us, those / this).  Heads of 32: at every size up to 256 keys
+// (1 x 8 x 64 keys 7.3 / 5.3, x 256 8.4 / 7.9; 256 x 8 x 64 53 / 27, x 128 52 / 39) and beyond where pairs of sequence and head are many (16 x 12 x 512
+// 37.8 / 33.4, 256 x 8 x 512 328 / 198, but 1 x 8 x 512 10.6 / 11.1, 4 x 8 x 640 12.5 / 15.5).  Keys that are not whole tiles, whose probabilities are
+// pairs: always (1 x 8 x 300 13.3 / 8.6, 256 x 8 x 200 163 / 79).  Heads of 64, with two CTAs an SM: only those, up to half a tile and behind the
+// first one (256 x 8 x 33 60 / 48, x 64 62 / 59, x 100 67 / 77, x 200 186 / 155, x 300 316 / 250; whole tiles x 256 level, 1 x 8 x 256 9.0 / 11.5).
 static bool fmha_prefers_mma(const FmhaArgs& a, long long keys) {
   const long long pairs = (long long)a.B * a.H;
-  if (a.D == 32 && pairs < 192) return false;
-  if (a.split_p) return keys <= 64 || (keys > 128 && keys <= (a.D == 32 ? 768 : 320));
-  return a.D == 32 && keys >= 256 && keys <= 768;
+  if (a.D == 32) return a.split_p || keys <= 256 || pairs >= 128;
+  return a.split_p && (keys <= 64 || keys > 128);
 }
 
 static int fmha_full(const void* q, int64_t q_batch_stride, int64_t q_row_stride, const dgpt_kv_layout* kv, const int32_t* kv_len,

@@ -23,9 +23,10 @@ def _reference(q, k, v, Tq, q_offset, kv_len, causal, gate):
     return y if gate is None else y.bfloat16().double() * torch.sigmoid(gate.double())
 
 
-# (batch, heads, head_dim, keys, query offset): whole tiles and ragged ones around the rule's edges, blocks of 16 and 32 rows, few rows
+# (batch, heads, head_dim, keys, query offset): whole tiles and ragged ones around the rule's edges, blocks of 16 rows, few rows
 CASES = [(24, 8, 32, 256, 0), (24, 8, 32, 384, 127), (96, 2, 32, 768, 0), (48, 4, 32, 40, 0), (48, 4, 32, 64, 17), (200, 1, 32, 129, 0),
-         (64, 3, 32, 700, 650), (2, 3, 64, 24, 0), (1, 2, 64, 64, 63), (3, 2, 64, 131, 0), (1, 8, 64, 320, 5), (9, 4, 64, 200, 199)]
+         (64, 3, 32, 700, 650), (1, 3, 32, 33, 0), (2, 8, 32, 128, 0),
+         (2, 3, 64, 24, 0), (1, 2, 64, 64, 63), (3, 2, 64, 131, 0), (1, 8, 64, 320, 5), (9, 4, 64, 200, 199)]
 
 
 @pytest.mark.parametrize("B,H,D,T,off", CASES)
