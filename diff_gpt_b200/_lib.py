@@ -125,6 +125,11 @@ PROTOTYPES = {
         C.c_int,
         [_p, _i64, _kvp, _p, _p, _p, _p, _p, _i64, _p, _i64, _p, _sz, _i32, _i32, _i32, _i32, _i32, _i32, _f32, _i32, _i32, _p, _p],
     ),
+    "dgpt_latent_attn_shared": (
+        C.c_int,
+        [_p, _i64, _kvp, _p, _p, _p, _p, _p, _i64, _p, _i64, _p, _sz, _i32, _i32, _i32, _i32, _i32, _i32, _f32, _i32, _i32, _i32, _i32,
+         _i32, _i32, _p, _p],
+    ),
     "dgpt_fmha_grouped": (
         C.c_int,
         [_p, _i64, _i64, _kvp, _i64, _i32, _p, _i64, _i64, _i32, _i32, _i32, _i32, _i32, _i32, _i32, _i32, _f32, _i32, _i32, _p, _p],
@@ -133,6 +138,11 @@ PROTOTYPES = {
         C.c_int,
         [_p, _i64, _kvp, _i32, _i32, _p, _p, _p, _p, _p, _i64, _p, _i64, _p, _sz, _i32, _i32, _i32, _i32, _i32, _i32, _i32, _i32, _i32,
          _f32, _i32, _i32, _p, _p],
+    ),
+    "dgpt_grouped_attn_shared": (
+        C.c_int,
+        [_p, _i64, _kvp, _i32, _i32, _p, _p, _p, _p, _p, _i64, _p, _i64, _p, _sz, _i32, _i32, _i32, _i32, _i32, _i32, _i32, _i32, _i32,
+         _f32, _i32, _i32, _i32, _i32, _i32, _i32, _p, _p],
     ),
     "dgpt_silu_mul": (C.c_int, [_p, _p, _i64, _i32, _p]),
     "dgpt_embed_streams": (

@@ -341,7 +341,8 @@ static int row_attn(const char* what, const void* q, int64_t q_row_stride, const
                     const int32_t* len0, const int32_t* start1, const int32_t* len1, const int32_t* step_ptr, const void* gate,
                     int64_t gate_row_stride, void* out, int64_t out_row_stride, void* workspace, size_t workspace_bytes,
                     int32_t n_splits, int32_t n_seq, int32_t T, int32_t H, int32_t G, int32_t dk, int32_t dv, int32_t window,
-                    int32_t keep_first, float scale, int32_t dtype, int32_t impl, int32_t* status, void* stream) {
+                    int32_t keep_first, float scale, int32_t dtype, int32_t impl, int32_t share, int32_t together, int32_t prompt_keys,
+                    int32_t own_keys, int32_t* status, void* stream) {
   DGPT_REQUIRE(q && out && start1 && len1, "%s: NULL pointer", what);
   DGPT_REQUIRE(n_seq >= 0 && T >= 0 && H > 0 && G > 0 && H % G == 0 && dk > 0 && dk % 8 == 0 && dv > 0 && dv % 8 == 0 && window >= 0 &&
                    keep_first >= 0,
@@ -354,6 +355,11 @@ static int row_attn(const char* what, const void* q, int64_t q_row_stride, const
   DGPT_REQUIRE((reinterpret_cast<uintptr_t>(q) & 15) == 0 && q_row_stride % 8 == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0 &&
                    out_row_stride % 8 == 0,
                "%s: q and out must be 16-byte aligned with row strides of a multiple of 8", what);
+  DGPT_REQUIRE(share >= 1 && n_seq % share == 0, "%s: %d sequences are not runs of %d", what, n_seq, share);
+  const int per = H / G;
+  DGPT_REQUIRE(together == 0 || together == 1 ||
+                   (together > 1 && (together & (together - 1)) == 0 && (per & (per - 1)) == 0 && per * together >= 16 && per * together <= 64),
+               "%s: 16, 32 or 64 heads of together rows are taken at once", what);
   if (int e = validate_kv(kv, row_w)) return e;
   const long long R = (long long)n_seq * T;
   if (R == 0) return DGPT_OK;
@@ -372,7 +378,8 @@ static int row_attn(const char* what, const void* q, int64_t q_row_stride, const
   a.ws_o = static_cast<float*>(workspace);
   a.ws_ml = workspace ? a.ws_o + (size_t)R * H * n_splits * dv : nullptr;
   a.n_splits = n_splits; a.n_seq = n_seq; a.Tn = T; a.H = H; a.window = window;
-  a.G = G; a.dk = dk; a.dv = dv; a.row_w = row_w; a.v_col = v_col; a.keep = keep_first;
+  a.G = G; a.dk = dk; a.dv = dv; a.row_w = row_w; a.v_col = v_col; a.keep = keep_first; a.share = share; a.together = together;
+  a.prompt_keys = prompt_keys > 0 ? prompt_keys : 0; a.own_keys = own_keys > 0 ? own_keys : 0;
   a.scale_log2 = scale * kLog2e;
   a.status = status;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
@@ -393,13 +400,37 @@ static int row_attn(const char* what, const void* q, int64_t q_row_stride, const
   return launch_status("latent_combine");
 }
 
+extern "C" int dgpt_latent_attn_shared(const void* q, int64_t q_row_stride, const dgpt_kv_layout* kv, const int32_t* len0,
+                                       const int32_t* start1, const int32_t* len1, const int32_t* step_ptr, const void* gate,
+                                       int64_t gate_row_stride, void* out, int64_t out_row_stride, void* workspace,
+                                       size_t workspace_bytes, int32_t n_splits, int32_t n_seq, int32_t T, int32_t H, int32_t r,
+                                       int32_t window, float scale, int32_t dtype, int32_t impl, int32_t share, int32_t together,
+                                       int32_t prompt_keys, int32_t own_keys, int32_t* status, void* stream) {
+  return row_attn("latent_attn", q, q_row_stride, kv, r, 0, len0, start1, len1, step_ptr, gate, gate_row_stride, out, out_row_stride,
+                  workspace, workspace_bytes, n_splits, n_seq, T, H, 1, r, r, window, 0, scale, dtype, impl, share, together,
+                  prompt_keys, own_keys, status, stream);
+}
+
 extern "C" int dgpt_latent_attn(const void* q, int64_t q_row_stride, const dgpt_kv_layout* kv, const int32_t* len0,
                                 const int32_t* start1, const int32_t* len1, const int32_t* step_ptr, const void* gate,
                                 int64_t gate_row_stride, void* out, int64_t out_row_stride, void* workspace,
                                 size_t workspace_bytes, int32_t n_splits, int32_t n_seq, int32_t T, int32_t H, int32_t r,
                                 int32_t window, float scale, int32_t dtype, int32_t impl, int32_t* status, void* stream) {
-  return row_attn("latent_attn", q, q_row_stride, kv, r, 0, len0, start1, len1, step_ptr, gate, gate_row_stride, out, out_row_stride,
-                  workspace, workspace_bytes, n_splits, n_seq, T, H, 1, r, r, window, 0, scale, dtype, impl, status, stream);
+  return dgpt_latent_attn_shared(q, q_row_stride, kv, len0, start1, len1, step_ptr, gate, gate_row_stride, out, out_row_stride, workspace,
+                                 workspace_bytes, n_splits, n_seq, T, H, r, window, scale, dtype, impl, 1, 0, 0, 0, status, stream);
+}
+
+extern "C" int dgpt_grouped_attn_shared(const void* q, int64_t q_row_stride, const dgpt_kv_layout* kv, int32_t row_width,
+                                        int32_t v_col, const int32_t* len0, const int32_t* start1, const int32_t* len1,
+                                        const int32_t* step_ptr, const void* gate, int64_t gate_row_stride, void* out,
+                                        int64_t out_row_stride, void* workspace, size_t workspace_bytes, int32_t n_splits,
+                                        int32_t n_seq, int32_t T, int32_t H, int32_t G, int32_t dk, int32_t dv, int32_t window,
+                                        int32_t keep_first, float scale, int32_t dtype, int32_t impl, int32_t share,
+                                        int32_t together, int32_t prompt_keys, int32_t own_keys, int32_t* status, void* stream) {
+  DGPT_REQUIRE(v_col > 0, "grouped_attn: the values follow the keys in a cache row");
+  return row_attn("grouped_attn", q, q_row_stride, kv, row_width, v_col, len0, start1, len1, step_ptr, gate, gate_row_stride, out,
+                  out_row_stride, workspace, workspace_bytes, n_splits, n_seq, T, H, G, dk, dv, window, keep_first, scale, dtype, impl,
+                  share, together, prompt_keys, own_keys, status, stream);
 }
 
 extern "C" int dgpt_grouped_attn(const void* q, int64_t q_row_stride, const dgpt_kv_layout* kv, int32_t row_width, int32_t v_col,
@@ -408,8 +439,7 @@ extern "C" int dgpt_grouped_attn(const void* q, int64_t q_row_stride, const dgpt
                                  size_t workspace_bytes, int32_t n_splits, int32_t n_seq, int32_t T, int32_t H, int32_t G,
                                  int32_t dk, int32_t dv, int32_t window, int32_t keep_first, float scale, int32_t dtype,
                                  int32_t impl, int32_t* status, void* stream) {
-  DGPT_REQUIRE(v_col > 0, "grouped_attn: the values follow the keys in a cache row");
-  return row_attn("grouped_attn", q, q_row_stride, kv, row_width, v_col, len0, start1, len1, step_ptr, gate, gate_row_stride, out,
-                  out_row_stride, workspace, workspace_bytes, n_splits, n_seq, T, H, G, dk, dv, window, keep_first, scale, dtype, impl,
-                  status, stream);
+  return dgpt_grouped_attn_shared(q, q_row_stride, kv, row_width, v_col, len0, start1, len1, step_ptr, gate, gate_row_stride, out,
+                                  out_row_stride, workspace, workspace_bytes, n_splits, n_seq, T, H, G, dk, dv, window, keep_first,
+                                  scale, dtype, impl, 1, 0, 0, 0, status, stream);
 }

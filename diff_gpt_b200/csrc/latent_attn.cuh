@@ -27,6 +27,9 @@ struct LatentArgs {
   int G, dk, dv;    // groups, query / key size, value size
   int row_w, v_col; // elements between rows; where the values start
   int keep;         // the first `keep` keys are seen from every distance
+  int share;        // each run of `share` rows sees the same slots below its first run's end, in the same pages (1: no such thing)
+  int together;     // rows of a prompt in one item of the tcgen05 kernel (0: chosen)
+  int prompt_keys, own_keys;  // about how many keys of the two runs a row sees, for that choice
   float scale_log2;
   int* status;
 };

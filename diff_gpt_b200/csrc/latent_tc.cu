@@ -11,9 +11,14 @@
 //   warp 5, lane 0  loader: Q of the item, then the units of its tiles into a ring, through TMA straight from the pages
 //   warp 4, lane 0  issuer: S^T into one of two TMEM buffers, O^T += V^T P^T; with room in the ring the scores of the
 //                   next tile are issued before the sums of this one
-//   warps 0-3       softmax, one thread per key: probabilities against a running reference per head that only moves when
-//                   it is exceeded by 2^8 (found with one barrier vote per tile), written as bf16 into shared memory;
+//   warps 0-3       softmax, one thread per key: probabilities against a running reference per head, kept in shared memory,
+//                   that only moves when it is exceeded by 2^8 (found with one barrier vote per tile), written as bf16 into
+//                   shared memory;
 //                   after the item's last tile, one thread per column: normalise, gate, store
+// Rows behind one prompt (ROWS): an item is a set of up to rg of them, whose heads together are the N of the products over
+// the prompt's tiles; then come the tiles of each row's own slots (those of two rows in one tile where they fit its halves),
+// whose products cover that row's columns only.  The columns' references move each for itself, so that a row's numbers do not
+// depend on its neighbours but for the order in which its weights are added.
 // A row of a unit that holds fewer than 64 columns leaves the block's other accumulator rows undefined; they are not read.
 // TMEM columns: S0 [0, N)  S1 [N, 2N)  O of unit u [2N + u N, +N).
 // Every mbarrier wait is bounded.  When one runs out the abort flag is raised, the loader and the issuer stop and drain
@@ -33,7 +38,10 @@ constexpr int kLtMaxUnits = 10;
 
 struct LtParams {
   LatentArgs a;
-  int n_rows, n_groups, n_items;  // item = (split * n_groups + group) * n_rows + row
+  int n_rows, n_groups, n_items;  // item = (split * n_groups + group) * n_sets + set
+  int n_sets;                     // sets of rows: one row each, or
+  int rg, per_log2;               // ROWS: up to rg rows of one prompt; log2 of the heads that share a row
+  int sets_per_prompt;
   int per, gpk;                   // heads that share a row, and item groups they make
   int n_units;                    // units in the ring
   uint32_t unit_bytes;
@@ -47,17 +55,25 @@ __device__ __forceinline__ int lt_blocks(int cols, int u) { return cols - u * 12
 
 struct LtItem {
   int row, seq, g, h0, nh, split;
+  int nr, n_shared, n_own;        // ROWS: rows of the set, tiles of their prompt, tiles of each one's own slots
+  bool pairs;                     // own slots fit half a tile: one holds those of two rows
   int begin[3], end[3], base[3];  // the slot ranges and where their tiles start
   int n_first, n_second;          // tiles of the first range, of the first two
   int t0, n;                      // this split's tiles
 };
 
 // KEPT: the cache holds first keys that are seen from every distance, a slot range of their own
-template <bool KEPT>
+template <bool KEPT, bool ROWS>
 __device__ __forceinline__ LtItem lt_item(const LtParams& p, int item, int N) {
   LtItem it;
-  const int gs = item / p.n_rows;
-  it.row = item - gs * p.n_rows;
+  const int gs = item / p.n_sets;
+  it.row = item - gs * p.n_sets;
+  it.nr = 1;
+  if (ROWS) {
+    const int prompt = it.row / p.sets_per_prompt, first = (it.row - prompt * p.sets_per_prompt) * p.rg;
+    it.nr = min(p.rg, p.a.share - first);
+    it.row = prompt * p.a.share + first;
+  }
   it.g = 0;
   it.h0 = 0;
   it.split = gs;
@@ -69,7 +85,7 @@ __device__ __forceinline__ LtItem lt_item(const LtParams& p, int item, int N) {
     first = (grp - it.g * p.gpk) * N;
     it.h0 = it.g * p.per + first;
   }
-  it.nh = min(N, p.per - first);
+  it.nh = ROWS ? it.nr << p.per_log2 : min(N, p.per - first);
   const LatentKeys k = latent_keys(p.a, it.row);
   it.seq = k.seq;
   // [0, ks) and [lo, n), cut where slots change from the first run to the second; the cut lies in one of the two
@@ -88,7 +104,10 @@ __device__ __forceinline__ LtItem lt_item(const LtParams& p, int item, int N) {
   }
   it.n_first = KEPT ? nt[0] : 0;
   it.n_second = it.n_first + nt[1];
-  const int total = it.n_second + nt[2];
+  it.n_shared = own ? it.n_first : it.n_second;
+  it.n_own = it.n_second + nt[2] - it.n_shared;
+  it.pairs = ROWS && p.box <= kLtKeys / 2 && it.n_own == 1 && nt[2] == 1 && it.end[2] - it.base[2] <= kLtKeys / 2;
+  const int total = it.n_shared + (it.pairs ? (it.nr + 1) / 2 : it.nr * it.n_own);
   if (p.a.n_splits == 1) {
     it.t0 = 0;
     it.n = total;
@@ -99,19 +118,34 @@ __device__ __forceinline__ LtItem lt_item(const LtParams& p, int item, int N) {
   }
   return it;
 }
-// first slot of tile j of the item, and the limits of its range
-template <bool KEPT>
-__device__ __forceinline__ int lt_tile(const LtItem& it, int j, int& begin, int& end) {
-  const int t = it.t0 + j;
+struct LtTile {
+  int slot, begin, end;  // first slot; the limits of the slots that are seen
+  int own;               // the row of the set whose slots they are, -1: those of all
+  bool pair;             // the second half of the tile: the same slots of the next row
+};
+template <bool KEPT, bool ROWS>
+__device__ __forceinline__ LtTile lt_tile(const LtItem& it, int j) {
+  LtTile x;
+  int t = it.t0 + j;
+  x.own = -1;
+  x.pair = false;
+  if (ROWS && t >= it.n_shared) {
+    t -= it.n_shared;
+    x.pair = it.pairs;
+    x.own = it.pairs ? 2 * t : t / it.n_own;
+    t = it.pairs ? it.n_shared : it.n_shared + t - x.own * it.n_own;
+  }
   if (KEPT && t < it.n_first) {
-    begin = it.begin[0];
-    end = it.end[0];
-    return it.base[0] + t * kLtKeys;
+    x.begin = it.begin[0];
+    x.end = it.end[0];
+    x.slot = it.base[0] + t * kLtKeys;
+    return x;
   }
   const bool last = t >= it.n_second;
-  begin = last ? it.begin[2] : it.begin[1];
-  end = last ? it.end[2] : it.end[1];
-  return (last ? it.base[2] : it.base[1]) + (t - (last ? it.n_second : it.n_first)) * kLtKeys;
+  x.begin = last ? it.begin[2] : it.begin[1];
+  x.end = last ? it.end[2] : it.end[1];
+  x.slot = (last ? it.base[2] : it.base[1]) + (t - (last ? it.n_second : it.n_first)) * kLtKeys;
+  return x;
 }
 
 __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1, int c2) {
@@ -160,12 +194,17 @@ __device__ __forceinline__ float lt_reduce16(const float* v, int lane, F op) {
   return op(d, __shfl_xor_sync(0xffffffffu, d, 16));
 }
 
-// NB: heads per group = 16 NB; HS <= 16 NB: heads the softmax looks after (a group may hold fewer than 16).
+// NB: columns of the products = 16 NB; HS <= 16 NB: heads the softmax looks after (a group may hold fewer than 16).
 // SHARED: a tile's values are its keys (latents), whose cache has no kept first keys.
-template <int NB, int HS, bool SHARED>
+// ROWS: a column is a head of one of rg rows, column c = row c >> per_log2, head c & (per - 1); HS = 16 NB.
+template <int NB, int HS, bool SHARED, bool ROWS>
 __global__ void __launch_bounds__(kLtThreads, NB == 4 ? 1 : 2)
 latent_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__ CUtensorMap mc, const LtParams p) {
   constexpr int N = 16 * NB;
+  // The sums of a tile that is not full go over the 16-key steps that hold a key only.  Latents of 512 / 256, 256 rows with
+  // 1000 keys: 106.5 -> 102.4 and 36.9 -> 33.8 us.  Rows of keys and values, each by itself, have products to spare (they
+  // wait for HBM) and took longer with them issued one by one: 64.3 -> 66.5 (4 groups of 64), 235 -> 241 (8 of 128).
+  constexpr bool kSome = SHARED || ROWS;
   constexpr uint32_t kIdescS = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | (8u << 24);
   constexpr uint32_t kIdescO = kIdescS | (1u << 15);  // A is read MN-major
   constexpr uint32_t kQBlock = N * 128;               // [N heads][64 columns]
@@ -188,7 +227,8 @@ latent_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__
   uint64_t* bars = reinterpret_cast<uint64_t*>(sP + (ahead ? 4 : 2) * kPBlock);
   float* red = reinterpret_cast<float*>(bars + 32);  // [4 warps][N]
   float* fac = red + 4 * N;                          // [4 warps][N]
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(fac + 4 * N);
+  float* ref = fac + 4 * N;                          // [N] what the probabilities of a head are relative to
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(ref + N);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   const uint32_t aU = smem_u32(sU), aQ = smem_u32(sQ), aP = smem_u32(sP);
   const uint32_t bar0 = smem_u32(bars);
@@ -222,7 +262,7 @@ latent_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__
       const int pt = p.a.kv.page_tokens;
       const LatentArgs& a = p.a;
       for (int item = blockIdx.x; ok && item < p.n_items; item += gridDim.x) {
-        const LtItem it = lt_item<!SHARED>(p, item, N);
+        const LtItem it = lt_item<!SHARED, ROWS>(p, item, N);
         if (it.n == 0) continue;
         if (items > 0) ok = wait_or_abort(bar_qf, (items - 1) & 1u, abort_flag, 50);  // the last scores of the item before are done
         if (!ok) break;
@@ -230,9 +270,10 @@ latent_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__
         for (int c = 0; c < nqb; ++c) tma_load_3d(aQ + c * kQBlock, &mq, bar_q, c * 64, it.h0, it.row);
         ++items;
         for (int j = 0; ok && j < it.n; ++j) {
-          int begin, end;
-          const int slot = lt_tile<!SHARED>(it, j, begin, end);
-          const int boxes = min(kLtKeys / p.box, (end - slot + p.box - 1) / p.box);
+          const LtTile x = lt_tile<!SHARED, ROWS>(it, j);
+          const int seq0 = it.seq + (ROWS ? max(x.own, 0) : 0);
+          const int half = min(kLtKeys / p.box, (x.end - x.slot + p.box - 1) / p.box);  // boxes of a row
+          const int boxes = ROWS && x.pair && x.own + 1 < it.nr ? 2 * half : half;
           for (int u = 0; ok && u < UT; ++u, ++un) {
             const unsigned s = un % (unsigned)NU, round = un / (unsigned)NU;
             if (round > 0) ok = wait_or_abort(bar_uf + 8 * s, (round - 1) & 1u, abort_flag, 51);
@@ -243,15 +284,17 @@ latent_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__
             const int col = SHARED ? u * 128 : key ? it.g * a.dk + u * 128 : a.v_col + it.g * a.dv + (u - UK) * 128;
             mbar_expect_tx(full, (uint32_t)boxes * p.box * 128u * blocks);
             for (int b = 0; b < boxes; ++b) {
-              const int at = slot + b * p.box;
-              int pg = it.seq, in = at;
+              const bool second = ROWS && b >= half;
+              const int seq = seq0 + (second ? 1 : 0), at = x.slot + (second ? b - half : b) * p.box;
+              const uint32_t to = dst + (second ? kLtBlock / 2 + (b - half) * p.box * 128 : b * p.box * 128);
+              int pg = seq, in = at;
               if (p.a.kv.page_table) {
                 const int lp = at / pt;
-                pg = p.a.kv.page_table[(long long)it.seq * p.a.kv.max_pages + lp];
+                pg = p.a.kv.page_table[(long long)seq * p.a.kv.max_pages + lp];
                 in = at - lp * pt;
               }
-              tma_load_3d(dst + b * p.box * 128, &mc, full, col, in, pg);
-              if (blocks == 2) tma_load_3d(dst + kLtBlock + b * p.box * 128, &mc, full, col + 64, in, pg);
+              tma_load_3d(to, &mc, full, col, in, pg);
+              if (blocks == 2) tma_load_3d(to + kLtBlock, &mc, full, col + 64, in, pg);
             }
           }
         }
@@ -267,35 +310,53 @@ latent_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__
     // ================= MMA issuer =================
     if (lane == 0) {
       const uint64_t dC = smem_desc(0, 16, 1024), dM = smem_desc(0, kLtBlock, 1024);  // K-major rows; MN-major pairs of blocks
+      // the products of rows' own slots: of their columns only
+      auto own_n = [&](const LtTile& x, uint32_t idesc) {
+        return !ROWS || x.own < 0 ? idesc : (idesc & ~(63u << 17)) | (uint32_t)max(2, (x.pair ? 2 : 1) * p.per >> 3) << 17;
+      };
+      auto own_block = [&](const LtTile& x) { return ROWS && x.own >= 0 ? (x.own << p.per_log2) >> 4 : 0; };
       unsigned g = 0u, items = 0u;  // tiles; items
       bool ok = true;
       for (int item = blockIdx.x; ok && item < p.n_items; item += gridDim.x) {
-        const LtItem it = lt_item<!SHARED>(p, item, N);
+        const LtItem it = lt_item<!SHARED, ROWS>(p, item, N);
         if (it.n == 0) continue;
         ok = wait_or_abort(bar_q, items & 1u, abort_flag, 52);
-        auto issue_s = [&](unsigned gt, bool last) {
-          const uint32_t d = tmem + (gt & 1u) * N;
+        unsigned started = 0u;  // 16-column blocks of O that hold sums
+        auto issue_s = [&](unsigned gt, int j) {
+          const bool last = j + 1 == it.n;
+          const LtTile x = lt_tile<!SHARED, ROWS>(it, j);
+          const int blk = own_block(x);
+          const uint32_t idesc = own_n(x, kIdescS);
+          const uint32_t d = tmem + (gt & 1u) * N + blk * 16;
           for (int u = 0; ok && u < UK; ++u) {
             const unsigned un = gt * (unsigned)UT + (unsigned)u, s = un % (unsigned)NU;
             ok = wait_or_abort(bar_u + 8 * s, (un / (unsigned)NU) & 1u, abort_flag, 53);
             if (!ok) return;
             tc_fence_after();
-            const uint64_t da = dC + ((aU + s * unit_bytes) >> 4), db = dC + ((aQ + 2 * u * kQBlock) >> 4);
-            if (SHARED || lt_blocks(p.a.dk, u) == 2) umma_ss8<2, kLtBlock / 16, 2, kQBlock / 16>(d, da, db, kIdescS, u > 0 ? 1u : 0u);
-            else umma_ss4<2, 2>(d, da, db, kIdescS, u > 0 ? 1u : 0u);
+            const uint64_t da = dC + ((aU + s * unit_bytes) >> 4), db = dC + ((aQ + 2 * u * kQBlock + blk * 2048) >> 4);
+            if (SHARED || lt_blocks(p.a.dk, u) == 2) umma_ss8<2, kLtBlock / 16, 2, kQBlock / 16>(d, da, db, idesc, u > 0 ? 1u : 0u);
+            else umma_ss4<2, 2>(d, da, db, idesc, u > 0 ? 1u : 0u);
             if (!SHARED) umma_commit(bar_uf + 8 * s);  // keys are done with
           }
           umma_commit(bar_s + 8 * (gt & 1u));
           if (last) umma_commit(bar_qf);
         };
-        if (ok) issue_s(g, it.n == 1);
+        if (ok) issue_s(g, 0);
         for (int j = 0; ok && j < it.n; ++j, ++g) {
           const unsigned b = g & 1u;
-          if (ahead && j + 1 < it.n) issue_s(g + 1, j + 2 == it.n);
+          if (ahead && j + 1 < it.n) issue_s(g + 1, j + 1);
           ok = ok && wait_or_abort(bar_p + 8 * b, (g >> 1) & 1u, abort_flag, 54);
           if (ok && j == 0 && items > 0) ok = wait_or_abort(bar_of, (items - 1) & 1u, abort_flag, 55);  // the last item's O has been read
           if (!ok) break;
           tc_fence_after();
+          const LtTile x = lt_tile<!SHARED, ROWS>(it, j);
+          // steps of 16 keys that hold one that is seen: the others' probabilities are zeros
+          const int k0 = kSome ? max(x.begin - x.slot, 0) >> 4 : 0, k1 = kSome ? min(kLtKeys, x.end - x.slot + 15) >> 4 : 8;
+          const int blk = own_block(x);
+          const uint32_t idesc = own_n(x, kIdescO);
+          const unsigned acc = (started >> blk) & 1u;
+          started |= ROWS && x.own >= 0 ? 1u << blk : 15u;  // a row's own blocks are always touched together
+          const bool second = ROWS && x.pair && x.own + 1 < it.nr;
           for (int u = 0; u < UV; ++u) {
             const unsigned un = g * (unsigned)UT + (unsigned)(v_unit + u), s = un % (unsigned)NU;
             if (!SHARED) {
@@ -303,13 +364,19 @@ latent_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__
               if (!ok) break;
               tc_fence_after();
             }
-            umma_ss8<128, 512, 2, kPBlock / 16>(tmem + 2 * N + u * N, dM + ((aU + s * unit_bytes) >> 4), dC + ((aP + (ahead ? 2 * b * kPBlock : 0u)) >> 4),
-                                            kIdescO, j > 0 ? 1u : 0u);
+            const uint32_t d = tmem + 2 * N + u * N + blk * 16;
+            const uint64_t da = dM + ((aU + s * unit_bytes) >> 4), db = dC + ((aP + (ahead ? 2 * b * kPBlock : 0u) + blk * 2048) >> 4);
+            if (k0 == 0 && k1 == 8) umma_ss8<128, 512, 2, kPBlock / 16>(d, da, db, idesc, acc);
+            else {
+              for (int k = k0; k < k1; ++k) umma_ss(d, da + 128 * k, db + (k >> 2) * (kPBlock / 16) + 2 * (k & 3), idesc, k > k0 ? 1u : acc);
+              if (second)
+                for (int k = k0; k < k1; ++k) umma_ss(d, da + 512 + 128 * k, db + kPBlock / 16 + 2 * k, idesc, 1u);
+            }
             umma_commit(bar_uf + 8 * s);
           }
           if (!ok) break;
           umma_commit(bar_o + 8 * b);
-          if (!ahead && j + 1 < it.n) issue_s(g + 1, j + 2 == it.n);
+          if (!ahead && j + 1 < it.n) issue_s(g + 1, j + 1);
         }
         ++items;
       }
@@ -325,13 +392,16 @@ latent_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__
     unsigned g = 0u;
     bool fail = false;
     const long long RH = (long long)p.n_rows * p.a.H;
-    if (HS < N) {  // heads nobody looks after: their probabilities are zeros, once
+    if (HS < N)  // heads nobody looks after: their probabilities are zeros, once
       for (int i = tid; i < (int)((ahead ? 4 : 2) * kPBlock / 16); i += 128) reinterpret_cast<uint4*>(sP)[i] = make_uint4(0u, 0u, 0u, 0u);
-      lt_sync();
-    }
+    if (tid < N) ref[tid] = -INFINITY;
+    lt_sync();
+    auto row_of = [&](int c) -> long long { return ROWS ? c >> p.per_log2 : 0; };
+    auto head_of = [&](int c) -> long long { return ROWS ? c & (p.per - 1) : c; };
     for (int item = blockIdx.x; item < p.n_items; item += gridDim.x) {
-      const LtItem it = lt_item<!SHARED>(p, item, N);
+      const LtItem it = lt_item<!SHARED, ROWS>(p, item, N);
       const int nh = it.nh;
+      unsigned started = 0u;  // 16-column blocks of O that hold sums
       constexpr int HL = (N + 31) / 32;  // heads a lane looks after at the end of the item
       float gate[HL];
 #pragma unroll
@@ -339,94 +409,147 @@ latent_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__
         const int h = lane + 32 * c;
         gate[c] = 1.f;
         if (p.a.gate && h < nh)
-          gate[c] = __bfloat162float(static_cast<const __nv_bfloat16*>(p.a.gate)[(long long)it.row * p.a.gate_rs + it.h0 + h]);
+          gate[c] = __bfloat162float(static_cast<const __nv_bfloat16*>(p.a.gate)[(it.row + row_of(h)) * p.a.gate_rs + it.h0 + head_of(h)]);
       }
-      float m[HS], l[HS];
+      float l[HS];
 #pragma unroll
-      for (int h = 0; h < HS; ++h) {
-        m[h] = -INFINITY;
-        l[h] = 0.f;
-      }
+      for (int h = 0; h < HS; ++h) l[h] = 0.f;
       for (int j = 0; j < it.n; ++j, ++g) {
         const unsigned b = g & 1u;
-        int begin, end;
-        const int slot = lt_tile<!SHARED>(it, j, begin, end) + tid;
+        const LtTile x = lt_tile<!SHARED, ROWS>(it, j);
+        const int half = ROWS && x.pair ? tid >> 6 : 0, slot = x.slot + tid - 64 * half, end = x.end;
+        // The tile concerns columns [c_lo, c_hi), this thread's key [k_lo, k_hi) of them.
+        const int c_lo = ROWS && x.own >= 0 ? x.own << p.per_log2 : 0;
+        const int c_hi = ROWS && x.own >= 0 ? c_lo + (x.pair ? 2 : 1) * p.per : HS;
+        const int k_lo = c_lo + half * p.per, k_hi = ROWS && x.own >= 0 ? k_lo + p.per : HS;
+        auto block = [&](int c) { return !ROWS || (c_lo < 16 * c + 16 && c_hi > 16 * c); };
+        const bool seen = slot >= x.begin && slot < end && (!ROWS || x.own + half < it.nr);
+        auto columns = [&](int c) -> unsigned {  // of block c, one bit each
+          if (!seen) return 0u;
+          if (ROWS && x.own < 0) return 0xffffu;
+          const int lo = max(k_lo - 16 * c, 0), hi = min(k_hi - 16 * c, 16);
+          return hi > lo ? (1u << hi) - (1u << lo) : 0u;
+        };
         if (!fail && !wait_or_abort(bar_s + 8 * b, (g >> 1) & 1u, abort_flag, 56)) fail = true;
         fail = __any_sync(0xffffffffu, fail);
         tc_fence_after();
-        const bool seen = slot >= begin && slot < end;
-        if (!fail && slot >= end) {  // nothing was loaded here, or rows nobody has written: 0 * x must stay 0
+        // Nothing was loaded here, or rows nobody has written: 0 * x must stay 0 where the sums go over the slot.  The whole warp
+        // waits for the unit: lanes that go apart in a wait need not have met again at the loads and barriers that follow, which
+        // are the warp's.
+        const bool blank = slot >= end && (!kSome || slot - x.slot < ((end - x.slot + 15) & ~15));
+        if (!fail && __any_sync(0xffffffffu, blank)) {
           for (int u = 0; u < UV; ++u) {
             const unsigned un = g * (unsigned)UT + (unsigned)(v_unit + u), us = un % (unsigned)NU;
             if (!SHARED && !wait_or_abort(bar_u + 8 * us, (un / (unsigned)NU) & 1u, abort_flag, 59)) break;  // still on its way
             uint8_t* unit = sU + (size_t)us * unit_bytes;
             const bool two = SHARED || lt_blocks(p.a.dv, u) == 2;
+            if (blank) {
 #pragma unroll
-            for (int c = 0; c < 8; ++c) {
-              reinterpret_cast<uint4*>(unit + tid * 128)[c] = make_uint4(0u, 0u, 0u, 0u);
-              if (two) reinterpret_cast<uint4*>(unit + kLtBlock + tid * 128)[c] = make_uint4(0u, 0u, 0u, 0u);
+              for (int c = 0; c < 8; ++c) {
+                reinterpret_cast<uint4*>(unit + tid * 128)[c] = make_uint4(0u, 0u, 0u, 0u);
+                if (two) reinterpret_cast<uint4*>(unit + kLtBlock + tid * 128)[c] = make_uint4(0u, 0u, 0u, 0u);
+              }
             }
           }
         }
-        float s[N];
+        __syncwarp();
+        float s[N];  // log2 of what is added for this key, against the heads' references
+        for (int pass = 0;; ++pass) {
 #pragma unroll
-        for (int c = 0; c < NB; ++c) tmem_ld16_nowait(lane_addr + b * N + c * 16, s + 16 * c);
-        tc_wait_ld();
-        bool over = false;
-#pragma unroll
-        for (int h = 0; h < HS; ++h) {
-          s[h] = seen ? s[h] * p.a.scale_log2 : -INFINITY;
-          over |= s[h] > m[h] + 8.f;
-        }
-        if (lt_any(over && !fail)) {  // some head's reference has to move: the tile's maxima, the same in every thread
-#pragma unroll
-          for (int h = HS; h < N; ++h) s[h] = -INFINITY;
+          for (int c = 0; c < NB; ++c) tmem_ld16_nowait(lane_addr + b * N + c * 16, s + 16 * c);
+          tc_wait_ld();
+          float top = -INFINITY;
 #pragma unroll
           for (int c = 0; c < NB; ++c) {
-            const float t = lt_reduce16(s + 16 * c, lane, [](float x, float y) { return fmaxf(x, y); });
+            if (!block(c)) continue;
+            const unsigned cols = columns(c);
+#pragma unroll
+            for (int i = 0; i < 16; i += 4) {
+              if (16 * c + i >= HS) continue;
+              const float4 m4 = *reinterpret_cast<const float4*>(ref + 16 * c + i);
+              const float mm[4] = {m4.x, m4.y, m4.z, m4.w};
+#pragma unroll
+              for (int k = 0; k < 4; ++k) {
+                const int h = 16 * c + i + k;
+                s[h] = (cols >> (i + k)) & 1u ? fmaf(s[h], p.a.scale_log2, -mm[k]) : -INFINITY;
+                top = fmaxf(top, s[h]);
+              }
+            }
+          }
+          if (pass || !lt_any(top > 8.f && !fail)) break;
+          // Some head's reference has to move.  Rare but for an item's first tile, so the loops stay rolled: with every
+          // block's code laid out the instructions of a first tile took longer to fetch than the tile.
+#pragma unroll 1
+          for (int c = c_lo >> 4; c < NB && 16 * c < c_hi; ++c) {
+            float v[16];
+            tmem_ld16_nowait(lane_addr + b * N + c * 16, v);
+            tc_wait_ld();
+            const unsigned cols = columns(c);
+#pragma unroll
+            for (int i = 0; i < 16; ++i) v[i] = (cols >> i) & 1u ? v[i] * p.a.scale_log2 : -INFINITY;
+            const float t = lt_reduce16(v, lane, [](float x, float y) { return fmaxf(x, y); });
             if (lane < 16) red[warp * N + 16 * c + lane] = t;
           }
           lt_sync();
-          float alpha[N];
-#pragma unroll
-          for (int h = HS; h < N; ++h) alpha[h] = 1.f;
-#pragma unroll
-          for (int h = 0; h < HS; ++h) {
-            const float mn = fmaxf(fmaxf(fmaxf(red[h], red[N + h]), fmaxf(red[2 * N + h], red[3 * N + h])), m[h]);
-            alpha[h] = mn == -INFINITY ? 1.f : ex2(m[h] - mn);  // -inf before the first tile: 0
-            m[h] = mn;
-            l[h] *= alpha[h];
+          if (tid < N) {
+            float alpha = 1.f;
+            if (tid >= c_lo && tid < c_hi) {
+              const float mn = fmaxf(fmaxf(red[tid], red[N + tid]), fmaxf(red[2 * N + tid], red[3 * N + tid])), mo = ref[tid];
+              if (mn > mo + 8.f) {  // only a head that needs it moves: what a row gets does not depend on the rows beside it
+                alpha = ex2(mo - mn);  // -inf before the first tile: 0
+                ref[tid] = mn;
+              }
+            }
+            fac[tid] = alpha;
           }
-          if (j > 0) {
+          __syncwarp();
+          lt_sync();  // and `red` may be written again
+#pragma unroll
+          for (int h = 0; h < HS; h += 4) {
+            const float4 f = *reinterpret_cast<const float4*>(fac + h);
+            l[h] *= f.x;
+            l[h + 1] *= f.y;
+            l[h + 2] *= f.z;
+            l[h + 3] *= f.w;
+          }
+          if (started) {
             // O may only be touched when no product is in flight on it: the tile before must be done, and this tile's
             // waits for this thread's arrival below
             if (!fail && !wait_or_abort(bar_o + 8 * (b ^ 1u), ((g - 1) >> 1) & 1u, abort_flag, 57)) fail = true;
             fail = __any_sync(0xffffffffu, fail);
             tc_fence_after();
-            for (int u = 0; u < UV; ++u) {
-#pragma unroll
-              for (int c = 0; c < NB; ++c) {
+#pragma unroll 1
+            for (int c = c_lo >> 4; c < NB && 16 * c < c_hi; ++c) {
+              if (!((started >> c) & 1u)) continue;
+#pragma unroll 1
+              for (int u = 0; u < UV; ++u) {
                 float v[16];
                 const uint32_t addr = lane_addr + 2 * N + u * N + c * 16;
                 tmem_ld16_nowait(addr, v);
                 tc_wait_ld();
                 uint32_t w[16];
 #pragma unroll
-                for (int i = 0; i < 16; ++i) w[i] = __float_as_uint(v[i] * alpha[16 * c + i]);
+                for (int i = 0; i < 16; ++i) w[i] = __float_as_uint(v[i] * fac[16 * c + i]);
                 tmem_st16(addr, w);
               }
             }
             tc_wait_st();
           }
-          lt_sync();  // `red` may be written again
         }
         uint8_t* pb = sP + ((ahead ? 2 * b : 0u) + (tid >> 6)) * kPBlock + (tid & 7) * 2;
         const int chunk = (tid & 63) >> 3;
 #pragma unroll
-        for (int h = 0; h < HS; ++h) {
-          const float e = ex2(s[h] - m[h]);  // not seen: 0 (m is finite: every tile holds a key that is seen)
-          l[h] += e;
-          *reinterpret_cast<__nv_bfloat16*>(pb + h * 128 + ((chunk ^ (h & 7)) << 4)) = __float2bfloat16_rn(e);
+        for (int c = 0; c < NB; ++c) {
+          if (!block(c)) continue;
+          started |= 1u << c;
+#pragma unroll
+          for (int i = 0; i < 16; ++i) {
+            const int h = 16 * c + i;
+            if (h >= HS) continue;
+            const float e = ex2(s[h]);  // not seen: 0
+            l[h % HS] += e;
+            *reinterpret_cast<__nv_bfloat16*>(pb + h * 128 + ((chunk ^ (h & 7)) << 4)) = __float2bfloat16_rn(e);
+          }
         }
         fence_async_smem();
         tc_fence_before();
@@ -448,8 +571,8 @@ latent_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__
         if (lane < 16) red[warp * N + 16 * c + lane] = t;
       }
       lt_sync();
-      const long long rh0 = (long long)it.row * p.a.H + it.h0;
-      const long long slot0 = (long long)it.split * RH + rh0;
+      // where column c's parts go
+      auto part = [&](int c) { return (long long)it.split * RH + (it.row + row_of(c)) * p.a.H + it.h0 + head_of(c); };
       // lane h: 1 / sum and gate of head h, or the sum itself for a split
 #pragma unroll
       for (int c = 0; c < HL; ++c) {
@@ -459,19 +582,19 @@ latent_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__
           float f = sum > 0.f ? 1.f / sum : 0.f;
           if (p.a.gate) f *= 1.f / (1.f + __expf(-gate[c]));
           fac[warp * N + h] = f;
-          if (p.a.n_splits > 1 && warp == 0 && h < nh) p.a.ws_ml[2 * (slot0 + h) + 1] = sum;
+          if (p.a.n_splits > 1 && warp == 0 && h < nh) {
+            p.a.ws_ml[2 * part(h)] = ref[h];
+            p.a.ws_ml[2 * part(h) + 1] = sum;
+          }
+          if (warp == 0) ref[h] = -INFINITY;
         }
-      }
-      if (p.a.n_splits > 1 && tid == 0) {
-#pragma unroll
-        for (int h = 0; h < HS; ++h)
-          if (h < nh) p.a.ws_ml[2 * (slot0 + h)] = m[h];
       }
       lt_sync();  // `red` may be written again, `fac` is complete
       if (it.n > 0) {
+#pragma unroll 1
         for (int u = 0; u < UV; ++u) {
           const int col = u * 128 + tid;
-#pragma unroll
+#pragma unroll 1
           for (int c = 0; c < NB; ++c) {
             float v[16];
             tmem_ld16_nowait(lane_addr + 2 * N + u * N + c * 16, v);
@@ -484,7 +607,7 @@ latent_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__
               if (col < p.a.dv) {
 #pragma unroll
                 for (int i = 0; i < 16; ++i)
-                  if (16 * c + i < nh) p.a.ws_o[(slot0 + 16 * c + i) * p.a.dv + col] = v[i];
+                  if (16 * c + i < nh) p.a.ws_o[part(16 * c + i) * p.a.dv + col] = v[i];
               }
               continue;
             }
@@ -498,7 +621,7 @@ latent_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__
               const float got = __shfl_xor_sync(0xffffffffu, odd ? x : y, 1);
               const int h = 16 * c + i + (odd ? 1 : 0);
               if (h < nh && col < p.a.dv)
-                *reinterpret_cast<__nv_bfloat162*>(dst + (long long)h * p.a.dv) = odd ? __floats2bfloat162_rn(got, y) : __floats2bfloat162_rn(x, got);
+                *reinterpret_cast<__nv_bfloat162*>(dst + row_of(h) * p.a.out_rs + head_of(h) * p.a.dv) = odd ? __floats2bfloat162_rn(got, y) : __floats2bfloat162_rn(x, got);
             }
           }
         }
@@ -506,7 +629,7 @@ latent_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__
         for (int u = 0; u < UV; ++u) {
           const int col = u * 128 + tid;
           for (int h = 0; h < nh && col < p.a.dv; ++h)
-            static_cast<__nv_bfloat16*>(p.a.out)[(long long)it.row * p.a.out_rs + (long long)(it.h0 + h) * p.a.dv + col] = __float2bfloat16_rn(0.f);
+            static_cast<__nv_bfloat16*>(p.a.out)[(it.row + row_of(h)) * p.a.out_rs + (it.h0 + head_of(h)) * p.a.dv + col] = __float2bfloat16_rn(0.f);
         }
       }
     }
@@ -536,7 +659,7 @@ struct LtShape {
   int N, uk, uv, upt;
   uint32_t unit_bytes;
   size_t bytes(int units) const {
-    return (size_t)2 * uk * N * 128 + (size_t)(units >= upt + uk ? 4 : 2) * N * 128 + 256 + (size_t)32 * N + 64 + 1024 + (size_t)units * unit_bytes +
+    return (size_t)2 * uk * N * 128 + (size_t)(units >= upt + uk ? 4 : 2) * N * 128 + 256 + (size_t)36 * N + 64 + 1024 + (size_t)units * unit_bytes +
            (unit_bytes < kLtUnit ? kLtBlock : 0);  // a value unit of one block is read as a pair of blocks: the last one's partner must exist
   }
   int units(size_t limit) const {
@@ -545,9 +668,9 @@ struct LtShape {
     return n;
   }
 };
-static LtShape lt_shape(const LatentArgs& a) {
+static LtShape lt_shape(const LatentArgs& a, int rows) {
   LtShape s;
-  s.N = lt_heads(a.H / a.G);
+  s.N = lt_heads(a.H / a.G * rows);
   s.uk = (a.dk + 127) / 128;
   s.uv = (a.dv + 127) / 128;
   s.upt = a.v_col == 0 ? s.uk : s.uk + s.uv;
@@ -555,14 +678,63 @@ static LtShape lt_shape(const LatentArgs& a) {
   return s;
 }
 
-template <int NB, int HS, bool SHARED>
+// Two CTAs per SM where half the shared memory holds a tile and a unit: while one waits for its scores or its
+// probabilities, the other has products to run.  (64 columns need the registers of a whole SM.)
+static int lt_per_sm(const LtShape& sh, long long items, int sms, int limit, int* units) {
+  *units = sh.units((size_t)limit);
+  if (sh.N < 64 && items > sms) {
+    const int half = sh.units((size_t)(limit - 1024) / 2);  // each CTA costs another KB of the SM's 228
+    if (half > sh.upt) {
+      *units = half;
+      return 2;
+    }
+  }
+  return 1;
+}
+
+// Rows of one prompt that an item takes together: the number for which the rounds of items over the CTAs take the least
+// time.  A tile's products cost the same for 16, 32 or 64 columns (A is read from shared memory at the same rate), its
+// softmax does not: an item of 1000 prompt keys takes 34 us alone, 34 to 37 with 16 columns of several rows, 37 to 39 with 32
+// and 53 to 57 with 64 (4 or 8 groups, heads of 128; latents of 256: 33, -, 37, 49; of 512: 53, -, 65, 84).  The keys of
+// the rows themselves are no less work together: a short tile for two rows, or a whole one each.  1000 rows of one prompt of
+// 1000, each by itself / together: 339 / 116 us (4 groups of 128), 570 / 156 (8 groups), 180 / 60 (4 groups of 64),
+// 124 / 92 (latents of 256), 314 / 161 (of 512); 64 prompts with 4 rows each, latents of 512: 97 / 65; 150 with 3 rows,
+// 300 keys, latents of 256, where it does not pay: 39 / 54.
+static int lt_rows(const LatentArgs& a, int sms, int limit) {
+  const int per = a.H / a.G;
+  if (a.share < 2 || a.Tn != 1 || !a.kv.page_table || (per & (per - 1)) != 0) return 1;
+  // Little to share: 1000 rows with 64 prompt keys and 400 of their own took 239 against 184 us (latents of 512) and 242 against
+  // 213 (4 groups of 128); with 128 and 200, 119 against 127 and 111 against 109.
+  if (!a.together && a.own_keys > kLtKeys / 2 && 2LL * a.prompt_keys < a.own_keys) return 1;
+  const double shared = 2 + (a.prompt_keys + kLtKeys - 1) / kLtKeys;  // an item's start and end are about two tiles
+  const double own = a.own_keys <= kLtKeys / 2 ? 0.3 : 0.8 * ((a.own_keys + kLtKeys - 1) / kLtKeys);
+  int best = 1;
+  double least = 0.;
+  for (int rg = 1; rg * per <= 64; rg *= 2) {
+    if (rg > 1 && (rg > 2 * a.share || rg * per < 16)) continue;
+    const LtShape sh = lt_shape(a, rg);
+    if (sh.units((size_t)limit) < sh.upt) continue;
+    if (rg == a.together) return rg;
+    const long long items = (long long)(a.n_seq / a.share) * ((a.share + rg - 1) / rg) * a.G * a.n_splits;
+    int units;
+    const long long ctas = (long long)lt_per_sm(sh, items, sms, limit, &units) * sms;
+    const double t = (double)((items + ctas - 1) / ctas) * ((rg == 1 ? 1. : sh.N == 64 ? 1.6 : 1.2) * shared + rg * own);
+    if (rg == 1 || t < least) {
+      least = t;
+      best = rg;
+    }
+  }
+  return a.together ? 1 : best;
+}
+
+template <int NB, int HS, bool SHARED, bool ROWS = false>
 static int lt_launch(const CUtensorMap& mq, const CUtensorMap& mc, const LtParams& p, int grid, size_t smem, cudaStream_t st) {
-  cudaError_t e = cudaFuncSetAttribute(latent_tc_kernel<NB, HS, SHARED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = cudaFuncSetAttribute(latent_tc_kernel<NB, HS, SHARED, ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) {
     set_error("latent_attn: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
     return DGPT_E_CUDA;
   }
-  launch_few(p.n_rows <= kFewRows, latent_tc_kernel<NB, HS, SHARED>, dim3(grid), dim3(kLtThreads), smem, st, mq, mc, p);
+  launch_few(p.n_rows <= kFewRows, latent_tc_kernel<NB, HS, SHARED, ROWS>, dim3(grid), dim3(kLtThreads), smem, st, mq, mc, p);
   return launch_status("latent_attn");
 }
 
@@ -588,7 +760,7 @@ bool latent_tc_supported(const LatentArgs& a, const dgpt_kv_layout& kv, int dtyp
   if (!tc::device_is_sm100() || tc::encode_fn() == nullptr) return false;
   int sms, smem;
   tc::lt_device(&sms, &smem);
-  const tc::LtShape sh = tc::lt_shape(a);
+  const tc::LtShape sh = tc::lt_shape(a, 1);
   return sh.units((size_t)smem) >= sh.upt;
 }
 
@@ -596,7 +768,8 @@ int latent_tc_launch(const LatentArgs& a, const dgpt_kv_layout& kv, cudaStream_t
   using namespace tc;
   int sms, limit;
   lt_device(&sms, &limit);
-  const LtShape sh = lt_shape(a);
+  const int rg = lt_rows(a, sms, limit);
+  const LtShape sh = lt_shape(a, rg);
   const int N = sh.N;
   LtParams p;
   p.a = a;
@@ -604,22 +777,17 @@ int latent_tc_launch(const LatentArgs& a, const dgpt_kv_layout& kv, cudaStream_t
   p.gpk = (p.per + N - 1) / N;
   p.n_rows = a.n_seq * a.Tn;
   p.n_groups = a.G * p.gpk;
-  p.n_items = p.n_rows * p.n_groups * a.n_splits;
+  p.rg = rg;
+  p.per_log2 = 0;
+  while (1 << p.per_log2 < p.per) ++p.per_log2;
+  p.sets_per_prompt = rg > 1 ? (a.share + rg - 1) / rg : 1;
+  p.n_sets = rg > 1 ? p.n_rows / a.share * p.sets_per_prompt : p.n_rows;
+  p.n_items = p.n_sets * p.n_groups * a.n_splits;
   p.uk = sh.uk;
   p.uv = sh.uv;
   p.upt = sh.upt;
   p.unit_bytes = sh.unit_bytes;
-  // Two CTAs per SM where half the shared memory holds a tile and a unit: while one waits for its scores or its
-  // probabilities, the other has products to run.  (NB = 4 needs the registers of a whole SM.)
-  int per_sm = 1;
-  p.n_units = sh.units((size_t)limit);
-  if (N < 64 && p.n_items > sms) {
-    const int half = sh.units((size_t)(limit - 1024) / 2);  // each CTA costs another KB of the SM's 228
-    if (half > p.upt) {
-      per_sm = 2;
-      p.n_units = half;
-    }
-  }
+  const int per_sm = lt_per_sm(sh, p.n_items, sms, limit, &p.n_units);
   const int pt = kv.page_tokens;
   p.box = kv.page_table && pt < kLtKeys ? pt : kLtKeys;
   p.align = kv.page_table ? p.box : 1;  // a dense run may be entered at any slot
@@ -627,7 +795,7 @@ int latent_tc_launch(const LatentArgs& a, const dgpt_kv_layout& kv, cudaStream_t
   {
     const cuuint64_t dims[3] = {(cuuint64_t)a.dk, (cuuint64_t)a.H, (cuuint64_t)p.n_rows};
     const cuuint64_t strides[2] = {(cuuint64_t)a.dk * 2, (cuuint64_t)a.q_rs * 2};
-    const cuuint32_t box[3] = {64, (cuuint32_t)N, 1};
+    const cuuint32_t box[3] = {64, (cuuint32_t)(N / rg), (cuuint32_t)rg};  // with several rows their heads make N
     if (!encode_3d(&mq, a.q, dims, strides, box)) return DGPT_E_CUDA;
   }
   {
@@ -639,6 +807,16 @@ int latent_tc_launch(const LatentArgs& a, const dgpt_kv_layout& kv, cudaStream_t
   }
   const size_t smem = sh.bytes(p.n_units);
   const int grid = p.n_items < per_sm * sms ? p.n_items : per_sm * sms;
+  if (rg > 1) {
+    if (a.v_col == 0) {
+      if (N == 16) return lt_launch<1, 16, true, true>(mq, mc, p, grid, smem, st);
+      if (N == 32) return lt_launch<2, 32, true, true>(mq, mc, p, grid, smem, st);
+      return lt_launch<4, 64, true, true>(mq, mc, p, grid, smem, st);
+    }
+    if (N == 16) return lt_launch<1, 16, false, true>(mq, mc, p, grid, smem, st);
+    if (N == 32) return lt_launch<2, 32, false, true>(mq, mc, p, grid, smem, st);
+    return lt_launch<4, 64, false, true>(mq, mc, p, grid, smem, st);
+  }
   if (a.v_col == 0) {
     if (N == 16) return lt_launch<1, 16, true>(mq, mc, p, grid, smem, st);
     if (N == 32) return lt_launch<2, 32, true>(mq, mc, p, grid, smem, st);

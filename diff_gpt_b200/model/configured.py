@@ -5,6 +5,7 @@ from __future__ import annotations
 
 import contextlib
 from abc import abstractmethod
+from dataclasses import dataclass
 from typing import Callable
 
 import torch
@@ -51,6 +52,26 @@ def pick_latent_splits(rows: int, head_groups: int, keys: int) -> int:
     if ctas >= _sm_count() or keys <= 128:
         return 1
     return max(1, min(_sm_count() // ctas, -(-keys // 128), 64))
+
+
+@dataclass(frozen=True)
+class Shared:
+    """Rows that decode behind one prompt: runs of `rows` sequences see the same pages of `prompt` tokens, and add up to `new`."""
+
+    rows: int = 1
+    prompt: int = 0
+    new: int = 0
+
+    @classmethod
+    def of(cls, cache) -> "Shared":
+        return cls(cache.rows_per_series, cache.prefix_len, cache.max_new)
+
+    def keys(self, window: int) -> dict[str, int]:
+        """The attention's arguments: what a row sees half way through."""
+        own = (self.new + 1) // 2
+        if window:
+            own = min(own, window)
+        return dict(share=self.rows, prompt_keys=min(self.prompt, window - own) if window else self.prompt, own_keys=own)
 
 
 class ConfiguredModel(DeviceModel):

@@ -33,7 +33,7 @@ import torch.nn.functional as F
 
 from .. import ops
 from .._lib import region
-from .configured import FUSED_FF_MIN_ROWS, ConfiguredModel, fp32_reductions, linear, pick_latent_splits, round_up
+from .configured import FUSED_FF_MIN_ROWS, ConfiguredModel, Shared, fp32_reductions, linear, pick_latent_splits, round_up
 from .kv_cache import LatentCache, PagedLatentCache
 
 EXPAND_MIN_TOKENS = 32  # query tokens per sequence from which keys and values are expanded
@@ -194,6 +194,7 @@ class LatentBinding:
     conv_in: torch.Tensor | None = None  # [n_layer, n_seq, taps - 1, C]
     conv_out: torch.Tensor | None = None
     fmha_impl: int = 0
+    share: Shared = Shared()
 
 
 class DelunexPlan:
@@ -270,7 +271,7 @@ class DelunexPlan:
                 ws = self._buf("ws", ops.latent_attn_workspace_bytes(n, H, r, splits) // 4, dtype=torch.float32)
             ops.latent_attn(
                 qa, b.layout(lw.owner), b.len0, b.start1, b.len1, b.step, oa, n_seq=n_seq, T=T, H=H, r=r, window=lw.window,
-                scale=lw.scale, gate=gate, workspace=ws, n_splits=splits, status=self.status,
+                scale=lw.scale, gate=gate, workspace=ws, n_splits=splits, **b.share.keys(lw.window), status=self.status,
             )
             with region("gemm_absorb"):
                 torch.bmm(oa.view(n, H, r).transpose(0, 1), lw.w_uv_t, out=o.view(n, H, D).transpose(0, 1))
@@ -433,6 +434,7 @@ class Delunex(ConfiguredModel):
         bind = LatentBinding(
             layout=layouts.__getitem__, slot0=slot0, start1=slot0, len0=prompt_lens.repeat_interleave(cache.rows_per_series).contiguous(),
             len1=torch.ones(R, dtype=torch.int32, device=dev), step=step, keys=max_keys, conv_in=cache.rows, conv_out=cache.rows,
+            share=Shared.of(cache),
         )
         return bind, DelunexPlan(self, R, 1, want_logits=want_logits, few_rows=few_rows)
 

@@ -37,7 +37,7 @@ import torch.nn.functional as F
 
 from .. import ops
 from .._lib import region
-from .configured import FUSED_FF_MIN_ROWS, ConfiguredModel, fp32_reductions, linear, pick_latent_splits, round_up
+from .configured import FUSED_FF_MIN_ROWS, ConfiguredModel, Shared, fp32_reductions, linear, pick_latent_splits, round_up
 from .kv_cache import PagedRowCache, RowCache, StateSpec
 from .rope import rotation_table
 
@@ -254,6 +254,7 @@ class RowBinding:
     context: int | None = None
     kv_layout: Callable[[int, int, int], object] | None = None
     fmha_impl: int = 0
+    share: Shared = Shared()
 
 
 class KipolixPlan:
@@ -322,7 +323,7 @@ class KipolixPlan:
             ws = self._buf("ws", ops.latent_attn_workspace_bytes(n, H, D, splits) // 4, dtype=torch.float32)
         ops.grouped_attn(
             q, b.layout(run), b.len0, b.start1, b.len1, b.step, o, row_width=width, v_col=v_col, n_seq=n_seq, T=T, H=H, G=G, dk=D, dv=D,
-            window=m.window, keep_first=m.keep_first, scale=m.scale, workspace=ws, n_splits=splits, status=self.status,
+            window=m.window, keep_first=m.keep_first, scale=m.scale, workspace=ws, n_splits=splits, **b.share.keys(m.window), status=self.status,
         )
         return o
 
@@ -499,7 +500,7 @@ class Kipolix(ConfiguredModel):
         bind = RowBinding(
             layout=layouts.__getitem__, slot0=slot0, pos0=row_len, start1=slot0, len0=row_len,
             len1=torch.ones(R, dtype=torch.int32, device=dev), step=step, keys=max_keys, tables=self.tables(max_keys),
-            state_in=cache.states, state_out=cache.states,
+            state_in=cache.states, state_out=cache.states, share=Shared.of(cache),
         )
         return bind, KipolixPlan(self, R, 1, want_logits=want_logits, few_rows=few_rows)
 

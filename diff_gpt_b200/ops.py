@@ -736,18 +736,24 @@ def latent_attn(
     workspace: torch.Tensor | None = None,
     n_splits: int = 1,
     impl: int = 0,
+    share: int = 1,
+    together: int = 0,
+    prompt_keys: int = 0,
+    own_keys: int = 0,
     status: torch.Tensor | None = None,
 ) -> None:
-    """q, out: [n_seq * T, H * r]; gate: [n_seq * T, H]."""
+    """q, out: [n_seq * T, H * r]; gate: [n_seq * T, H].  share: runs of so many sequences see the same prompt pages; prompt_keys,
+    own_keys: about how many keys of the prompt and after it a row sees."""
     _cuda(q, len0, start1, len1, step, out, gate, workspace, status)
     assert q.shape == out.shape == (n_seq * T, H * r) and q.stride(1) == out.stride(1) == 1 and q.dtype == out.dtype
     assert gate is None or (gate.shape == (n_seq * T, H) and gate.stride(1) == 1 and gate.dtype == q.dtype)
     ws_bytes = 0 if workspace is None else workspace.numel() * workspace.element_size()
     check(
-        lib.dgpt_latent_attn(
+        lib.dgpt_latent_attn_shared(
             q.data_ptr(), q.stride(0), C.byref(kv), _ptr(len0), start1.data_ptr(), len1.data_ptr(), _ptr(step), _ptr(gate),
             0 if gate is None else gate.stride(0), out.data_ptr(), out.stride(0), _ptr(workspace), ws_bytes, n_splits, n_seq, T, H,
-            r, window, scale, dtype_code(q), impl, _ptr(status), _stream(),
+            r, window, scale, dtype_code(q), impl, share, together, prompt_keys, own_keys,
+            _ptr(status), _stream(),
         )
     )
 
@@ -929,19 +935,25 @@ def grouped_attn(
     workspace: torch.Tensor | None = None,
     n_splits: int = 1,
     impl: int = 0,
+    share: int = 1,
+    together: int = 0,
+    prompt_keys: int = 0,
+    own_keys: int = 0,
     status: torch.Tensor | None = None,
 ) -> None:
-    """q: [n_seq * T, H * dk]; out: [n_seq * T, H * dv]; gate: [n_seq * T, H]."""
+    """q: [n_seq * T, H * dk]; out: [n_seq * T, H * dv]; gate: [n_seq * T, H].  share: runs of so many sequences see the same prompt pages; prompt_keys,
+    own_keys: about how many keys of the prompt and after it a row sees."""
     _cuda(q, len0, start1, len1, step, out, gate, workspace, status)
     n = n_seq * T
     assert q.shape == (n, H * dk) and out.shape == (n, H * dv) and q.stride(1) == out.stride(1) == 1 and q.dtype == out.dtype
     assert gate is None or (gate.shape == (n, H) and gate.stride(1) == 1 and gate.dtype == q.dtype)
     ws_bytes = 0 if workspace is None else workspace.numel() * workspace.element_size()
     check(
-        lib.dgpt_grouped_attn(
+        lib.dgpt_grouped_attn_shared(
             q.data_ptr(), q.stride(0), C.byref(kv), row_width, v_col, _ptr(len0), start1.data_ptr(), len1.data_ptr(), _ptr(step),
             _ptr(gate), 0 if gate is None else gate.stride(0), out.data_ptr(), out.stride(0), _ptr(workspace), ws_bytes, n_splits, n_seq,
-            T, H, G, dk, dv, window, keep_first, scale, dtype_code(q), impl, _ptr(status), _stream(),
+            T, H, G, dk, dv, window, keep_first, scale, dtype_code(q), impl, share, together, prompt_keys, own_keys,
+            _ptr(status), _stream(),
         )
     )
 

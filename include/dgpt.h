@@ -464,6 +464,18 @@ int dgpt_latent_attn(const void* q, int64_t q_row_stride, const dgpt_kv_layout* 
                      const int32_t* len1, const int32_t* step_ptr, const void* gate, int64_t gate_row_stride, void* out,
                      int64_t out_row_stride, void* workspace, size_t workspace_bytes, int32_t n_splits, int32_t n_seq, int32_t T,
                      int32_t H, int32_t r, int32_t window, float scale, int32_t dtype, int32_t impl, int32_t* status, void* stream);
+/* The same for sequences that share prompts: each run of `share` sequences (n_seq is a multiple of it) has the same len0,
+ * start1 and len1 and the same page table entries for the slots below len0, which the tcgen05 kernel then reads once for
+ * several rows.  Results are those of dgpt_latent_attn but for the order in which a row's weights are added.  together: rows
+ * that are taken at once, 0 = choose, 1 = each by itself, or a power of two by which the heads that share a cache row become
+ * 16, 32 or 64 (T = 1 and pages only).  prompt_keys, own_keys: about how many keys below and from len0 on a row sees, for
+ * the choice. */
+int dgpt_latent_attn_shared(const void* q, int64_t q_row_stride, const dgpt_kv_layout* kv, const int32_t* len0,
+                            const int32_t* start1, const int32_t* len1, const int32_t* step_ptr, const void* gate,
+                            int64_t gate_row_stride, void* out, int64_t out_row_stride, void* workspace, size_t workspace_bytes,
+                            int32_t n_splits, int32_t n_seq, int32_t T, int32_t H, int32_t r, int32_t window, float scale,
+                            int32_t dtype, int32_t impl, int32_t share, int32_t together, int32_t prompt_keys, int32_t own_keys,
+                            int32_t* status, void* stream);
 
 /* Grouped-query attention over cached rows [keys of G groups | values of G groups], with a sliding window and first tokens
  * that stay visible:
@@ -480,6 +492,13 @@ int dgpt_grouped_attn(const void* q, int64_t q_row_stride, const dgpt_kv_layout*
                       size_t workspace_bytes, int32_t n_splits, int32_t n_seq, int32_t T, int32_t H, int32_t G, int32_t dk,
                       int32_t dv, int32_t window, int32_t keep_first, float scale, int32_t dtype, int32_t impl,
                       int32_t* status, void* stream);
+/* share, together, prompt_keys, own_keys: as in dgpt_latent_attn_shared. */
+int dgpt_grouped_attn_shared(const void* q, int64_t q_row_stride, const dgpt_kv_layout* kv, int32_t row_width, int32_t v_col,
+                             const int32_t* len0, const int32_t* start1, const int32_t* len1, const int32_t* step_ptr,
+                             const void* gate, int64_t gate_row_stride, void* out, int64_t out_row_stride, void* workspace,
+                             size_t workspace_bytes, int32_t n_splits, int32_t n_seq, int32_t T, int32_t H, int32_t G, int32_t dk,
+                             int32_t dv, int32_t window, int32_t keep_first, float scale, int32_t dtype, int32_t impl,
+                             int32_t share, int32_t together, int32_t prompt_keys, int32_t own_keys, int32_t* status, void* stream);
 
 /* out = scale * emb[ids] in fp32.  ids: device int32 [n_tokens]; emb: [V, C] in dtype; out: fp32 [n_tokens, C]. */
 int dgpt_embed_scale(const int32_t* ids, const void* emb, float* out, int64_t n_tokens, int32_t C, int32_t V, float scale,
