@@ -67,7 +67,7 @@ template <bool KEPT, bool ROWS>
 __device__ __forceinline__ LtItem lt_item(const LtParams& p, int item, int N) {
   LtItem it;
   // Groups change fastest: those of a row lie beside each other in memory and are read at the same time, so DRAM pages are opened once.
-  // 256 rows of 545 keys, 4 groups of 128: 84 -> 80.5 us, 200 rows of 1450, 8 groups: 236 -> 231, 1000 rows of one prompt, 8 groups,
+  // 256 rows of 545 keys, 4 groups of 128: 83 -> 81 us, 200 rows of 1450, 8 groups: 236 -> 232, 1000 rows of one prompt, 8 groups,
   // 32 rows together: 157 -> 141, 4 groups, 16 together: 115 -> 107.
   const int sp = item / p.n_groups, grp = item - sp * p.n_groups;
   it.split = sp / p.n_sets;
