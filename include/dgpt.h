@@ -120,8 +120,10 @@ int dgpt_rope_qknorm_kvappend(const void* q, const void* k, const void* v, int64
  * kv: sequence index = b;  kv_len: device int32 [B] or NULL (then kv_len_all is used).
  * impl: 0 = choose (bf16 with D = 32, 64 or 128 and whole tiles of 128 keys, or pages that make them up, runs on the tcgen05
  * tensor cores: the warp-specialised kernel from 640 keys on and where one CTA per SM holds every query tile, the two-CTAs-per-SM
- * one otherwise.  Dense keys of any other length run on the two-CTAs-per-SM one with each probability as a pair of bf16 numbers,
- * from 24 keys on (D = 32: 33) and unless the output is fp32.  Everything else takes the warp-level online-softmax kernel),
+ * one otherwise; D = 32 up to 256 keys, and from 128 pairs of sequence and head on, a kernel with the products in registers.
+ * Dense keys of any other length keep each probability as a pair of bf16 numbers, from 24 keys on (D = 32: 33) and unless the
+ * output is fp32: on that kernel for D = 32 and, but for 65 to 128 keys, D = 64 while K and V of a pair fit its shared memory, on the
+ * two-CTAs-per-SM one otherwise.  Everything else takes the warp-level online-softmax kernel),
  * 1 = warp-level kernel, 2 = warp-specialised
  * tensor-core kernel or fail, 3 = tensor-core kernel with two CTAs per SM or fail, 4 = persistent tensor-core kernel
  * with two query tiles per CTA or fail.
