@@ -11,14 +11,15 @@
 //   warp 5, lane 0  loader: Q of the item, then the units of its tiles into a ring, through TMA straight from the pages
 //   warp 4, lane 0  issuer: S^T into one of two TMEM buffers, O^T += V^T P^T; with room in the ring the scores of the
 //                   next tile are issued before the sums of this one
-//   warps 0-3       softmax, one thread per key: probabilities against a running reference per head, kept in shared memory,
-//                   that only moves when it is exceeded by 2^8 (found with one barrier vote per tile), written as bf16 into
-//                   shared memory;
+//   warps 0-3       softmax, one thread per key: probabilities against a running reference per head, kept in shared memory;
+//                   when one of a row's is exceeded by 2^8 (found with one barrier vote per tile) all of that row's move to
+//                   its maxima so far; written as bf16 into shared memory;
 //                   after the item's last tile, one thread per column: normalise, gate, store
 // Rows behind one prompt (ROWS): an item is a set of up to rg of them, whose heads together are the N of the products over
 // the prompt's tiles; then come the tiles of each row's own slots (those of two rows in one tile where they fit its halves),
-// whose products cover that row's columns only.  The columns' references move each for itself, so that a row's numbers do not
-// depend on its neighbours but for the order in which its weights are added.
+// whose products cover that row's columns only.  A row's result has the bits that it gets by itself, so that the tokens drawn from it do not depend on
+// how many rows there are: a split is cut at the same tiles, references move row by row, and where a tile holds two rows' slots the second row's
+// weights are handed to the threads that would have had them (tests/test_gpu_shared_rows.py).
 // A row of a unit that holds fewer than 64 columns leaves the block's other accumulator rows undefined; they are not read.
 // TMEM columns: S0 [0, N)  S1 [N, 2N)  O of unit u [2N + u N, +N).
 // Every mbarrier wait is bounded.  When one runs out the abort flag is raised, the loader and the issuer stop and drain
@@ -40,7 +41,7 @@ struct LtParams {
   LatentArgs a;
   int n_rows, n_groups, n_items;  // item = (split * n_sets + set) * n_groups + group
   int n_sets;                     // sets of rows: one row each, or
-  int rg, per_log2;               // ROWS: up to rg rows of one prompt; log2 of the heads that share a row
+  int rg, cols, cols_log2;        // ROWS: up to rg rows of one prompt, each in `cols` columns: the heads that share a cache row, or four
   int sets_per_prompt;
   int per, gpk;                   // heads that share a row, and item groups they make
   int n_units;                    // units in the ring
@@ -55,7 +56,8 @@ __device__ __forceinline__ int lt_blocks(int cols, int u) { return cols - u * 12
 
 struct LtItem {
   int row, seq, g, h0, nh, split;
-  int nr, n_shared, n_own;        // ROWS: rows of the set, tiles of their prompt, tiles of each one's own slots
+  int nr, n_shared;               // ROWS: rows of the set, tiles of their prompt
+  int n_mine, own0, n_own;        // ROWS: this split's tiles of the prompt; its first tile of each row's own slots, and how many
   bool pairs;                     // own slots fit half a tile: one holds those of two rows
   int begin[3], end[3], base[3];  // the slot ranges and where their tiles start
   int n_first, n_second;          // tiles of the first range, of the first two
@@ -67,8 +69,7 @@ template <bool KEPT, bool ROWS>
 __device__ __forceinline__ LtItem lt_item(const LtParams& p, int item, int N) {
   LtItem it;
   // Groups change fastest: those of a row lie beside each other in memory and are read at the same time, so DRAM pages are opened once.
-  // 256 rows of 545 keys, 4 groups of 128: 83 -> 81 us, 200 rows of 1450, 8 groups: 236 -> 232, 1000 rows of one prompt, 8 groups,
-  // 32 rows together: 157 -> 141, 4 groups, 16 together: 115 -> 107.
+  // 256 rows of 545 keys, 4 groups of 128: 83 -> 81 us, 200 rows of 1450, 8 groups: 236 -> 232.
   const int sp = item / p.n_groups, grp = item - sp * p.n_groups;
   it.split = sp / p.n_sets;
   it.row = sp - it.split * p.n_sets;
@@ -86,7 +87,7 @@ __device__ __forceinline__ LtItem lt_item(const LtParams& p, int item, int N) {
     first = (grp - it.g * p.gpk) * N;
     it.h0 = it.g * p.per + first;
   }
-  it.nh = ROWS ? it.nr << p.per_log2 : min(N, p.per - first);
+  it.nh = ROWS ? it.nr << p.cols_log2 : min(N, p.per - first);
   const LatentKeys k = latent_keys(p.a, it.row);
   it.seq = k.seq;
   // [0, ks) and [lo, n), cut where slots change from the first run to the second; the cut lies in one of the two
@@ -106,16 +107,23 @@ __device__ __forceinline__ LtItem lt_item(const LtParams& p, int item, int N) {
   it.n_first = KEPT ? nt[0] : 0;
   it.n_second = it.n_first + nt[1];
   it.n_shared = own ? it.n_first : it.n_second;
-  it.n_own = it.n_second + nt[2] - it.n_shared;
-  it.pairs = ROWS && p.box <= kLtKeys / 2 && it.n_own == 1 && nt[2] == 1 && it.end[2] - it.base[2] <= kLtKeys / 2;
-  const int total = it.n_shared + (it.pairs ? (it.nr + 1) / 2 : it.nr * it.n_own);
-  if (p.a.n_splits == 1) {
-    it.t0 = 0;
-    it.n = total;
-  } else {
+  // the tiles of one row, and those of them that are this split's
+  const int total = it.n_second + nt[2];
+  int t1 = total;
+  it.t0 = 0;
+  if (p.a.n_splits > 1) {
     const int per = (total + p.a.n_splits - 1) / p.a.n_splits;
     it.t0 = min(total, it.split * per);
-    it.n = min(total, it.t0 + per) - it.t0;
+    t1 = min(total, it.t0 + per);
+  }
+  it.n = t1 - it.t0;
+  it.pairs = false;
+  if (ROWS) {
+    it.n_mine = max(0, min(t1, it.n_shared) - it.t0);
+    it.own0 = max(it.t0, it.n_shared);
+    it.n_own = max(0, t1 - it.own0);
+    it.pairs = p.box <= kLtKeys / 2 && total - it.n_shared == 1 && nt[2] == 1 && it.end[2] - it.base[2] <= kLtKeys / 2;
+    it.n = it.n_mine + (it.pairs ? (it.nr + 1) / 2 * it.n_own : it.nr * it.n_own);
   }
   return it;
 }
@@ -130,11 +138,11 @@ __device__ __forceinline__ LtTile lt_tile(const LtItem& it, int j) {
   int t = it.t0 + j;
   x.own = -1;
   x.pair = false;
-  if (ROWS && t >= it.n_shared) {
-    t -= it.n_shared;
+  if (ROWS && j >= it.n_mine) {
+    t = j - it.n_mine;
     x.pair = it.pairs;
     x.own = it.pairs ? 2 * t : t / it.n_own;
-    t = it.pairs ? it.n_shared : it.n_shared + t - x.own * it.n_own;
+    t = it.own0 + (it.pairs ? 0 : t - x.own * it.n_own);
   }
   if (KEPT && t < it.n_first) {
     x.begin = it.begin[0];
@@ -197,7 +205,7 @@ __device__ __forceinline__ float lt_reduce16(const float* v, int lane, F op) {
 
 // NB: columns of the products = 16 NB; HS <= 16 NB: heads the softmax looks after (a group may hold fewer than 16).
 // SHARED: a tile's values are its keys (latents), whose cache has no kept first keys.
-// ROWS: a column is a head of one of rg rows, column c = row c >> per_log2, head c & (per - 1); HS = 16 NB.
+// ROWS: a column is a head of one of rg rows, column c = row c >> cols_log2, head c & (cols - 1); HS = 16 NB.
 template <int NB, int HS, bool SHARED, bool ROWS>
 __global__ void __launch_bounds__(kLtThreads, NB == 4 ? 1 : 2)
 latent_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__ CUtensorMap mc, const LtParams p) {
@@ -229,7 +237,8 @@ latent_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__
   float* red = reinterpret_cast<float*>(bars + 32);  // [4 warps][N]
   float* fac = red + 4 * N;                          // [4 warps][N]
   float* ref = fac + 4 * N;                          // [N] what the probabilities of a head are relative to
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(ref + N);
+  float* hand = ref + N;                             // ROWS, half tiles: [N / 2][64 keys] weights of second rows
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(ROWS && p.box <= kLtKeys / 2 ? hand + 32 * N : hand);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   const uint32_t aU = smem_u32(sU), aQ = smem_u32(sQ), aP = smem_u32(sP);
   const uint32_t bar0 = smem_u32(bars);
@@ -313,9 +322,9 @@ latent_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__
       const uint64_t dC = smem_desc(0, 16, 1024), dM = smem_desc(0, kLtBlock, 1024);  // K-major rows; MN-major pairs of blocks
       // the products of rows' own slots: of their columns only
       auto own_n = [&](const LtTile& x, uint32_t idesc) {
-        return !ROWS || x.own < 0 ? idesc : (idesc & ~(63u << 17)) | (uint32_t)max(2, (x.pair ? 2 : 1) * p.per >> 3) << 17;
+        return !ROWS || x.own < 0 ? idesc : (idesc & ~(63u << 17)) | (uint32_t)max(2, (x.pair ? 2 : 1) * p.cols >> 3) << 17;
       };
-      auto own_block = [&](const LtTile& x) { return ROWS && x.own >= 0 ? (x.own << p.per_log2) >> 4 : 0; };
+      auto own_block = [&](const LtTile& x) { return ROWS && x.own >= 0 ? (x.own << p.cols_log2) >> 4 : 0; };
       unsigned g = 0u, items = 0u;  // tiles; items
       bool ok = true;
       for (int item = blockIdx.x; ok && item < p.n_items; item += gridDim.x) {
@@ -397,8 +406,9 @@ latent_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__
       for (int i = tid; i < (int)((ahead ? 4 : 2) * kPBlock / 16); i += 128) reinterpret_cast<uint4*>(sP)[i] = make_uint4(0u, 0u, 0u, 0u);
     if (tid < N) ref[tid] = -INFINITY;
     lt_sync();
-    auto row_of = [&](int c) -> long long { return ROWS ? c >> p.per_log2 : 0; };
-    auto head_of = [&](int c) -> long long { return ROWS ? c & (p.per - 1) : c; };
+    auto row_of = [&](int c) -> long long { return ROWS ? c >> p.cols_log2 : 0; };
+    auto head_of = [&](int c) -> long long { return ROWS ? c & (p.cols - 1) : c; };
+    auto there = [&](int c, int nh) { return c < nh && (!ROWS || head_of(c) < p.per); };  // the column is a head's
     for (int item = blockIdx.x; item < p.n_items; item += gridDim.x) {
       const LtItem it = lt_item<!SHARED, ROWS>(p, item, N);
       const int nh = it.nh;
@@ -409,7 +419,7 @@ latent_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__
       for (int c = 0; c < HL; ++c) {  // wanted at the end only
         const int h = lane + 32 * c;
         gate[c] = 1.f;
-        if (p.a.gate && h < nh)
+        if (p.a.gate && there(h, nh))
           gate[c] = __bfloat162float(static_cast<const __nv_bfloat16*>(p.a.gate)[(it.row + row_of(h)) * p.a.gate_rs + it.h0 + head_of(h)]);
       }
       float l[HS];
@@ -420,9 +430,9 @@ latent_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__
         const LtTile x = lt_tile<!SHARED, ROWS>(it, j);
         const int half = ROWS && x.pair ? tid >> 6 : 0, slot = x.slot + tid - 64 * half, end = x.end;
         // The tile concerns columns [c_lo, c_hi), this thread's key [k_lo, k_hi) of them.
-        const int c_lo = ROWS && x.own >= 0 ? x.own << p.per_log2 : 0;
-        const int c_hi = ROWS && x.own >= 0 ? c_lo + (x.pair ? 2 : 1) * p.per : HS;
-        const int k_lo = c_lo + half * p.per, k_hi = ROWS && x.own >= 0 ? k_lo + p.per : HS;
+        const int c_lo = ROWS && x.own >= 0 ? x.own << p.cols_log2 : 0;
+        const int c_hi = ROWS && x.own >= 0 ? c_lo + (x.pair ? 2 : 1) * p.cols : HS;
+        const int k_lo = c_lo + half * p.cols, k_hi = ROWS && x.own >= 0 ? k_lo + p.cols : HS;
         auto block = [&](int c) { return !ROWS || (c_lo < 16 * c + 16 && c_hi > 16 * c); };
         const bool seen = slot >= x.begin && slot < end && (!ROWS || x.own + half < it.nr);
         auto columns = [&](int c) -> unsigned {  // of block c, one bit each
@@ -454,7 +464,7 @@ latent_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__
           }
         }
         __syncwarp();
-        float s[N];  // log2 of what is added for this key, against the heads' references
+        float s[N];  // log2 of what is added for this key, against the heads' references (a score is rounded before its reference is taken off)
         for (int pass = 0;; ++pass) {
 #pragma unroll
           for (int c = 0; c < NB; ++c) tmem_ld16_nowait(lane_addr + b * N + c * 16, s + 16 * c);
@@ -472,13 +482,13 @@ latent_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__
 #pragma unroll
               for (int k = 0; k < 4; ++k) {
                 const int h = 16 * c + i + k;
-                s[h] = (cols >> (i + k)) & 1u ? fmaf(s[h], p.a.scale_log2, -mm[k]) : -INFINITY;
+                s[h] = (cols >> (i + k)) & 1u ? __fmul_rn(s[h], p.a.scale_log2) - mm[k] : -INFINITY;
                 top = fmaxf(top, s[h]);
               }
             }
           }
-          if (pass || !lt_any(top > 8.f && !fail)) break;
-          // Some head's reference has to move.  Rare but for an item's first tile, so the loops stay rolled: with every
+          if (pass || !lt_any(top >= 8.f && !fail)) break;  // (a score above the rounded reference + 8 is 8 above the reference)
+          // Some row's references have to move.  Rare but for an item's first tile, so the loops stay rolled: with every
           // block's code laid out the instructions of a first tile took longer to fetch than the tile.
 #pragma unroll 1
           for (int c = c_lo >> 4; c < NB && 16 * c < c_hi; ++c) {
@@ -487,21 +497,25 @@ latent_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__
             tc_wait_ld();
             const unsigned cols = columns(c);
 #pragma unroll
-            for (int i = 0; i < 16; ++i) v[i] = (cols >> i) & 1u ? v[i] * p.a.scale_log2 : -INFINITY;
+            for (int i = 0; i < 16; ++i) v[i] = (cols >> i) & 1u ? __fmul_rn(v[i], p.a.scale_log2) : -INFINITY;
             const float t = lt_reduce16(v, lane, [](float x, float y) { return fmaxf(x, y); });
             if (lane < 16) red[warp * N + 16 * c + lane] = t;
           }
           lt_sync();
-          if (tid < N) {
+          if (warp < (N + 31) / 32) {
+            const bool in = tid >= c_lo && tid < c_hi;  // (c_hi <= N)
+            const float mo = in ? ref[tid] : 0.f;
+            const float mt = in ? fmaxf(fmaxf(red[tid], red[N + tid]), fmaxf(red[2 * N + tid], red[3 * N + tid])) : 0.f;
+            const unsigned want = __ballot_sync(0xffffffffu, in && mt > mo + 8.f);
+            // rows together: those of the row in whose columns one wants to (there are at most 32 of them, within the warp)
+            const bool move = in && (!ROWS || (want >> (lane & ~(p.cols - 1)) & (p.cols == 32 ? ~0u : (1u << p.cols) - 1u)) != 0u);
             float alpha = 1.f;
-            if (tid >= c_lo && tid < c_hi) {
-              const float mn = fmaxf(fmaxf(red[tid], red[N + tid]), fmaxf(red[2 * N + tid], red[3 * N + tid])), mo = ref[tid];
-              if (mn > mo + 8.f) {  // only a head that needs it moves: what a row gets does not depend on the rows beside it
-                alpha = ex2(mo - mn);  // -inf before the first tile: 0
-                ref[tid] = mn;
-              }
+            if (move) {
+              const float mn = fmaxf(mt, mo);
+              alpha = mn == -INFINITY ? 1.f : ex2(mo - mn);  // -inf before the first tile: 0
+              ref[tid] = mn;
             }
-            fac[tid] = alpha;
+            if (tid < N) fac[tid] = alpha;
           }
           __syncwarp();
           lt_sync();  // and `red` may be written again
@@ -537,6 +551,21 @@ latent_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__
             tc_wait_st();
           }
         }
+        // The second row of a tile: its weights go to the sums of the threads that would have had them were the row by itself.
+        const float mine = half ? 0.f : 1.f;
+        if (ROWS && half && x.own + 1 < it.nr) {
+#pragma unroll 1
+          for (int c = k_lo >> 4; 16 * c < k_hi; ++c) {
+            float v[16];
+            tmem_ld16_nowait(lane_addr + b * N + c * 16, v);
+            tc_wait_ld();
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
+              const int h = 16 * c + i;
+              if (h >= k_lo && h < k_hi) hand[((x.own >> 1) * p.cols + h - k_lo) * 64 + (tid & 63)] = seen ? ex2(__fmul_rn(v[i], p.a.scale_log2) - ref[h]) : 0.f;
+            }
+          }
+        }
         uint8_t* pb = sP + ((ahead ? 2 * b : 0u) + (tid >> 6)) * kPBlock + (tid & 7) * 2;
         const int chunk = (tid & 63) >> 3;
 #pragma unroll
@@ -548,7 +577,7 @@ latent_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__
             const int h = 16 * c + i;
             if (h >= HS) continue;
             const float e = ex2(s[h]);  // not seen: 0
-            l[h % HS] += e;
+            l[h % HS] = ROWS ? fmaf(e, mine, l[h % HS]) : l[h % HS] + e;
             *reinterpret_cast<__nv_bfloat16*>(pb + h * 128 + ((chunk ^ (h & 7)) << 4)) = __float2bfloat16_rn(e);
           }
         }
@@ -562,6 +591,19 @@ latent_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__
         if (!fail && !wait_or_abort(bar_o + 8 * (last & 1u), (last >> 1) & 1u, abort_flag, 58)) fail = true;
         fail = __any_sync(0xffffffffu, fail);
         tc_fence_after();
+      }
+      if (ROWS && it.pairs && it.n_own > 0) {
+        lt_sync();
+        if (tid < 64) {
+#pragma unroll
+          for (int h = 4; h < HS; h += 4) {  // (a row's columns are four or more)
+            const int r = h >> p.cols_log2;
+            if (!(r & 1) || h >= nh) continue;
+            const float* from = hand + ((r >> 1 << p.cols_log2) + (h & (p.cols - 1))) * 64 + tid;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) l[h + i] += from[64 * i];
+          }
+        }
       }
 #pragma unroll
       for (int c = 0; c < NB; ++c) {
@@ -583,7 +625,7 @@ latent_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__
           float f = sum > 0.f ? 1.f / sum : 0.f;
           if (p.a.gate) f *= 1.f / (1.f + __expf(-gate[c]));
           fac[warp * N + h] = f;
-          if (p.a.n_splits > 1 && warp == 0 && h < nh) {
+          if (p.a.n_splits > 1 && warp == 0 && there(h, nh)) {
             p.a.ws_ml[2 * part(h)] = ref[h];
             p.a.ws_ml[2 * part(h) + 1] = sum;
           }
@@ -608,7 +650,7 @@ latent_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__
               if (col < p.a.dv) {
 #pragma unroll
                 for (int i = 0; i < 16; ++i)
-                  if (16 * c + i < nh) p.a.ws_o[part(16 * c + i) * p.a.dv + col] = v[i];
+                  if (there(16 * c + i, nh)) p.a.ws_o[part(16 * c + i) * p.a.dv + col] = v[i];
               }
               continue;
             }
@@ -621,7 +663,7 @@ latent_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__
               const float x = v[i] * fac[warp * N + 16 * c + i], y = v[i + 1] * fac[warp * N + 16 * c + i + 1];
               const float got = __shfl_xor_sync(0xffffffffu, odd ? x : y, 1);
               const int h = 16 * c + i + (odd ? 1 : 0);
-              if (h < nh && col < p.a.dv)
+              if (there(h, nh) && col < p.a.dv)
                 *reinterpret_cast<__nv_bfloat162*>(dst + row_of(h) * p.a.out_rs + head_of(h) * p.a.dv) = odd ? __floats2bfloat162_rn(got, y) : __floats2bfloat162_rn(x, got);
             }
           }
@@ -630,7 +672,7 @@ latent_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__
         for (int u = 0; u < UV; ++u) {
           const int col = u * 128 + tid;
           for (int h = 0; h < nh && col < p.a.dv; ++h)
-            static_cast<__nv_bfloat16*>(p.a.out)[(it.row + row_of(h)) * p.a.out_rs + (it.h0 + head_of(h)) * p.a.dv + col] = __float2bfloat16_rn(0.f);
+            if (there(h, nh)) static_cast<__nv_bfloat16*>(p.a.out)[(it.row + row_of(h)) * p.a.out_rs + (it.h0 + head_of(h)) * p.a.dv + col] = __float2bfloat16_rn(0.f);
         }
       }
     }
@@ -656,11 +698,14 @@ static bool encode_3d(CUtensorMap* map, const void* base, const cuuint64_t (&dim
 
 // heads per group (per = heads that share a row), and what fits beside Q and P in the shared memory (limit: opt-in bytes per CTA)
 static int lt_heads(int per) { return per <= 16 ? 16 : (per <= 32 ? 32 : 64); }
+// columns that a row has where rows are taken together: four at least, as the row by itself has with values of its own; its references move
+// when any of the four is exceeded, the other groups' heads among them
+static int lt_cols(const LatentArgs& a) { return a.H / a.G < 4 ? 4 : a.H / a.G; }
 struct LtShape {
-  int N, uk, uv, upt;
+  int N, uk, uv, upt, hand;
   uint32_t unit_bytes;
   size_t bytes(int units) const {
-    return (size_t)2 * uk * N * 128 + (size_t)(units >= upt + uk ? 4 : 2) * N * 128 + 256 + (size_t)36 * N + 64 + 1024 + (size_t)units * unit_bytes +
+    return (size_t)2 * uk * N * 128 + (size_t)(units >= upt + uk ? 4 : 2) * N * 128 + 256 + (size_t)36 * N + hand + 64 + 1024 + (size_t)units * unit_bytes +
            (unit_bytes < kLtUnit ? kLtBlock : 0);  // a value unit of one block is read as a pair of blocks: the last one's partner must exist
   }
   int units(size_t limit) const {
@@ -671,7 +716,8 @@ struct LtShape {
 };
 static LtShape lt_shape(const LatentArgs& a, int rows) {
   LtShape s;
-  s.N = lt_heads(a.H / a.G * rows);
+  s.N = lt_heads(rows > 1 ? lt_cols(a) * rows : a.H / a.G);
+  s.hand = rows > 1 && a.kv.page_tokens <= kLtKeys / 2 ? s.N * 128 : 0;
   s.uk = (a.dk + 127) / 128;
   s.uv = (a.dv + 127) / 128;
   s.upt = a.v_col == 0 ? s.uk : s.uk + s.uv;
@@ -695,31 +741,43 @@ static int lt_per_sm(const LtShape& sh, long long items, int sms, int limit, int
 
 // Rows of one prompt that an item takes together: the number for which the rounds of items over the CTAs take the least
 // time.  A tile's products cost the same for 16, 32 or 64 columns (A is read from shared memory at the same rate), its
-// softmax does not: an item of 1000 prompt keys takes 34 us alone, 34 to 37 with 16 columns of several rows, 37 to 39 with 32
-// and 53 to 57 with 64 (4 or 8 groups, heads of 128; latents of 256: 33, -, 37, 49; of 512: 53, -, 65, 84).  The keys of
+// softmax does not: an item of 1000 prompt keys takes 27 us alone, 32 with 16 columns of several rows, 39 with 32
+// and 55 with 64 (4 or 8 groups, heads of 128; latents of 256: 31, -, 37, 53; of 512: 53, -, 66, 92).  The keys of
 // the rows themselves are no less work together: a short tile for two rows, or a whole one each.  1000 rows of one prompt of
-// 1000, each by itself / together: 339 / 107 us (4 groups of 128), 570 / 141 (8 groups), 180 / 60 (4 groups of 64),
-// 124 / 92 (latents of 256), 314 / 161 (of 512); 64 prompts with 4 rows each, latents of 512: 97 / 65; 150 with 3 rows,
-// 300 keys, latents of 256, where it does not pay: 39 / 54.
+// 1000, each by itself / together: 307 / 125 us (4 groups of 128), 590 / 220 (8 groups), 253 / 78 (4 groups of 64),
+// 123 / 95 (latents of 256), 313 / 166 (of 512); 64 prompts with 4 rows each, latents of 512: 94 / 66; 150 with 3 rows, 300 keys, latents
+// of 512, where it does not pay: 90 / 98.
+// Latents, in tiles of one row with a CTA to each SM, fitted to 14 jobs of 12 to 1200 rows: an item's start and end, a tile of its prompt, a tile of a
+// row's own keys (half of one where they are 64 or fewer and two rows come in one).  Two CTAs of an SM take 1.4 times as long for a tile.
+// With the model of the grouped form 1000 rows with 128 prompt keys and 200 of their own took 150 against 125 us, 40 x 15 rows, 35 and 10 keys, 76 against 66.
+static double lt_item_cost(const LatentArgs& a, const LtShape& sh, int rg, int per_sm) {
+  const int prompt = (a.prompt_keys + kLtKeys - 1) / kLtKeys, tiles = a.own_keys > 0 ? (a.own_keys + kLtKeys - 1) / kLtKeys : 1;
+  const bool pairs = a.own_keys <= kLtKeys / 2;
+  if (a.v_col == 0) {
+    if (rg == 1) return (per_sm == 2 ? 1.4 : 1.) * (0.5 + prompt + tiles);
+    return sh.N == 64 ? 3.9 + 1.4 * prompt + rg * (pairs ? 0.57 : 1.3 * tiles) : 1.6 + 1.15 * prompt + rg * (pairs ? 0.75 : 1.2 * tiles);
+  }
+  return (rg == 1 ? 1. : sh.N == 64 ? 1.6 : 1.2) * (2 + prompt) + rg * (pairs ? 0.3 : 0.8 * tiles);
+}
 static int lt_rows(const LatentArgs& a, int sms, int limit) {
   const int per = a.H / a.G;
   if (a.share < 2 || a.Tn != 1 || !a.kv.page_table || (per & (per - 1)) != 0) return 1;
-  // Little to share: 1000 rows with 64 prompt keys and 400 of their own took 239 against 184 us (latents of 512) and 242 against
-  // 213 (4 groups of 128); with 128 and 200, 119 against 127 and 111 against 109.
+  // Little to share: 1000 rows with 64 prompt keys and 400 of their own took 301 against 234 us with 8 rows together (4 groups of 128), 230 with 4;
+  // with 128 and 200, 144 against 137.
   if (!a.together && a.own_keys > kLtKeys / 2 && 2LL * a.prompt_keys < a.own_keys) return 1;
-  const double shared = 2 + (a.prompt_keys + kLtKeys - 1) / kLtKeys;  // an item's start and end are about two tiles
-  const double own = a.own_keys <= kLtKeys / 2 ? 0.3 : 0.8 * ((a.own_keys + kLtKeys - 1) / kLtKeys);
+  const int cols = lt_cols(a);
   int best = 1;
   double least = 0.;
-  for (int rg = 1; rg * per <= 64; rg *= 2) {
-    if (rg > 1 && (rg > 2 * a.share || rg * per < 16)) continue;
+  for (int rg = 1; rg == 1 || rg * cols <= 64; rg *= 2) {
+    if (rg > 1 && (rg > 2 * a.share || rg * cols < 16)) continue;
     const LtShape sh = lt_shape(a, rg);
     if (sh.units((size_t)limit) < sh.upt) continue;
     if (rg == a.together) return rg;
     const long long items = (long long)(a.n_seq / a.share) * ((a.share + rg - 1) / rg) * a.G * a.n_splits;
     int units;
-    const long long ctas = (long long)lt_per_sm(sh, items, sms, limit, &units) * sms;
-    const double t = (double)((items + ctas - 1) / ctas) * ((rg == 1 ? 1. : sh.N == 64 ? 1.6 : 1.2) * shared + rg * own);
+    const int per_sm = lt_per_sm(sh, items, sms, limit, &units);
+    const long long ctas = (long long)per_sm * sms;
+    const double t = (double)((items + ctas - 1) / ctas) * lt_item_cost(a, sh, rg, per_sm);
     if (rg == 1 || t < least) {
       least = t;
       best = rg;
@@ -779,8 +837,9 @@ int latent_tc_launch(const LatentArgs& a, const dgpt_kv_layout& kv, cudaStream_t
   p.n_rows = a.n_seq * a.Tn;
   p.n_groups = a.G * p.gpk;
   p.rg = rg;
-  p.per_log2 = 0;
-  while (1 << p.per_log2 < p.per) ++p.per_log2;
+  p.cols = lt_cols(a);
+  p.cols_log2 = 0;
+  while (1 << p.cols_log2 < p.cols) ++p.cols_log2;
   p.sets_per_prompt = rg > 1 ? (a.share + rg - 1) / rg : 1;
   p.n_sets = rg > 1 ? p.n_rows / a.share * p.sets_per_prompt : p.n_rows;
   p.n_items = p.n_sets * p.n_groups * a.n_splits;

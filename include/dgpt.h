@@ -468,9 +468,9 @@ int dgpt_latent_attn(const void* q, int64_t q_row_stride, const dgpt_kv_layout* 
                      int32_t H, int32_t r, int32_t window, float scale, int32_t dtype, int32_t impl, int32_t* status, void* stream);
 /* The same for sequences that share prompts: each run of `share` sequences (n_seq is a multiple of it) has the same len0,
  * start1 and len1 and the same page table entries for the slots below len0, which the tcgen05 kernel then reads once for
- * several rows.  Results are those of dgpt_latent_attn but for the order in which a row's weights are added.  together: rows
- * that are taken at once, 0 = choose, 1 = each by itself, or a power of two by which the heads that share a cache row become
- * 16, 32 or 64 (T = 1 and pages only).  prompt_keys, own_keys: about how many keys below and from len0 on a row sees, for
+ * several rows.  Results are those of dgpt_latent_attn, bit for bit.  together: rows that are taken at once, 0 = choose,
+ * 1 = each by itself, or a power of two by which the heads that share a cache row (four columns at least) become 16, 32 or 64 (T = 1
+ * and pages only; a number that does not fit the kernel is taken as 1).  prompt_keys, own_keys: about how many keys below and from len0 on a row sees, for
  * the choice. */
 int dgpt_latent_attn_shared(const void* q, int64_t q_row_stride, const dgpt_kv_layout* kv, const int32_t* len0,
                             const int32_t* start1, const int32_t* len1, const int32_t* step_ptr, const void* gate,

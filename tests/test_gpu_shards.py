@@ -67,3 +67,41 @@ def test_tiles_at_any_number_of_rows():
         out = torch.empty(M, 1040, dtype=torch.bfloat16, device="cuda")
         ops.linear(a[:M], w, out, tiles=True)
         assert torch.equal(out, whole[:M])
+
+
+def _configured(family):
+    if family == "delunex":
+        from delunex_cases import build, config, mixer
+
+        layers = [(mixer(16, 64, 64, 128, 200), 512), (mixer(16, 64, 64, 128, 90, kv_from=0), 512)]
+        return build(config(256, 512, 3, layers), 3, torch.bfloat16)[0]
+    from kipolix_cases import attention, build, config
+
+    return build(config(256, 512, [(attention(16, 4, 64, 64, 200, 4), 512), (attention(16, 2, 64, 64, 90, 0), 512)]), 3, torch.bfloat16)[0]
+
+
+@pytest.mark.parametrize("family", ["delunex", "kipolix"])
+@pytest.mark.parametrize("P,N,n", [(300, 1024, 256), (40, 640, 320)])
+def test_a_shard_of_rows_behind_one_prompt(family, P, N, n):
+    """The number of rows chooses how many of them the attention takes together, which may not show in any of them.  (Numbers of rows for
+    which the products run on the same kernels.)"""
+    from diff_gpt_b200 import Engine, TemperatureSampler
+    from diff_gpt_b200.model.engine import DecodeRun
+
+    model, G = _configured(family), 40
+    prompt = torch.randint(0, 512, (P,), generator=torch.Generator().manual_seed(P)).tolist()
+    force = [[(7 * g) % 500 for g in range(G - 1)] + [None]]
+
+    def logits(rows):
+        with torch.inference_mode():
+            r = DecodeRun(model, [prompt], rows, G, TemperatureSampler(1.0), 42, force, fused_head=False, whole_job=False)
+            r.start()
+            r.advance(G)
+            r.check_status()
+            return r.logits.clone()
+
+    assert torch.equal(logits(N)[:n], logits(n))
+    whole, _ = Engine(model).generate_many([prompt], N, 30, TemperatureSampler(1.0), seed=3)
+    for i in range(0, N, 2 * n):
+        part, _ = Engine(model).generate_many([prompt], n, 30, TemperatureSampler(1.0), seed=3, traj_offset=i)
+        assert torch.equal(part, whole[:, i : i + n]), i

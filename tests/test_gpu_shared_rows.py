@@ -95,3 +95,45 @@ def test_a_prompt_is_shared_by_whole_runs_of_rows():
     for kw in (dict(share=2), dict(share=0), dict(share=3, together=3), dict(share=3, together=8)):
         with pytest.raises(DgptError):
             ops.latent_attn(x, lay, None, one, one, None, x, n_seq=3, T=1, H=16, r=64, window=0, scale=1.0, **kw)
+
+
+@pytest.mark.parametrize("H,G,dk", [(16, 0, 512), (16, 0, 64), (8, 0, 136), (32, 0, 128), (16, 4, 128), (16, 8, 64), (32, 4, 96), (32, 1, 64), (64, 2, 64)])
+@pytest.mark.parametrize("case", CASES + [(6, 2, 200, 64, 0, 0, 32, 2), (8, 3, 130, 129, 0, 3, 64, 3), (31, 1, 260, 30, 120, 2, 16, 3)],
+                         ids=lambda c: "x".join(map(str, c)))
+def test_a_row_has_the_bits_that_it_gets_by_itself(case, H, G, dk):
+    """However many rows are taken together, with splits and without: the order of a row's sums is its own."""
+    from diff_gpt_b200 import ops
+
+    share, prompts, n_prompt, n_own, window, keep, pt, splits = case
+    keep, groups = (0, 1) if G == 0 else (keep, G)
+    width = dk if G == 0 else 2 * G * dk
+    R, per = share * prompts, H // groups
+    g = torch.Generator(device="cuda").manual_seed(R + H + dk)
+    pp, op = -(-n_prompt // pt), -(-n_own // pt)
+    n_pages = prompts * pp + R * op
+    store = torch.randn((n_pages, pt, width), generator=g, device="cuda").bfloat16()
+    perm = torch.randperm(n_pages, generator=g, device="cuda").int()
+    table = torch.cat([perm[: prompts * pp].view(prompts, pp).repeat_interleave(share, 0), perm[prompts * pp :].view(R, op)], 1).contiguous()
+    # some rows' largest scores come late in the prompt or among their own keys, by more than the 2^8 that moves a reference
+    q = torch.randn((R, H * dk), generator=g, device="cuda") * torch.rand((R, 1), generator=g, device="cuda") * 12
+    q, gate = q.bfloat16(), torch.randn((R, H), generator=g, device="cuda").bfloat16()
+    i32 = lambda x: torch.full((R,), x, dtype=torch.int32, device="cuda")  # noqa: E731
+    step = torch.full((1,), n_own - 1, dtype=torch.int32, device="cuda")
+    lay = ops.kv_layout(store, store, store.stride(0), 0, pt, table, n_pages)
+
+    def run(together):
+        out = torch.full((R, H * dk), float("nan"), dtype=torch.bfloat16, device="cuda")
+        ws = torch.empty(max(4, ops.latent_attn_workspace_bytes(R, H, dk, splits) // 4), device="cuda").fill_(float("nan")) if splits > 1 else None
+        kw = dict(n_seq=R, T=1, H=H, window=window, scale=dk**-0.5, gate=gate, workspace=ws, n_splits=splits, share=share, together=together)
+        args = (q, lay, i32(n_prompt), i32(pp * pt), i32(1), step, out)
+        if G == 0:
+            ops.latent_attn(*args, r=dk, **kw)
+        else:
+            ops.grouped_attn(*args, row_width=width, v_col=G * dk, G=G, dk=dk, dv=dk, keep_first=keep, **kw)
+        return out
+
+    want = run(1)
+    assert bool(torch.isfinite(want).all())
+    for t in (2, 4, 8, 16):
+        if 16 <= per * t <= 64:
+            assert torch.equal(run(t), want), t
