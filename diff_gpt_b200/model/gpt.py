@@ -207,27 +207,6 @@ def prefix_ctas(units: int, key_tiles: int, own_us: float, n_sm: int) -> int:
     return many if units > few and estimate(many) < 0.97 * estimate(few) else few
 
 
-PREFIX_SINGLE_HEADS = 8
-
-
-def prefix_choice(series: int, rows: int, heads: int, keys: int, own_us: float, ctas: int, n_sm: int) -> tuple[int, int]:
-    """(impl, SMs) of the shared-prompt phase for `rows` trajectories of each series: the kernel with two query tiles per CTA on `ctas` SMs, or
-    for up to 8 heads, which seldom make pairs of tiles enough for the SMs, the one with a single query tile per CTA, on as many SMs as
-    are estimated best (fitted to 18 jobs).  The two kernels round differently and a shard must take the whole job's, so the number of
-    rows and series does not choose between them.  Measured per layer, us, two tiles / one: 8 heads of 64, 1 x 200 rows, 1400 keys 70.1 / 60.8,
-    48 x 20, 400 keys 106 / 92, 3 x 333, 777 keys 77.1 / 72.8, 1 x 1200, 1000 keys 91.7 / 91.0; 8 of 32, 20 x 33, 1400 keys 97.0 / 80.7, 1 x 1000, 500 keys
-    59.8 / 60.0.  12 heads: 40 x 20, 1000 keys 148 / 130, but 3 x 333, 777 keys 88.1 / 91.7, 1 x 1200, 1400 keys 120 / 122, 1 x 4096 x 1024 409 / 407."""
-    if heads > PREFIX_SINGLE_HEADS:
-        return PREFIX_IMPL, ctas
-    items, tiles = series * heads * -(-rows // 128), -(-keys // 128)
-
-    def estimate(sms: int) -> float:
-        phase = -(-items // sms) * tiles * 1.28
-        return phase + max(0.0, own_us - phase * min(1.0, 2.7 * (n_sm - min(items, sms)) / n_sm))
-
-    return 2, min((n_sm, n_sm * 3 // 4, n_sm // 2), key=estimate)
-
-
 SIDE_PRIORITY = -1  # stream of the shared-prompt attention phase: ahead of the per-row phase it runs beside
 
 
@@ -387,7 +366,7 @@ class ForwardPlan:
         self.part_o = None
         self.part_lse = None
         self.prefix_on_tc = False
-        self.prefix_ctas, self.prefix_impl = 0, PREFIX_IMPL
+        self.prefix_ctas = 0
         self.workspace = None
 
     def _mix(self, cands: list, partial: torch.Tensor, w: torch.Tensor, known: set) -> None:
@@ -443,10 +422,6 @@ class ForwardPlan:
             # the per-row phase: its bytes at the copy rate, and what a warp per (row, head) costs however few its keys
             own_us = self.n * H * (2 * D * size * b.own_keys / 6.65e6 + 4e-4)
             self.prefix_ctas = prefix_ctas(units, -(-b.shared_keys // 128), own_us, n_sm)
-            self.prefix_impl = PREFIX_IMPL
-            if PREFIX_IMPL:
-                own = self.n * H * max(2 * D * size * b.own_keys / 6.55e6 + 7.5e-5, 1.6e-3)
-                self.prefix_impl, self.prefix_ctas = prefix_choice(self.n // rows, rows, H, b.shared_keys, own, self.prefix_ctas, n_sm)
             # the persistent tensor-core kernel covers bf16 heads of 32, 64 or 128 in pages that tile its 128-key
             # blocks; other models leave the choice to the library (its warp-level kernel)
             pt = int(b.shared_layouts[0].page_tokens)
@@ -505,7 +480,7 @@ class ForwardPlan:
                         self.q, b.shared_layouts[i], self.prefix_o, B=n_seq // N, H=H, Tq=N, D=D,
                         q_batch_stride=N * C, q_row_stride=C, o_batch_stride=N * C, o_row_stride=C,
                         kv_len=b.shared_len, causal=False, lse=self.prefix_lse,
-                        impl=self.prefix_impl if (self.side is not None and PREFIX_IMPL and self.prefix_on_tc) else b.fmha_impl,
+                        impl=PREFIX_IMPL if (self.side is not None and PREFIX_IMPL and self.prefix_on_tc) else b.fmha_impl,
                         status=self.status,
                         max_ctas=self.prefix_ctas if self.side is not None else 0,
                     )
