@@ -72,8 +72,7 @@ __global__ void __launch_bounds__(kMmThreads, D == 32 ? 3 : 2) fmha_mma_kernel(c
   const int j = blockIdx.x % p.splits, bh = blockIdx.x / p.splits, h = bh % p.H, b = bh / p.H;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   const int n_blk = (p.Tq + kRows - 1) / kRows, G = p.splits * kMmWarps, me = j * kMmWarps + warp;
-  const int cap = p.kv.page_table ? p.kv.max_pages * p.kv.page_tokens : p.kv.page_tokens;
-  const int klen = min(min(p.kv_len ? p.kv_len[b] : p.kv_len_all, cap), p.room);
+  const int klen = min(min(p.kv_len ? p.kv_len[b] : p.kv_len_all, p.kv.page_tokens), p.room);
   // keys that the CTA's last rows see
   int last_blk = 0;
   for (int r = 0; r * G < n_blk; ++r) last_blk = max(last_blk, min(n_blk - 1, (r & 1) ? r * G + G - 1 - j * kMmWarps : r * G + j * kMmWarps + kMmWarps - 1));
@@ -91,12 +90,7 @@ __global__ void __launch_bounds__(kMmThreads, D == 32 ? 3 : 2) fmha_mma_kernel(c
   for (int i = threadIdx.x; i < rows * kChunks; i += kMmThreads) {
     const int row = i / kChunks, c = i - row * kChunks;
     long long off = -1;
-    if (row < need) {
-      const int lp = p.kv.page_table ? row / p.kv.page_tokens : 0;
-      const long long pg = p.kv.page_table ? (long long)p.kv.page_table[(long long)b * p.kv.max_pages + lp] : (long long)b;
-      if (!(p.kv.page_table && (pg < 0 || (p.kv.n_pages > 0 && pg >= p.kv.n_pages))))
-        off = pg * p.kv.page_stride + (long long)h * p.kv.head_stride + (long long)(row - lp * p.kv.page_tokens) * (p.kv.token_stride ? p.kv.token_stride : D) + c * 8;
-    }
+    if (row < need) off = b * p.kv.page_stride + h * p.kv.head_stride + (long long)row * (p.kv.token_stride ? p.kv.token_stride : D) + c * 8;
     const uint32_t at = mm_at<D>(row, c);
     const int bytes = off >= 0 ? 16 : 0;  // 0: filled with zeros, so that 0 * x stays 0
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(sK + at), "l"(kb + (off >= 0 ? off : 0)), "r"(bytes) : "memory");
@@ -262,12 +256,14 @@ __global__ void __launch_bounds__(kMmThreads, D == 32 ? 3 : 2) fmha_mma_kernel(c
   }
 }
 
-// What the kernel covers: whole sequences or portions without window, log-sum-exp or fp32 output, `keys` of them at most.
+// What the kernel covers: whole sequences or portions over dense keys without window, log-sum-exp or fp32 output, `keys` of them at most.
+// Not pages: those are the prompts of decode jobs, whose draws follow the rounding of the tcgen05 kernels.  One job's prompts must not change their kernel
+// with the number of pairs either, as they may be prefilled by several ranks.
 bool fmha_mma_supported(const FmhaArgs& a, const KvView& kv, long long keys) {
   auto al16 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
   return a.dtype == DGPT_BF16 && (a.D == 32 || a.D == 64) && !a.lse && !a.o_f32 && a.window == 0 && !a.hgate &&
          (a.kv_heads == 0 || a.kv_heads == a.H) && a.max_ctas == 0 && keys >= 1 && keys * a.D * 4 <= 96 * 1024 && al16(a.q) && al16(a.o) &&
-         al16(a.egate) && a.egate_rs % 8 == 0 && (kv.token_stride == 0 || kv.token_stride % 8 == 0) && (a.scale == 0.f);
+         kv.page_table == nullptr && al16(a.egate) && a.egate_rs % 8 == 0 && (kv.token_stride == 0 || kv.token_stride % 8 == 0) && (a.scale == 0.f);
 }
 
 template <int D, bool SPLIT>
