@@ -551,9 +551,11 @@ class StepRunner:
     cache records its launches as a graph, and the following ones replay it until something that the launches were made for
     changes: the weights, the cache's storage or state buffer, the key splits, the numbers a GPT carries (soft-cap, SwiGLU).
     A cache has two recordings at most (a GPT's one), and there are as many caches as requests were live at one time; a
-    recording that holds replaced weights or outgrown storage goes with the next step.  All of them run on one stream of the
+    recording that holds replaced weights or outgrown storage goes with the next step.  They run on one stream of the
     runner, between two waits with the caller's, so that requests stepped from several streams never share cuBLAS's workspace
-    at the same time.
+    at the same time.  A token that is one launch (a small fp32 GPT), which needs no such workspace, is replayed on the caller's stream.
+
+    A request may be stepped from one stream and then from another: whatever runs behind its cache waits for what ran there before.
 
     Different requests may be stepped from different threads: one thread at a time enqueues on the runner's stream (what
     another put there meanwhile would be recorded instead of run), and a thread records only after it has run a step
@@ -565,6 +567,8 @@ class StepRunner:
         self._live: dict = {}
         self._free: list = []
         self._single: dict = {}  # (cache, state buffer): its SingleStep
+        self._last: dict = {}  # cache: the caller's stream that its newest tokens are on, or have been waited for by
+        self._replayed: dict = {}  # cache: that stream's handle, if the newest token was replayed there
         self._stream: torch.cuda.Stream | None = None
         self._lock = threading.Lock()  # the dictionaries, and what is enqueued on the runner's stream
         self._ran = threading.local()
@@ -587,6 +591,8 @@ class StepRunner:
             out = self._one(cache, int(tokens[0]))
             if out is not None:
                 return out
+        with self._lock:
+            self._follow(cache)
         dev = self.model.embedding.device
         idx = torch.tensor([tokens], dtype=torch.int64, device=dev)
         rows = torch.tensor(want, dtype=torch.int64, device=dev)
@@ -596,6 +602,17 @@ class StepRunner:
                 self._drop_stale(cache)
         return out
 
+    def _follow(self, cache) -> None:
+        """The caller's stream waits for the stream that `cache`'s newest tokens are on."""
+        if cache in self._replayed and self._replayed[cache] == ops._stream():
+            return  # without a Stream object: 4 us a token
+        caller, last = torch.cuda.current_stream(), self._last.get(cache)
+        self._replayed.pop(cache, None)
+        if last != caller:
+            if last is not None:
+                caller.wait_stream(last)
+            self._last[cache] = caller
+
     def _drop_stale(self, cache) -> None:
         """Let go of what recordings hold that nothing else does any more: replaced weights, and storage that `cache` has outgrown."""
         weights, storage = self.model.last_packed, self.model.cache_storage(cache)
@@ -603,8 +620,8 @@ class StepRunner:
         if stale:
             self._stream.synchronize()  # their memory belongs to other streams
         for key in stale:
-            if self._single[key].last is not None:
-                self._single[key].last.synchronize()
+            if self._single[key].streams:
+                self._last[key[0]].synchronize()  # it has waited for the others
         for key in stale:
             del self._single[key]
 
@@ -620,6 +637,7 @@ class StepRunner:
         key = (cache, 0 if state is None else state.current)  # a portion of several tokens changes the buffer
         if self._stream is None:
             self._stream = torch.cuda.Stream(device=self.model.embedding.device)
+        self._follow(cache)  # before the cache's storage may grow
         old = self._single.get(key)
         one = self.model.single_step(cache, old, self._stream)
         if one is None:
@@ -657,14 +675,13 @@ class StepRunner:
         return one, out
 
     def _replay_here(self, one, cache, token: int) -> torch.Tensor:
-        """A recorded token of one launch, which needs nothing of cuBLAS's: on the caller's stream, behind the stream it ran on last.
-        (The change of streams and its two waits are 35 us of a token's 105.)"""
-        if one.last is None or one.last.cuda_stream != ops._stream():
-            caller = torch.cuda.current_stream()
-            caller.wait_stream(self._stream if one.last is None else one.last)
-            for t in (one.numbers, one.plan.logits, one.plan.status):
-                t.record_stream(caller)
-            one.last = caller
+        """A recorded token of one launch, which needs nothing of cuBLAS's: on the caller's stream, which waits for the tokens before it
+        (`_follow`).  (The change of streams and its two waits are 35 us of a token's 105.)"""
+        here = self._replayed[cache] = ops._stream()
+        if here not in one.streams:
+            for t in (one.numbers, one.bind.len0, one.plan.logits, one.plan.status):
+                t.record_stream(torch.cuda.current_stream())
+            one.streams.add(here)
         one.numbers.copy_(torch.tensor([token, cache.pos, cache.pos, cache.pos + 1], dtype=torch.int32))
         one.graph.replay()
         _lib.stats.launches += one.launches

@@ -21,7 +21,7 @@ There is no CPU implementation: CPU tensors raise.
 from __future__ import annotations
 
 from abc import ABC, abstractmethod
-from dataclasses import dataclass
+from dataclasses import dataclass, field
 
 import torch
 import torch.nn as nn
@@ -228,7 +228,7 @@ class SingleStep:
     graph: torch.cuda.CUDAGraph | None = None
     launches: int = 0
     runs: int = 0
-    last: torch.cuda.Stream | None = None  # where it was replayed last, if not on the runner's stream
+    streams: set = field(default_factory=set)  # handles of the streams that it was replayed on, but for the runner's
 
     def fits(self, kind: tuple, held: tuple) -> bool:
         return self.kind == kind and len(self.held) == len(held) and all(a is b for a, b in zip(self.held, held))

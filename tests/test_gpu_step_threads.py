@@ -46,3 +46,37 @@ def test_requests_from_their_own_threads(family, dtype):
     assert all(one.graph is not None for one in runner._single.values())
     for k in ids:
         assert torch.equal(torch.cat(got[k]), want[k]), k
+
+
+def test_one_request_on_two_streams():
+    """A small fp32 GPT, whose tokens are replayed on the caller's stream: the streams take turns without synchronising, past the 256 and 512 keys
+    where another plan takes over, around portions and where the cache grows; a second request takes the cache over."""
+    from diff_gpt_b200 import GPT, StepRunner
+
+    torch.manual_seed(0)
+    model = GPT(vocab_size=128, n_embd=64, block_size=2048, n_head=4, n_layer=2)
+    for p in model.parameters():
+        torch.nn.init.normal_(p, std=0.1)
+    model = model.cuda().eval()
+    streams, runner = [torch.cuda.Stream() for _ in range(2)], StepRunner(model)
+    for seed in range(2):
+        ids = torch.randint(0, 128, (530,), generator=torch.Generator().manual_seed(seed)).tolist()
+        portions, at, got, ends = {0: 200, 240: 3, 300: 180}, 0, [], []
+        torch.cuda.synchronize()
+        busy = torch.randn(2048, 2048, device="cuda")
+        torch.cuda.synchronize()
+        while at < len(ids):
+            n = portions.get(at, 1)
+            with torch.cuda.stream(streams[len(ends) % 2]):
+                if len(ends) % 3 == 0:
+                    busy @ busy  # the other stream would run ahead
+                got.append(runner.step("r", ids[at : at + n], [n - 1]))
+            at += n
+            ends.append(at - 1)
+        torch.cuda.synchronize()
+        runner.finish("r")
+        with torch.inference_mode():
+            want = model(torch.tensor([ids], device="cuda"))[0][0, ends]
+        assert all(one.graph is not None for one in runner._single.values())
+        err = (torch.cat(got) - want).norm(dim=1) / want.norm(dim=1)
+        assert bool((err < 1e-5).all()), err.max()  # fp32, sums in another order

@@ -193,3 +193,94 @@ def test_replaced_weights_and_outgrown_storage_are_let_go(cuda, tokens):
     gc.collect()
     assert storage() is None and weights() is None
     assert all(one.held[0] is model.last_packed for one in runner._single.values())
+
+
+class _Line:
+    """A stream that knows which pieces of work it, and what it has waited for, have behind them."""
+
+    def __init__(self, number):
+        self.cuda_stream, self.behind = number, set()
+
+    def wait_stream(self, other):
+        self.behind |= other.behind
+
+    def synchronize(self):
+        pass
+
+
+@pytest.mark.parametrize("whole", [True, False])
+def test_a_request_that_moves_from_stream_to_stream(monkeypatch, whole):
+    """Every step runs behind the one before, also where the plan changes (every fifth token), where the cache grows and around portions."""
+    from diff_gpt_b200 import StepRunner, ops
+    from diff_gpt_b200.model.gpt import SingleStep
+
+    callers, current, recording = [_Line(1), _Line(2)], [None], [False]
+    done, missed = [0], []
+
+    def work():
+        if not recording[0]:
+            line = current[0]
+            missed.extend(set(range(done[0])) - line.behind)
+            line.behind.add(done[0])
+            done[0] += 1
+
+    class Graph:
+        def capture_begin(self, **k):
+            recording[0] = True
+
+        def capture_end(self):
+            recording[0] = False
+
+        def replay(self):
+            work()
+
+    @contextlib.contextmanager
+    def on(line):
+        was, current[0] = current[0], line
+        yield
+        current[0] = was
+
+    monkeypatch.setattr(torch.cuda, "Stream", lambda **k: _Line(9))
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda *a: current[0])
+    monkeypatch.setattr(torch.cuda, "stream", on)
+    monkeypatch.setattr(torch.cuda, "CUDAGraph", Graph)
+    monkeypatch.setattr(ops, "_stream", lambda: current[0].cuda_stream)
+
+    class Cache:
+        def reset(self):
+            self.pos = 0
+
+    class Tensor(_Logits):
+        def copy_(self, x):
+            pass
+
+        def record_stream(self, s):
+            pass
+
+    class Model:
+        vocab_size, embedding, last_packed = 8, torch.zeros(1), _Storage()
+        new_cache = Cache
+        single_step_allowed = lambda self: True  # noqa: E731
+        cache_storage = lambda self, cache: ()  # noqa: E731
+
+        def single_step(self, cache, old, stream):
+            kind = (cache.pos // 5,)
+            if old is not None and old.fits(kind, (self.last_packed,)):
+                return old
+            work()  # the storage grows
+            plan = SimpleNamespace(whole=whole, logits=Tensor(), status=Tensor(), run=lambda ids, bind: work())
+            return SingleStep(plan, SimpleNamespace(len0=Tensor()), Tensor(), kind, (self.last_packed,), checks=False)
+
+        def logits_at(self, idx, cache, rows):
+            work()
+            cache.pos += idx.shape[1]
+            return torch.zeros(rows.numel(), 8)
+
+    monkeypatch.setattr(SingleStep, "enqueue", lambda self: self.plan.run(None, None))
+    runner = StepRunner(Model())
+    for request in ("a", "b"):  # b takes a's cache over
+        for i, n in enumerate([3, 1, 1, 1, 1, 1, 1, 1, 1, 2, 1, 1, 1, 1, 4, 1, 1, 1]):
+            with on(callers[i // 2 % 2 if i < 9 else i % 2]):
+                runner.step(request, [1] * n, [0])
+        runner.finish(request)
+    assert done[0] > 36 and not missed, missed
