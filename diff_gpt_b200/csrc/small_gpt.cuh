@@ -53,6 +53,16 @@ __device__ __forceinline__ int tid_here() {
 // The barrier of the warps that compute.
 __device__ __forceinline__ void sg_sync() { asm volatile("bar.sync 1, %0;" ::"n"(kSgThreads) : "memory"); }
 
+// The same, telling every thread whether any of them said yes.
+__device__ __forceinline__ bool sg_any(bool mine) {
+  int r;
+  asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.s32 p, %1, 0;\n\tbarrier.red.or.pred q, 1, %2, p;\n\tselp.s32 %0, 1, 0, q;\n\t}"
+               : "=r"(r)
+               : "r"((int)mine), "n"(kSgThreads)
+               : "memory");
+  return r != 0;
+}
+
 // One product of the CTA's M rows: out[m][n] = sum_k a[m][k] w[n][k], w as [K / 4 / KS][N][KS][4] in kChunks slots of the ring: KS lanes
 // side by side share a column, so that a warp reads 512 bytes in a row.  (As [K / 4][N][4] its lanes meet in the same banks, KS deep: the
 // 64 x 128 product of one row took 3000 clocks.)
@@ -566,6 +576,7 @@ __global__ void __launch_bounds__(kSgThreads + 32, 1) small_gpt_kernel(const __g
 #pragma unroll 1
   for (int i = tid; i < L * 2 * C; i += kSgThreads) mixw[i] = __ldg(p.w + p.n_w + i);
   sg_sync();
+  bool lost = false;  // a wait ran out.  Every thread goes by the same answer, so that those that leave do not leave others at a barrier.
 #pragma unroll 1
   for (int it = 0; it < p.n_steps; ++it) {
     if (resident) w_ring.slot = w_ring.asked = 0;
@@ -709,11 +720,11 @@ __global__ void __launch_bounds__(kSgThreads + 32, 1) small_gpt_kernel(const __g
       Down::run(w_ring, act, [&](int m, int n, float v, bool mine) {
         if (mine) now[m * C + n] += v;
       });
-      sg_sync();
+      lost = sg_any(stuck);
       w_ring.release(Down::kGroup);
-      if (stuck) break;
+      if (lost) break;
     }
-    if (stuck) break;
+    if (lost) break;
     if (!head) continue;  // (a chunk has one step)
     // ---- head: one token's logits a row ----
     if (warp < M) mix_row<C, M>(cand, warp, 1u << L, 1, nullptr, u);
