@@ -505,7 +505,7 @@ __global__ void __launch_bounds__(kSgThreads + 32, 1) small_gpt_kernel(const __g
   unsigned* at = reinterpret_cast<unsigned*>(p.out_tok ? ex + M * (V + 33) : lg);  // [rows, or 1][max_keys] where keys are, / 16 bytes
   __shared__ __align__(8) uint64_t full[kSgMaxSlots];
   __shared__ long long traj[M], append[M];  // append: where the token's key goes, -1 where it is out of range
-  __shared__ int tok[M], pos[M], n_keys[M];
+  __shared__ int tok[M], pos[M], n_keys[M], fresh_key[M];  // fresh_key: which key is the step's own token's, -1 where that is not the last one
   __shared__ uint32_t bits[M];  // the random words of the step's draws
   __shared__ volatile int stuck, chunks_there, chunks_read;  // a bounded wait ran out; chunks that have come, that everyone is done with
   const bool chunk = p.T > 0;
@@ -591,6 +591,7 @@ __global__ void __launch_bounds__(kSgThreads + 32, 1) small_gpt_kernel(const __g
       pos[tid] = in ? r_pos + it : 0;
       append[tid] = to == kNoKey ? -1 : 4ll * to;
       n_keys[tid] = tid < live ? min(n, p.max_keys) : 0;
+      fresh_key[tid] = in && newest ? n - 1 : -1;
     }
     sg_sync();
     // ---- embedding and its norm; cos and sin of the positions ----
@@ -633,10 +634,10 @@ __global__ void __launch_bounds__(kSgThreads + 32, 1) small_gpt_kernel(const __g
       const float* kb = static_cast<const float*>(p.kv.k) + l * p.layer_stride;
       const float* vb = static_cast<const float*>(p.kv.v) + l * p.layer_stride;
       KeyRound<D> round;
-      // the first keys of this warp's first task do not depend on the token at hand (in a chunk they do)
-      if (const int w = tid_here() >> 5, m = w / kParts / H; !chunk && w < kTasks && m < live) {
+      // the first keys of this warp's first task do not depend on the token at hand (in a chunk they do, and where its key lies among them)
+      if (const int w = tid_here() >> 5, m = w / kParts / H; w < kTasks && m < live && fresh_key[m] >= 0) {
         const long long o = (long long)(w / kParts % H) * p.kv.head_stride;
-        round.load(at + m * p.max_keys, n_keys[m], kb + o, vb + o, qkvg, qkvg, n_keys[m] - 1, (w % kParts) * KeyRound<D>::G * KeyRound<D>::U);
+        round.load(at + m * p.max_keys, n_keys[m], kb + o, vb + o, qkvg, qkvg, fresh_key[m], (w % kParts) * KeyRound<D>::G * KeyRound<D>::U);
       }
       // ---- rotation, norm over the head, append ----
       constexpr int kHalf = D / 2;
@@ -674,10 +675,10 @@ __global__ void __launch_bounds__(kSgThreads + 32, 1) small_gpt_kernel(const __g
         const int pair = task / kParts, sp = task % kParts, m = pair / H, h = pair % H;
         if (m >= live) continue;
         const unsigned* keys = at + (chunk ? 0 : m * p.max_keys);
-        const int n = n_keys[m], newest = chunk ? -1 : n - 1;  // a decode step's newest key is taken from where it has just been made
+        const int n = n_keys[m], newest = fresh_key[m];  // taken from where it has just been made
         const float* row = qkvg + m * 4 * C + h * D;
         const float *kh = kb + (long long)h * p.kv.head_stride, *vh = vb + (long long)h * p.kv.head_stride;
-        if (chunk || task >= kSgWarps) round.load(keys, n, kh, vh, row + C, row + 2 * C, newest, sp * KeyRound<D>::G * KeyRound<D>::U);
+        if (newest < 0 || task >= kSgWarps) round.load(keys, n, kh, vh, row + C, row + 2 * C, newest, sp * KeyRound<D>::G * KeyRound<D>::U);
         attend<D>(keys, n, kh, vh, round, row, row + C, row + 2 * C, newest, sp, kParts, part + task * kPart);
       }
       sg_sync();

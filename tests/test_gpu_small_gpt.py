@@ -116,3 +116,32 @@ def test_out_of_range_is_reported(monkeypatch):
         r.advance(1)
         with pytest.raises(RuntimeError, match="status 1"):
             r.check_status()
+
+
+@pytest.mark.parametrize("R", [3, 200, 700])  # one, two and eight rows a CTA
+@pytest.mark.parametrize("slot,start,length,keys", [(20, 0, 21, 21), (20, 0, 20, 21), (20, 0, 12, 40), (5, 0, 20, 20), (9, 4, 15, 32)])
+def test_tokens_whose_own_key_is_not_the_last(R, slot, start, length, keys):
+    """slot: where the token's key goes; start, length: the keys that it sees, its own the last of them, in between or not among them."""
+    from diff_gpt_b200.model.gpt import ForwardPlan, KvBinding
+    from diff_gpt_b200.model.kv_cache import KVCache
+
+    m = _model(32, 4, 3, 64)
+    g = torch.Generator(device="cuda").manual_seed(R + slot)
+    ids = torch.randint(0, 64, (R,), generator=g, device="cuda", dtype=torch.int32)
+    storage = torch.randn((3, 2, R, 4, 48, 8), generator=g, device="cuda")
+    i32 = lambda x: torch.full((R,), x, dtype=torch.int32, device="cuda")  # noqa: E731
+
+    def run(whole):
+        cache = KVCache(R, 4, 48, 8, 3)
+        cache.kv_cache = storage.clone()
+        bind = KvBinding(layouts=[cache.layer_layout(i) for i in range(3)], pos0=i32(20), slot0=i32(slot), decode=True, len0=i32(0), start1=i32(start),
+                         len1=i32(length), n_splits=1)
+        with torch.inference_mode():
+            plan = ForwardPlan(m, R, 1, keys=keys if whole else None)
+            assert plan.whole == whole
+            return plan.run(ids, bind).clone(), cache.kv_cache, int(plan.status)
+
+    (za, ca, sa), (zb, cb, sb) = run(True), run(False)
+    _close(za, zb)
+    _close(ca, cb)
+    assert sa == sb == 0
