@@ -359,7 +359,7 @@ __device__ __forceinline__ int draw_row(const float* z, int V, float temperature
     if (on && e[i] > 0.f) pick = c0 + i;
     on = on && !(e[i] > 0.f && c > local);
   }
-  return __shfl_sync(0xffffffffu, pick, max(who, 0));
+  return who < 0 ? best.i : __shfl_sync(0xffffffffu, pick, who);  // no sum to walk along, as sample_row
 }
 
 // What the ring receives, in the order of use: per layer the four matrices, then the head's blocks of 256 columns, and again.
@@ -698,7 +698,7 @@ __global__ void __launch_bounds__(kSgThreads + 32, 1) small_gpt_kernel(const __g
             sum = fmaf(f, src[s * kPart + D + 1], sum);
           }
           const float g = qkvg[m * 4 * C + 3 * C + c];
-          v = sum > 0.f ? __fdividef(v, sum) * __fdividef(1.f, 1.f + __expf(-g)) : 0.f;
+          v = (sum > 0.f ? __fdividef(v, sum) : 0.f * v) * __fdividef(1.f, 1.f + __expf(-g));  // no keys: 0; not a number stays that
         }
         y[i] = v;
       }

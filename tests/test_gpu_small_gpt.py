@@ -145,3 +145,28 @@ def test_tokens_whose_own_key_is_not_the_last(R, slot, start, length, keys):
     _close(za, zb)
     _close(ca, cb)
     assert sa == sb == 0
+
+
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+@pytest.mark.parametrize("temperature,V", [(0.0, 256), (1.0, 256), (0.7, 512)])
+def test_numbers_that_are_none(monkeypatch, bad, temperature, V):
+    """A token whose vector is not finite: the logits of every token that sees it are not either, and the draws from such rows go by one rule."""
+    m = _model(64, 4, 2, V, cap=0.0)
+    with torch.no_grad():
+        m.token_embedding_table.weight[5] = bad
+    idx = torch.randint(6, V, (3, 40), device="cuda")
+    idx[1, 17] = 5
+
+    one, plain = (x.isfinite() for x in _both(monkeypatch, lambda: m(idx)[0]))
+    assert not bool(one[1, 17:].any()) and bool(one[1, :17, 6:].all()) and bool(one[::2, :, 6:].all())
+    assert not bool((plain & ~one).any())  # (the general path multiplies what a row does not see by 0, and so loses more rows)
+
+    def draws():
+        with torch.inference_mode():
+            r = DecodeRun(m, idx[:, :30].to(torch.int32).contiguous(), 20, 5, TemperatureSampler(temperature), 11, None)
+            r.start()
+            r.advance(5)
+            return r.tokens_so_far().clone()
+
+    a, b = _both(monkeypatch, draws)
+    assert torch.equal(a, b)
