@@ -268,7 +268,7 @@ def whole_f32(C: int, H: int, L: int, V: int, n_seq: int, T: int, keys: int) -> 
     101 / 76, 900 keys 141 / 146; 128, 60 keys 211 / 189, 300 keys 246 / 295).  Every CTA reads all weights and its rows' prompt by itself.
     Whole sequences, us a call with its host work: 2 layers of 64, 1 x 256 tokens 520 / 256, 1 x 1024 590 / 979; 4 layers of 128, 1 x 128
     855 / 365, 1 x 512 983 / 1334; many sequences pay while their CTAs are two a multiprocessor (8 x 256 565 / 382, 32 x 64 578 / 247)."""
-    if T < 1 or not ops.small_gpt_supported(C, H, L, V, keys):  # (no tokens: empty logits)
+    if not ops.small_gpt_supported(C, H, L, V, keys):
         return False
     sms = _sm_count()
     if T == 1:

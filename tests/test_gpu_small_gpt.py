@@ -170,11 +170,3 @@ def test_numbers_that_are_none(monkeypatch, bad, temperature, V):
 
     a, b = _both(monkeypatch, draws)
     assert torch.equal(a, b)
-
-
-def test_no_tokens_behind_a_cache():
-    m = _model(64, 4, 2, 256)
-    cache = m.new_cache(2, 40)
-    idx = torch.randint(0, 256, (2, 30), device="cuda")
-    m(idx, kv_cache=cache)
-    assert m(idx[:, :0], kv_cache=cache)[0].shape == (2, 0, 256) and cache.get_pos() == 30

@@ -15,11 +15,3 @@ def test_threads_leave_the_step_loop_by_one_answer():
     loop = kernel[kernel.index("for (int it = 0; it < p.n_steps; ++it)") : kernel.index("if (stuck && tid == 0)")]
     assert re.findall(r"if \((\w+)\) break;", loop) == ["lost", "lost"]
     assert [line.strip() for line in loop.splitlines() if "stuck" in line] == ["lost = sg_any(stuck);"]
-
-
-def test_no_tokens_are_not_a_decode_step():
-    """0 tokens behind a cache take the general path, which has empty logits for them."""
-    from diff_gpt_b200.model.gpt import whole_f32
-
-    assert whole_f32(64, 4, 2, 256, 1, 1, 40) and whole_f32(64, 4, 2, 256, 2, 7, 40)
-    assert not whole_f32(64, 4, 2, 256, 2, 0, 40) and not whole_f32(64, 4, 2, 256, 2, 0, 0)
