@@ -608,7 +608,7 @@ class StepRunner:
             return  # without a Stream object: 4 us a token
         caller, last = torch.cuda.current_stream(), self._last.get(cache)
         self._replayed.pop(cache, None)
-        if last != caller:
+        if last is None or not last == caller:  # (`!=` of torch's streams is not the opposite of `==`)
             if last is not None:
                 caller.wait_stream(last)
             self._last[cache] = caller

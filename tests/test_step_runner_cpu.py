@@ -204,6 +204,9 @@ class _Line:
     def wait_stream(self, other):
         self.behind |= other.behind
 
+    def __ne__(self, other):  # as torch's streams, whose `!=` may be False where `==` is False too
+        return False
+
     def synchronize(self):
         pass
 
