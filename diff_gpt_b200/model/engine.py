@@ -586,6 +586,7 @@ class StepRunner:
         """fp32 [len(want), V] on the device; `want` names places among `tokens`."""
         assert len(tokens) > 0 and all(0 <= t < self.model.vocab_size for t in tokens), "tokens must be ids of the vocabulary"
         assert all(0 <= w < len(tokens) for w in want), "wanted places must lie among the tokens of the step"
+        self._check_late()
         cache = self._cache(request)
         if len(tokens) == 1 and len(want) == 1 and _lib.stats.timer is None and self.model.single_step_allowed():
             out = self._one(cache, int(tokens[0]))
@@ -679,7 +680,7 @@ class StepRunner:
         (`_follow`).  (The change of streams and its two waits are 35 us of a token's 105.)"""
         here = self._replayed[cache] = ops._stream()
         if here not in one.streams:
-            for t in (one.numbers, one.bind.len0, one.plan.logits, one.plan.status):
+            for t in (one.numbers, one.bind.len0, one.plan.logits):
                 t.record_stream(torch.cuda.current_stream())
             one.streams.add(here)
         one.numbers.copy_(torch.tensor([token, cache.pos, cache.pos, cache.pos + 1], dtype=torch.int32))
@@ -689,11 +690,23 @@ class StepRunner:
         cache.pos += 1
         return one.plan.logits.to(torch.float32, copy=True)
 
+    def _check_late(self) -> None:
+        late = getattr(self.model, "late_status", None)
+        if late is not None:
+            late.check()
+
     def finish(self, request) -> None:
+        """The request's cache is free for another one.  Where launches report late (`LateStatus`), waits for the request's last ones and raises
+        what they have to report."""
         with self._lock:
             cache = self._live.pop(request, None)
             if cache is not None:
                 self._free.append(cache)
+            last = self._last.get(cache)
+        late = getattr(self.model, "late_status", None)
+        if late is not None and late.used and last is not None:
+            last.synchronize()
+            late.check()
 
 
 def _generate_generic(model, tokens, num_samples, G, sampler, seed, force_schedule):

@@ -60,6 +60,37 @@ class BaseGPT(nn.Module, ABC):
         ...
 
 
+class LateStatus:
+    """A status word in pinned host memory for launches that nobody waits for: a kernel writes there only when something went wrong, and the
+    host looks without a copy or a wait, when it next comes by.  Copies and pickles of its owner get one of their own."""
+
+    def __init__(self) -> None:
+        self._word = self._view = None
+
+    def word(self) -> torch.Tensor | None:
+        """The word, or None where it cannot be made now (a stream is being captured)."""
+        if self._word is None and not torch.cuda.is_current_stream_capturing():
+            self._word = torch.zeros(1, dtype=torch.int32).pin_memory()
+            self._view = self._word.numpy()
+        return self._word
+
+    @property
+    def used(self) -> bool:
+        return self._word is not None
+
+    def check(self) -> None:
+        if self._view is not None and self._view[0]:
+            bad, self._view[0] = int(self._view[0]), 0
+            raise RuntimeError(f"device-side status {bad}: in an earlier forward a cache slot or position was out of range, or a bounded wait ran out; "
+                               "its logits are not to be used")
+
+    def __deepcopy__(self, memo) -> "LateStatus":
+        return LateStatus()
+
+    def __reduce__(self):
+        return LateStatus, ()
+
+
 class DeviceModel(BaseGPT):
     """A model whose forward is enqueued by a plan of this library's kernels: what the Engine, the step-by-step
     runner and the facade need from it, whatever its layers are."""
@@ -112,6 +143,9 @@ class DeviceModel(BaseGPT):
         """The launches of one more token behind `cache`, which has room for it afterwards: `old` where it still fits, or None
         where a single token takes the general path.  What it allocates for itself belongs to `stream`, where it will run."""
         return None
+
+    # what launches that nobody has waited for have to report, if the model has such
+    late_status: LateStatus | None = None
 
     # -- batched decode (DecodeRun) --
     @abstractmethod
@@ -318,9 +352,10 @@ class ForwardPlan:
     """
 
     def __init__(self, model: "GPT", n_seq: int, T: int, last_only: bool = False, want_logits: bool = True,
-                 cap: float = 0.0, few_rows: bool = True, keys: int | None = None) -> None:
+                 cap: float = 0.0, few_rows: bool = True, keys: int | None = None, late: bool = False) -> None:
         """`cap`: soft-cap the logits as they are stored (0 = raw logits).  `few_rows`: see `DeviceModel.prefill_plan`.  `keys`: the
-        most keys that a token sees, where the kernel of small fp32 models may run the whole forward (see whole_f32)."""
+        most keys that a token sees, where the kernel of small fp32 models may run the whole forward (see whole_f32).  `late`: nobody reads
+        the plan's status; that kernel's goes to the model's `late_status`."""
         emb = model.token_embedding_table.weight
         dev, dt = emb.device, emb.dtype
         C, V, L = model.n_embd, model.vocab_size, model.n_layer
@@ -332,12 +367,14 @@ class ForwardPlan:
 
         n_out = n_seq if last_only else n
         self.cap = cap
-        self.status = torch.zeros(1, dtype=torch.int32, device=dev)
         self.logits = buf(n_out, V) if want_logits else None
         self.keys = keys
         self.whole = (
             keys is not None and want_logits and dt == torch.float32 and emb.is_contiguous() and whole_f32(C, model.n_head, L, V, n_seq, T, keys)
         )
+        self.status = model.report() if late and self.whole else None
+        if self.status is None:
+            self.status = torch.zeros(1, dtype=torch.int32, device=dev)
         self.side = None
         if self.whole:
             return
@@ -649,6 +686,11 @@ class GPT(DeviceModel):
         self.attn_res_layers_per_block = attn_res_layers_per_block
         self._packed: _Packed | None = None
 
+    def report(self) -> torch.Tensor | None:
+        if self.late_status is None:
+            self.late_status = LateStatus()
+        return self.late_status.word()
+
     # ---- weights as the kernels want them -------------------------------------------
     def packed_weights(self) -> _Packed:
         """Fused QKVG weight and transposed views, rebuilt when a parameter was modified or moved."""
@@ -727,7 +769,7 @@ class GPT(DeviceModel):
                 layouts=[cache.layer_layout(i) for i in range(self.n_layer)], pos0=numbers[2:3], slot0=numbers[1:2], decode=True,
                 len0=zero, start1=zero, len1=numbers[3:4], n_splits=splits,
             )
-            return SingleStep(ForwardPlan(self, 1, 1, cap=self.logit_softcap, keys=keys), bind, numbers, kind, held, checks=False)
+            return SingleStep(ForwardPlan(self, 1, 1, cap=self.logit_softcap, keys=keys, late=True), bind, numbers, kind, held, checks=False)
 
     def paged_cache(self, n_series, rows_per_series, prefix_len, max_new, page_tokens, pool=None) -> PagedKVCache:
         emb = self.embedding
@@ -798,7 +840,9 @@ class GPT(DeviceModel):
         dt = self.token_embedding_table.weight.dtype
         t0 = 0 if kv_cache is None else kv_cache.get_pos()
         assert t0 + T <= self.freqs_cis.shape[0]
-        plan = ForwardPlan(self, B, T, cap=self.logit_softcap, keys=t0 + T)
+        if self.late_status is not None:
+            self.late_status.check()
+        plan = ForwardPlan(self, B, T, cap=self.logit_softcap, keys=t0 + T, late=True)
         if kv_cache is None:
             # every layer reuses the same scratch K/V, unless one kernel's CTAs work on different layers at one time
             scratch = KVCache(batch_size=B, num_heads=H, seq_len=T, head_dim=D, num_layers=L if plan.whole else 1)

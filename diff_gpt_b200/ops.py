@@ -406,8 +406,9 @@ def small_gpt(
     draw: _lib.SmallGptDraw | None = None,
 ) -> None:
     """Whole forwards of a small fp32 GPT: T tokens of each sequence of `pos0`, or (T = 0) `n_steps` decode steps of its rows, none
-    of which sees more than `max_keys` keys."""
-    _cuda(ids, pos0, slot0, step, logits, status, len0, start1, len1)
+    of which sees more than `max_keys` keys.  `status` may lie in pinned host memory."""
+    _cuda(ids, pos0, slot0, step, logits, len0, start1, len1)
+    assert status.dtype == torch.int32 and (status.is_cuda or status.is_pinned())
     assert ids.dtype == torch.int32 and ids.is_contiguous() and logits.is_contiguous() and logits.dtype == torch.float32
     n_seq = pos0.numel()
     assert ids.numel() >= n_seq * max(T, 1) and slot0.numel() == n_seq and logits.shape[-1] == model.V

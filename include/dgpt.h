@@ -275,8 +275,8 @@ int dgpt_small_gpt_supported(int32_t C, int32_t H, int32_t L, int32_t V, int32_t
  *            n_steps of them: step i runs at step + i, draws for column step + i + 1 and goes on with the token drawn; *step_ptr is not
  *            advanced.  The logits of the last step remain.
  * kv: layer 0's storage; layer l's lies l * kv_layer_stride elements behind it, through the same page table.  logit_cap > 0: logits are
- * stored soft-capped.  Rows do not depend on one another.  max_keys: the most keys that any token of the call sees.  status: device
- * int32, set to 1 if a position or slot is out of range (nothing is written there) or a token sees more keys than that (they are left
+ * stored soft-capped.  Rows do not depend on one another.  max_keys: the most keys that any token of the call sees.  status: int32
+ * in device or pinned host memory, set to 1 if a position or slot is out of range (nothing is written there) or a token sees more keys than that (they are left
  * out), to 2 if a bounded wait ran out. */
 int dgpt_small_gpt(const dgpt_small_gpt_model* model, const dgpt_kv_layout* kv, int64_t kv_layer_stride, const int32_t* ids,
                    const int32_t* pos0, const int32_t* slot0, const int32_t* step_ptr, const int32_t* len0, const int32_t* start1,

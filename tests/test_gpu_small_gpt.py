@@ -170,3 +170,41 @@ def test_numbers_that_are_none(monkeypatch, bad, temperature, V):
 
     a, b = _both(monkeypatch, draws)
     assert torch.equal(a, b)
+
+
+def test_a_late_status_is_raised(monkeypatch):
+    """Nobody waits for a forward or a recorded token: what its kernel reports is raised by the next call, and by `finish` at the latest.  (Made by
+    positions beyond the table, which the kernel clamps; a copy of the model has a word of its own.)"""
+    import copy
+
+    m = _model(32, 4, 1, 64)
+    idx = torch.randint(0, 64, (1, 8), device="cuda")
+    m(idx)
+    torch.cuda.synchronize()
+    m(idx)
+    other, table = copy.deepcopy(m), m.freqs_cis.shape[0]
+    real = gpt_module.ops.small_gpt
+
+    def far(model, kv, stride, ids, pos0, *a, **kw):
+        real(model, kv, stride, ids, pos0 + table, *a, **kw)
+
+    with monkeypatch.context() as mp:
+        mp.setattr(gpt_module.ops, "small_gpt", far)
+        m(idx)
+    torch.cuda.synchronize()
+    other(idx)
+    with pytest.raises(RuntimeError, match="status 1"):
+        m(idx)
+    m(idx)  # raised once
+    r = StepRunner(m)
+    r.step("a", [1, 2, 3], [2])
+    for _ in range(3):
+        r.step("a", [4], [0])
+    with monkeypatch.context() as mp:
+        mp.setattr(gpt_module.ops, "small_gpt", far)
+        r.step("b", [1, 2], [1])
+    with pytest.raises(RuntimeError, match="status 1"):
+        r.finish("b")
+    r.step("a", [5], [0])
+    r.finish("a")
+    torch.cuda.synchronize()
