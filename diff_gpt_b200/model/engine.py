@@ -603,16 +603,17 @@ class StepRunner:
                 self._drop_stale(cache)
         return out
 
-    def _follow(self, cache) -> None:
-        """The caller's stream waits for the stream that `cache`'s newest tokens are on."""
+    def _follow(self, cache) -> "torch.cuda.Stream":
+        """The caller's stream waits for the stream that `cache`'s newest tokens are on.  Returns it."""
         if cache in self._replayed and self._replayed[cache] == ops._stream():
-            return  # without a Stream object: 4 us a token
+            return self._last[cache]  # without another Stream object: 4 us a token
         caller, last = torch.cuda.current_stream(), self._last.get(cache)
         self._replayed.pop(cache, None)
         if last is None or not last == caller:  # (`!=` of torch's streams is not the opposite of `==`)
             if last is not None:
                 caller.wait_stream(last)
             self._last[cache] = caller
+        return caller
 
     def _drop_stale(self, cache) -> None:
         """Let go of what recordings hold that nothing else does any more: replaced weights, and storage that `cache` has outgrown."""
@@ -638,7 +639,7 @@ class StepRunner:
         key = (cache, 0 if state is None else state.current)  # a portion of several tokens changes the buffer
         if self._stream is None:
             self._stream = torch.cuda.Stream(device=self.model.embedding.device)
-        self._follow(cache)  # before the cache's storage may grow
+        caller, mine = self._follow(cache), self._stream  # before the cache's storage may grow
         old = self._single.get(key)
         one = self.model.single_step(cache, old, self._stream)
         if one is None:
@@ -648,7 +649,6 @@ class StepRunner:
             self._single[key] = one
         if one.graph is not None and getattr(one.plan, "whole", False):
             return one, self._replay_here(one, cache, token)
-        caller, mine = torch.cuda.current_stream(), self._stream
         mine.wait_stream(caller)
         with torch.cuda.stream(mine):
             slot = cache.pos if state is None else cache.slot
@@ -681,7 +681,7 @@ class StepRunner:
         here = self._replayed[cache] = ops._stream()
         if here not in one.streams:
             for t in (one.numbers, one.bind.len0, one.plan.logits):
-                t.record_stream(torch.cuda.current_stream())
+                t.record_stream(self._last[cache])
             one.streams.add(here)
         one.numbers.copy_(torch.tensor([token, cache.pos, cache.pos, cache.pos + 1], dtype=torch.int32))
         one.graph.replay()
