@@ -17,11 +17,12 @@
 //                   after the item's last tile, one thread per column: normalise, gate, store
 // Rows behind one prompt (ROWS): an item is a set of up to rg of them, whose heads together are the N of the products over
 // the prompt's tiles; then come the tiles of each row's own slots (those of two rows in one tile where they fit its halves),
-// whose products cover that row's columns only.  A row's result has the bits that it gets by itself, so that the tokens drawn from it do not depend on
+// whose products cover that row's columns only, so that a row with numbers that are none spoils no other (0 * NaN).  A product has 16 columns at
+// least: rows with fewer heads (PACK) lie side by side for the prompt's tiles, and their sums move to 16 columns each before their own.  A row's result has the bits that it gets by itself, so that the tokens drawn from it do not depend on
 // how many rows there are: a split is cut at the same tiles, references move row by row, and where a tile holds two rows' slots the second row's
 // weights are handed to the threads that would have had them (tests/test_gpu_shared_rows.py).
 // A row of a unit that holds fewer than 64 columns leaves the block's other accumulator rows undefined; they are not read.
-// TMEM columns: S0 [0, N)  S1 [N, 2N)  O of unit u [2N + u N, +N).
+// TMEM columns: S0 [0, N)  S1 [N, 2N)  O of unit u [2N + u N, +N)  PACK: O of unit u and row r [2N + UV N + 16 (u rg + r), +16).
 // Every mbarrier wait is bounded.  When one runs out the abort flag is raised, the loader and the issuer stop and drain
 // what they have in flight, the softmax warps run through their remaining tiles without waiting (so that every CTA
 // barrier is still met by all of them), TMEM is freed and the status word names the wait.
@@ -41,7 +42,7 @@ struct LtParams {
   LatentArgs a;
   int n_rows, n_groups, n_items;  // item = (split * n_sets + set) * n_groups + group
   int n_sets;                     // sets of rows: one row each, or
-  int rg, cols, cols_log2;        // ROWS: up to rg rows of one prompt, each in `cols` columns: the heads that share a cache row, or four
+  int rg, cols, cols_log2;        // ROWS: up to rg rows of one prompt, each in `cols` columns: the heads that share a cache row, or 4 (latents: 16)
   int sets_per_prompt;
   int per, gpk;                   // heads that share a row, and item groups they make
   int n_units;                    // units in the ring
@@ -205,11 +206,12 @@ __device__ __forceinline__ float lt_reduce16(const float* v, int lane, F op) {
 
 // NB: columns of the products = 16 NB; HS <= 16 NB: heads the softmax looks after (a group may hold fewer than 16).
 // SHARED: a tile's values are its keys (latents), whose cache has no kept first keys.
-// ROWS: a column is a head of one of rg rows, column c = row c >> cols_log2, head c & (cols - 1); HS = 16 NB.
+// ROWS: a column is a head of one of rg rows, column c = row c >> cols_log2, head c & (cols - 1); HS = min(cols, 16).
 template <int NB, int HS, bool SHARED, bool ROWS>
 __global__ void __launch_bounds__(kLtThreads, NB == 4 ? 1 : 2)
 latent_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__ CUtensorMap mc, const LtParams p) {
-  constexpr int N = 16 * NB;
+  constexpr int N = 16 * NB, CW = ROWS ? N : HS;  // columns, and those that the softmax looks after
+  constexpr bool PACK = ROWS && HS < 16;
   // The sums of a tile that is not full go over the 16-key steps that hold a key only.  Latents of 512 / 256, 256 rows with
   // 1000 keys: 106.5 -> 102.4 and 36.9 -> 33.8 us.  Rows of keys and values, each by itself, have products to spare (they
   // wait for HBM) and took longer with them issued one by one: 64.3 -> 66.5 (4 groups of 64), 235 -> 241 (8 of 128).
@@ -218,7 +220,7 @@ latent_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__
   constexpr uint32_t kIdescO = kIdescS | (1u << 15);  // A is read MN-major
   constexpr uint32_t kQBlock = N * 128;               // [N heads][64 columns]
   constexpr uint32_t kPBlock = N * 128;               // [N heads][64 keys]
-  constexpr uint32_t kTmemCols = NB == 1 ? 128 : (NB == 2 ? 256 : 512);  // N (2 + 4) columns at most
+  constexpr uint32_t kTmemCols = NB == 1 ? 128 : (NB == 2 ? 256 : 512);  // N (2 + 4) columns at most; PACK: as lt_rows allows
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const int UT = p.upt, UK = p.uk, UV = p.uv, NU = p.n_units;
@@ -321,8 +323,8 @@ latent_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__
     if (lane == 0) {
       const uint64_t dC = smem_desc(0, 16, 1024), dM = smem_desc(0, kLtBlock, 1024);  // K-major rows; MN-major pairs of blocks
       // the products of rows' own slots: of their columns only
-      auto own_n = [&](const LtTile& x, uint32_t idesc) {
-        return !ROWS || x.own < 0 ? idesc : (idesc & ~(63u << 17)) | (uint32_t)max(2, (x.pair ? 2 : 1) * p.cols >> 3) << 17;
+      auto own_n = [&](const LtTile& x, uint32_t idesc, int rows) {
+        return !ROWS || x.own < 0 ? idesc : (idesc & ~(63u << 17)) | (uint32_t)max(2, rows * p.cols >> 3) << 17;
       };
       auto own_block = [&](const LtTile& x) { return ROWS && x.own >= 0 ? (x.own << p.cols_log2) >> 4 : 0; };
       unsigned g = 0u, items = 0u;  // tiles; items
@@ -331,12 +333,12 @@ latent_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__
         const LtItem it = lt_item<!SHARED, ROWS>(p, item, N);
         if (it.n == 0) continue;
         ok = wait_or_abort(bar_q, items & 1u, abort_flag, 52);
-        unsigned started = 0u;  // 16-column blocks of O that hold sums
+        unsigned started = 0u;  // 16-column blocks of O that hold sums; PACK: from bit 4 on those of the rows
         auto issue_s = [&](unsigned gt, int j) {
           const bool last = j + 1 == it.n;
           const LtTile x = lt_tile<!SHARED, ROWS>(it, j);
           const int blk = own_block(x);
-          const uint32_t idesc = own_n(x, kIdescS);
+          const uint32_t idesc = own_n(x, kIdescS, x.pair ? 2 : 1);
           const uint32_t d = tmem + (gt & 1u) * N + blk * 16;
           for (int u = 0; ok && u < UK; ++u) {
             const unsigned un = gt * (unsigned)UT + (unsigned)u, s = un % (unsigned)NU;
@@ -362,11 +364,14 @@ latent_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__
           const LtTile x = lt_tile<!SHARED, ROWS>(it, j);
           // steps of 16 keys that hold one that is seen: the others' probabilities are zeros
           const int k0 = kSome ? max(x.begin - x.slot, 0) >> 4 : 0, k1 = kSome ? min(kLtKeys, x.end - x.slot + 15) >> 4 : 8;
-          const int blk = own_block(x);
-          const uint32_t idesc = own_n(x, kIdescO);
-          const unsigned acc = (started >> blk) & 1u;
-          started |= ROWS && x.own >= 0 ? 1u << blk : 15u;  // a row's own blocks are always touched together
+          const bool apart = PACK && x.own >= 0;  // sums in the row's own 16 columns, P in the first 16 rows of its buffer
+          const int blk = apart ? 0 : own_block(x), bit = apart ? 4 + x.own : blk;
+          const uint32_t idesc = own_n(x, kIdescO, 1);
           const bool second = ROWS && x.pair && x.own + 1 < it.nr;
+          const int more = PACK ? 1 : p.cols >> 4;  // from a row's blocks to the next row's
+          if (PACK && x.own >= 0 && it.n_mine > 0) started = ~0u;  // the prompt's sums have been moved there
+          const unsigned acc = (started >> bit) & 1u, acc2 = (started >> (bit + more)) & 1u;
+          started |= ROWS && x.own >= 0 ? (1u << bit) | (second ? 1u << (bit + more) : 0u) : 15u;  // a row's own blocks are always touched together
           for (int u = 0; u < UV; ++u) {
             const unsigned un = g * (unsigned)UT + (unsigned)(v_unit + u), s = un % (unsigned)NU;
             if (!SHARED) {
@@ -374,13 +379,14 @@ latent_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__
               if (!ok) break;
               tc_fence_after();
             }
-            const uint32_t d = tmem + 2 * N + u * N + blk * 16;
+            const uint32_t d = tmem + (apart ? 2 * N + UV * N + (u * p.rg + x.own) * 16 : 2 * N + u * N + blk * 16);
             const uint64_t da = dM + ((aU + s * unit_bytes) >> 4), db = dC + ((aP + (ahead ? 2 * b * kPBlock : 0u) + blk * 2048) >> 4);
             if (k0 == 0 && k1 == 8) umma_ss8<128, 512, 2, kPBlock / 16>(d, da, db, idesc, acc);
             else {
               for (int k = k0; k < k1; ++k) umma_ss(d, da + 128 * k, db + (k >> 2) * (kPBlock / 16) + 2 * (k & 3), idesc, k > k0 ? 1u : acc);
               if (second)
-                for (int k = k0; k < k1; ++k) umma_ss(d, da + 512 + 128 * k, db + kPBlock / 16 + 2 * k, idesc, 1u);
+                for (int k = k0; k < k1; ++k)
+                  umma_ss(d + 16 * more, da + 512 + 128 * k, db + kPBlock / 16 + (PACK ? 0 : 128 * more) + 2 * k, idesc, k > k0 ? 1u : acc2);
             }
             umma_commit(bar_uf + 8 * s);
           }
@@ -402,7 +408,7 @@ latent_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__
     unsigned g = 0u;
     bool fail = false;
     const long long RH = (long long)p.n_rows * p.a.H;
-    if (HS < N)  // heads nobody looks after: their probabilities are zeros, once
+    if (CW < N)  // heads nobody looks after: their probabilities are zeros, once
       for (int i = tid; i < (int)((ahead ? 4 : 2) * kPBlock / 16); i += 128) reinterpret_cast<uint4*>(sP)[i] = make_uint4(0u, 0u, 0u, 0u);
     if (tid < N) ref[tid] = -INFINITY;
     lt_sync();
@@ -412,7 +418,7 @@ latent_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__
     for (int item = blockIdx.x; item < p.n_items; item += gridDim.x) {
       const LtItem it = lt_item<!SHARED, ROWS>(p, item, N);
       const int nh = it.nh;
-      unsigned started = 0u;  // 16-column blocks of O that hold sums
+      unsigned started = 0u;  // 16-column blocks of O that hold sums; PACK: from bit 4 on those of the rows
       constexpr int HL = (N + 31) / 32;  // heads a lane looks after at the end of the item
       float gate[HL];
 #pragma unroll
@@ -422,17 +428,17 @@ latent_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__
         if (p.a.gate && there(h, nh))
           gate[c] = __bfloat162float(static_cast<const __nv_bfloat16*>(p.a.gate)[(it.row + row_of(h)) * p.a.gate_rs + it.h0 + head_of(h)]);
       }
-      float l[HS];
+      float l[CW];
 #pragma unroll
-      for (int h = 0; h < HS; ++h) l[h] = 0.f;
+      for (int h = 0; h < CW; ++h) l[h] = 0.f;
       for (int j = 0; j < it.n; ++j, ++g) {
         const unsigned b = g & 1u;
         const LtTile x = lt_tile<!SHARED, ROWS>(it, j);
         const int half = ROWS && x.pair ? tid >> 6 : 0, slot = x.slot + tid - 64 * half, end = x.end;
         // The tile concerns columns [c_lo, c_hi), this thread's key [k_lo, k_hi) of them.
         const int c_lo = ROWS && x.own >= 0 ? x.own << p.cols_log2 : 0;
-        const int c_hi = ROWS && x.own >= 0 ? c_lo + (x.pair ? 2 : 1) * p.cols : HS;
-        const int k_lo = c_lo + half * p.cols, k_hi = ROWS && x.own >= 0 ? k_lo + p.cols : HS;
+        const int c_hi = ROWS && x.own >= 0 ? c_lo + (x.pair ? 2 : 1) * p.cols : CW;
+        const int k_lo = c_lo + half * p.cols, k_hi = ROWS && x.own >= 0 ? k_lo + p.cols : CW;
         auto block = [&](int c) { return !ROWS || (c_lo < 16 * c + 16 && c_hi > 16 * c); };
         const bool seen = slot >= x.begin && slot < end && (!ROWS || x.own + half < it.nr);
         auto columns = [&](int c) -> unsigned {  // of block c, one bit each
@@ -464,6 +470,30 @@ latent_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__
           }
         }
         __syncwarp();
+        // the rows' columns in O, and whether a product on them may be in flight or done
+        auto rows_at = [&](int u, int r) { return lane_addr + 2 * N + UV * N + (u * p.rg + r) * 16; };
+        const bool apart = PACK && x.own >= 0;
+        if (apart && it.n_mine > 0 && started < 16u) {  // the prompt's sums move to the rows' own columns
+          if (!fail && !wait_or_abort(bar_o + 8 * (b ^ 1u), ((g - 1) >> 1) & 1u, abort_flag, 57)) fail = true;
+          fail = __any_sync(0xffffffffu, fail);
+          tc_fence_after();
+#pragma unroll 1
+          for (int i = 0; i < UV * NB; ++i) {
+            const int u = i / NB, c = i - u * NB;
+            float v[16];
+            tmem_ld16_nowait(lane_addr + 2 * N + u * N + c * 16, v);
+            tc_wait_ld();
+#pragma unroll
+            for (int q = 0; q < 16 / HS; ++q) {
+              uint32_t w[16];
+#pragma unroll
+              for (int k = 0; k < 16; ++k) w[k] = k < HS ? __float_as_uint(v[(q * HS + k) % 16]) : 0u;
+              tmem_st16(rows_at(u, c * (16 / HS) + q), w);
+            }
+          }
+          tc_wait_st();
+          started = ~0u;
+        }
         float s[N];  // log2 of what is added for this key, against the heads' references (a score is rounded before its reference is taken off)
         for (int pass = 0;; ++pass) {
 #pragma unroll
@@ -476,7 +506,7 @@ latent_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__
             const unsigned cols = columns(c);
 #pragma unroll
             for (int i = 0; i < 16; i += 4) {
-              if (16 * c + i >= HS) continue;
+              if (16 * c + i >= CW) continue;
               const float4 m4 = *reinterpret_cast<const float4*>(ref + 16 * c + i);
               const float mm[4] = {m4.x, m4.y, m4.z, m4.w};
 #pragma unroll
@@ -520,19 +550,33 @@ latent_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__
           __syncwarp();
           lt_sync();  // and `red` may be written again
 #pragma unroll
-          for (int h = 0; h < HS; h += 4) {
+          for (int h = 0; h < CW; h += 4) {
             const float4 f = *reinterpret_cast<const float4*>(fac + h);
             l[h] *= f.x;
             l[h + 1] *= f.y;
             l[h + 2] *= f.z;
             l[h + 3] *= f.w;
           }
-          if (started) {
+          if (apart ? (started >> (4 + x.own)) & 3u : started) {
             // O may only be touched when no product is in flight on it: the tile before must be done, and this tile's
             // waits for this thread's arrival below
             if (!fail && !wait_or_abort(bar_o + 8 * (b ^ 1u), ((g - 1) >> 1) & 1u, abort_flag, 57)) fail = true;
             fail = __any_sync(0xffffffffu, fail);
             tc_fence_after();
+            if (apart) {
+#pragma unroll 1
+              for (int i = 0; i < UV * (x.pair ? 2 : 1); ++i) {
+                const int u = i % UV, r = x.own + i / UV;
+                if (!((started >> (4 + r)) & 1u)) continue;
+                float v[16];
+                tmem_ld16_nowait(rows_at(u, r), v);
+                tc_wait_ld();
+                uint32_t w[16];
+#pragma unroll
+                for (int k = 0; k < 16; ++k) w[k] = k < HS ? __float_as_uint(v[k] * fac[r * HS + k]) : 0u;
+                tmem_st16(rows_at(u, r), w);
+              }
+            } else
 #pragma unroll 1
             for (int c = c_lo >> 4; c < NB && 16 * c < c_hi; ++c) {
               if (!((started >> c) & 1u)) continue;
@@ -571,16 +615,18 @@ latent_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__
 #pragma unroll
         for (int c = 0; c < NB; ++c) {
           if (!block(c)) continue;
-          started |= 1u << c;
+          if (!apart) started |= 1u << c;
 #pragma unroll
           for (int i = 0; i < 16; ++i) {
             const int h = 16 * c + i;
-            if (h >= HS) continue;
+            if (h >= CW) continue;
             const float e = ex2(s[h]);  // not seen: 0
-            l[h % HS] = ROWS ? fmaf(e, mine, l[h % HS]) : l[h % HS] + e;
-            *reinterpret_cast<__nv_bfloat16*>(pb + h * 128 + ((chunk ^ (h & 7)) << 4)) = __float2bfloat16_rn(e);
+            l[h % CW] = ROWS ? fmaf(e, mine, l[h % CW]) : l[h % CW] + e;
+            const int at = apart ? (i - k_lo) & 15 : h;  // a row apart: its columns first
+            *reinterpret_cast<__nv_bfloat16*>(pb + at * 128 + ((chunk ^ (at & 7)) << 4)) = __float2bfloat16_rn(e);
           }
         }
+        if (apart) started |= (x.pair ? 3u : 1u) << (4 + x.own);
         fence_async_smem();
         tc_fence_before();
         mbar_arrive(bar_p + 8 * b);
@@ -596,7 +642,7 @@ latent_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__
         lt_sync();
         if (tid < 64) {
 #pragma unroll
-          for (int h = 4; h < HS; h += 4) {  // (a row's columns are four or more)
+          for (int h = 4; h < CW; h += 4) {  // (a row's columns are four or more)
             const int r = h >> p.cols_log2;
             if (!(r & 1) || h >= nh) continue;
             const float* from = hand + ((r >> 1 << p.cols_log2) + (h & (p.cols - 1))) * 64 + tid;
@@ -609,7 +655,7 @@ latent_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__
       for (int c = 0; c < NB; ++c) {
         float ls[16];
 #pragma unroll
-        for (int i = 0; i < 16; ++i) ls[i] = 16 * c + i < HS ? l[(16 * c + i) % HS] : 0.f;
+        for (int i = 0; i < 16; ++i) ls[i] = 16 * c + i < CW ? l[(16 * c + i) % CW] : 0.f;
         const float t = lt_reduce16(ls, lane, [](float x, float y) { return x + y; });
         if (lane < 16) red[warp * N + 16 * c + lane] = t;
       }
@@ -640,8 +686,19 @@ latent_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__
 #pragma unroll 1
           for (int c = 0; c < NB; ++c) {
             float v[16];
-            tmem_ld16_nowait(lane_addr + 2 * N + u * N + c * 16, v);
-            tc_wait_ld();
+            if (PACK && it.n_own > 0) {
+#pragma unroll
+              for (int q = 0; q < 16 / HS; ++q) {
+                float t[16];
+                tmem_ld16_nowait(lane_addr + 2 * N + UV * N + (u * p.rg + c * (16 / HS) + q) * 16, t);
+                tc_wait_ld();
+#pragma unroll
+                for (int k = 0; k < HS; ++k) v[(q * HS + k) % 16] = t[k];
+              }
+            } else {
+              tmem_ld16_nowait(lane_addr + 2 * N + u * N + c * 16, v);
+              tc_wait_ld();
+            }
             if (u == UV - 1 && c == NB - 1) {
               tc_fence_before();
               mbar_arrive(bar_of);  // the next item may overwrite O
@@ -698,9 +755,12 @@ static bool encode_3d(CUtensorMap* map, const void* base, const cuuint64_t (&dim
 
 // heads per group (per = heads that share a row), and what fits beside Q and P in the shared memory (limit: opt-in bytes per CTA)
 static int lt_heads(int per) { return per <= 16 ? 16 : (per <= 32 ? 32 : 64); }
-// columns that a row has where rows are taken together: four at least, as the row by itself has with values of its own; its references move
-// when any of the four is exceeded, the other groups' heads among them
-static int lt_cols(const LatentArgs& a) { return a.H / a.G < 4 ? 4 : a.H / a.G; }
+// columns that a row has where rows are taken together: as many as the softmax looks after where the row is by itself, since all its references move
+// when any of them is exceeded, the other groups' heads among them
+static int lt_cols(const LatentArgs& a) {
+  const int per = a.H / a.G;
+  return a.v_col == 0 ? (per < 16 ? 16 : per) : per < 4 ? 4 : per;
+}
 struct LtShape {
   int N, uk, uv, upt, hand;
   uint32_t unit_bytes;
@@ -741,15 +801,15 @@ static int lt_per_sm(const LtShape& sh, long long items, int sms, int limit, int
 
 // Rows of one prompt that an item takes together: the number for which the rounds of items over the CTAs take the least
 // time.  A tile's products cost the same for 16, 32 or 64 columns (A is read from shared memory at the same rate), its
-// softmax does not: an item of 1000 prompt keys takes 27 us alone, 32 with 16 columns of several rows, 39 with 32
-// and 55 with 64 (4 or 8 groups, heads of 128; latents of 256: 31, -, 37, 53; of 512: 53, -, 66, 92).  The keys of
+// softmax does not: an item of 1000 prompt keys takes 27 us alone, 33 with 16 columns of several rows, 42 with 32
+// and 69 with 64 (4 or 8 groups, heads of 128; latents of 256: 31, -, 39, 55; of 512: 53, -, 68, 90).  The keys of
 // the rows themselves are no less work together: a short tile for two rows, or a whole one each.  1000 rows of one prompt of
-// 1000, each by itself / together: 307 / 125 us (4 groups of 128), 590 / 220 (8 groups), 253 / 78 (4 groups of 64),
+// 1000, each by itself / together: 307 / 156 us (4 groups of 128), 586 / 293 (8 groups), 252 / 90 (4 groups of 64),
 // 123 / 95 (latents of 256), 313 / 166 (of 512); 64 prompts with 4 rows each, latents of 512: 94 / 66; 150 with 3 rows, 300 keys, latents
 // of 512, where it does not pay: 90 / 98.
-// Latents, in tiles of one row with a CTA to each SM, fitted to 14 jobs of 12 to 1200 rows: an item's start and end, a tile of its prompt, a tile of a
-// row's own keys (half of one where they are 64 or fewer and two rows come in one).  Two CTAs of an SM take 1.4 times as long for a tile.
-// With the model of the grouped form 1000 rows with 128 prompt keys and 200 of their own took 150 against 125 us, 40 x 15 rows, 35 and 10 keys, 76 against 66.
+// In tiles of one row: an item's start and end, a tile of its prompt, a tile of a row's own keys (half of one where they are 64 or fewer and two
+// rows come in one), fitted to 14 jobs of 12 to 1200 rows for each of five shapes.  Two CTAs of an SM share its pipes.  Before the fit
+// 1000 rows with 128 prompt keys and 200 of their own took 150 against 125 us (latents of 512), 162 against 136 (4 groups of 128).
 static double lt_item_cost(const LatentArgs& a, const LtShape& sh, int rg, int per_sm) {
   const int prompt = (a.prompt_keys + kLtKeys - 1) / kLtKeys, tiles = a.own_keys > 0 ? (a.own_keys + kLtKeys - 1) / kLtKeys : 1;
   const bool pairs = a.own_keys <= kLtKeys / 2;
@@ -757,13 +817,15 @@ static double lt_item_cost(const LatentArgs& a, const LtShape& sh, int rg, int p
     if (rg == 1) return (per_sm == 2 ? 1.4 : 1.) * (0.5 + prompt + tiles);
     return sh.N == 64 ? 3.9 + 1.4 * prompt + rg * (pairs ? 0.57 : 1.3 * tiles) : 1.6 + 1.15 * prompt + rg * (pairs ? 0.75 : 1.2 * tiles);
   }
-  return (rg == 1 ? 1. : sh.N == 64 ? 1.6 : 1.2) * (2 + prompt) + rg * (pairs ? 0.3 : 0.8 * tiles);
+  if (rg == 1) return 2 + prompt + tiles;
+  if (sh.N == 16) return 1.6 * prompt + rg * (pairs ? 1.1 : 2.3 * tiles);
+  if (sh.N == 32) return (per_sm == 2 ? 1.4 : 1.) * (2.5 + 1.4 * prompt + rg * (pairs ? 0.67 : 1.15 * tiles));
+  return 6.5 + 1.6 * prompt + rg * (pairs ? 1.05 : 1.4 * tiles);
 }
 static int lt_rows(const LatentArgs& a, int sms, int limit) {
   const int per = a.H / a.G;
   if (a.share < 2 || a.Tn != 1 || !a.kv.page_table || (per & (per - 1)) != 0) return 1;
-  // Little to share: 1000 rows with 64 prompt keys and 400 of their own took 301 against 234 us with 8 rows together (4 groups of 128), 230 with 4;
-  // with 128 and 200, 144 against 137.
+  // Little to share: 1000 rows with 64 prompt keys and 400 of their own took 255 us with 4 rows together against 234 (4 groups of 128).
   if (!a.together && a.own_keys > kLtKeys / 2 && 2LL * a.prompt_keys < a.own_keys) return 1;
   const int cols = lt_cols(a);
   int best = 1;
@@ -772,6 +834,7 @@ static int lt_rows(const LatentArgs& a, int sms, int limit) {
     if (rg > 1 && (rg > 2 * a.share || rg * cols < 16)) continue;
     const LtShape sh = lt_shape(a, rg);
     if (sh.units((size_t)limit) < sh.upt) continue;
+    if (rg > 1 && cols < 16 && 2 * sh.N + sh.uv * (sh.N + 16 * rg) > 8 * sh.N) continue;  // TMEM
     if (rg == a.together) return rg;
     const long long items = (long long)(a.n_seq / a.share) * ((a.share + rg - 1) / rg) * a.G * a.n_splits;
     int units;
@@ -868,14 +931,12 @@ int latent_tc_launch(const LatentArgs& a, const dgpt_kv_layout& kv, cudaStream_t
   const size_t smem = sh.bytes(p.n_units);
   const int grid = p.n_items < per_sm * sms ? p.n_items : per_sm * sms;
   if (rg > 1) {
-    if (a.v_col == 0) {
-      if (N == 16) return lt_launch<1, 16, true, true>(mq, mc, p, grid, smem, st);
-      if (N == 32) return lt_launch<2, 32, true, true>(mq, mc, p, grid, smem, st);
-      return lt_launch<4, 64, true, true>(mq, mc, p, grid, smem, st);
-    }
-    if (N == 16) return lt_launch<1, 16, false, true>(mq, mc, p, grid, smem, st);
-    if (N == 32) return lt_launch<2, 32, false, true>(mq, mc, p, grid, smem, st);
-    return lt_launch<4, 64, false, true>(mq, mc, p, grid, smem, st);
+#define DGPT_LT(NB, HS, SHARED) lt_launch<NB, HS, SHARED, true>(mq, mc, p, grid, smem, st)
+    if (a.v_col == 0) return N == 32 ? DGPT_LT(2, 16, true) : DGPT_LT(4, 16, true);
+    if (p.cols == 4) return N == 16 ? DGPT_LT(1, 4, false) : N == 32 ? DGPT_LT(2, 4, false) : DGPT_LT(4, 4, false);
+    if (p.cols == 8) return N == 16 ? DGPT_LT(1, 8, false) : N == 32 ? DGPT_LT(2, 8, false) : DGPT_LT(4, 8, false);
+    return N == 32 ? DGPT_LT(2, 16, false) : DGPT_LT(4, 16, false);
+#undef DGPT_LT
   }
   if (a.v_col == 0) {
     if (N == 16) return lt_launch<1, 16, true>(mq, mc, p, grid, smem, st);

@@ -469,7 +469,7 @@ int dgpt_latent_attn(const void* q, int64_t q_row_stride, const dgpt_kv_layout* 
 /* The same for sequences that share prompts: each run of `share` sequences (n_seq is a multiple of it) has the same len0,
  * start1 and len1 and the same page table entries for the slots below len0, which the tcgen05 kernel then reads once for
  * several rows.  Results are those of dgpt_latent_attn, bit for bit.  together: rows that are taken at once, 0 = choose,
- * 1 = each by itself, or a power of two by which the heads that share a cache row (four columns at least) become 16, 32 or 64 (T = 1
+ * 1 = each by itself, or a power of two by which the heads that share a cache row become 16, 32 or 64 (T = 1
  * and pages only; a number that does not fit the kernel is taken as 1).  prompt_keys, own_keys: about how many keys below and from len0 on a row sees, for
  * the choice. */
 int dgpt_latent_attn_shared(const void* q, int64_t q_row_stride, const dgpt_kv_layout* kv, const int32_t* len0,

@@ -124,7 +124,8 @@ def test_a_row_has_the_bits_that_it_gets_by_itself(case, H, G, dk):
     def run(together):
         out = torch.full((R, H * dk), float("nan"), dtype=torch.bfloat16, device="cuda")
         ws = torch.empty(max(4, ops.latent_attn_workspace_bytes(R, H, dk, splits) // 4), device="cuda").fill_(float("nan")) if splits > 1 else None
-        kw = dict(n_seq=R, T=1, H=H, window=window, scale=dk**-0.5, gate=gate, workspace=ws, n_splits=splits, share=share, together=together)
+        kw = dict(n_seq=R, T=1, H=H, window=window, scale=dk**-0.5, gate=gate, workspace=ws, n_splits=splits, share=share, together=together,
+                  prompt_keys=5000, own_keys=1)  # (so that a number is chosen which shares)
         args = (q, lay, i32(n_prompt), i32(pp * pt), i32(1), step, out)
         if G == 0:
             ops.latent_attn(*args, r=dk, **kw)
@@ -132,8 +133,17 @@ def test_a_row_has_the_bits_that_it_gets_by_itself(case, H, G, dk):
             ops.grouped_attn(*args, row_width=width, v_col=G * dk, G=G, dk=dk, dv=dk, keep_first=keep, **kw)
         return out
 
+    counts = [0] + [t for t in (2, 4, 8, 16) if 16 <= per * t <= 64]
     want = run(1)
     assert bool(torch.isfinite(want).all())
-    for t in (2, 4, 8, 16):
-        if 16 <= per * t <= 64:
-            assert torch.equal(run(t), want), t
+    for t in counts:
+        assert torch.equal(run(t), want), t
+    # one row's own numbers are none: the rows beside it keep their bits
+    bad = min(1, share - 1)
+    store[table[bad, pp:].long()] = float("inf")
+    store[table[bad, pp].long(), 0, ::3] = float("nan")
+    want = run(1)
+    others = torch.arange(R, device="cuda") != bad
+    assert bool(torch.isfinite(want[others]).all())
+    for t in counts:
+        assert torch.equal(run(t)[others], want[others]), t
