@@ -644,7 +644,7 @@ def _config1(dev, cpu: bool) -> dict:
     t = _wall(lambda: dg.predict_samples(df, max_new_points=h, num_samples=n, sampler=TemperatureSampler(1.0)), dev, repeat=10)
     line = {"workload": "BASELINE config 1: DiffGPT.predict_samples, 100 trajectories x 48 points, fp32, 89-token prompt",
             "value": n * h / t, "unit": "tokens/s", "ms_per_call": 1e3 * t, "us_per_decode_step": 1e6 * t / h, "dtype": "f32",
-            "bound": "launch latency (0.43 MB of weights, 137 cached positions): one graph replay per step",
+            "bound": "a chain of dependent phases (0.43 MB of weights from L2, 137 cached positions): the whole decode loop is one launch",
             "api": "DiffGPT.predict_samples(host frame) -> host float64 [100, 48, 1]"}
     ref = reference_side()
     if cpu and ref.available:

@@ -412,9 +412,10 @@ class Engine:
 
         Returns (tokens, masks): int32 device tensors of shape (S, num_samples, G); masks are 1 where a
         token was sampled and 0 where it was forced.  `traj_offset`/`series_offset` shift the ids that key
-        the random stream, so a shard of the trajectories draws what its part of the full run draws, for a bf16 model token
+        the random stream, so a shard of the trajectories draws what its part of the full run draws, for a bf16 GPT token
         for token.  (fp32 products go to kernels by their number of rows, which order their sums differently: logits
-        equal to 1e-6 or so, and a draw that falls that close to a seam between two tokens may go to the other.)
+        equal to 1e-6 or so, and a draw that falls that close to a seam between two tokens may go to the other.  So do bf16 products
+        of the other families, on cuBLAS, and their attention below one row per multiprocessor, which is then split along the keys.)
         `shared_prefix` (None = decide from `num_samples`) fixes whether the prompt's keys are read once per series
         by the tensor-core phase or per row, so that a shard can take the path the whole job takes; `whole_job` says that
         this is no shard, and lets one or two rows take kernels of their own.

@@ -46,7 +46,8 @@ def test_dense(B, H, D, T, off, gated):
 
 @pytest.mark.parametrize("causal", [True, False])
 def test_pages_and_lengths(causal):
-    """Scrambled pages, a length per sequence (one of none at all), rows of a wider buffer."""
+    """Scrambled pages, a length per sequence (one of none at all), rows of a wider buffer: on the tcgen05 kernels, by the same reference.  (Lengths of
+    dense sequences: test_gpu_prompt_kernels.py.)"""
     g = torch.Generator(device="cuda").manual_seed(3)
     B, H, D, pt, n_pages, Tq = 40, 5, 32, 64, 5, 320
     C = H * D
