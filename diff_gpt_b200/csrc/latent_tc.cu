@@ -595,23 +595,9 @@ latent_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__
             tc_wait_st();
           }
         }
-        // The second row of a tile: its weights go to the sums of the threads that would have had them were the row by itself.
-        const float mine = half ? 0.f : 1.f;
-        if (ROWS && half && x.own + 1 < it.nr) {
-#pragma unroll 1
-          for (int c = k_lo >> 4; 16 * c < k_hi; ++c) {
-            float v[16];
-            tmem_ld16_nowait(lane_addr + b * N + c * 16, v);
-            tc_wait_ld();
-#pragma unroll
-            for (int i = 0; i < 16; ++i) {
-              const int h = 16 * c + i;
-              if (h >= k_lo && h < k_hi) hand[((x.own >> 1) * p.cols + h - k_lo) * 64 + (tid & 63)] = seen ? ex2(__fmul_rn(v[i], p.a.scale_log2) - ref[h]) : 0.f;
-            }
-          }
-        }
         uint8_t* pb = sP + ((ahead ? 2 * b : 0u) + (tid >> 6)) * kPBlock + (tid & 7) * 2;
         const int chunk = (tid & 63) >> 3;
+        const float mine = half ? 0.f : 1.f;
 #pragma unroll
         for (int c = 0; c < NB; ++c) {
           if (!block(c)) continue;
@@ -620,16 +606,34 @@ latent_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__
           for (int i = 0; i < 16; ++i) {
             const int h = 16 * c + i;
             if (h >= CW) continue;
-            const float e = ex2(s[h]);  // not seen: 0
-            l[h % CW] = ROWS ? fmaf(e, mine, l[h % CW]) : l[h % CW] + e;
-            const int at = apart ? (i - k_lo) & 15 : h;  // a row apart: its columns first
-            *reinterpret_cast<__nv_bfloat16*>(pb + at * 128 + ((chunk ^ (at & 7)) << 4)) = __float2bfloat16_rn(e);
+            s[h] = ex2(s[h]);  // not seen: 0
+            l[h % CW] = ROWS ? fmaf(s[h], mine, l[h % CW]) : l[h % CW] + s[h];
+            if (!apart) *reinterpret_cast<__nv_bfloat16*>(pb + h * 128 + ((chunk ^ (h & 7)) << 4)) = __float2bfloat16_rn(s[h]);
+          }
+          if (apart) {  // one block: the row's columns first
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
+              const int at = (i - k_lo) & 15;
+              *reinterpret_cast<__nv_bfloat16*>(pb + at * 128 + ((chunk ^ (at & 7)) << 4)) = __float2bfloat16_rn(s[(16 * c + i) % N]);
+            }
           }
         }
         if (apart) started |= (x.pair ? 3u : 1u) << (4 + x.own);
         fence_async_smem();
         tc_fence_before();
         mbar_arrive(bar_p + 8 * b);
+        if (ROWS && half && x.own + 1 < it.nr) {  // the second row of a tile: its weights are summed by the threads that would have had them were it by itself
+          float* to = hand + (x.own >> 1) * p.cols * 64 + (tid & 63);
+#pragma unroll
+          for (int c = 0; c < NB; ++c) {
+            if (!block(c)) continue;
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
+              const int j = 16 * c + i - k_lo;
+              if (j >= 0 && j < p.cols) to[j * 64] = s[(16 * c + i) % N];
+            }
+          }
+        }
       }
       // ---- the item's result ----
       if (it.n > 0) {
