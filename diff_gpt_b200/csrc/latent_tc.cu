@@ -805,11 +805,11 @@ static int lt_per_sm(const LtShape& sh, long long items, int sms, int limit, int
 
 // Rows of one prompt that an item takes together: the number for which the rounds of items over the CTAs take the least
 // time.  A tile's products cost the same for 16, 32 or 64 columns (A is read from shared memory at the same rate), its
-// softmax does not: an item of 1000 prompt keys takes 27 us alone, 33 with 16 columns of several rows, 42 with 32
-// and 69 with 64 (4 or 8 groups, heads of 128; latents of 256: 31, -, 39, 55; of 512: 53, -, 68, 90).  The keys of
+// softmax does not: an item of 1000 prompt keys takes 27 us alone, 35 with 16 columns of several rows, 43 with 32
+// and 68 with 64 (4 or 8 groups, heads of 128; latents of 256: 31, -, 39, 55; of 512: 53, -, 68, 90).  The keys of
 // the rows themselves are no less work together: a short tile for two rows, or a whole one each.  1000 rows of one prompt of
-// 1000, each by itself / together: 307 / 156 us (4 groups of 128), 586 / 293 (8 groups), 252 / 90 (4 groups of 64),
-// 123 / 95 (latents of 256), 313 / 166 (of 512); 64 prompts with 4 rows each, latents of 512: 94 / 66; 150 with 3 rows, 300 keys, latents
+// 1000, each by itself / together: 307 / 139 us (4 groups of 128), 588 / 237 (8 groups), 252 / 86 (4 groups of 64),
+// 123 / 96 (latents of 256), 313 / 166 (of 512); 64 prompts with 4 rows each, latents of 512: 94 / 66; 150 with 3 rows, 300 keys, latents
 // of 512, where it does not pay: 90 / 98.
 // In tiles of one row: an item's start and end, a tile of its prompt, a tile of a row's own keys (half of one where they are 64 or fewer and two
 // rows come in one), fitted to 14 jobs of 12 to 1200 rows for each of five shapes.  Two CTAs of an SM share its pipes.  Before the fit
@@ -829,7 +829,7 @@ static double lt_item_cost(const LatentArgs& a, const LtShape& sh, int rg, int p
 static int lt_rows(const LatentArgs& a, int sms, int limit) {
   const int per = a.H / a.G;
   if (a.share < 2 || a.Tn != 1 || !a.kv.page_table || (per & (per - 1)) != 0) return 1;
-  // Little to share: 1000 rows with 64 prompt keys and 400 of their own took 255 us with 4 rows together against 234 (4 groups of 128).
+  // Little to share: 1000 rows with 64 prompt keys and 400 of their own took 249 us with 4 rows together against 234 (4 groups of 128).
   if (!a.together && a.own_keys > kLtKeys / 2 && 2LL * a.prompt_keys < a.own_keys) return 1;
   const int cols = lt_cols(a);
   int best = 1;
